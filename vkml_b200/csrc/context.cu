@@ -216,8 +216,9 @@ GemmProblem matmul_problem(const b200_node& node) {
     if (node.out.ndim != 4 || node.src[0].ndim != 4 || node.src[1].ndim != 4) {
         fail(B200_SHAPE_ERROR, "matmul expects rank-4 operands");
     }
-    if (out.dtype != B200_F32 || a.dtype != B200_F32 || b.dtype != B200_F32) {
-        fail(B200_DTYPE_ERROR, "matmul: only f32 is implemented");
+    const bool half = out.dtype == B200_F16 && a.dtype == B200_F16 && b.dtype == B200_F16;  // (pointers to halves then)
+    if (!half && (out.dtype != B200_F32 || a.dtype != B200_F32 || b.dtype != B200_F32)) {
+        fail(B200_DTYPE_ERROR, "matmul: operands and result are f32, or all f16");
     }
     if (!out.contiguous) {
         fail(B200_NOT_IMPLEMENTED, "matmul output must be contiguous");
@@ -244,10 +245,58 @@ GemmProblem matmul_problem(const b200_node& node) {
 
 void dispatch_matmul(b200_ctx* ctx, const b200_node& node) {
     const GemmProblem p = matmul_problem(node);
-    if (ctx->gemm_precision != B200_GEMM_FP32 && gemm_tc_eligible(ctx, p)) {
+    if (gemm_h16_serves(ctx, p) && gemm_tc_eligible(ctx, p)) {
+        gemm_h16(ctx, p);
+    } else if (ctx->gemm_precision != B200_GEMM_FP32 && gemm_tc_eligible(ctx, p)) {
         gemm_tc(ctx, p, ctx->gemm_precision == B200_GEMM_3XTF32);
     } else {
         gemm_simt(ctx, p);
+    }
+}
+
+bool touches_f16(const b200_node& n) {
+    if (n.op == B200_OP_CAST || n.op == B200_OP_FULL) return false;  // these handle F16 themselves
+    if (n.out.dtype == B200_F16) return true;
+    for (uint32_t s = 0; s < n.n_src && s < B200_MAX_SRC; ++s) {
+        if (n.src[s].dtype == B200_F16) return true;
+    }
+    return false;
+}
+
+size_t tensor_span_bytes(const b200_tensor& t) {
+    size_t n = dtype_size(t.dtype);
+    for (int d = 0; d < t.ndim; ++d) n *= static_cast<size_t>(t.dims[d]);
+    return n;
+}
+
+// Notes the large products whose result this span compares with something -- a ReLU and its mask, a pooling
+// maximum -- directly or with a bias added.  There the last bits of a sum decide whole paths of the
+// gradient, so these products keep the TF32 terms, bit for bit, and a training run its masks: half terms
+// round elsewhere (five times closer to the exact result at K = 8192, but elsewhere), and one switched unit of a wide
+// MLP was measured to move single weight gradients by half of their rms.
+void note_compared_products(b200_ctx* ctx, const b200_node* nodes, size_t n_nodes) {
+    ctx->compared.clear();
+    for (size_t i = 0; i + 1 < n_nodes; ++i) {
+        const b200_node& m = nodes[i];
+        if (m.op != B200_OP_MATMUL || m.out.data == nullptr || m.out.dtype != B200_F32) continue;
+        const char* at[2] = {static_cast<const char*>(m.out.data), nullptr};
+        size_t bytes[2] = {tensor_span_bytes(m.out), 0};
+        for (size_t j = i + 1; j < n_nodes; ++j) {
+            const b200_node& n = nodes[j];
+            bool reads = false;
+            for (uint32_t k = 0; k < n.n_src && k < B200_MAX_SRC; ++k) {
+                const char* p = static_cast<const char*>(n.src[k].data);
+                for (int q = 0; q < 2; ++q) reads = reads || (at[q] != nullptr && p >= at[q] && p < at[q] + bytes[q]);
+            }
+            if (!reads) continue;
+            if (n.op == B200_OP_ADD && at[1] == nullptr) {
+                at[1] = static_cast<const char*>(n.out.data);
+                bytes[1] = tensor_span_bytes(n.out);
+            } else if (n.op == B200_OP_RELU || n.op == B200_OP_MAX_POOL2D || (n.op >= B200_OP_MAXIMUM && n.op <= B200_OP_NOT_EQUAL)) {
+                ctx->compared.insert(m.out.data);
+                break;
+            }
+        }
     }
 }
 
@@ -266,23 +315,16 @@ void count_matmul_operands(b200_ctx* ctx, const b200_node* nodes, size_t n_nodes
             continue;
         }
         try {
+            if (touches_f16(node)) continue;  // half operands need no planes
             const GemmProblem p = matmul_problem(node);
             if (p.b0 * p.b1 * p.m * p.n * p.k != 0 && gemm_tc_eligible(ctx, p)) {
-                gemm_tc_note_uses(ctx, p);
+                if (gemm_h16_serves(ctx, p)) gemm_h16_note_uses(ctx, p);
+                else gemm_tc_note_uses(ctx, p);
             }
         } catch (const Error&) {
             // reported when the node is dispatched
         }
     }
-}
-
-bool touches_f16(const b200_node& n) {
-    if (n.op == B200_OP_CAST || n.op == B200_OP_FULL) return false;  // these handle F16 themselves
-    if (n.out.dtype == B200_F16) return true;
-    for (uint32_t s = 0; s < n.n_src && s < B200_MAX_SRC; ++s) {
-        if (n.src[s].dtype == B200_F16) return true;
-    }
-    return false;
 }
 
 b200_tensor dense_f32_like(const b200_tensor& like, void* data) {
@@ -367,6 +409,9 @@ void dispatch_node(b200_ctx* ctx, const b200_node& node) {
         for (uint32_t s = 0; s < node.n_src && s < B200_MAX_SRC; ++s) {
             all_half = all_half && node.src[s].dtype != B200_F32;
         }
+        const bool half_matmul = op == B200_OP_MATMUL && node.n_src >= 2 && node.src[0].dtype == B200_F16 &&
+                                 node.src[1].dtype == B200_F16 && node.out.dtype == B200_F16;
+        if (half_matmul && gemm_f16_storage(ctx, matmul_problem(node))) return;
         if (elementwise && all_half && node.out.dtype != B200_F32) {
             ProfScope scope(ctx, op_label(op));
             launch_elementwise(ctx, node);
@@ -569,12 +614,16 @@ int b200_create(int cuda_ordinal, b200_ctx** out) {
         B200_CUDA_CHECK(cudaMemset(ctx->d_status, 0, sizeof(uint32_t)));
         B200_CUDA_CHECK(cudaMalloc(&ctx->d_counters, sizeof(unsigned) * kArrivalCounters));
         B200_CUDA_CHECK(cudaMemset(ctx->d_counters, 0, sizeof(unsigned) * kArrivalCounters));
+        B200_CUDA_CHECK(cudaMalloc(&ctx->d_ranges, sizeof(RangeSlot) * kRangeSlots));
         B200_CUDA_CHECK(cudaMallocHost(&ctx->h_status, sizeof(uint32_t)));
         *ctx->h_status = 0;
         // VKML_B200_GEMM_PRECISION = 3xtf32 (default) | tf32 | fp32, read once per context:
         // the counterpart of the VKML_GEMM_* switches (vulkan_backend.cpp:2160-2178)
         if (const char* e = std::getenv("VKML_B200_GEMM_GROUP_M")) {
             ctx->gemm_group_m = std::max(0, std::min(1024, std::atoi(e)));
+        }
+        if (const char* e = std::getenv("VKML_B200_GEMM_HALF_TERMS")) {
+            ctx->gemm_half_terms = std::string(e) != "0";
         }
         if (const char* e = std::getenv("VKML_B200_GEMM_BN")) {
             ctx->gemm_bn_override = std::atoi(e);
@@ -660,6 +709,7 @@ void b200_destroy(b200_ctx* ctx) {
     if (ctx->stream != nullptr) cudaStreamDestroy(ctx->stream);
     if (ctx->d_status != nullptr) cudaFree(ctx->d_status);
     if (ctx->d_counters != nullptr) cudaFree(ctx->d_counters);
+    if (ctx->d_ranges != nullptr) cudaFree(ctx->d_ranges);
     if (ctx->h_status != nullptr) cudaFreeHost(ctx->h_status);
     for (cudaEvent_t ev : ctx->event_pool) cudaEventDestroy(ev);
     if (ctx->timer_begin != nullptr) cudaEventDestroy(ctx->timer_begin);
@@ -731,6 +781,7 @@ static void compute_span(b200_ctx* ctx, const b200_node* nodes, size_t n_nodes, 
             gemm_tc_end_span(c);
         }
     } span_guard{ctx};
+    note_compared_products(ctx, nodes, n_nodes);
     count_matmul_operands(ctx, nodes, n_nodes);
     std::vector<char> is_sink;
     if (grad_sync && ctx->grads.empty()) {
@@ -1414,6 +1465,7 @@ int b200_matmul_kernel(b200_ctx* ctx, const b200_node* node, char* name, size_t 
     if (ctx == nullptr || node == nullptr || name == nullptr || name_len == 0) return B200_INVALID_ARGUMENT;
     return guarded(ctx, [&] {
         if (node->op != B200_OP_MATMUL) fail(B200_INVALID_ARGUMENT, "b200_matmul_kernel: not a matmul node");
+        if (touches_f16(*node)) fail(B200_DTYPE_ERROR, "b200_matmul_kernel: an f32 node is wanted");
         const GemmProblem p = matmul_problem(*node);
         const char* kernel = "fp32_simt";
         const char* why = "the shape is too small or too ragged for a tensor-core tile";
@@ -1421,7 +1473,10 @@ int b200_matmul_kernel(b200_ctx* ctx, const b200_node* node, char* name, size_t 
             why = "plain fp32 arithmetic was asked for";
         } else if (gemm_tc_eligible(ctx, p)) {
             const bool three = ctx->gemm_precision == B200_GEMM_3XTF32;
-            if (gemm_tc_streams(ctx, p)) {
+            if (gemm_h16_serves(ctx, p)) {
+                kernel = "tcgen05_3xf16";
+                why = "bound by the tensor cores: two half terms per operand (TF32 planes where an operand's range is too wide for them)";
+            } else if (gemm_tc_streams(ctx, p)) {
                 kernel = three ? "tcgen05_3xtf32_stream" : "tcgen05_tf32_stream";
                 why = "bound by memory (a small left operand or a short K): the right operand is read as fp32 and split on the way";
             } else if (gemm_tc_reads_directly(ctx, p)) {

@@ -65,17 +65,17 @@ struct GradBuffer {
 // forward and, transposed, in the weight-gradient product) give the same key.
 struct PlaneKey {
     const void* src;
-    int64_t v[8];  // rows, cols, row stride, column stride, inner batch extent, batch strides, batches
+    int64_t v[9];  // rows, cols, row stride, column stride, inner batch extent, batch strides, batches, 0: TF32 planes, 1: half planes
     bool operator<(const PlaneKey& o) const {
         if (src != o.src) return src < o.src;
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < 9; ++i) {
             if (v[i] != o.v[i]) return v[i] < o.v[i];
         }
         return false;
     }
 };
 
-// The TF32 hi / lo planes of one operand, kept for the rest of the compute span.
+// The hi / lo planes of one operand, kept for the rest of the compute span.
 struct PlaneEntry {
     float* hi;
     float* lo;
@@ -83,7 +83,11 @@ struct PlaneEntry {
     int uses_left;
     const char* src_begin;
     const char* src_end;
+    void* range = nullptr;  // half planes: the matrix's RangeSlot
 };
+
+// Ranges of the matrices that one span's half-term products split (gemm_h16.cu).
+constexpr int kRangeSlots = 1024;
 
 }  // namespace b200
 
@@ -129,6 +133,12 @@ struct b200_ctx {
     // where the layout allows it and no other operand scheme was asked for by name; 0: never; 1:
     // every product whose layout allows it, whatever its size (A/B runs).
     int gemm_stream = -1;
+    // VKML_B200_GEMM_HALF_TERMS: large F32 products from two half terms per operand where their range allows
+    // it (gemm_h16.cu); 0: TF32 terms everywhere (A/B runs).
+    bool gemm_half_terms = true;
+    void* d_ranges = nullptr;  // RangeSlot[kRangeSlots], cleared at a span's first use
+    int range_next = 0;        // slots taken in the current span
+    std::set<const void*> compared;  // results of the current span's products that keep TF32 terms (note_compared_products)
     int gemm_group_m = 0;      // VKML_B200_GEMM_GROUP_M: M-tiles per L2 group of the tile walk (0: the built-in 16)
     int gemm_bn_override = 0;  // VKML_B200_GEMM_BN: force the N extent of the tensor-core tile (tuning aid)
     // SMs the persistent GEMM kernel leaves free while a span's gradients are being all-reduced,
@@ -211,6 +221,27 @@ inline void launch_kernel(b200_ctx* ctx, void (*kernel)(Params...), dim3 grid, d
     cfg.attrs = attr;
     cfg.numAttrs = ctx->pdl ? 1 : 0;
     // a failed launch is picked up by check_last_launch() at the call site
+    (void)cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
+
+// The same for a kernel whose blocks work in clusters of `cluster` along x.
+template <typename... Params, typename... Args>
+inline void launch_kernel_clustered(b200_ctx* ctx, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, int cluster,
+                                    Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = ctx->pdl ? 2 : 1;
     (void)cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 

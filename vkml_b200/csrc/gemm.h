@@ -18,12 +18,38 @@ struct GemmProblem {
     int64_t b_s[4];  // element strides of b over (b0, b1, k, n)
 };
 
+// The range of one operand matrix, found on the device (gemm_h16.cu): the bits of the largest magnitude in
+// a sample of it, how many nonzero elements are too small beside that for the half split, and whether one is too large.
+struct RangeSlot {
+    uint32_t max_bits;
+    uint32_t strays;
+    uint32_t spoiled;
+    uint32_t unused;
+};
+
+// Launches carrying a guard run only if one of the two matrices is wide (see gemm_h16.cu); a == null: always.
+struct RangeGuard {
+    const RangeSlot* a;
+    const RangeSlot* b;
+    uint32_t limit_a, limit_b;
+};
+
 // fp32 FMA on the CUDA cores; any strides, any size. gemm_simt.cu
 void gemm_simt(b200_ctx* ctx, const GemmProblem& p);
 
 // tcgen05 tensor-core path (3xTF32 or single-pass TF32). gemm_tc.cu
 bool gemm_tc_eligible(const b200_ctx* ctx, const GemmProblem& p);
 void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass);
+// The TF32 planes for the case that an operand turns out wide on the device: queued behind gemm_h16's kernel.
+void gemm_tc_if_wide(b200_ctx* ctx, const GemmProblem& p, const RangeGuard& guard, void* planes);
+size_t gemm_tc_plane_bytes(const GemmProblem& p);  // bytes that gemm_tc_if_wide wants at `planes`
+
+// tcgen05 kind::f16: F32 products from two half terms per operand, F16 products directly. gemm_h16.cu
+bool gemm_h16_serves(const b200_ctx* ctx, const GemmProblem& p);
+void gemm_h16(b200_ctx* ctx, const GemmProblem& p);
+void gemm_h16_note_uses(b200_ctx* ctx, const GemmProblem& p);
+// Half storage: `p`'s pointers are to halves.  False: not a case for this kernel.
+bool gemm_f16_storage(b200_ctx* ctx, const GemmProblem& p);
 // True when gemm_tc would serve `p` with the streamed-operand kernel (a small left operand, the
 // right operand read once from HBM) rather than from operand planes.
 bool gemm_tc_streams(const b200_ctx* ctx, const GemmProblem& p);

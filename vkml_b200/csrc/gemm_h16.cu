@@ -1,0 +1,983 @@
+// GEMM on the tensor cores with half-precision operand terms: tcgen05.mma kind::f16, fp32 accumulators.
+//
+// Two uses of one kernel.
+//
+// F16 storage (one pass).  Half operands are the MMA's own format: products are exact, the accumulator
+// is fp32, the result is narrowed once on the way out -- what the reference computes by widening, in
+// the layout the caller already has.
+//
+// F32 storage (three passes).  Each operand x is scaled by a power of two s and split into
+// hi = half(s x) and lo = half(2^11 (s x - hi)): 11 + 11 significant bits, the same 22 that the TF32
+// split keeps, at twice the MMA rate and half the operand bytes.  hi.hi goes into one TMEM
+// accumulator, the cross terms lo.hi + hi.lo, which carry the factor 2^11, into a second one; the
+// epilogue adds them and takes the scales out again.  (8192^3: 4.22 -> 2.43 ms for the kernel, and a
+// relative error of 9.7e-6 instead of 5.7e-5: half as many truncating additions per accumulator.)
+//
+// Half has five exponent bits, so s has to suit the matrix.  A first pass looks for the largest magnitude
+// in a sample -- 128-element pieces spread over the whole matrix, all of it where it is small -- and s puts
+// that into [2^11, 2^12): room for elements sixteen times larger, and all 22 bits for elements down to
+// 2^-24 of it (below, an absolute error of at most 2^-36/s).  The split checks every element against both
+// ends.  A matrix that overflows, that holds an infinity or a NaN, or in which more than a few elements
+// lie below the lower end (kStrayFloor plus one in 2^21: N(0,1) data has one in 7e6) is WIDE, and a product
+// with a wide operand is computed by the TF32 planes queued behind this kernel instead (gemm_tc_if_wide;
+// its launches return at once otherwise).  No host synchronisation decides this.
+#include "gemm.h"
+#include "tcgen05.cuh"
+
+#include <algorithm>
+
+#include <cuda_fp16.h>
+
+namespace b200 {
+namespace {
+
+constexpr int kRowsM = 128;   // accumulator lanes of one CTA
+constexpr int kBlockK = 64;   // halves per K-block: one 128-byte swizzle row
+constexpr int kStepK = 16;    // K of one kind::f16 instruction
+constexpr int kThreads = 192;
+constexpr int kPatchPitch = 36;
+constexpr int kGroupRows = 2048;  // M rows walked together before moving along N (L2 reuse of the B tiles)
+
+// ---------------------------------------------------------------------------
+// range of a matrix, and the split
+// ---------------------------------------------------------------------------
+
+struct MatrixArgs {
+    const float* src;
+    __half* hi;
+    __half* lo;
+    RangeSlot* range;
+    int64_t b1, n_batches;            // inner batch extent, batches
+    int64_t s_b0, s_b1, s_r, s_c;     // element strides
+    int64_t rows, cols, pitch;        // pitch: halves per plane row (a multiple of 8)
+    int vec;                          // rows start on 16 bytes and columns are dense
+};
+
+struct MatrixPair {
+    MatrixArgs m[2];
+};
+
+__device__ __forceinline__ const float* row_of(const MatrixArgs& a, int64_t rb, int64_t& r) {
+    const int64_t b = a.n_batches == 1 ? 0 : rb / a.rows;
+    r = rb - b * a.rows;
+    const int64_t bo = a.s_b0 == 0 && a.b1 == 1 ? 0 : b / a.b1;
+    return a.src + bo * a.s_b0 + (b - bo * a.b1) * a.s_b1 + r * a.s_r;
+}
+
+// Eight consecutive columns of one row, zeros past the end.
+__device__ __forceinline__ void load8(const MatrixArgs& a, const float* row, int64_t c, float (&v)[8]) {
+    if (a.vec && c + 8 <= a.cols) {
+        const float4 x = __ldg(reinterpret_cast<const float4*>(row + c));
+        const float4 y = __ldg(reinterpret_cast<const float4*>(row + c + 4));
+        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+        v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        v[j] = c + j < a.cols ? __ldg(row + (c + j) * a.s_c) : 0.0F;
+    }
+}
+
+// The largest magnitude in a sample of each matrix, as the bits of its absolute value (infinities and
+// NaNs included: they compare above every finite value).  Looking at all of both operands took 98 us at
+// 8192^3 and 53 us at 512 x 65536 x 512; one piece in `stride` takes a few.
+constexpr int kPiece = 16;  // consecutive groups of eight columns that are looked at together
+constexpr int64_t kSampleGroups = int64_t(1) << 17;
+
+__device__ __forceinline__ int64_t row_number(int64_t i, int64_t per_row, int64_t total) {
+    return total < (int64_t(1) << 31) ? int64_t(uint32_t(i) / uint32_t(per_row)) : i / per_row;
+}
+
+__global__ void __launch_bounds__(256) range_kernel(MatrixPair pair) {
+    pdl_prologue();
+    const MatrixArgs& a = pair.m[blockIdx.y];
+    const int64_t per_row = (a.cols + 7) / 8;
+    const int64_t total = per_row * a.rows * a.n_batches;
+    const int64_t stride = max(int64_t(1), total / kSampleGroups);  // of the pieces, one in so many
+    const int64_t groups = (total + stride - 1) / stride;
+    const int64_t step = int64_t(gridDim.x) * blockDim.x;
+    uint32_t top = 0;
+    for (int64_t j = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < groups; j += step) {
+        const int64_t piece = j / kPiece;
+        // (a piece's place inside its stretch varies, so that no column pattern of the matrix is in step with it)
+        const int64_t i = min(total - 1, (piece * stride + (piece * 7919) % stride) * kPiece + j % kPiece);
+        float v[8];
+        int64_t r;
+        const int64_t rb = row_number(i, per_row, total);
+        load8(a, row_of(a, rb, r), (i - rb * per_row) * 8, v);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) top = max(top, __float_as_uint(v[q]) & 0x7FFFFFFFu);
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    __shared__ uint32_t tops[8];
+    if ((threadIdx.x & 31) == 0) tops[threadIdx.x >> 5] = top;
+    __syncthreads();
+    if (threadIdx.x < 8) {
+        top = __reduce_max_sync(0xffu, tops[threadIdx.x]);
+        if (threadIdx.x == 0 && top != 0) atomicMax(&a.range->max_bits, top);
+    }
+}
+
+// Writes each matrix's two half planes, [batch][row][pitch], in the orientation the matrix has in memory: 4 bytes read, 4 written per element.
+__global__ void __launch_bounds__(256) split_half_kernel(MatrixPair pair) {
+    pdl_prologue();
+    const MatrixArgs& a = pair.m[blockIdx.y];
+    const uint32_t top = __ldcg(&a.range->max_bits);
+    if (top >= 0x7F800000u) return;  // the planes will not be read
+    const int up = range_shift(top);
+    const float s1 = exp2_int(up / 2), s2 = exp2_int(up - up / 2);
+    const int64_t per_row = a.pitch / 8;
+    const int64_t total = per_row * a.rows * a.n_batches;
+    const int64_t step = int64_t(gridDim.x) * blockDim.x;
+    uint32_t strays = 0;
+    bool over = false;
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += step) {
+        float v[8];
+        int64_t r;
+        const int64_t rb = row_number(i, per_row, total);
+        const int64_t c = (i - rb * per_row) * 8;
+        load8(a, row_of(a, rb, r), c, v);
+        __half2 hi[4], lo[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float x = v[2 * j] * s1 * s2, y = v[2 * j + 1] * s1 * s2;  // exact: powers of two
+            strays += (fabsf(x) < kStrayBelow && v[2 * j] != 0.0F) + (fabsf(y) < kStrayBelow && v[2 * j + 1] != 0.0F);
+            over = over || !(fmaxf(fabsf(x), fabsf(y)) < 65504.0F) || x != x || y != y;
+            hi[j] = __floats2half2_rn(x, y);
+            const float2 h = __half22float2(hi[j]);
+            lo[j] = __floats2half2_rn((x - h.x) * 2048.0F, (y - h.y) * 2048.0F);
+        }
+        *reinterpret_cast<uint4*>(a.hi + rb * a.pitch + c) = *reinterpret_cast<const uint4*>(hi);
+        *reinterpret_cast<uint4*>(a.lo + rb * a.pitch + c) = *reinterpret_cast<const uint4*>(lo);
+    }
+    strays = __reduce_add_sync(0xffffffffu, strays);
+    if ((threadIdx.x & 31) == 0 && strays != 0) atomicAdd(&a.range->strays, strays);
+    if (over) a.range->spoiled = 1;
+}
+
+// A half matrix that TMA cannot read as it lies (odd pitch, misaligned base, two strided axes): a dense copy.
+__global__ void __launch_bounds__(256) pack_half_kernel(const __half* __restrict__ src, __half* __restrict__ dst, int64_t b1,
+                                                        int64_t s_b0, int64_t s_b1, int64_t s_r, int64_t s_c, int64_t rows,
+                                                        int64_t cols, int64_t pitch, int64_t batches) {
+    pdl_prologue();
+    const int64_t per_row = pitch / 8;
+    const int64_t total = per_row * rows * batches;
+    const int64_t step = int64_t(gridDim.x) * blockDim.x;
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += step) {
+        const int64_t rb = i / per_row, c = (i - rb * per_row) * 8;
+        const int64_t b = rb / rows, r = rb - b * rows;
+        const __half* row = src + (b / b1) * s_b0 + (b % b1) * s_b1 + r * s_r;
+        __half v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = c + j < cols ? row[(c + j) * s_c] : __half(0.0F);
+        *reinterpret_cast<uint4*>(dst + rb * pitch + c) = *reinterpret_cast<const uint4*>(v);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Main kernel
+// ---------------------------------------------------------------------------
+
+struct H16Args {
+    void* out;             // C (f32 or half), or the f32 partial planes when splits > 1
+    int out_half;
+    int64_t m, n, batches;
+    int a_b1, b_b1;        // inner batch extents of the operand maps; 0: one matrix for every batch
+    int64_t k_blocks, kb_per_split;
+    int splits;
+    int64_t split_stride;  // elements between partial planes
+    int64_t tiles_m, tiles_n;
+    int group_m;           // M-tiles walked together
+    const RangeSlot* range_a;  // three passes: the operands' ranges
+    const RangeSlot* range_b;
+    uint32_t limit_a, limit_b;
+    uint32_t* status;
+};
+
+// CG CTAs share one tile of CG*128 rows x BN columns: with CG = 2 each CTA of a cluster holds its 128
+// rows of A and half of B, and one instruction issued by the even CTA drives both tensor cores
+// (cta_group::2), so B's tile is fetched and stored once for 256 rows.
+template <int CG, int BN, int PASSES>
+struct H16Tile {
+    static constexpr int kPlanes = PASSES == 3 ? 2 : 1;
+    static constexpr int kABytes = kRowsM * kBlockK * 2;
+    static constexpr int kBBytes = (BN / CG) * kBlockK * 2;
+    static constexpr int kStageBytes = kPlanes * (kABytes + kBBytes);
+    static constexpr int kFit = 200 * 1024 / kStageBytes;
+    static constexpr int kStages = kFit < 8 ? kFit : 8;
+    static constexpr int kAccCols = (PASSES == 3 ? 2 : 1) * BN;  // main terms, then cross terms
+    static constexpr int kAccs = 2 * kAccCols <= 512 ? 2 : 1;
+    static constexpr int kTmemCols = kAccs * kAccCols;
+    static constexpr int kBars = kStages * kStageBytes;
+    static constexpr int kTotal = kBars + 256 + 1024;
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+
+// The address, in the cluster's shared window, of the even CTA's copy of a shared-memory location.
+__device__ __forceinline__ uint32_t lead_addr(uint32_t addr) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+    return r;
+}
+
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+}
+
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <int CG>
+__device__ __forceinline__ void tma_tile(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2, int c3) {
+    if constexpr (CG == 2) {
+        asm volatile(
+            "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+            ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+            : "memory");
+    } else {
+        tma_load_4d(dst, map, bar, c0, c1, c2, c3);
+    }
+}
+
+template <int CG>
+__device__ __forceinline__ void umma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+    if constexpr (CG == 2) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+    } else {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+            ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
+    }
+}
+
+// Arrives on `bar` of every CTA of the tile once the MMAs issued so far are done.
+template <int CG>
+__device__ __forceinline__ void commit_all(uint32_t bar) {
+    if constexpr (CG == 2) {
+        asm volatile(
+            "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+            ::"r"(bar), "h"(static_cast<uint16_t>(3)) : "memory");
+    } else {
+        umma_commit(bar);
+    }
+}
+
+template <int CG>
+__device__ __forceinline__ void tmem_get(uint32_t dst_smem, uint32_t cols) {
+    if constexpr (CG == 2) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(cols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+        tmem_alloc(dst_smem, cols);
+    }
+}
+
+template <int CG>
+__device__ __forceinline__ void tmem_put(uint32_t taddr, uint32_t cols) {
+    if constexpr (CG == 2) {
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
+    } else {
+        tmem_dealloc(taddr, cols);
+    }
+}
+
+// D = f32, A = B = f16.
+__host__ __device__ constexpr uint32_t h16_idesc(int m, int n, bool a_mn, bool b_mn) {
+    return (1u << 4) | (a_mn ? (1u << 15) : 0u) | (b_mn ? (1u << 16) : 0u) | (static_cast<uint32_t>(n >> 3) << 17) |
+           (static_cast<uint32_t>(m >> 4) << 24);
+}
+
+// Tiles of 16-bit elements, 128-byte swizzle.  K-major: rows of 64 halves, 8-row groups 1024 bytes apart,
+// one K-step is 32 bytes further.  MN-major: atoms of 64 K-rows x 128 bytes (64 elements along MN), 8-row
+// groups again 1024 bytes apart, the next atom along MN 8192 bytes further, one K-step 16 rows further.
+constexpr uint32_t kAtomBytes = kBlockK * 128;
+
+template <bool MN>
+__device__ __forceinline__ uint64_t h16_desc(uint32_t addr) {
+    return smem_desc(addr, MN ? kAtomBytes : 0, 1024, 2);
+}
+
+// Bounded by the tensor cores for the large products.  Layout of the roles as in gemm_tc_kernel: warp 0 TMA,
+// warp 1 tensor memory and MMA, warps 2-5 epilogue, tiles from a fixed walk.
+template <int CG, int BN, int PASSES, bool A_MN, bool B_MN>
+__global__ void __launch_bounds__(kThreads, 1)
+gemm_h16_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_constant__ CUtensorMap map_a_lo,
+                const __grid_constant__ CUtensorMap map_b_hi, const __grid_constant__ CUtensorMap map_b_lo, H16Args g) {
+    using T = H16Tile<CG, BN, PASSES>;
+    constexpr int STAGES = T::kStages;
+    constexpr uint32_t kIdesc = h16_idesc(CG * kRowsM, BN, A_MN, B_MN);
+    constexpr int kTileM = CG * kRowsM;
+    static_assert(8 * (2 * STAGES + 2 * T::kAccs) <= 256, "barrier block");
+
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t bars = base + T::kBars;
+    auto full_bar = [&](int s) { return bars + 8u * s; };              // the even CTA's: both CTAs' tiles landed
+    auto empty_bar = [&](int s) { return bars + 8u * (STAGES + s); };
+    auto acc_full = [&](int a) { return bars + 8u * (2 * STAGES + a); };
+    auto acc_empty = [&](int a) { return bars + 8u * (2 * STAGES + T::kAccs + a); };  // the even CTA's
+    __shared__ uint32_t tmem_base_slot;
+    __shared__ int abort_flag;
+    __shared__ __align__(16) float epi_patch[4][32][kPatchPitch];
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    const uint32_t rank = CG == 2 ? cluster_rank() : 0;
+
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(full_bar(s), 1);
+            mbar_init(empty_bar(s), 1);
+        }
+        for (int a = 0; a < T::kAccs; ++a) {
+            mbar_init(acc_full(a), 1);
+            mbar_init(acc_empty(a), 4 * CG);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (warp == 1) {
+        tmem_get<CG>(smem_u32(&tmem_base_slot), T::kTmemCols);
+        tc_fence_before();
+    }
+    __syncthreads();
+    if (CG == 2) cluster_sync();  // the other CTA's barriers are initialised
+    tc_fence_after();
+    const uint32_t tmem_base = tmem_base_slot;
+    volatile int* abort_p = &abort_flag;
+    pdl_prologue();
+
+    int64_t n_units = g.tiles_m * g.tiles_n * g.batches * g.splits;
+    if (PASSES == 3 && (range_wide(g.range_a, g.limit_a) || range_wide(g.range_b, g.limit_b))) {
+        n_units = 0;  // the TF32 planes behind this kernel serve the product
+    }
+    const int64_t unit0 = blockIdx.x / CG, unit_step = gridDim.x / CG;
+    auto decode = [&](int64_t u, int& split, int64_t& batch, int64_t& tm, int64_t& tn) {
+        split = static_cast<int>(u % g.splits);
+        int64_t t = u / g.splits;
+        const int64_t per_batch = g.tiles_m * g.tiles_n;
+        batch = t / per_batch;
+        t -= batch * per_batch;
+        const int64_t group_size = int64_t(g.group_m) * g.tiles_n;
+        const int64_t group = t / group_size;
+        const int64_t first_m = group * g.group_m;
+        const int64_t rows_in_group = min(int64_t(g.group_m), g.tiles_m - first_m);
+        const int64_t in_group = t - group * group_size;
+        tm = first_m + in_group % rows_in_group;
+        tn = in_group / rows_in_group;
+    };
+
+    if (warp == 0) {
+        // ---------------- TMA producer (one per CTA, signalling the even CTA's barrier) ----------------
+        if (lane == 0) {
+            uint32_t it = 0;
+            bool ok = true;
+            for (int64_t u = unit0; u < n_units && ok; u += unit_step) {
+                int split;
+                int64_t batch, tm, tn;
+                decode(u, split, batch, tm, tn);
+                const int m0 = static_cast<int>(tm * kTileM + rank * kRowsM);
+                const int n0 = static_cast<int>(tn * BN + rank * (BN / CG));
+                const int a3 = g.a_b1 == 0 ? 0 : static_cast<int>(batch / g.a_b1), a2 = g.a_b1 == 0 ? 0 : static_cast<int>(batch - int64_t(a3) * g.a_b1);
+                const int b3 = g.b_b1 == 0 ? 0 : static_cast<int>(batch / g.b_b1), b2 = g.b_b1 == 0 ? 0 : static_cast<int>(batch - int64_t(b3) * g.b_b1);
+                const int64_t kb0 = int64_t(split) * g.kb_per_split;
+                const int64_t kb1 = min(kb0 + g.kb_per_split, g.k_blocks);
+                for (int64_t kb = kb0; kb < kb1; ++kb, ++it) {
+                    const int s = it % STAGES;
+                    if (!mbar_wait(empty_bar(s), ((it / STAGES) & 1) ^ 1, abort_p, g.status)) {
+                        ok = false;
+                        break;
+                    }
+                    const uint32_t stage = base + s * T::kStageBytes;
+                    const int kc = static_cast<int>(kb * kBlockK);
+                    const uint32_t bar = CG == 2 ? lead_addr(full_bar(s)) : full_bar(s);
+                    if (rank == 0) mbar_arrive_expect_tx(full_bar(s), CG * T::kStageBytes);
+                    auto load = [&](uint32_t dst, const CUtensorMap* map, bool mn, int rows, int r0, int c2, int c3) {
+                        if (mn) {
+                            for (int atom = 0; atom < rows / 64; ++atom) {
+                                tma_tile<CG>(dst + atom * kAtomBytes, map, bar, r0 + 64 * atom, kc, c2, c3);
+                            }
+                        } else {
+                            tma_tile<CG>(dst, map, bar, kc, r0, c2, c3);
+                        }
+                    };
+                    load(stage, &map_a_hi, A_MN, kRowsM, m0, a2, a3);
+                    load(stage + T::kPlanes * T::kABytes, &map_b_hi, B_MN, BN / CG, n0, b2, b3);
+                    if (PASSES == 3) {
+                        load(stage + T::kABytes, &map_a_lo, A_MN, kRowsM, m0, a2, a3);
+                        load(stage + 2 * T::kABytes + T::kBBytes, &map_b_lo, B_MN, BN / CG, n0, b2, b3);
+                    }
+                }
+            }
+        }
+    } else if (warp == 1) {
+        // ---------------- MMA issuer (the even CTA's) ----------------
+        if (lane == 0 && rank == 0) {
+            uint32_t it = 0, tile_it = 0;
+            bool ok = true;
+            for (int64_t u = unit0; u < n_units && ok; u += unit_step, ++tile_it) {
+                const int split = static_cast<int>(u % g.splits);
+                const int acc = tile_it % T::kAccs;
+                if (!mbar_wait(acc_empty(acc), ((tile_it / T::kAccs) & 1) ^ 1, abort_p, g.status)) break;
+                tc_fence_after();
+                const uint32_t d_main = tmem_base + acc * T::kAccCols;
+                const uint32_t d_cross = d_main + BN;
+                const int64_t kb0 = int64_t(split) * g.kb_per_split;
+                const int64_t kb1 = min(kb0 + g.kb_per_split, g.k_blocks);
+                for (int64_t kb = kb0; kb < kb1; ++kb, ++it) {
+                    const int s = it % STAGES;
+                    if (!mbar_wait(full_bar(s), (it / STAGES) & 1, abort_p, g.status)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t stage = base + s * T::kStageBytes;
+                    const uint64_t a_hi = h16_desc<A_MN>(stage);
+                    const uint64_t a_lo = h16_desc<A_MN>(stage + T::kABytes);
+                    const uint64_t b_hi = h16_desc<B_MN>(stage + T::kPlanes * T::kABytes);
+                    const uint64_t b_lo = h16_desc<B_MN>(stage + T::kPlanes * T::kABytes + T::kBBytes);
+#pragma unroll
+                    for (int kk = 0; kk < kBlockK / kStepK; ++kk) {
+                        const uint64_t adv_a = static_cast<uint64_t>((A_MN ? kk * kStepK * 128 : kk * kStepK * 2) >> 4);
+                        const uint64_t adv_b = static_cast<uint64_t>((B_MN ? kk * kStepK * 128 : kk * kStepK * 2) >> 4);
+                        const uint32_t more = (kb == kb0 && kk == 0) ? 0u : 1u;
+                        if (PASSES == 3) {
+                            umma_f16<CG>(d_cross, a_lo + adv_a, b_hi + adv_b, kIdesc, more);
+                            umma_f16<CG>(d_cross, a_hi + adv_a, b_lo + adv_b, kIdesc, 1u);
+                        }
+                        umma_f16<CG>(d_main, a_hi + adv_a, b_hi + adv_b, kIdesc, more);
+                    }
+                    commit_all<CG>(empty_bar(s));
+                }
+                if (ok) commit_all<CG>(acc_full(acc));
+            }
+        }
+    } else {
+        // ---------------- epilogue (warps 2..5) ----------------
+        const int quarter = warp & 3;
+        float f1 = 1.0F, f2 = 1.0F, f3 = 1.0F;  // 2^-(shift_a + shift_b) in factors that stay in range
+        if (PASSES == 3 && n_units > 0) {
+            const int e = -range_shift(__ldcg(&g.range_a->max_bits)) - range_shift(__ldcg(&g.range_b->max_bits));
+            const int e1 = max(-126, min(126, e));
+            const int e2 = max(-126, min(126, e - e1));
+            f1 = exp2_int(e1);
+            f2 = exp2_int(e2);
+            f3 = exp2_int(e - e1 - e2);
+        }
+        const bool vec = g.n % 4 == 0 && g.split_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(g.out) & (g.out_half ? 7 : 15)) == 0;
+        uint32_t tile_it = 0;
+        for (int64_t u = unit0; u < n_units; u += unit_step, ++tile_it) {
+            int split;
+            int64_t batch, tm, tn;
+            decode(u, split, batch, tm, tn);
+            const int acc = tile_it % T::kAccs;
+            if (!mbar_wait(acc_full(acc), (tile_it / T::kAccs) & 1, abort_p, g.status)) break;
+            tc_fence_after();
+            const int64_t row_base = tm * kTileM + rank * kRowsM + quarter * 32;
+            const int64_t col0 = tn * BN;
+            const int64_t at = int64_t(split) * g.split_stride + (batch * g.m + row_base) * g.n + col0;
+            const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * T::kAccCols;
+#pragma unroll 1
+            for (int c = 0; c < BN / 32; ++c) {
+                if (col0 + c * 32 >= g.n || row_base >= g.m) break;  // uniform across the warp
+                uint32_t r[32];
+                tmem_ld32(t_acc + c * 32, r);
+                if (PASSES == 3) {
+                    uint32_t x[32];
+                    tmem_ld32(t_acc + BN + c * 32, x);
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        r[j] = __float_as_uint(fmaf(__uint_as_float(x[j]), 0x1p-11F, __uint_as_float(r[j])) * f1 * f2 * f3);
+                    }
+                }
+                const int64_t left = g.n - (col0 + c * 32);
+                if (vec && left >= 32) {
+                    // through a padded patch, so that a warp stores whole row segments
+                    float* patch = &epi_patch[quarter][0][0];
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        *reinterpret_cast<uint4*>(patch + lane * kPatchPitch + 4 * j) =
+                            make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+                    }
+                    __syncwarp();
+                    const int sub = lane >> 3, seg = lane & 7;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int rl = i * 4 + sub;
+                        if (row_base + rl < g.m) {
+                            const float4 v = *reinterpret_cast<const float4*>(patch + rl * kPatchPitch + seg * 4);
+                            const int64_t o = at + int64_t(rl) * g.n + c * 32 + seg * 4;
+                            if (g.out_half) {
+                                __half2 h[2] = {__floats2half2_rn(v.x, v.y), __floats2half2_rn(v.z, v.w)};
+                                *reinterpret_cast<uint2*>(static_cast<__half*>(g.out) + o) = *reinterpret_cast<const uint2*>(h);
+                            } else {
+                                *reinterpret_cast<float4*>(static_cast<float*>(g.out) + o) = v;
+                            }
+                        }
+                    }
+                    __syncwarp();
+                } else if (row_base + lane < g.m) {
+                    const int64_t o = at + int64_t(lane) * g.n + c * 32;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        if (j < left) {
+                            if (g.out_half) static_cast<__half*>(g.out)[o + j] = __float2half_rn(__uint_as_float(r[j]));
+                            else static_cast<float*>(g.out)[o + j] = __uint_as_float(r[j]);
+                        }
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                if (CG == 2) mbar_arrive_cluster(lead_addr(acc_empty(acc)));
+                else mbar_arrive(acc_empty(acc));
+            }
+        }
+    }
+
+    __syncthreads();
+    if (abort_flag != 0) {
+        for (int i = 0; i < 200; ++i) __nanosleep(1000);  // copies in flight land before the CTA retires
+        __syncthreads();
+    }
+    tc_fence_before();
+    if (CG == 2) cluster_sync();  // nothing of the pair is addressed after this
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_put<CG>(tmem_base, T::kTmemCols);
+    }
+}
+
+// Sums the K-slices' partial planes in split order.
+template <typename Out>
+__global__ void __launch_bounds__(256) fold_kernel(Out* __restrict__ out, const float* __restrict__ part, int64_t n, int splits,
+                                                   H16Args g, int passes) {
+    pdl_prologue();
+    if (passes == 3 && (range_wide(g.range_a, g.limit_a) || range_wide(g.range_b, g.limit_b))) return;
+    const int64_t step = int64_t(gridDim.x) * blockDim.x;
+    if (n % 4 == 0) {
+        for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n / 4; i += step) {
+            float4 s = __ldcg(reinterpret_cast<const float4*>(part) + i);
+            for (int k = 1; k < splits; ++k) {
+                const float4 v = __ldcg(reinterpret_cast<const float4*>(part + int64_t(k) * n) + i);
+                s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+            }
+            if constexpr (sizeof(Out) == 2) {
+                __half2 h[2] = {__floats2half2_rn(s.x, s.y), __floats2half2_rn(s.z, s.w)};
+                if (reinterpret_cast<uintptr_t>(out) % 8 == 0) {
+                    reinterpret_cast<uint2*>(out)[i] = *reinterpret_cast<const uint2*>(h);
+                } else {
+                    for (int j = 0; j < 4; ++j) out[4 * i + j] = reinterpret_cast<const __half*>(h)[j];
+                }
+            } else if (reinterpret_cast<uintptr_t>(out) % 16 == 0) {
+                reinterpret_cast<float4*>(out)[i] = s;
+            } else {
+                out[4 * i] = s.x; out[4 * i + 1] = s.y; out[4 * i + 2] = s.z; out[4 * i + 3] = s.w;
+            }
+        }
+        return;
+    }
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += step) {
+        float s = __ldcg(part + i);
+        for (int k = 1; k < splits; ++k) s += __ldcg(part + int64_t(k) * n + i);
+        out[i] = static_cast<Out>(s);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Host side
+// ---------------------------------------------------------------------------
+
+// A half matrix as a 4-D tensor: (unit-stride axis, the other axis, inner batch, outer batch), boxes of 64 x box_rows.
+CUtensorMap half_map(const __half* base, int64_t cols, int64_t rows, int64_t pitch, int64_t b1, int64_t s_b1, int64_t b0,
+                     int64_t s_b0, int box_rows) {
+    CUtensorMap m;
+    const int64_t plane = std::max<int64_t>(rows * pitch, 8);
+    if (b1 <= 1) { b1 = 1; s_b1 = plane; }
+    if (b0 <= 1) { b0 = 1; s_b0 = std::max(plane, s_b1 * b1); }
+    const cuuint64_t dims[4] = {cuuint64_t(cols), cuuint64_t(rows), cuuint64_t(b1), cuuint64_t(b0)};
+    const cuuint64_t strides[3] = {cuuint64_t(pitch) * 2, cuuint64_t(s_b1) * 2, cuuint64_t(s_b0) * 2};
+    const cuuint32_t box[4] = {kBlockK, cuuint32_t(box_rows), 1, 1};
+    const cuuint32_t elem[4] = {1, 1, 1, 1};
+    const CUresult rc = encode_tiled()(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<__half*>(base), dims, strides, box,
+                                       elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (rc != CUDA_SUCCESS) {
+        fail(B200_INTERNAL_ERROR, "cuTensorMapEncodeTiled (half operand) failed with code " + std::to_string(rc));
+    }
+    return m;
+}
+
+// One operand as the matrix it is in memory: rows x cols with `cols` the unit-stride axis where there is one.
+// An operand whose M (or N) axis is that axis is consumed MN-major: nothing is transposed.
+struct HalfOperand {
+    bool mn = false, bcast = false;
+    int64_t rows = 0, cols = 0, nb = 1, b1 = 1, s_b0 = 0, s_b1 = 0, s_r = 0, s_c = 0, pitch = 0;
+    const void* src = nullptr;
+    const __half* hi = nullptr;  // (one pass: the operand itself, or its packed copy)
+    const __half* lo = nullptr;
+    int64_t map_b1 = 1, map_s_b1 = 0, map_b0 = 1, map_s_b0 = 0;
+    RangeSlot* range = nullptr;
+    PlaneKey key{};
+    bool cached = false, fresh = false;
+
+    int64_t numel() const { return nb * rows * cols; }
+    size_t plane_bytes() const { return static_cast<size_t>(align_up(nb * rows * pitch * 2, 1024)); }
+    uint32_t limit() const { return kStrayFloor + static_cast<uint32_t>(std::min<int64_t>(numel() >> 21, 1 << 30)); }
+    CUtensorMap map(const __half* plane, int tile) const {
+        return half_map(plane, cols, rows, pitch, map_b1, map_s_b1, map_b0, map_s_b0, mn ? kBlockK : tile);
+    }
+};
+
+HalfOperand half_operand(const void* src, const int64_t (&s)[4], int mn_axis, int k_axis, int64_t mn_extent, int64_t k_extent,
+                         const GemmProblem& p) {
+    HalfOperand o;
+    o.src = src;
+    o.bcast = (s[0] == 0 || p.b0 == 1) && (s[1] == 0 || p.b1 == 1);
+    o.nb = o.bcast ? 1 : p.b0 * p.b1;
+    o.b1 = o.bcast ? 1 : p.b1;
+    o.s_b0 = o.bcast ? 0 : s[0];
+    o.s_b1 = o.bcast ? 0 : s[1];
+    o.mn = s[mn_axis] == 1 && s[k_axis] != 1;
+    o.rows = o.mn ? k_extent : mn_extent;
+    o.cols = o.mn ? mn_extent : k_extent;
+    o.s_r = o.mn ? s[k_axis] : s[mn_axis];
+    o.s_c = o.mn ? s[mn_axis] : s[k_axis];
+    return o;
+}
+
+HalfOperand operand_a(const GemmProblem& p) { return half_operand(p.a, p.a_s, 2, 3, p.m, p.k, p); }
+HalfOperand operand_b(const GemmProblem& p) { return half_operand(p.b, p.b_s, 3, 2, p.n, p.k, p); }
+
+// The dense layout of planes and packed copies: [batch][row][pitch].
+void lay_out_planes(HalfOperand& o) {
+    o.pitch = align_up(o.cols, 8);
+    o.map_b1 = o.nb;
+    o.map_s_b1 = o.rows * o.pitch;
+    o.map_b0 = 1;
+    o.map_s_b0 = 0;
+    o.key.src = o.src;
+    const int64_t kv[9] = {o.rows, o.cols, o.s_r, o.s_c, o.b1, o.s_b0, o.s_b1, o.nb, 1};
+    for (int i = 0; i < 9; ++i) o.key.v[i] = kv[i];
+}
+
+template <int CG, int BN, int PASSES, bool A_MN, bool B_MN>
+void launch_tile(b200_ctx* ctx, const HalfOperand& a, const HalfOperand& b, const H16Args& g, int64_t units) {
+    using T = H16Tile<CG, BN, PASSES>;
+    auto kernel = gemm_h16_kernel<CG, BN, PASSES, A_MN, B_MN>;
+    B200_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kTotal));
+    const CUtensorMap ah = a.map(a.hi, kRowsM), bh = b.map(b.hi, BN / CG);
+    const CUtensorMap al = PASSES == 3 ? a.map(a.lo, kRowsM) : ah, bl = PASSES == 3 ? b.map(b.lo, BN / CG) : bh;
+    int sms = ctx->prop.multiProcessorCount;
+    if (ctx->in_grad_sync_span && ctx->comm_pending) sms = std::max(sms - ctx->comm_sms, sms / 2);
+    const int grid = static_cast<int>(std::min<int64_t>(units, sms / CG)) * CG;
+    launch_kernel_clustered(ctx, kernel, grid, kThreads, T::kTotal, CG, ah, al, bh, bl, g);
+    ctx->count_launch();
+}
+
+template <int CG, int BN, int PASSES>
+void launch_major(b200_ctx* ctx, const HalfOperand& a, const HalfOperand& b, const H16Args& g, int64_t units) {
+    if constexpr (BN / CG >= 64) {  // (an MN-major atom is 64 wide)
+        if (b.mn) {
+            if (a.mn) launch_tile<CG, BN, PASSES, true, true>(ctx, a, b, g, units);
+            else launch_tile<CG, BN, PASSES, false, true>(ctx, a, b, g, units);
+            return;
+        }
+    }
+    if (a.mn) launch_tile<CG, BN, PASSES, true, false>(ctx, a, b, g, units);
+    else launch_tile<CG, BN, PASSES, false, false>(ctx, a, b, g, units);
+}
+
+struct TileChoice {
+    int cg, bn;
+    int64_t tiles_m, tiles_n, splits, kb_per_split, units;
+};
+
+// The tile whose whole waves cost least.  `width` x 128 rows of cg CTAs; a narrower or single-CTA tile moves more
+// operand bytes per product (relative cost per unit of work beside the widest), so it is taken only
+// where the widest one would leave SMs idle: few tiles, or a nearly empty last wave.
+TileChoice choose_tile(const GemmProblem& p, int passes, bool b_mn, int sms) {
+    struct Form { int cg, bn; double cost; };
+    // cost of one K-block of a tile, in units of a 256 x 128 tile's
+    static const Form three[] = {{2, 128, 1.0}, {2, 64, 0.56}, {1, 128, 1.08}, {1, 64, 0.6}};
+    static const Form one[] = {{2, 256, 1.9}, {2, 128, 1.0}, {1, 128, 1.08}, {1, 64, 0.6}};
+    const Form* forms = passes == 3 ? three : one;
+    const int64_t batches = p.b0 * p.b1, k_blocks = ceil_div(p.k, kBlockK);
+    TileChoice best{};
+    double least = 0;
+    for (int i = 0; i < 4; ++i) {
+        const Form& f = forms[i];
+        if (b_mn && f.bn / f.cg < 64) continue;  // an MN-major atom is 64 wide
+        TileChoice c{f.cg, f.bn, ceil_div(p.m, int64_t(f.cg) * kRowsM), ceil_div(p.n, int64_t(f.bn)), 1, k_blocks, 0};
+        const int64_t tiles = c.tiles_m * c.tiles_n * batches, slots = sms / f.cg;
+        if (tiles < slots && k_blocks >= 8) {
+            // as many K-slices as keep every unit in one wave, none shorter than four K-blocks
+            c.splits = std::max<int64_t>(1, std::min({slots / tiles, k_blocks / 4, int64_t(64)}));
+            c.kb_per_split = ceil_div(k_blocks, c.splits);
+            c.splits = ceil_div(k_blocks, c.kb_per_split);
+        }
+        c.units = tiles * c.splits;
+        const double waves = double(ceil_div(c.units, slots));
+        // a tile's fill and drain come to about two K-blocks; slices write and fold partial planes
+        const double cost = waves * f.cost * (double(c.kb_per_split) + 2.0) + (c.splits > 1 ? 4.0 : 0.0);
+        if (i == 0 || cost < least) {
+            least = cost;
+            best = c;
+        }
+    }
+    return best;
+}
+
+void run_h16(b200_ctx* ctx, const GemmProblem& p, int passes, const TileChoice& t, const HalfOperand& a, const HalfOperand& b,
+             float* partial, bool out_half, const char* label) {
+    H16Args g{};
+    const int64_t batches = p.b0 * p.b1, out_elems = batches * p.m * p.n;
+    g.out = t.splits > 1 ? static_cast<void*>(partial) : static_cast<void*>(p.out);
+    g.out_half = t.splits > 1 ? 0 : (out_half ? 1 : 0);
+    g.m = p.m;
+    g.n = p.n;
+    g.batches = batches;
+    g.a_b1 = a.bcast ? 0 : static_cast<int>(a.map_b1);
+    g.b_b1 = b.bcast ? 0 : static_cast<int>(b.map_b1);
+    g.k_blocks = ceil_div(p.k, kBlockK);
+    g.kb_per_split = t.kb_per_split;
+    g.splits = static_cast<int>(t.splits);
+    g.split_stride = out_elems;
+    g.tiles_m = t.tiles_m;
+    g.tiles_n = t.tiles_n;
+    g.group_m = ctx->gemm_group_m > 0 ? ctx->gemm_group_m : kGroupRows / (t.cg * kRowsM);
+    g.range_a = a.range;
+    g.range_b = b.range;
+    g.limit_a = a.limit();
+    g.limit_b = b.limit();
+    g.status = ctx->d_status;
+    {
+        ProfScope scope(ctx, label);
+#define B200_H16_CASE(CG, BN, P)                                  \
+    if (t.cg == CG && t.bn == BN && passes == P) launch_major<CG, BN, P>(ctx, a, b, g, t.units);
+        B200_H16_CASE(2, 128, 3)
+        B200_H16_CASE(2, 64, 3)
+        B200_H16_CASE(1, 128, 3)
+        B200_H16_CASE(1, 64, 3)
+        B200_H16_CASE(2, 256, 1)
+        B200_H16_CASE(2, 128, 1)
+        B200_H16_CASE(1, 128, 1)
+        B200_H16_CASE(1, 64, 1)
+#undef B200_H16_CASE
+    }
+    check_last_launch("matmul (tcgen05, half terms)");
+    if (t.splits > 1) {
+        ProfScope scope(ctx, "matmul.fold");
+        const int blocks = grid_for(ceil_div(out_elems, 4), 256);
+        if (out_half) {
+            launch_kernel(ctx, fold_kernel<__half>, blocks, 256, 0, reinterpret_cast<__half*>(p.out), partial, out_elems,
+                          static_cast<int>(t.splits), g, passes);
+        } else {
+            launch_kernel(ctx, fold_kernel<float>, blocks, 256, 0, p.out, partial, out_elems, static_cast<int>(t.splits), g, passes);
+        }
+        ctx->count_launch();
+        check_last_launch("matmul (fold)");
+    }
+}
+
+bool fits_tma(const GemmProblem& p) {
+    const int64_t lim = int64_t(1) << 31;
+    return p.m < lim && p.n < lim && p.k < lim && p.b0 * p.b1 < lim;
+}
+
+MatrixArgs matrix_args(const HalfOperand& o) {
+    MatrixArgs a{};
+    a.src = static_cast<const float*>(o.src);
+    a.hi = const_cast<__half*>(o.hi);
+    a.lo = const_cast<__half*>(o.lo);
+    a.range = o.range;
+    a.b1 = o.b1;
+    a.n_batches = o.nb;
+    a.s_b0 = o.s_b0;
+    a.s_b1 = o.s_b1;
+    a.s_r = o.s_r;
+    a.s_c = o.s_c;
+    a.rows = o.rows;
+    a.cols = o.cols;
+    a.pitch = o.pitch;
+    a.vec = o.s_c == 1 && o.s_r % 4 == 0 && o.s_b0 % 4 == 0 && o.s_b1 % 4 == 0 && reinterpret_cast<uintptr_t>(o.src) % 16 == 0;
+    return a;
+}
+
+}  // namespace
+
+// Products above 2^32 operations: the range pass (one more read of each operand than the TF32 planes need)
+// and the three launches that stand by for a wide operand cost about 10 us together, which the halved
+// MMA time does not return on smaller ones.  What the streamed-operand kernel or the direct operands serve stays there.
+bool gemm_h16_serves(const b200_ctx* ctx, const GemmProblem& p) {
+    if (ctx->gemm_precision != B200_GEMM_3XTF32 || !ctx->gemm_half_terms || ctx->gemm_operands >= 0 || ctx->gemm_stream > 0 ||
+        ctx->gemm_schedule == 1 || ctx->gemm_bn_override != 0 || !fits_tma(p)) {
+        return false;
+    }
+    const double flops = 2.0 * double(p.m) * double(p.n) * double(p.k) * double(p.b0 * p.b1);
+    return flops >= 4294967296.0 && !gemm_tc_streams(ctx, p) && ctx->compared.count(p.out) == 0;
+}
+
+void gemm_h16_note_uses(b200_ctx* ctx, const GemmProblem& p) {
+    HalfOperand a = operand_a(p), b = operand_b(p);
+    lay_out_planes(a);
+    lay_out_planes(b);
+    ++ctx->plane_uses[a.key];
+    ++ctx->plane_uses[b.key];
+}
+
+void gemm_h16(b200_ctx* ctx, const GemmProblem& p) {
+    HalfOperand a = operand_a(p), b = operand_b(p);
+    const TileChoice t = choose_tile(p, 3, b.mn, ctx->prop.multiProcessorCount);
+    if (ctx->range_next + 2 > kRangeSlots) {
+        gemm_tc(ctx, p, true);
+        return;
+    }
+    if (ctx->range_next == 0) {
+        B200_CUDA_CHECK(cudaMemsetAsync(ctx->d_ranges, 0, sizeof(RangeSlot) * kRangeSlots, ctx->stream));
+    }
+    const size_t cache_limit = std::min<size_t>(size_t(16) << 30, ctx->prop.totalGlobalMem / 8);
+    auto place = [&](HalfOperand& o) {
+        lay_out_planes(o);
+        if (auto it = ctx->plane_cache.find(o.key); it != ctx->plane_cache.end()) {
+            o.hi = reinterpret_cast<const __half*>(it->second.hi);
+            o.lo = reinterpret_cast<const __half*>(it->second.lo);
+            o.range = static_cast<RangeSlot*>(it->second.range);
+            o.cached = true;
+            ++ctx->plane_hits;
+            return;
+        }
+        o.fresh = true;
+        o.range = static_cast<RangeSlot*>(ctx->d_ranges) + ctx->range_next++;
+        const auto uses = ctx->plane_uses.find(o.key);
+        const size_t bytes = 2 * o.plane_bytes();
+        if (uses != ctx->plane_uses.end() && uses->second >= 2 && ctx->plane_cache_bytes + bytes <= cache_limit) {
+            char* block = static_cast<char*>(ctx->scratch.allocate(bytes));
+            o.hi = reinterpret_cast<const __half*>(block);
+            o.lo = reinterpret_cast<const __half*>(block + o.plane_bytes());
+            const char* begin = static_cast<const char*>(o.src);
+            auto mag = [](int64_t v) { return v < 0 ? -v : v; };
+            const int64_t span = (o.nb / o.b1 - 1) * mag(o.s_b0) + (o.b1 - 1) * mag(o.s_b1) + (o.rows - 1) * mag(o.s_r) +
+                                 (o.cols - 1) * mag(o.s_c) + 1;
+            ctx->plane_cache[o.key] = PlaneEntry{reinterpret_cast<float*>(block), reinterpret_cast<float*>(block + o.plane_bytes()),
+                                                 bytes, uses->second, begin, begin + span * 4, o.range};
+            ctx->plane_cache_bytes += bytes;
+            o.cached = true;
+        }
+    };
+    place(a);
+    place(b);  // (B may be the very matrix A just put there)
+
+    const int64_t out_elems = p.b0 * p.b1 * p.m * p.n;
+    const size_t partial_bytes = t.splits > 1 ? static_cast<size_t>(align_up(out_elems * t.splits * 4, 1024)) : 0;
+    const size_t tf32_bytes = gemm_tc_plane_bytes(p);
+    size_t bytes = partial_bytes + tf32_bytes + 1024;
+    if (!a.cached) bytes += 2 * a.plane_bytes();
+    if (!b.cached) bytes += 2 * b.plane_bytes();
+    char* ws = static_cast<char*>(ctx->ensure_workspace(bytes));
+    ws = reinterpret_cast<char*>(align_up(reinterpret_cast<int64_t>(ws), 1024));
+    for (HalfOperand* o : {&a, &b}) {
+        if (o->cached) continue;
+        o->hi = reinterpret_cast<const __half*>(ws);
+        o->lo = reinterpret_cast<const __half*>(ws + o->plane_bytes());
+        ws += 2 * o->plane_bytes();
+    }
+    float* partial = reinterpret_cast<float*>(ws);
+    ws += partial_bytes;
+
+    MatrixPair pair{};
+    int fresh = 0;
+    int64_t largest = 0;
+    for (HalfOperand* o : {&a, &b}) {
+        if (!o->fresh) continue;
+        pair.m[fresh++] = matrix_args(*o);
+        largest = std::max(largest, o->nb * o->rows * (o->pitch / 8));
+    }
+    if (fresh > 0) {
+        const dim3 grid(grid_for(largest, 256), static_cast<unsigned>(fresh));
+        {
+            ProfScope scope(ctx, "matmul.range");
+            launch_kernel(ctx, range_kernel, dim3(grid_for(std::min(largest, kSampleGroups), 256), grid.y), 256, 0, pair);
+        }
+        {
+            ProfScope scope(ctx, "matmul.split");
+            launch_kernel(ctx, split_half_kernel, grid, 256, 0, pair);
+        }
+        ctx->count_launch(2);
+        check_last_launch("matmul (operand range and split)");
+    }
+    run_h16(ctx, p, 3, t, a, b, partial, false, "matmul.tcgen05_3xf16");
+    gemm_tc_if_wide(ctx, p, RangeGuard{a.range, b.range, a.limit(), b.limit()}, ws);
+    for (HalfOperand* o : {&a, &b}) {
+        if (!o->cached) continue;
+        const auto it = ctx->plane_cache.find(o->key);
+        if (it != ctx->plane_cache.end() && --it->second.uses_left <= 0) {
+            ctx->scratch.release(it->second.hi);  // the stream is in order: only later work reuses it
+            ctx->plane_cache_bytes -= it->second.bytes;
+            ctx->plane_cache.erase(it);
+        }
+    }
+}
+
+// Half storage: products of at least 2^25 operations with a row for most of a tile's lanes (smaller ones are
+// launch-bound, and served through widened copies by the CUDA cores).
+bool gemm_f16_storage(b200_ctx* ctx, const GemmProblem& p) {
+    if (ctx->prop.major != 10 || encode_tiled() == nullptr || ctx->gemm_precision == B200_GEMM_FP32 || !fits_tma(p) ||
+        p.m < 32 || p.n < 16 || p.k < 16) {
+        return false;
+    }
+    if (2.0 * double(p.m) * double(p.n) * double(p.k) * double(p.b0 * p.b1) < double(1 << 25)) return false;
+    HalfOperand a = operand_a(p), b = operand_b(p);
+    const TileChoice t = choose_tile(p, 1, b.mn, ctx->prop.multiProcessorCount);
+    size_t bytes = 2048;
+    auto direct = [](HalfOperand& o) {
+        const bool ok = o.s_c == 1 && o.s_r % 8 == 0 && o.s_r >= o.cols && reinterpret_cast<uintptr_t>(o.src) % 16 == 0 &&
+                        o.s_b0 % 8 == 0 && o.s_b1 % 8 == 0 && (o.nb == 1 || ((o.b1 == 1 || o.s_b1 > 0) && (o.nb == o.b1 || o.s_b0 > 0)));
+        if (ok) {
+            o.pitch = o.s_r;
+            o.hi = static_cast<const __half*>(o.src);
+            o.map_b1 = o.b1;
+            o.map_s_b1 = o.s_b1;
+            o.map_b0 = o.nb / o.b1;
+            o.map_s_b0 = o.s_b0;
+        } else {
+            lay_out_planes(o);
+        }
+        return ok;
+    };
+    const bool da = direct(a), db = direct(b);
+    const int64_t out_elems = p.b0 * p.b1 * p.m * p.n;
+    if (!da) bytes += a.plane_bytes();
+    if (!db) bytes += b.plane_bytes();
+    if (t.splits > 1) bytes += static_cast<size_t>(out_elems * t.splits * 4);
+    char* ws = static_cast<char*>(ctx->ensure_workspace(bytes));
+    ws = reinterpret_cast<char*>(align_up(reinterpret_cast<int64_t>(ws), 1024));
+    for (HalfOperand* o : {&a, &b}) {
+        if (o == &a ? da : db) continue;
+        o->hi = reinterpret_cast<const __half*>(ws);
+        ws += o->plane_bytes();
+        ProfScope scope(ctx, "matmul.pack");
+        launch_kernel(ctx, pack_half_kernel, grid_for(o->nb * o->rows * (o->pitch / 8), 256), 256, 0,
+                      static_cast<const __half*>(o->src), const_cast<__half*>(o->hi), o->b1, o->s_b0, o->s_b1, o->s_r, o->s_c,
+                      o->rows, o->cols, o->pitch, o->nb);
+        ctx->count_launch();
+    }
+    run_h16(ctx, p, 1, t, a, b, reinterpret_cast<float*>(ws), true, "matmul.tcgen05_f16");
+    return true;
+}
+
+}  // namespace b200

@@ -39,8 +39,7 @@
 // their loops, TMEM is freed and the kernel returns; the host reports
 // B200_TIMEOUT at the next synchronize.
 #include "gemm.h"
-
-#include <cuda.h>  // CUtensorMap and the cuTensorMapEncodeTiled prototype (types only)
+#include "tcgen05.cuh"
 
 namespace b200 {
 namespace {
@@ -54,111 +53,6 @@ constexpr int kThreadsDirect = kThreads + kProducerThreads;
 constexpr int kGroupM = 16;
 constexpr int kEpiPitch = 36;   // words per row of the epilogue's staging patch (16-byte aligned rows)
 constexpr int kSchedRing = 4;  // published-but-unconsumed tile numbers per CTA
-constexpr uint64_t kWaitLimitNs = 4000000000ULL;  // 4 s
-
-// ---------------------------------------------------------------------------
-// PTX wrappers
-// ---------------------------------------------------------------------------
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-                 : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-// The same test, but the hardware may park the thread for up to `hint_ns` while the phase is
-// still open (it is woken when the phase completes).  For the many warps that wait for one
-// event, a parked warp leaves the issue slots and the shared-memory pipe to the warps that work.
-__device__ __forceinline__ bool mbar_try_wait_parked(uint32_t bar, uint32_t parity, uint32_t hint_ns) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity), "r"(hint_ns)
-        : "memory");
-    return ok != 0;
-}
-
-__device__ __forceinline__ uint64_t global_ns() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Bounded wait. Returns false (and raises the abort flag) when the limit ran out
-// or another role already aborted.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          uint32_t* status, uint64_t limit_ns = kWaitLimitNs) {
-    // The clock is only consulted every 1024 polls (reading %globaltimer costs far more than a
-    // poll, and the converter warps wait here once per K-block), so the limit is the stated time
-    // plus at most 1024 polls.
-    uint64_t start = 0;
-    uint32_t spins = 0;
-    while (!mbar_try_wait(bar, parity)) {
-        if ((++spins & 0x3ff) == 0) {
-            if (*abort_flag != 0) {
-                return false;
-            }
-            const uint64_t now = global_ns();
-            if (start == 0) {
-                start = now;
-            } else if (now - start > limit_ns) {
-                *abort_flag = 1;
-                atomicOr(status, kStatusWaitTimedOut);
-                return false;
-            }
-        }
-    }
-    return true;
-}
-
-// Bounded wait for the warps of a many-waiter role: parked polls, the clock read every 64 of them.
-__device__ __forceinline__ bool mbar_wait_parked(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                                 uint32_t* status) {
-    uint64_t start = 0;
-    uint32_t spins = 0;
-    while (!mbar_try_wait_parked(bar, parity, 2000u)) {
-        if ((++spins & 0x3f) == 0) {
-            if (*abort_flag != 0) {
-                return false;
-            }
-            const uint64_t now = global_ns();
-            if (start == 0) {
-                start = now;
-            } else if (now - start > kWaitLimitNs) {
-                *abort_flag = 1;
-                atomicOr(status, kStatusWaitTimedOut);
-                return false;
-            }
-        }
-    }
-    return true;
-}
 
 // One block that waits, through the very mbar_wait the GEMM kernels use, on a barrier nobody will
 // ever arrive on: the wait runs out after `limit_ns`, records kStatusWaitTimedOut and the kernel
@@ -175,65 +69,6 @@ __global__ void wait_probe_kernel(uint32_t* status, uint64_t limit_ns) {
     }
 }
 
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0,
-                                            int c1) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1)
-        : "memory");
-}
-
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1,
-                                            int c2, int c3) {
-    asm volatile(
-        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
-        ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
-        : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t cols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(cols)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
-}
-
-__device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-// Arrives on `bar` once every tcgen05.mma issued so far by this thread has finished.
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-                 : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
 // Shared-memory matrix descriptors, 128-byte swizzle, 32-bit elements.
 //
 // K-major tile ([rows][32 floats], one swizzle row per matrix row): 8-row groups are 1024
@@ -248,17 +83,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 // so the stride-dimension offset is 512 bytes; the next atom along MN starts kMnAtomBytes
 // later (leading-dimension offset).  One K step (8 K-rows) advances the start by 1024 bytes.
 constexpr uint32_t kMnAtomBytes = BK * 128;  // 32 K-rows x 128 bytes
-
-__device__ __forceinline__ uint64_t smem_desc(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes,
-                                              uint32_t layout_type) {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((smem_addr & 0x3FFFF) >> 4);   // start address, bits 0-13
-    d |= static_cast<uint64_t>(lbo_bytes >> 4) << 16;         // leading-dimension byte offset, bits 16-29
-    d |= static_cast<uint64_t>(sbo_bytes >> 4) << 32;         // stride-dimension byte offset, bits 32-45
-    d |= static_cast<uint64_t>(1) << 46;                      // descriptor version for sm_100
-    d |= static_cast<uint64_t>(layout_type) << 61;            // 2: 128-byte swizzle, 1: same with 32-byte atoms
-    return d;
-}
 
 template <bool MN_MAJOR>
 __device__ __forceinline__ uint64_t operand_desc(uint32_t smem_addr) {
@@ -345,8 +169,7 @@ struct SplitArgs {
 
 // Source rows dense along K and 16-byte aligned: one thread per four K-elements, 128-bit
 // loads and stores, no shared memory.
-__global__ void __launch_bounds__(256) split_rows_kernel(SplitArgs a) {
-    pdl_prologue();
+__device__ __forceinline__ void split_rows(const SplitArgs& a) {
     const int64_t kp4 = a.kp / 4;
     const int64_t total = kp4 * a.out_rows * a.n_batches;
     const int64_t step = int64_t(gridDim.x) * blockDim.x;
@@ -386,8 +209,7 @@ __global__ void __launch_bounds__(256) split_rows_kernel(SplitArgs a) {
 // thread in flight in each phase.
 constexpr int kSplitTile = 64;
 
-__global__ void __launch_bounds__(256) split_kernel(SplitArgs a) {
-    pdl_prologue();
+__device__ __forceinline__ void split_tiles(const SplitArgs& a) {
     __shared__ float tile[kSplitTile][kSplitTile + 1];  // [row][k]
     const int fast = threadIdx.x & 63, slow = threadIdx.x >> 6;
     const int64_t tiles_k = a.kp / kSplitTile + (a.kp % kSplitTile != 0);
@@ -439,11 +261,39 @@ __global__ void __launch_bounds__(256) split_kernel(SplitArgs a) {
     }
 }
 
+__global__ void __launch_bounds__(256) split_rows_kernel(SplitArgs a) {
+    pdl_prologue();
+    split_rows(a);
+}
+
+__global__ void __launch_bounds__(256) split_kernel(SplitArgs a) {
+    pdl_prologue();
+    split_tiles(a);
+}
+
+bool rows_dense(const SplitArgs& s) {
+    return s.s_k == 1 && s.s_r % 4 == 0 && s.s_b0 % 4 == 0 && s.s_b1 % 4 == 0 && reinterpret_cast<uintptr_t>(s.src) % 16 == 0;
+}
+
+// Both operands of a product in one launch, for the planes that stand by for a wide operand: nearly always
+// there is nothing to do, and then a launch of a few hundred blocks costs less than two full ones.
+struct SplitPair {
+    SplitArgs s[2];
+    int dense[2];
+    RangeGuard guard;
+};
+
+__global__ void __launch_bounds__(256) split_if_wide_kernel(SplitPair p) {
+    pdl_prologue();
+    if (guard_idle(p.guard)) return;
+    const SplitArgs& a = p.s[blockIdx.y];
+    if (p.dense[blockIdx.y]) split_rows(a);
+    else split_tiles(a);
+}
+
 void launch_split(b200_ctx* ctx, const SplitArgs& s, const char* label) {
     ProfScope scope(ctx, label);
-    const bool rows_dense = s.s_k == 1 && s.s_r % 4 == 0 && s.s_b0 % 4 == 0 && s.s_b1 % 4 == 0 &&
-                            reinterpret_cast<uintptr_t>(s.src) % 16 == 0;
-    if (rows_dense) {
+    if (rows_dense(s)) {
         const int64_t total = (s.kp / 4) * s.out_rows * s.n_batches;
         launch_kernel(ctx, split_rows_kernel, grid_for(ceil_div(total, 2), 256), 256, 0, s);
     } else {
@@ -474,6 +324,7 @@ struct TcArgs {
     // zeroed counter from which CTAs draw their units after the first, so a CTA that starts late
     // or shares its SM with another kernel (an all-reduce) simply takes fewer tiles.
     unsigned int* sched;
+    RangeGuard guard;
 };
 
 // Direct-operand variant: TMA brings the fp32 operand tiles themselves into the `hi` slots of a
@@ -559,7 +410,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_consta
     pdl_prologue();
 
     const int64_t tiles_per_batch = g.tiles_m * g.tiles_n;
-    const int64_t n_units = tiles_per_batch * g.batches * g.splits;
+    const int64_t n_units = guard_idle(g.guard) ? 0 : tiles_per_batch * g.batches * g.splits;
 
     // unit -> (split, batch, m tile, n tile); M-tiles walked in groups of kGroupM
     auto decode = [&](int64_t u, int& split, int64_t& batch, int64_t& tm, int64_t& tn) {
@@ -1421,25 +1272,6 @@ fold_partials_kernel(float* __restrict__ out, const float* __restrict__ partial,
 // Host side
 // ---------------------------------------------------------------------------
 
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                   CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                   CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled() {
-    static EncodeTiledFn fn = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess) {
-            cudaGetLastError();
-            return static_cast<EncodeTiledFn>(nullptr);
-        }
-        return reinterpret_cast<EncodeTiledFn>(p);
-    }();
-    return fn;
-}
-
 // Plane [rows][pitch] of f32 (pitch in floats, a multiple of 4), boxes of 32 floats x box_rows,
 // 128-byte swizzle.  K-major planes: pitch = Kp, rows = matrix rows, box_rows = tile rows.
 // MN-major planes: pitch = padded M or N, rows = batches * Kp, box_rows = 32 K-rows.
@@ -1458,8 +1290,6 @@ CUtensorMap make_map(float* plane, int64_t rows, int64_t pitch, int box_rows, bo
     }
     return m;
 }
-
-int64_t align_up(int64_t v, int64_t a) { return (v + a - 1) / a * a; }
 
 // The caller's own matrix as a 4-D tensor: (unit-stride axis, the other matrix axis, inner
 // batch, outer batch), f32, boxes of 32 floats x box_rows, zero fill outside.  A broadcast
@@ -2100,6 +1930,64 @@ void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass) {
     release_use(ctx, ob);
 }
 
+size_t gemm_tc_plane_bytes(const GemmProblem& p) {
+    const bool a_bcast = (p.a_s[0] == 0 || p.b0 == 1) && (p.a_s[1] == 0 || p.b1 == 1);
+    const bool b_bcast = (p.b_s[0] == 0 || p.b0 == 1) && (p.b_s[1] == 0 || p.b1 == 1);
+    return 2 * plan_operand(p.a, p.a_s[0], p.a_s[1], p.a_s[2], p.a_s[3], p.m, p.k, a_bcast, p).plane_bytes +
+           2 * plan_operand(p.b, p.b_s[0], p.b_s[1], p.b_s[3], p.b_s[2], p.n, p.k, b_bcast, p).plane_bytes;
+}
+
+void gemm_tc_if_wide(b200_ctx* ctx, const GemmProblem& p, const RangeGuard& guard, void* planes) {
+    const bool a_bcast = (p.a_s[0] == 0 || p.b0 == 1) && (p.a_s[1] == 0 || p.b1 == 1);
+    const bool b_bcast = (p.b_s[0] == 0 || p.b0 == 1) && (p.b_s[1] == 0 || p.b1 == 1);
+    Operand oa = plan_operand(p.a, p.a_s[0], p.a_s[1], p.a_s[2], p.a_s[3], p.m, p.k, a_bcast, p);
+    Operand ob = plan_operand(p.b, p.b_s[0], p.b_s[1], p.b_s[3], p.b_s[2], p.n, p.k, b_bcast, p);
+    char* ws = static_cast<char*>(planes);
+    SplitPair pair{};
+    pair.guard = guard;
+    int i = 0;
+    for (Operand* o : {&oa, &ob}) {
+        o->split.hi = o->hi = reinterpret_cast<float*>(ws);
+        o->split.lo = o->lo = reinterpret_cast<float*>(ws + o->plane_bytes);
+        ws += 2 * o->plane_bytes;
+        pair.s[i] = o->split;
+        pair.dense[i++] = rows_dense(o->split) ? 1 : 0;
+    }
+    {
+        ProfScope scope(ctx, "matmul.if_wide");
+        launch_kernel(ctx, split_if_wide_kernel, dim3(ctx->prop.multiProcessorCount * 2, 2), 256, 0, pair);
+    }
+    ctx->count_launch();
+    constexpr int bn = 128;
+    auto map_of = [&](float* plane, const Operand& o, int tile) {
+        return o.mn ? make_map(plane, o.nb * o.rows_pad, o.cols_pad, BK, true)
+                    : make_map(plane, o.nb * o.rows_pad, o.cols_pad, tile, false);
+    };
+    TcArgs g{};
+    g.out = p.out;
+    g.m = p.m;
+    g.n = p.n;
+    g.batches = p.b0 * p.b1;
+    g.a_batch_rows = a_bcast ? 0 : oa.rows_pad;
+    g.b_batch_rows = b_bcast ? 0 : ob.rows_pad;
+    g.k_blocks = ceil_div(p.k, BK);
+    g.kb_per_split = g.k_blocks;  // (no K-slices: what is queued here almost never runs)
+    g.splits = 1;
+    g.tiles_m = ceil_div(p.m, BM);
+    g.tiles_n = ceil_div(p.n, bn);
+    g.group_m = kGroupM;
+    g.status = ctx->d_status;
+    g.guard = guard;
+    const int grid = static_cast<int>(std::min<int64_t>(g.tiles_m * g.tiles_n * g.batches, ctx->prop.multiProcessorCount));
+    {
+        ProfScope scope(ctx, "matmul.if_wide");
+        launch_main<bn, 3>(ctx, true, oa.mn, ob.mn, map_of(oa.hi, oa, BM), map_of(oa.lo, oa, BM), map_of(ob.hi, ob, bn),
+                           map_of(ob.lo, ob, bn), g, grid);
+    }
+    ctx->count_launch();
+    check_last_launch("matmul (TF32 planes of a wide operand)");
+}
+
 void gemm_tc_note_uses(b200_ctx* ctx, const GemmProblem& p) {
     const int64_t batches = p.b0 * p.b1;
     (void)batches;
@@ -2134,6 +2022,7 @@ void gemm_tc_end_span(b200_ctx* ctx) {
     ctx->plane_cache.clear();
     ctx->plane_uses.clear();
     ctx->plane_cache_bytes = 0;
+    ctx->range_next = 0;
 }
 
 }  // namespace b200
