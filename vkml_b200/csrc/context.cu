@@ -970,6 +970,30 @@ static void compute_span(b200_ctx* ctx, const b200_node* nodes, size_t n_nodes, 
         }
         const size_t i = exec[p];
         const b200_node& node = nodes[i];
+        if (ctx->fuse && (node.op == B200_OP_FULL || node.op == B200_OP_CONTIGUOUS || node.op == B200_OP_LOG_SOFTMAX || node.op == B200_OP_MUL)) {
+            constexpr size_t kLook = 16;
+            const b200_node* seq[kLook];
+            size_t run = 0;
+            while (run < kLook && p + run < exec.size() && !done[p + run]) {
+                const size_t idx = exec[p + run];
+                // (a gradient that this span all-reduces is exchanged as soon as its own kernel is queued)
+                if (!is_sink.empty() && is_sink[idx]) break;
+                if (grad_sync && is_sink.empty() && !ctx->grads.empty()) break;
+                seq[run++] = &nodes[idx];
+            }
+            const size_t taken = run > 0 ? loss_group(ctx, seq, run, false) : 0;
+            if (taken > 0) {
+                for (size_t k = 0; k < taken; ++k) prepare(exec[p + k]);
+                ctx->current_op = node.op;
+                loss_group(ctx, seq, run, true);
+                for (size_t k = 0; k < taken; ++k) {
+                    constants.erase(seq[k]->out.data);
+                    finish(exec[p + k]);
+                }
+                p += taken;
+                continue;
+            }
+        }
         if (ctx->fuse && exec.size() - p >= 2 &&
             (node.op == B200_OP_ADD || node.op == B200_OP_FULL || node.op == B200_OP_EQUAL ||
              node.op == B200_OP_EXP)) {

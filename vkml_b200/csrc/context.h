@@ -45,6 +45,7 @@ private:
 // Words behind b200_ctx::d_counters: 4096 arrival counters of split reductions, 64 words for the
 // persistent GEMM's tile counter, 1024 arrival counters of the streamed-operand GEMM's split-K fold.
 constexpr size_t kArrivalCounters = 4096 + 64 + 1024;
+constexpr size_t kLossCounter = 4096 + 32;  // (of the 64) blocks of the loss's mean
 
 struct DistState;  // dist.cu
 
@@ -261,8 +262,11 @@ size_t launch_fused(b200_ctx* ctx, const b200_node* const* seq, size_t avail);
 // movement.cu: max_pool2d_backward + the where() of ReLU's backward rule behind it, one launch; false: not that case
 bool launch_pool_backward_where(b200_ctx* ctx, const b200_node& pool, const b200_node& where, int result_is_x,
                                 const void* constant);
+constexpr int64_t kTinyElements = 4096;  // one block: beyond a few thousand elements a node is faster as its own launch
 // elementwise.cu: the leading run of tiny elementwise nodes (a loss prologue) as one single-block launch
 size_t launch_tiny_chain(b200_ctx* ctx, const b200_node* const* seq, size_t avail);
+// loss.cu: a cross-entropy's head, backward and value, one launch each; how many nodes of `seq` it covers
+size_t loss_group(b200_ctx* ctx, const b200_node* const* seq, size_t avail, bool launch);
 size_t launch_scaled_add_group(b200_ctx* ctx, const b200_node* const* seq, size_t avail, bool* picked);
 
 // dist.cu

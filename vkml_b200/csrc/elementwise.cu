@@ -1138,7 +1138,6 @@ void run_float(b200_ctx* ctx, const b200_node& node, const typename F::P& p, con
 namespace {
 
 constexpr int kTinyNodes = 12;
-constexpr int64_t kTinyElems = 4096;  // one block: beyond a few thousand elements a node is faster as its own launch
 enum TinyKind : int {
     kTinyFull, kTinyArange, kTinyCopy4, kTinyCastI64, kTinyCastBool, kTinyNeg, kTinyAdd, kTinySub, kTinyMul, kTinyDiv, kTinyEqual
 };
@@ -1199,7 +1198,7 @@ __global__ void __launch_bounds__(1024) tiny_chain_kernel(const __grid_constant_
 // Fills `t` when the node is one the chain kernel serves as it stands.
 bool tiny_node(const b200_node& node, TinyNode& t) {
     const View out = make_view(node.out);
-    if (!out.contiguous || out.numel <= 0 || out.numel > kTinyElems || out.data == nullptr) return false;
+    if (!out.contiguous || out.numel <= 0 || out.numel > kTinyElements || out.data == nullptr) return false;
     const int dt = out.dtype;
     int n_src = 0;
     int want[2] = {B200_F32, B200_F32};
