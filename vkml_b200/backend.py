@@ -8,6 +8,7 @@ types vkML maps to Python (bindings/module.cpp:243-250).
 from __future__ import annotations
 
 import ctypes as C
+import struct
 from typing import Sequence
 
 import numpy as np
@@ -160,13 +161,14 @@ class Backend:
 
     def copy_device_to_device(self, copies: Sequence[tuple]) -> None:
         """copies: (dst Storage, dst_offset, src Storage, src_offset, nbytes); disjoint ranges."""
-        arr = (_abi.Copy * max(len(copies), 1))()
-        for i, (d, doff, s, soff, n) in enumerate(copies):
+        words = []
+        for d, doff, s, soff, n in copies:
             if doff < 0 or doff + n > d.nbytes or soff < 0 or soff + n > s.nbytes:
                 raise IndexError("copy_device_to_device range exceeds a storage")
-            arr[i].dst = (d.data + doff) or None
-            arr[i].src = (s.data + soff) or None
-            arr[i].nbytes = n
+            words += (d.data + doff, s.data + soff, n)
+        if not words:
+            return
+        arr = (_abi.Copy * len(copies)).from_buffer_copy(struct.pack("<%dQ" % len(words), *words))
         self._check(self._lib.b200_copy_device_to_device(self._ctx, arr, len(copies)),
                     "copy_device_to_device")
 

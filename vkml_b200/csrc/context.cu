@@ -1351,6 +1351,8 @@ int b200_copy_to_host(b200_ctx* ctx, void* dst_host, const void* src_device, siz
 int b200_copy_device_to_device(b200_ctx* ctx, const b200_copy* copies, size_t n) {
     if (ctx == nullptr || (copies == nullptr && n != 0)) return B200_INVALID_ARGUMENT;
     return guarded(ctx, [&] {
+        std::vector<b200_copy> todo;
+        todo.reserve(n);
         for (size_t i = 0; i < n; ++i) {
             if (copies[i].nbytes == 0) continue;
             if (copies[i].dst == nullptr || copies[i].src == nullptr) {
@@ -1358,8 +1360,12 @@ int b200_copy_device_to_device(b200_ctx* ctx, const b200_copy* copies, size_t n)
             }
             dist_wait_range(ctx, copies[i].dst, static_cast<const char*>(copies[i].dst) + copies[i].nbytes);
             dist_wait_range(ctx, copies[i].src, static_cast<const char*>(copies[i].src) + copies[i].nbytes);
-            B200_CUDA_CHECK(cudaMemcpyAsync(copies[i].dst, copies[i].src, copies[i].nbytes,
-                                            cudaMemcpyDeviceToDevice, ctx->stream));
+            todo.push_back(copies[i]);
+        }
+        if (todo.size() == 1) {
+            B200_CUDA_CHECK(cudaMemcpyAsync(todo[0].dst, todo[0].src, todo[0].nbytes, cudaMemcpyDeviceToDevice, ctx->stream));
+        } else if (!todo.empty()) {
+            launch_copies(ctx, todo.data(), todo.size());
         }
     });
 }

@@ -265,6 +265,8 @@ bool launch_pool_backward_where(b200_ctx* ctx, const b200_node& pool, const b200
 constexpr int64_t kTinyElements = 4096;  // one block: beyond a few thousand elements a node is faster as its own launch
 // elementwise.cu: the leading run of tiny elementwise nodes (a loss prologue) as one single-block launch
 size_t launch_tiny_chain(b200_ctx* ctx, const b200_node* const* seq, size_t avail);
+// movement.cu: disjoint byte ranges of device memory, as few launches as possible
+void launch_copies(b200_ctx* ctx, const b200_copy* copies, size_t n);
 // loss.cu: a cross-entropy's head, backward and value, one launch each; how many nodes of `seq` it covers
 size_t loss_group(b200_ctx* ctx, const b200_node* const* seq, size_t avail, bool launch);
 size_t launch_scaled_add_group(b200_ctx* ctx, const b200_node* const* seq, size_t avail, bool* picked);
