@@ -168,8 +168,44 @@ class NodeDesc:
         return n
 
 
+# A node is packed from the bytes of its tensors, each of which keeps its own until one of its fields is assigned
+# again: setting the ctypes structures field by field took 12 us of a scripting language's time for a node with
+# two operands, joining kept bytes takes 2.
+_TENSOR_WORDS = struct.Struct("<Q8q2i")
+_NODE_HEAD = struct.Struct("<2I")
+_NO_TENSORS = [bytes(_TENSOR_WORDS.size * n) for n in range(_abi.MAX_SRC + 1)]
+_NO_PARAMS = bytes(_abi.PARAM_BYTES)
+assert _TENSOR_WORDS.size == ctypes.sizeof(_abi.Tensor)
+assert _NODE_HEAD.size + (1 + _abi.MAX_SRC) * _TENSOR_WORDS.size + _abi.PARAM_BYTES == ctypes.sizeof(_abi.Node)
+_MORE_DIMS = [(1,) * (_abi.MAX_DIMS - n) for n in range(_abi.MAX_DIMS + 1)]
+_MORE_STRIDES = [(0,) * (_abi.MAX_DIMS - n) for n in range(_abi.MAX_DIMS + 1)]
+
+
+def _tensor_bytes(t: TensorDesc) -> bytes:
+    f = t.__dict__
+    kept = f.get("_packed")
+    if (kept is not None and kept[0] is f["data"] and kept[1] is f["dims"] and kept[2] is f["strides"] and
+            kept[3] is f["dtype"]):
+        return kept[4]
+    n = len(t.dims)
+    if n > _abi.MAX_DIMS:
+        raise ValueError(f"rank {n} exceeds {_abi.MAX_DIMS}")
+    packed = _TENSOR_WORDS.pack(t.data or 0, *t.dims, *_MORE_DIMS[n], *t.strides, *_MORE_STRIDES[n], n, int(t.dtype))
+    if type(t.dims) is tuple and type(t.strides) is tuple:  # (a list could change in place)
+        f["_packed"] = (t.data, t.dims, t.strides, t.dtype, packed)
+    return packed
+
+
 def pack_nodes(nodes: Sequence[NodeDesc]):
-    arr = (_abi.Node * max(len(nodes), 1))()
-    for i, n in enumerate(nodes):
-        arr[i] = n.to_c()
-    return arr
+    if not nodes:
+        return (_abi.Node * 1)()
+    parts = []
+    for n in nodes:
+        src = n.src
+        parts.append(_NODE_HEAD.pack(n.op, len(src)))
+        parts.append(_tensor_bytes(n.out))
+        for s in src:
+            parts.append(_tensor_bytes(s))
+        parts.append(_NO_TENSORS[_abi.MAX_SRC - len(src)])
+        parts.append(bytes(n.params[:_abi.PARAM_BYTES]).ljust(_abi.PARAM_BYTES, b"\0") if n.params else _NO_PARAMS)
+    return (_abi.Node * len(nodes)).from_buffer_copy(b"".join(parts))
