@@ -1673,7 +1673,7 @@ bool gemm_tc_eligible(const b200_ctx* ctx, const GemmProblem& p) {
         return false;
     }
     const double flops = 2.0 * double(p.m) * double(p.n) * double(p.k) * double(batches);
-    if (flops < double(1 << 25)) {
+    if (flops <= double(1 << 25)) {
         return false;  // launch-bound either way: the single CUDA-core kernel is cheaper than split + GEMM
     }
     // TMA coordinates are 32-bit
