@@ -997,19 +997,31 @@ static void compute_span(b200_ctx* ctx, const b200_node* nodes, size_t n_nodes, 
         if (ctx->fuse && exec.size() - p >= 2 &&
             (node.op == B200_OP_ADD || node.op == B200_OP_FULL || node.op == B200_OP_EQUAL ||
              node.op == B200_OP_EXP)) {
-            const size_t avail = std::min<size_t>(exec.size() - p, 5);
-            const b200_node* seq[5];
-            bool eligible = true;
-            for (size_t k = 0; k < avail; ++k) {
-                seq[k] = &nodes[exec[p + k]];
+            constexpr size_t kLater = 20;
+            const b200_node* seq[kLater];
+            size_t later = 0;
+            for (; later < kLater && p + later < exec.size() && !done[p + later]; ++later) {
+                const size_t idx = exec[p + later];
                 // a gradient that this span all-reduces is exchanged as soon as its own kernel is queued
-                eligible = eligible && (is_sink.empty() || !is_sink[exec[p + k]]) && seq[k]->out.data != nullptr;
-                eligible = eligible && (!grad_sync || !is_sink.empty() || ctx->grads.empty());
+                if ((!is_sink.empty() && is_sink[idx]) || nodes[idx].out.data == nullptr ||
+                    (grad_sync && is_sink.empty() && !ctx->grads.empty())) {
+                    break;
+                }
+                seq[later] = &nodes[idx];
             }
-            if (eligible) {
-                for (size_t k = 0; k < avail; ++k) prepare(exec[p + k]);
+            const size_t avail = std::min<size_t>(later, 5);
+            if (avail >= 2) {
+                for (size_t k = 0; k < later; ++k) {
+                    if (k < avail || seq[k]->op == B200_OP_RELU) prepare(exec[p + k]);  // (a relu may be served early)
+                }
                 ctx->current_op = node.op;
-                const size_t taken = launch_fused(ctx, seq, avail);
+                size_t early = 0;
+                const size_t taken = launch_fused(ctx, seq, avail, later, &early);
+                if (early > 0) {
+                    constants.erase(seq[early]->out.data);
+                    finish(exec[p + early]);
+                    done[p + early] = 1;
+                }
                 if (taken > 0) {
                     for (size_t k = 0; k < taken; ++k) {
                         if (seq[k]->op == B200_OP_FULL && seq[k]->out.dtype == B200_F32) {

@@ -152,7 +152,9 @@ bool bias_layout(const b200_tensor& b, int64_t& inner, int64_t& count) {
 // The forms this group takes in a recorded step: all five nodes (a hidden Linear layer), without
 // the relu (the layer before the loss, whose relu is emitted later), add + relu alone (a
 // convolution, whose mask nodes come with the backward pass) and the mask alone.
-size_t fuse_bias_group(b200_ctx* ctx, const b200_node* const* seq, size_t avail) {
+// A relu(y) that comes only after other nodes (the layer before the loss, whose relu follows the loss's head) is served
+// here all the same, if it is among `later`: nothing but y is read for it.  `early` then tells its place there.
+size_t fuse_bias_group(b200_ctx* ctx, const b200_node* const* seq, size_t avail, size_t later, size_t* early) {
     BiasGroup g{};
     size_t at = 0;
     const b200_tensor* y = nullptr;  // what the mask compares and the relu reads
@@ -203,6 +205,15 @@ size_t fuse_bias_group(b200_ctx* ctx, const b200_node* const* seq, size_t avail)
         reads(seq[at]->src[0], *y) && same_shape(seq[at]->out, *y) && aligned16(seq[at]->out.data)) {
         g.relu = static_cast<float*>(seq[at]->out.data);
         ++at;
+    } else if (at >= 3) {
+        for (size_t k = at; k < later; ++k) {
+            if (seq[k]->op == B200_OP_RELU && seq[k]->out.dtype == B200_F32 && seq[k]->n_src == 1 && reads(seq[k]->src[0], *y) &&
+                same_shape(seq[k]->out, *y) && aligned16(seq[k]->out.data)) {
+                g.relu = static_cast<float*>(seq[k]->out.data);
+                *early = k;
+                break;
+            }
+        }
     }
     if (at < 2) return 0;  // a lone add: nothing to fuse
     const int64_t n = numel_of(*y);
@@ -403,6 +414,8 @@ struct ScaledAddGroup {
     float alpha[kGroupTensors], beta[kGroupTensors];
     uint32_t first_block[kGroupTensors + 1];
     uint32_t vec_mask;  // bit t: tensor t may be walked in 16-byte quads
+    uint32_t turned_mask;  // bit t: b is the transposed view of a dense [cols, rows] matrix, taken in 64x64 tiles
+    uint32_t rows[kGroupTensors], cols[kGroupTensors];  // (of such a tensor)
     int n;
 };
 
@@ -413,6 +426,29 @@ __global__ void __launch_bounds__(kThreads) scaled_add_group_kernel(const __grid
     const int64_t base = int64_t(blockIdx.x - g.first_block[t]) * kGroupTile;
     const int64_t count = g.count[t];
     const float alpha = g.alpha[t], beta = g.beta[t];
+    if ((g.turned_mask >> t) & 1u) {
+        __shared__ float tile[64][65];
+        const uint32_t rows = g.rows[t], cols = g.cols[t], across = (cols + 63) / 64;
+        const uint32_t i = blockIdx.x - g.first_block[t], r0 = i / across * 64, c0 = i % across * 64;
+        const uint32_t lane = threadIdx.x & 63, line = threadIdx.x >> 6;
+        float x[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+            const uint32_t c = line + 4 * u;
+            if (c0 + c < cols && r0 + lane < rows) tile[c][lane] = g.b[t][size_t(c0 + c) * rows + r0 + lane];
+            const uint32_t r = line + 4 * u;
+            x[u] = r0 + r < rows && c0 + lane < cols ? g.a[t][size_t(r0 + r) * cols + c0 + lane] : 0.0F;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+            const uint32_t r = line + 4 * u;
+            if (r0 + r < rows && c0 + lane < cols) {
+                g.out[t][size_t(r0 + r) * cols + c0 + lane] = __fadd_rn(__fmul_rn(x[u], alpha), __fmul_rn(tile[lane][r], beta));
+            }
+        }
+        return;
+    }
     if ((g.vec_mask >> t) & 1u) {
         const float4* __restrict__ a = reinterpret_cast<const float4*>(g.a[t] + base);
         const float4* __restrict__ b = reinterpret_cast<const float4*>(g.b[t] + base);
@@ -464,6 +500,7 @@ size_t launch_scaled_add_group(b200_ctx* ctx, const b200_node* const* seq, size_
     ScaledAddGroup g{};
     uint64_t blocks = 0;
     size_t n = 0;
+    constexpr int64_t kTurnedElements = 1 << 20;
     auto bytes_of = [](const b200_tensor& t) {
         // the span of addresses the tensor can touch (strided views included)
         int64_t hi = static_cast<int64_t>(dtype_size(t.dtype));
@@ -488,9 +525,15 @@ size_t launch_scaled_add_group(b200_ctx* ctx, const b200_node* const* seq, size_
         if (node.op != B200_OP_SCALED_ADD || node.n_src != 2) continue;
         const b200_tensor& o = node.out;
         bool ok = o.dtype == B200_F32 && dense_tensor(o) && o.data != nullptr;
+        bool turned = false;
         for (int s = 0; s < 2 && ok; ++s) {
-            ok = node.src[s].dtype == B200_F32 && same_shape(node.src[s], o) && dense_tensor(node.src[s]) &&
-                 node.src[s].data != nullptr;
+            const b200_tensor& in = node.src[s];
+            ok = in.dtype == B200_F32 && same_shape(in, o) && in.data != nullptr;
+            // a Linear layer's gradient comes as the transposed view of [in, out].  Small ones join the group for the
+            // launch they save; a large one is faster by itself (elementwise.cu moves its tiles in 16-byte runs)
+            turned = s == 1 && ok && !dense_tensor(in) && in.ndim == 2 && in.strides[0] == 4 && in.strides[1] == 4 * in.dims[0] &&
+                     numel_of(in) <= kTurnedElements;
+            ok = ok && (turned || dense_tensor(in));
         }
         for (int d = 0; d < o.ndim && ok; ++d) ok = o.strides[d] >= 0;
         for (size_t e = 0; e < k && ok; ++e) ok = independent(node, *seq[e]);  // members and the nodes it jumps over
@@ -505,8 +548,15 @@ size_t launch_scaled_add_group(b200_ctx* ctx, const b200_node* const* seq, size_
         g.alpha[n] = prm.alpha;
         g.beta[n] = prm.beta;
         g.first_block[n] = static_cast<uint32_t>(blocks);
-        if (count % 4 == 0 && aligned16(g.out[n]) && aligned16(g.a[n]) && aligned16(g.b[n])) g.vec_mask |= 1u << n;
-        blocks += static_cast<uint64_t>((count + kGroupTile - 1) / kGroupTile);
+        if (turned) {
+            g.turned_mask |= 1u << n;
+            g.rows[n] = static_cast<uint32_t>(o.dims[0]);
+            g.cols[n] = static_cast<uint32_t>(o.dims[1]);
+            blocks += static_cast<uint64_t>((o.dims[0] + 63) / 64) * static_cast<uint64_t>((o.dims[1] + 63) / 64);
+        } else {
+            if (count % 4 == 0 && aligned16(g.out[n]) && aligned16(g.a[n]) && aligned16(g.b[n])) g.vec_mask |= 1u << n;
+            blocks += static_cast<uint64_t>((count + kGroupTile - 1) / kGroupTile);
+        }
         picked[k] = true;
         ++n;
     }
@@ -525,8 +575,11 @@ size_t launch_scaled_add_group(b200_ctx* ctx, const b200_node* const* seq, size_
 
 // Tries every pattern at the head of `seq` (the span's remaining computed nodes, in execution
 // order); returns how many nodes one fused launch served, or 0.
-size_t launch_fused(b200_ctx* ctx, const b200_node* const* seq, size_t avail) {
-    if (size_t n = fuse_bias_group(ctx, seq, avail)) return n;
+// `later` >= avail nodes of `seq` may be looked at for one that a group can serve ahead of its turn; `early` is its
+// place in `seq` then (0: none).
+size_t launch_fused(b200_ctx* ctx, const b200_node* const* seq, size_t avail, size_t later, size_t* early) {
+    *early = 0;
+    if (size_t n = fuse_bias_group(ctx, seq, avail, later, early)) return n;
     if (size_t n = fuse_one_hot(ctx, seq, avail)) return n;
     if (size_t n = fuse_lsm_backward(ctx, seq, avail)) return n;
     return 0;

@@ -829,7 +829,7 @@ bool gemm_h16_serves(const b200_ctx* ctx, const GemmProblem& p) {
         return false;
     }
     const double flops = 2.0 * double(p.m) * double(p.n) * double(p.k) * double(p.b0 * p.b1);
-    return flops >= 4294967296.0 && !gemm_tc_streams(ctx, p) && ctx->compared.count(p.out) == 0;
+    return flops > 2147483648.0 && !gemm_tc_streams(ctx, p) && ctx->compared.count(p.out) == 0;
 }
 
 void gemm_h16_note_uses(b200_ctx* ctx, const GemmProblem& p) {

@@ -580,11 +580,9 @@ uint32_t axes_of(const b200_node& n, bool& keepdim) {
 size_t match_head(const b200_node* const* seq, size_t avail, LossArgs& a) {
     size_t at = 0, lead = 0;
     if (seq[0]->op == B200_OP_FULL) {
-        // the scalars in front are taken along where the rows' vectors are too long for the chain of tiny nodes,
-        // which serves the scalars together with those vectors otherwise
         if (avail < 11 || seq[1]->op != B200_OP_FULL || seq[2]->op != B200_OP_DIV || seq[3]->op != B200_OP_CONTIGUOUS || seq[3]->out.ndim != 1 ||
-            seq[3]->out.dims[0] <= kTinyElements || seq[2]->n_src != 2 || seq[2]->src[0].data != seq[0]->out.data ||
-            seq[2]->src[1].data != seq[1]->out.data || seq[3]->src[0].data != seq[2]->out.data) {
+            seq[2]->n_src != 2 || seq[2]->src[0].data != seq[0]->out.data || seq[2]->src[1].data != seq[1]->out.data ||
+            seq[3]->src[0].data != seq[2]->out.data) {
             return 0;
         }
         for (int i = 0; i < 3; ++i) {
@@ -804,7 +802,8 @@ size_t loss_group(b200_ctx* ctx, const b200_node* const* seq, size_t avail, bool
         n = head + back;
         if (n == 0 || !launch) return n;
         if (back > 0) a = both;
-        ProfScope scope(ctx, back > 0 ? "fused.log_softmax_backward" : "fused.loss_head");
+        // (a head by itself, scalars and all, goes by the name of the single-block chain that it takes the place of)
+        ProfScope scope(ctx, back > 0 ? "fused.log_softmax_backward" : a.scalars[0] != nullptr ? "fused.tiny_chain" : "fused.loss_head");
         if (head > 0 && back > 0) launch_rows<true, true>(ctx, a);
         else if (head > 0) launch_rows<true, false>(ctx, a);
         else launch_rows<false, true>(ctx, a);
