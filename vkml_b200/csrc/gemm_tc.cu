@@ -165,10 +165,11 @@ struct SplitArgs {
     int64_t s_b0, s_b1, s_r, s_k;  // element strides of src
     int64_t n_batches;
     int64_t out_rows;    // plane rows per batch (>= rows; the extra rows are written as zero)
+    int unit, vec;       // dense along K; and every row on 16 bytes
 };
 
-// Source rows dense along K and 16-byte aligned: one thread per four K-elements, 128-bit
-// loads and stores, no shared memory.
+// Source rows dense along K: one thread per four K-elements, 128-bit stores and, where every row lies on 16
+// bytes, 128-bit loads; no shared memory.
 __device__ __forceinline__ void split_rows(const SplitArgs& a) {
     const int64_t kp4 = a.kp / 4;
     const int64_t total = kp4 * a.out_rows * a.n_batches;
@@ -182,12 +183,13 @@ __device__ __forceinline__ void split_rows(const SplitArgs& a) {
         float4 v = make_float4(0.0F, 0.0F, 0.0F, 0.0F);
         if (r < a.rows) {
             const float* src = a.src + (b / a.b1) * a.s_b0 + (b % a.b1) * a.s_b1 + r * a.s_r;
-            if (k + 3 < a.k) {
+            if (a.vec && k + 3 < a.k) {
                 v = *reinterpret_cast<const float4*>(src + k);
             } else {
                 if (k < a.k) v.x = src[k];
                 if (k + 1 < a.k) v.y = src[k + 1];
                 if (k + 2 < a.k) v.z = src[k + 2];
+                if (k + 3 < a.k) v.w = src[k + 3];
             }
         }
         float4 h, l;
@@ -271,35 +273,30 @@ __global__ void __launch_bounds__(256) split_kernel(SplitArgs a) {
     split_tiles(a);
 }
 
-bool rows_dense(const SplitArgs& s) {
-    return s.s_k == 1 && s.s_r % 4 == 0 && s.s_b0 % 4 == 0 && s.s_b1 % 4 == 0 && reinterpret_cast<uintptr_t>(s.src) % 16 == 0;
-}
-
-// Both operands of a product in one launch, for the planes that stand by for a wide operand: nearly always
-// there is nothing to do, and then a launch of a few hundred blocks costs less than two full ones.
+// Both operands of a product in one launch: the planes that stand by for a wide operand.  There is nearly always nothing
+// to do, and then one launch of a few hundred blocks costs less than two full ones.
 struct SplitPair {
     SplitArgs s[2];
-    int dense[2];
     RangeGuard guard;
 };
 
-__global__ void __launch_bounds__(256) split_if_wide_kernel(SplitPair p) {
+__global__ void __launch_bounds__(256) split_pair_kernel(SplitPair p) {
     pdl_prologue();
     if (guard_idle(p.guard)) return;
     const SplitArgs& a = p.s[blockIdx.y];
-    if (p.dense[blockIdx.y]) split_rows(a);
+    if (a.unit) split_rows(a);
     else split_tiles(a);
+}
+
+int64_t split_blocks(const SplitArgs& s) {
+    if (s.unit) return grid_for(ceil_div((s.kp / 4) * s.out_rows * s.n_batches, 2), 256);
+    return grid_for(ceil_div(s.kp, kSplitTile) * ceil_div(s.rows, kSplitTile) * s.n_batches, 1, 8);
 }
 
 void launch_split(b200_ctx* ctx, const SplitArgs& s, const char* label) {
     ProfScope scope(ctx, label);
-    if (rows_dense(s)) {
-        const int64_t total = (s.kp / 4) * s.out_rows * s.n_batches;
-        launch_kernel(ctx, split_rows_kernel, grid_for(ceil_div(total, 2), 256), 256, 0, s);
-    } else {
-        const int64_t tiles = ceil_div(s.kp, kSplitTile) * ceil_div(s.rows, kSplitTile) * s.n_batches;
-        launch_kernel(ctx, split_kernel, grid_for(tiles, 1, 8), 256, 0, s);
-    }
+    if (s.unit) launch_kernel(ctx, split_rows_kernel, static_cast<unsigned>(split_blocks(s)), 256, 0, s);
+    else launch_kernel(ctx, split_kernel, static_cast<unsigned>(split_blocks(s)), 256, 0, s);
     ctx->count_launch();
 }
 
@@ -667,10 +664,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_consta
                 break;
             }
             tc_fence_after();
-            const int64_t row = tm * BM + quarter * 32 + lane;
             const int64_t col0 = tn * BN;
-            float* dst = g.out + int64_t(split) * g.split_stride + (batch * g.m + row) * g.n + col0;
-            const bool row_ok = row < g.m;
             const bool vec_ok = (g.n % 4 == 0) && ((reinterpret_cast<uintptr_t>(g.out) & 15) == 0) &&
                                 ((g.split_stride % 4) == 0);
             const bool warp_rows_live = tm * BM + quarter * 32 < g.m;  // else nothing of this warp's is stored
@@ -714,16 +708,23 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_consta
                     __syncwarp();
                     continue;
                 }
-                if (row_ok) {
-                    // ragged right edge, or an output that cannot take 128-bit stores
-                    float* p = dst + c * 32;
+                // a ragged right edge, or rows that do not begin on 16 bytes: a row's 32 columns per store
+                float* patch = &epi_patch[quarter][0][0];
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        if (j < left) {
-                            p[j] = __uint_as_float(r[j]);
-                        }
+                for (int j = 0; j < 8; ++j) {
+                    *reinterpret_cast<uint4*>(patch + lane * kEpiPitch + 4 * j) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+                }
+                __syncwarp();
+                const int64_t row_base = tm * BM + quarter * 32;
+                if (lane < left) {
+                    const int rows = static_cast<int>(min(int64_t(32), g.m - row_base));
+                    float* q = g.out + int64_t(split) * g.split_stride + (batch * g.m + row_base) * g.n + col0 + c * 32 + lane;
+                    for (int rl = 0; rl < rows; ++rl) {
+                        *q = patch[rl * kEpiPitch + lane];
+                        q += g.n;
                     }
                 }
+                __syncwarp();
             }
             tc_fence_before();
             __syncwarp();
@@ -1376,15 +1377,15 @@ struct Operand {
 
 // `s_mn` / `s_k` are the element strides along the operand's M (or N) axis and along K.
 // An operand whose M (or N) axis is contiguous keeps its [K][MN] layout and is consumed
-// MN-major; everything else becomes a K-major plane [MN][Kp].  Planes of densely readable
-// sources are padded to 32 rows and 32 columns of zeros, so the same plane serves a later use
+// MN-major; everything else becomes a K-major plane [MN][Kp].  Planes of sources with a unit-stride
+// axis are padded to 32 rows and 32 columns of zeros, so the same plane serves a later use
 // of the same memory in the other orientation.
 Operand plan_operand(const float* ptr, int64_t s_b0, int64_t s_b1, int64_t s_mn, int64_t s_k, int64_t mn_extent,
                      int64_t k_extent, bool bcast, const GemmProblem& p) {
     Operand o;
     const int64_t sb0 = bcast ? 0 : s_b0, sb1 = bcast ? 0 : s_b1;
     const bool aligned = reinterpret_cast<uintptr_t>(ptr) % 16 == 0 && sb0 % 4 == 0 && sb1 % 4 == 0;
-    o.mn = s_mn == 1 && s_k != 1 && aligned && s_k % 4 == 0;
+    o.mn = s_mn == 1 && s_k != 1;
     o.nb = bcast ? 1 : p.b0 * p.b1;
     int64_t s_r, s_c;
     if (o.mn) {
@@ -1398,9 +1399,11 @@ Operand plan_operand(const float* ptr, int64_t s_b0, int64_t s_b1, int64_t s_mn,
         s_r = s_mn;
         s_c = s_k;
     }
-    const bool dense = s_c == 1 && s_r % 4 == 0 && aligned;  // the 128-bit split kernel's condition
-    o.dense = dense;
-    o.rows_pad = dense ? align_up(o.rows, 32) : o.rows;
+    const bool unit = s_c == 1;
+    o.dense = unit && s_r % 4 == 0 && aligned;  // as TMA and 128-bit loads want it
+    o.rows_pad = unit ? align_up(o.rows, 32) : o.rows;
+    o.split.unit = unit ? 1 : 0;
+    o.split.vec = o.dense ? 1 : 0;
     o.cols_pad = align_up(o.cols, 32);
     o.plane_bytes = static_cast<size_t>(align_up(o.nb * o.rows_pad * o.cols_pad * 4, 1024));
     const int64_t b1 = bcast ? 1 : p.b1;
@@ -1430,19 +1433,18 @@ Operand plan_operand(const float* ptr, int64_t s_b0, int64_t s_b1, int64_t s_mn,
 // in-kernel split is bound by shared-memory traffic (the converter's loads and stores contend
 // with the tensor core's operand reads) at about 147 TFLOP/s of algorithmic work -- 7.5 ms against
 // 4.5 ms at 8192^3, 0.32 against 0.31 ms at 512 x 65536 x 512 -- while the plane scheme moves each
-// operand five times (read, two planes written, two planes read).  It pays where that traffic is
-// what the product costs and nobody else in the span uses the planes: the CNN's first
-// weight gradient, g[256][64x1024] . cols^T[256][1024x27], 74 us against 105; the CNN's head,
-// 19 against 24 us.
+// operand five times (read, two planes written, two planes read).  It pays where
+// that traffic is what the product costs: the CNN's first weight gradient, g[256][64x1024] . cols^T[256][1024x27], 74 us
+// against 105; the CNN's head, 19 against 24 us (planes that another product of the span uses too cost each half) --
+// and below 2^28 operations, which take under 2 us either way while a plane pass is one more launch per operand.
 bool direct_pays(const b200_ctx* ctx, const GemmProblem& p, int64_t batches, const Operand& oa, const Operand& ob) {
-    auto shared = [&](const Operand& o) {
+    auto share = [&](const Operand& o) {
         const auto it = ctx->plane_uses.find(o.key);
-        return it != ctx->plane_uses.end() && it->second >= 2;
+        return it != ctx->plane_uses.end() && it->second >= 2 ? 0.5 : 1.0;
     };
-    if (shared(oa) || shared(ob)) return false;
     const double flops = 2.0 * double(p.m) * double(p.n) * double(p.k) * double(batches);
-    const double operand_bytes = double(oa.plane_bytes) + double(ob.plane_bytes);
-    return flops / 147e12 < 4.0 * operand_bytes / 6.5e12;
+    if (flops < double(1 << 28)) return true;
+    return flops / 147e12 < 4.0 * (double(oa.plane_bytes) * share(oa) + double(ob.plane_bytes) * share(ob)) / 6.5e12;
 }
 
 size_t plane_cache_limit(const b200_ctx* ctx) {
@@ -1854,16 +1856,12 @@ void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass) {
     from_workspace(ob);
     float* partial = splits > 1 ? reinterpret_cast<float*>(ws) : nullptr;
 
-    if (!a_hit) {
-        oa.split.hi = oa.hi;
-        oa.split.lo = oa.lo;
-        launch_split(ctx, oa.split, "matmul.split_a");
-    }
-    if (!b_hit) {
-        ob.split.hi = ob.hi;
-        ob.split.lo = ob.lo;
-        launch_split(ctx, ob.split, "matmul.split_b");
-    }
+    oa.split.hi = oa.hi;
+    oa.split.lo = oa.lo;
+    ob.split.hi = ob.hi;
+    ob.split.lo = ob.lo;
+    if (!a_hit) launch_split(ctx, oa.split, "matmul.split_a");
+    if (!b_hit) launch_split(ctx, ob.split, "matmul.split_b");
     if (!a_hit || !b_hit) {
         check_last_launch("matmul (operand split)");
     }
@@ -1950,12 +1948,11 @@ void gemm_tc_if_wide(b200_ctx* ctx, const GemmProblem& p, const RangeGuard& guar
         o->split.hi = o->hi = reinterpret_cast<float*>(ws);
         o->split.lo = o->lo = reinterpret_cast<float*>(ws + o->plane_bytes);
         ws += 2 * o->plane_bytes;
-        pair.s[i] = o->split;
-        pair.dense[i++] = rows_dense(o->split) ? 1 : 0;
+        pair.s[i++] = o->split;
     }
     {
         ProfScope scope(ctx, "matmul.if_wide");
-        launch_kernel(ctx, split_if_wide_kernel, dim3(ctx->prop.multiProcessorCount * 2, 2), 256, 0, pair);
+        launch_kernel(ctx, split_pair_kernel, dim3(ctx->prop.multiProcessorCount * 2, 2), 256, 0, pair);
     }
     ctx->count_launch();
     constexpr int bn = 128;
