@@ -87,9 +87,22 @@ struct BiasGroup {
     float* relu;        // null: no relu
     float value_a, value_b;
     int64_t n4;           // quads
+    int rest;             // elements behind the last quad
     uint32_t inner4;      // quads that share one bias element (0: the bias runs along the quad)
     uint32_t count;       // bias elements
+    int loose;            // quads and bias elements are not in step: `by_inner` and `by_count` find each element's
+    FastDiv by_inner, by_count;
 };
+
+__device__ __forceinline__ float loose_bias(const BiasGroup& g, int64_t i) {
+    const uint32_t q = g.by_inner.div(static_cast<uint32_t>(i));
+    return g.bias[q - g.by_count.div(q) * g.count];
+}
+
+__device__ __forceinline__ float relu_of(float v) {
+    // relu(x) = x <= 0 ? 0 : x, so a NaN goes through (src/backend/cpu/kernels_elementwise.cpp:223-231)
+    return v <= 0.0F ? 0.0F : v;
+}
 
 __global__ void __launch_bounds__(kThreads) bias_relu_group_kernel(BiasGroup g) {
     pdl_prologue();
@@ -98,7 +111,9 @@ __global__ void __launch_bounds__(kThreads) bias_relu_group_kernel(BiasGroup g) 
         float4 s = reinterpret_cast<const float4*>(g.x)[i];
         if (g.bias != nullptr) {
             float4 b;
-            if (g.inner4 != 0) {
+            if (g.loose) {
+                b = make_float4(loose_bias(g, 4 * i), loose_bias(g, 4 * i + 1), loose_bias(g, 4 * i + 2), loose_bias(g, 4 * i + 3));
+            } else if (g.inner4 != 0) {
                 const float v = g.bias[(i / g.inner4) % g.count];
                 b = make_float4(v, v, v, v);
             } else {
@@ -121,14 +136,22 @@ __global__ void __launch_bounds__(kThreads) bias_relu_group_kernel(BiasGroup g) 
             reinterpret_cast<uchar4*>(g.mask)[i] = m;
         }
         if (g.relu != nullptr) {
-            // relu(x) = x <= 0 ? 0 : x, so a NaN goes through (src/backend/cpu/kernels_elementwise.cpp:223-231)
-            float4 r;
-            r.x = s.x <= 0.0F ? 0.0F : s.x;
-            r.y = s.y <= 0.0F ? 0.0F : s.y;
-            r.z = s.z <= 0.0F ? 0.0F : s.z;
-            r.w = s.w <= 0.0F ? 0.0F : s.w;
-            reinterpret_cast<float4*>(g.relu)[i] = r;
+            reinterpret_cast<float4*>(g.relu)[i] = make_float4(relu_of(s.x), relu_of(s.y), relu_of(s.z), relu_of(s.w));
         }
+    }
+    if (blockIdx.x == 0 && static_cast<int>(threadIdx.x) < g.rest) {
+        const int64_t i = 4 * g.n4 + threadIdx.x;
+        float s = g.x[i];
+        if (g.bias != nullptr) {
+            s = __fadd_rn(s, loose_bias(g, i));
+            g.add[i] = s;
+        }
+        if (g.full_a != nullptr) {
+            g.full_a[i] = g.value_a;
+            g.full_b[i] = g.value_b;
+            g.mask[i] = s <= g.value_a ? 1 : 0;
+        }
+        if (g.relu != nullptr) g.relu[i] = relu_of(s);
     }
 }
 
@@ -165,8 +188,11 @@ size_t fuse_bias_group(b200_ctx* ctx, const b200_node* const* seq, size_t avail,
         int64_t inner = 0, count = 0;
         if (!bias_layout(add.src[1], inner, count)) return 0;
         const bool along = inner == 1 && count % 4 == 0 && aligned16(add.src[1].data);
-        if (!along && inner % 4 != 0) return 0;
-        if (inner / 4 >= (int64_t(1) << 31) || count >= (int64_t(1) << 31)) return 0;
+        if (numel_of(add.out) >= (int64_t(1) << 31) && ((!along && inner % 4 != 0) || numel_of(add.out) % 4 != 0)) return 0;
+        if (inner >= (int64_t(1) << 31) || count >= (int64_t(1) << 31)) return 0;
+        g.loose = !along && inner % 4 != 0 ? 1 : 0;
+        g.by_inner = FastDiv(static_cast<uint32_t>(inner));
+        g.by_count = FastDiv(static_cast<uint32_t>(count));
         if (!aligned16(add.src[0].data) || !aligned16(add.out.data)) return 0;
         g.x = static_cast<const float*>(add.src[0].data);
         g.bias = static_cast<const float*>(add.src[1].data);
@@ -217,13 +243,14 @@ size_t fuse_bias_group(b200_ctx* ctx, const b200_node* const* seq, size_t avail,
     }
     if (at < 2) return 0;  // a lone add: nothing to fuse
     const int64_t n = numel_of(*y);
-    if (n == 0 || n % 4 != 0) return 0;
+    if (n == 0) return 0;
     g.n4 = n / 4;
+    g.rest = static_cast<int>(n % 4);
     const char* label = g.bias != nullptr ? (g.full_a != nullptr ? (g.relu != nullptr ? "fused.bias_mask_relu" : "fused.bias_mask")
                                                                  : "fused.bias_relu")
                                           : "fused.mask";
     ProfScope scope(ctx, label);
-    launch_kernel(ctx, bias_relu_group_kernel, grid_for(g.n4, kThreads), kThreads, 0, g);
+    launch_kernel(ctx, bias_relu_group_kernel, grid_for(g.n4 + 1, kThreads), kThreads, 0, g);
     ctx->count_launch();
     check_last_launch("fused bias / mask / relu");
     return at;
@@ -580,6 +607,7 @@ size_t launch_scaled_add_group(b200_ctx* ctx, const b200_node* const* seq, size_
 size_t launch_fused(b200_ctx* ctx, const b200_node* const* seq, size_t avail, size_t later, size_t* early) {
     *early = 0;
     if (size_t n = fuse_bias_group(ctx, seq, avail, later, early)) return n;
+    *early = 0;
     if (size_t n = fuse_one_hot(ctx, seq, avail)) return n;
     if (size_t n = fuse_lsm_backward(ctx, seq, avail)) return n;
     return 0;
