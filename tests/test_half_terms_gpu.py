@@ -105,3 +105,28 @@ def test_f16_storage_products(backend, m, k, n, layout):
     err = np.abs(got.reshape(want.shape).astype(np.float64) - want)
     # one rounding to half, and the fp32 accumulator's error where it decides between neighbours
     assert np.all(err <= 0.5 * ulp + 1e-5 * np.sqrt(k))
+
+
+# a tile and its remainder in rows, one pair of accumulators and several, with and without the relu; sizes that keep the nodes apart
+@pytest.mark.parametrize("relu", [False, True])
+@pytest.mark.parametrize("m,k,n", [(300, 512, 4096), (1023, 256, 1088), (2048, 64, 1024), (200, 512, 1000)])
+def test_f16_linear_layers(backend, m, k, n, relu):
+    rng = np.random.default_rng(m + n)
+    x, w = rng.standard_normal((m, k)).astype(np.float16), rng.standard_normal((n, k)).astype(np.float16)
+    bias = (8 * rng.standard_normal(n)).astype(np.float16)
+    dx, dw = (DeviceTensor.from_host(backend, t.reshape((1, 1) + t.shape)) for t in (x, w))
+    y, z, h = (DeviceTensor.empty(backend, (m, n), DType.F16) for _ in range(3))
+    nodes = [NodeDesc(int(Op.MATMUL), y.reshape((1, 1, m, n)).desc, [dx.desc, dw.transpose(2, 3).desc]),
+             NodeDesc(int(Op.ADD), z.desc, [y.desc, DeviceTensor.from_host(backend, bias).broadcast_to((m, n)).desc])]
+    if relu:
+        nodes.append(NodeDesc(int(Op.RELU), h.desc, [z.desc]))
+    keep = DeviceTensor.from_host(backend, bias)
+    nodes[1].src[1] = keep.broadcast_to((m, n)).desc
+    backend.compute(nodes)
+    got = y.numpy()
+    want = x.astype(np.float64) @ w.astype(np.float64).T
+    assert np.all(np.abs(got - want) <= 0.5 * np.spacing(np.abs(want).astype(np.float16)).astype(np.float64) + 1e-5 * np.sqrt(k))
+    summed = (got.astype(np.float32) + bias.astype(np.float32)).astype(np.float16)
+    assert np.array_equal(z.numpy().view(np.uint16), summed.view(np.uint16))
+    if relu:
+        assert np.array_equal(h.numpy(), np.where(summed <= 0, np.float16(0), summed))

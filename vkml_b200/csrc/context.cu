@@ -263,6 +263,30 @@ bool touches_f16(const b200_node& n) {
     return false;
 }
 
+// matmul(f16), add(y, bias vector along the rows) and perhaps relu on the sum, all dense halves.
+bool half_linear(const b200_node& mm, const b200_node& add, const b200_node* relu, HalfEpilogue& epi) {
+    auto half_matrix = [&](const b200_tensor& t) {
+        return t.dtype == B200_F16 && t.ndim == 2 && t.dims[0] == mm.out.dims[2] && t.dims[1] == mm.out.dims[3] && t.data != nullptr &&
+               t.strides[0] == t.dims[1] * 2 && t.strides[1] == 2;
+    };
+    if (mm.n_src != 2 || mm.src[0].dtype != B200_F16 || mm.src[1].dtype != B200_F16 || mm.out.ndim != 4 || mm.out.dims[0] * mm.out.dims[1] != 1 ||
+        add.op != B200_OP_ADD || add.n_src != 2 || !half_matrix(add.out) || !half_matrix(add.src[0]) || add.src[0].data != mm.out.data) {
+        return false;
+    }
+    const b200_tensor& b = add.src[1];
+    if (b.dtype != B200_F16 || b.ndim != 2 || b.dims[0] != mm.out.dims[2] || b.dims[1] != mm.out.dims[3] || b.strides[0] != 0 || b.strides[1] != 2 ||
+        b.data == nullptr) {
+        return false;
+    }
+    epi.bias = b.data;
+    epi.biased = add.out.data;
+    if (relu != nullptr && relu->op == B200_OP_RELU && relu->n_src == 1 && half_matrix(relu->out) && half_matrix(relu->src[0]) &&
+        relu->src[0].data == add.out.data) {
+        epi.rectified = relu->out.data;
+    }
+    return true;
+}
+
 size_t tensor_span_bytes(const b200_tensor& t) {
     size_t n = dtype_size(t.dtype);
     for (int d = 0; d < t.ndim; ++d) n *= static_cast<size_t>(t.dims[d]);
@@ -992,6 +1016,25 @@ static void compute_span(b200_ctx* ctx, const b200_node* nodes, size_t n_nodes, 
                 }
                 p += taken;
                 continue;
+            }
+        }
+        if (ctx->fuse && node.op == B200_OP_MATMUL && node.out.dtype == B200_F16 && p + 1 < exec.size() && !done[p + 1]) {
+            // a Linear layer over half storage: its bias and relu in the product's epilogue
+            const b200_node& add = nodes[exec[p + 1]];
+            const b200_node* relu = p + 2 < exec.size() && !done[p + 2] ? &nodes[exec[p + 2]] : nullptr;
+            HalfEpilogue epi{};
+            if (is_sink.empty() && !grad_sync && half_linear(node, add, relu, epi)) {
+                const size_t taken = epi.rectified != nullptr ? 3 : 2;
+                for (size_t k = 0; k < taken; ++k) prepare(exec[p + k]);
+                ctx->current_op = node.op;
+                if (gemm_f16_storage(ctx, matmul_problem(node), &epi)) {
+                    for (size_t k = 0; k < taken; ++k) {
+                        constants.erase(nodes[exec[p + k]].out.data);
+                        finish(exec[p + k]);
+                    }
+                    p += taken;
+                    continue;
+                }
             }
         }
         if (ctx->fuse && exec.size() - p >= 2 &&

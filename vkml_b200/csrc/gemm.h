@@ -48,8 +48,14 @@ size_t gemm_tc_plane_bytes(const GemmProblem& p);  // bytes that gemm_tc_if_wide
 bool gemm_h16_serves(const b200_ctx* ctx, const GemmProblem& p);
 void gemm_h16(b200_ctx* ctx, const GemmProblem& p);
 void gemm_h16_note_uses(b200_ctx* ctx, const GemmProblem& p);
-// Half storage: `p`'s pointers are to halves.  False: not a case for this kernel.
-bool gemm_f16_storage(b200_ctx* ctx, const GemmProblem& p);
+// Half storage: `p`'s pointers are to halves.  False: not a case for this kernel.  With an epilogue the nodes behind the
+// product -- add(y, bias along the rows) and perhaps relu -- are served as well.
+struct HalfEpilogue {
+    const void* bias;
+    void* biased;
+    void* rectified;  // may be null
+};
+bool gemm_f16_storage(b200_ctx* ctx, const GemmProblem& p, const HalfEpilogue* epilogue = nullptr);
 // True when gemm_tc would serve `p` with the streamed-operand kernel (a small left operand, the
 // right operand read once from HBM) rather than from operand planes.
 bool gemm_tc_streams(const b200_ctx* ctx, const GemmProblem& p);

@@ -182,6 +182,10 @@ __global__ void __launch_bounds__(256) pack_half_kernel(const __half* __restrict
 struct H16Args {
     void* out;             // C (f32 or half), or the f32 partial planes when splits > 1
     int out_half;
+    // half output: the bias that a following add spreads over the rows, its result, and a relu's (each may be null)
+    const __half* bias;
+    __half* biased;
+    __half* rectified;
     int64_t m, n, batches;
     int a_b1, b_b1;        // inner batch extents of the operand maps; 0: one matrix for every batch
     int64_t k_blocks, kb_per_split;
@@ -477,7 +481,7 @@ gemm_h16_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_const
             f2 = exp2_int(e2);
             f3 = exp2_int(e - e1 - e2);
         }
-        const bool vec = g.n % 4 == 0 && g.split_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(g.out) & (g.out_half ? 7 : 15)) == 0;
+        const bool vec = g.n % 4 == 0 && g.split_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(g.out) & 15) == 0;
         uint32_t tile_it = 0;
         for (int64_t u = unit0; u < n_units; u += unit_step, ++tile_it) {
             int split;
@@ -490,8 +494,64 @@ gemm_h16_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_const
             const int64_t col0 = tn * BN;
             const int64_t at = int64_t(split) * g.split_stride + (batch * g.m + row_base) * g.n + col0;
             const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + acc * T::kAccCols;
+            int done_cols = 0;
+            if (PASSES == 1 && g.out_half && vec && g.n % 8 == 0 && row_base < g.m) {
+                // 64 columns at a time, narrowed before they go through the patch: whole 128-byte rows of halves per store
+                __half* patch = reinterpret_cast<__half*>(&epi_patch[quarter][0][0]);
+                constexpr int kPitch = 72;
 #pragma unroll 1
-            for (int c = 0; c < BN / 32; ++c) {
+                for (; done_cols + 64 <= BN && col0 + done_cols + 64 <= g.n; done_cols += 64) {
+                    uint32_t r[32];
+#pragma unroll
+                    for (int half = 0; half < 2; ++half) {
+                        tmem_ld32(t_acc + done_cols + 32 * half, r);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            __half2 h[4];
+#pragma unroll
+                            for (int q = 0; q < 4; ++q) {
+                                h[q] = __floats2half2_rn(__uint_as_float(r[8 * j + 2 * q]), __uint_as_float(r[8 * j + 2 * q + 1]));
+                            }
+                            *reinterpret_cast<uint4*>(patch + lane * kPitch + 32 * half + 8 * j) = *reinterpret_cast<const uint4*>(h);
+                        }
+                    }
+                    __syncwarp();
+                    const int sub = lane >> 3, seg = lane & 7;
+                    uint4 bias4 = make_uint4(0, 0, 0, 0);
+                    if (g.bias != nullptr) bias4 = __ldg(reinterpret_cast<const uint4*>(g.bias + col0 + done_cols + seg * 8));
+                    const __half2* b = reinterpret_cast<const __half2*>(&bias4);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int rl = i * 4 + sub;
+                        if (row_base + rl < g.m) {
+                            uint4 bits = *reinterpret_cast<const uint4*>(patch + rl * kPitch + seg * 8);
+                            const int64_t o = at + int64_t(rl) * g.n + done_cols + seg * 8;
+                            *reinterpret_cast<uint4*>(static_cast<__half*>(g.out) + o) = bits;
+                            if (g.bias != nullptr) {
+                                // every node narrows its own result (HalfIO, elementwise.cu): the sum is that of the stored halves
+                                __half2* h = reinterpret_cast<__half2*>(&bits);
+#pragma unroll
+                                for (int q = 0; q < 4; ++q) {
+                                    const float2 y = __half22float2(h[q]), w = __half22float2(b[q]);
+                                    h[q] = __floats2half2_rn(__fadd_rn(y.x, w.x), __fadd_rn(y.y, w.y));
+                                }
+                                *reinterpret_cast<uint4*>(g.biased + o) = bits;
+                                if (g.rectified != nullptr) {
+#pragma unroll
+                                    for (int q = 0; q < 4; ++q) {
+                                        const float2 y = __half22float2(h[q]);
+                                        h[q] = __floats2half2_rn(y.x <= 0.0F ? 0.0F : y.x, y.y <= 0.0F ? 0.0F : y.y);
+                                    }
+                                    *reinterpret_cast<uint4*>(g.rectified + o) = bits;
+                                }
+                            }
+                        }
+                    }
+                    __syncwarp();
+                }
+            }
+#pragma unroll 1
+            for (int c = done_cols / 32; c < BN / 32; ++c) {
                 if (col0 + c * 32 >= g.n || row_base >= g.m) break;  // uniform across the warp
                 uint32_t r[32];
                 tmem_ld32(t_acc + c * 32, r);
@@ -529,15 +589,25 @@ gemm_h16_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_const
                         }
                     }
                     __syncwarp();
-                } else if (row_base + lane < g.m) {
-                    const int64_t o = at + int64_t(lane) * g.n + c * 32;
+                } else {
+                    // a ragged right edge, or rows that do not begin on 16 bytes: a row's 32 columns per store
+                    float* patch = &epi_patch[quarter][0][0];
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        if (j < left) {
-                            if (g.out_half) static_cast<__half*>(g.out)[o + j] = __float2half_rn(__uint_as_float(r[j]));
-                            else static_cast<float*>(g.out)[o + j] = __uint_as_float(r[j]);
+                    for (int j = 0; j < 8; ++j) {
+                        *reinterpret_cast<uint4*>(patch + lane * kPatchPitch + 4 * j) =
+                            make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+                    }
+                    __syncwarp();
+                    if (lane < left) {
+                        const int rows = static_cast<int>(min(int64_t(32), g.m - row_base));
+                        for (int rl = 0; rl < rows; ++rl) {
+                            const float v = patch[rl * kPatchPitch + lane];
+                            const int64_t o = at + int64_t(rl) * g.n + c * 32 + lane;
+                            if (g.out_half) static_cast<__half*>(g.out)[o] = __float2half_rn(v);
+                            else static_cast<float*>(g.out)[o] = v;
                         }
                     }
+                    __syncwarp();
                 }
             }
             tc_fence_before();
@@ -711,15 +781,17 @@ struct TileChoice {
 // operand bytes per product (relative cost per unit of work beside the widest), so it is taken only
 // where the widest one would leave SMs idle: few tiles, or a nearly empty last wave.
 TileChoice choose_tile(const GemmProblem& p, int passes, bool b_mn, int sms) {
-    struct Form { int cg, bn; double cost; };
-    // cost of one K-block of a tile, in units of a 256 x 128 tile's
-    static const Form three[] = {{2, 128, 1.0}, {2, 64, 0.56}, {1, 128, 1.08}, {1, 64, 0.6}};
-    static const Form one[] = {{2, 256, 1.9}, {2, 128, 1.0}, {1, 128, 1.08}, {1, 64, 0.6}};
+    struct Form { int cg, bn; double cost, drain; };
+    // cost of one K-block of a tile in units of a 256 x 128 tile's, and K-blocks that its fill and drain come to.  Three
+    // passes over 256 columns leave room for one pair of accumulators, so that tile's epilogue is not hidden; its operand
+    // traffic per product is two thirds, which at the power cap is worth 14 % (8192^3: 3.15 -> 2.69 ms sustained).
+    static const Form three[] = {{2, 256, 1.65, 6}, {2, 128, 1.0, 2}, {2, 64, 0.56, 2}, {1, 128, 1.08, 2}, {1, 64, 0.6, 2}};
+    static const Form one[] = {{2, 256, 1.75, 2}, {2, 128, 1.0, 2}, {1, 128, 1.08, 2}, {1, 64, 0.6, 2}};
     const Form* forms = passes == 3 ? three : one;
     const int64_t batches = p.b0 * p.b1, k_blocks = ceil_div(p.k, kBlockK);
     TileChoice best{};
     double least = 0;
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < (passes == 3 ? 5 : 4); ++i) {
         const Form& f = forms[i];
         if (b_mn && f.bn / f.cg < 64) continue;  // an MN-major atom is 64 wide
         TileChoice c{f.cg, f.bn, ceil_div(p.m, int64_t(f.cg) * kRowsM), ceil_div(p.n, int64_t(f.bn)), 1, k_blocks, 0};
@@ -732,8 +804,8 @@ TileChoice choose_tile(const GemmProblem& p, int passes, bool b_mn, int sms) {
         }
         c.units = tiles * c.splits;
         const double waves = double(ceil_div(c.units, slots));
-        // a tile's fill and drain come to about two K-blocks; slices write and fold partial planes
-        const double cost = waves * f.cost * (double(c.kb_per_split) + 2.0) + (c.splits > 1 ? 4.0 : 0.0);
+        // (slices write and fold partial planes)
+        const double cost = waves * f.cost * (double(c.kb_per_split) + f.drain) + (c.splits > 1 ? 4.0 : 0.0);
         if (i == 0 || cost < least) {
             least = cost;
             best = c;
@@ -743,8 +815,13 @@ TileChoice choose_tile(const GemmProblem& p, int passes, bool b_mn, int sms) {
 }
 
 void run_h16(b200_ctx* ctx, const GemmProblem& p, int passes, const TileChoice& t, const HalfOperand& a, const HalfOperand& b,
-             float* partial, bool out_half, const char* label) {
+             float* partial, bool out_half, const char* label, const HalfEpilogue* epi = nullptr) {
     H16Args g{};
+    if (epi != nullptr) {
+        g.bias = static_cast<const __half*>(epi->bias);
+        g.biased = static_cast<__half*>(epi->biased);
+        g.rectified = static_cast<__half*>(epi->rectified);
+    }
     const int64_t batches = p.b0 * p.b1, out_elems = batches * p.m * p.n;
     g.out = t.splits > 1 ? static_cast<void*>(partial) : static_cast<void*>(p.out);
     g.out_half = t.splits > 1 ? 0 : (out_half ? 1 : 0);
@@ -769,6 +846,7 @@ void run_h16(b200_ctx* ctx, const GemmProblem& p, int passes, const TileChoice& 
         ProfScope scope(ctx, label);
 #define B200_H16_CASE(CG, BN, P)                                  \
     if (t.cg == CG && t.bn == BN && passes == P) launch_major<CG, BN, P>(ctx, a, b, g, t.units);
+        B200_H16_CASE(2, 256, 3)
         B200_H16_CASE(2, 128, 3)
         B200_H16_CASE(2, 64, 3)
         B200_H16_CASE(1, 128, 3)
@@ -935,7 +1013,7 @@ void gemm_h16(b200_ctx* ctx, const GemmProblem& p) {
 
 // Half storage: products of at least 2^25 operations with a row for most of a tile's lanes (smaller ones are
 // launch-bound, and served through widened copies by the CUDA cores).
-bool gemm_f16_storage(b200_ctx* ctx, const GemmProblem& p) {
+bool gemm_f16_storage(b200_ctx* ctx, const GemmProblem& p, const HalfEpilogue* epi) {
     if (ctx->prop.major != 10 || encode_tiled() == nullptr || ctx->gemm_precision == B200_GEMM_FP32 || !fits_tma(p) ||
         p.m < 32 || p.n < 16 || p.k < 16) {
         return false;
@@ -943,6 +1021,13 @@ bool gemm_f16_storage(b200_ctx* ctx, const GemmProblem& p) {
     if (2.0 * double(p.m) * double(p.n) * double(p.k) * double(p.b0 * p.b1) < double(1 << 25)) return false;
     HalfOperand a = operand_a(p), b = operand_b(p);
     const TileChoice t = choose_tile(p, 1, b.mn, ctx->prop.multiProcessorCount);
+    if (epi != nullptr) {
+        // the epilogue adds where it stores 64 whole columns: no K-slices, no ragged edge
+        for (const void* q : {static_cast<const void*>(p.out), epi->bias, static_cast<const void*>(epi->biased), static_cast<const void*>(epi->rectified)}) {
+            if (reinterpret_cast<uintptr_t>(q) % 16 != 0) return false;
+        }
+        if (t.splits > 1 || p.n % 64 != 0 || p.b0 * p.b1 != 1) return false;
+    }
     size_t bytes = 2048;
     auto direct = [](HalfOperand& o) {
         const bool ok = o.s_c == 1 && o.s_r % 8 == 0 && o.s_r >= o.cols && reinterpret_cast<uintptr_t>(o.src) % 16 == 0 &&
@@ -976,7 +1061,7 @@ bool gemm_f16_storage(b200_ctx* ctx, const GemmProblem& p) {
                       o->rows, o->cols, o->pitch, o->nb);
         ctx->count_launch();
     }
-    run_h16(ctx, p, 1, t, a, b, reinterpret_cast<float*>(ws), true, "matmul.tcgen05_f16");
+    run_h16(ctx, p, 1, t, a, b, reinterpret_cast<float*>(ws), true, epi != nullptr ? "matmul.tcgen05_f16_bias" : "matmul.tcgen05_f16", epi);
     return true;
 }
 
