@@ -43,8 +43,8 @@ private:
 };
 
 // Words behind b200_ctx::d_counters: 4096 arrival counters of split reductions, 64 words for the
-// persistent GEMM's tile counter, 1024 arrival counters of the streamed-operand GEMM's split-K fold.
-constexpr size_t kArrivalCounters = 4096 + 64 + 1024;
+// persistent GEMM's tile counter and the loss.
+constexpr size_t kArrivalCounters = 4096 + 64;
 constexpr size_t kLossCounter = 4096 + 32;  // (of the 64) blocks of the loss's mean
 
 struct DistState;  // dist.cu

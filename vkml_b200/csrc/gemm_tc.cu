@@ -785,20 +785,18 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_consta
 // side by side on neighbouring SMs, so S's tile is fetched from HBM once and from L2 after that.
 //
 // When N is shorter than 128 and W is broadcast over the batch, one tile spans several batches
-// (lanes = batch x n).  K is split across CTAs when the tiles alone cannot fill the machine;
-// the warp that arrives last at its quarter of a tile folds the partial planes in split order in
-// the same launch (deterministic, no atomics on data).
+// (lanes = batch x n).  K is split across CTAs when the tiles alone cannot fill the machine, into
+// partial planes that a second launch folds in split order.  (Folded in the same launch by the warp that arrived last
+// at its quarter of a tile, 64 x 4096 x 4096 took 10 us longer: one warp per quarter adds up what the whole
+// machine reads in 3 us.)
 constexpr int kStreamStages = 4;          // W's ring in shared memory and S's ring in tensor memory
 constexpr int kStreamConverters = 16;     // converter warps: four per tensor-memory lane quarter, 8 K columns each
 constexpr int kStreamThreads = (7 + kStreamConverters) * 32;  // + two TMA warps, MMA and four epilogue warps
 constexpr int kStreamTileBytes = BK * 128 * 4;  // one fp32 tile of S: 32 K-rows x 128 lanes
 constexpr uint32_t kStreamTmemCols = 512;
-constexpr int kStreamCounters = 1024;     // arrival counters of the in-kernel split-K fold: 4 per tile
-constexpr int kStreamCounterBase = 4096 + 64;  // their place behind b200_ctx::d_counters
 
 struct StreamArgs {
     float* out;            // C, or the partial planes when splits > 1
-    float* folded;         // C when splits > 1 (target of the in-kernel fold)
     int64_t m, n;          // per batch
     int64_t batches;
     int64_t w_batch_rows;  // rows between consecutive batches in W's planes (0: broadcast)
@@ -810,7 +808,6 @@ struct StreamArgs {
     int bpt;               // batches per tile (nt * bpt == 128 when bpt > 1)
     int64_t batch_groups;  // ceil(batches / bpt)
     uint32_t* status;
-    unsigned int* counters;
 };
 
 
@@ -1101,59 +1098,6 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_const
             if (lane == 0) {
                 mbar_arrive(acc_empty(acc));
             }
-            if (g.splits > 1) {
-                // Split K: each epilogue warp owns 32 lanes of the tile in every K-slice.  The warp
-                // that completes its lanes' last slice folds the slices, in split order -- a
-                // per-warp arrival counter, so no warp ever waits for another one.
-                __threadfence();
-                __syncwarp();
-                unsigned old = 0;
-                if (lane == 0) {
-                    const int64_t tile = (bg * g.tiles_n + tn) * g.tiles_m + tm;
-                    old = atomicInc(g.counters + tile * 4 + quarter, static_cast<unsigned>(g.splits - 1));
-                }
-                old = __shfl_sync(0xffffffffu, old, 0);
-                if (old == static_cast<unsigned>(g.splits - 1)) {
-                    __threadfence();
-                    if (lane_ok) {
-                        // Eight rows and up to four K-slices at a time, all 32 loads issued before
-                        // the first add: the partial planes come from L2, and a chain that waits for
-                        // one load before issuing the next would pay that latency per element.  The
-                        // adds keep the split order.
-                        const int64_t rows = min(int64_t(BNW), g.m - m0);
-                        const float* __restrict__ part = g.out + col + m0 * g.n;
-                        float* __restrict__ dstf = g.folded + col + m0 * g.n;
-                        for (int64_t j0 = 0; j0 < rows; j0 += 8) {
-                            float sum[8];
-                            for (int sp0 = 0; sp0 < g.splits; sp0 += 4) {
-                                float t[4][8];
-#pragma unroll
-                                for (int q = 0; q < 4; ++q) {
-#pragma unroll
-                                    for (int j = 0; j < 8; ++j) {
-                                        t[q][j] = (sp0 + q < g.splits && j0 + j < rows)
-                                                      ? __ldcg(part + int64_t(sp0 + q) * g.split_stride + (j0 + j) * g.n)
-                                                      : 0.0F;
-                                    }
-                                }
-#pragma unroll
-                                for (int q = 0; q < 4; ++q) {
-                                    if (sp0 + q < g.splits) {
-#pragma unroll
-                                        for (int j = 0; j < 8; ++j) {
-                                            sum[j] = (sp0 + q == 0) ? t[q][j] : sum[j] + t[q][j];
-                                        }
-                                    }
-                                }
-                            }
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) {
-                                if (j0 + j < rows) dstf[(j0 + j) * g.n] = sum[j];
-                            }
-                        }
-                    }
-                }
-            }
         }
     } else if (warp < 6 + kStreamConverters) {
         // ---------------- converters (warps 6..21): S tile -> hi / lo in tensor memory ----------------
@@ -1227,6 +1171,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_const
                         split_tf32_select(v[j], hi[j], lo[j]);  // infinities, NaNs, values that round past the range
                     }
                 }
+                __syncwarp();  // (the rare branch above may have parted the warp: the stores below are one warp's)
                 const uint32_t t_hi = tmem_base + lane_field + kStageCol0 + s * 64 + part * 8;
                 tmem_st8(t_hi, hi);
                 if (THREE_PASS) {
@@ -1257,16 +1202,42 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_const
 }
 
 __global__ void __launch_bounds__(256)
-fold_partials_kernel(float* __restrict__ out, const float* __restrict__ partial, int64_t n, int splits) {
+fold_partials_kernel(float* __restrict__ out, const float* __restrict__ partial, int64_t n, int splits, int quads) {
     pdl_prologue();
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
+    if (quads) {
+        for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n / 4; i += stride) {
+            float4 acc = __ldcg(reinterpret_cast<const float4*>(partial) + i);
+#pragma unroll 4
+            for (int s = 1; s < splits; ++s) {
+                const float4 v = __ldcg(reinterpret_cast<const float4*>(partial + int64_t(s) * n) + i);
+                acc.x += v.x;
+                acc.y += v.y;
+                acc.z += v.z;
+                acc.w += v.w;
+            }
+            reinterpret_cast<float4*>(out)[i] = acc;
+        }
+        return;
+    }
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
-        float acc = partial[i];
+        float acc = __ldcg(partial + i);
+#pragma unroll 4
         for (int s = 1; s < splits; ++s) {
-            acc += partial[int64_t(s) * n + i];
+            acc += __ldcg(partial + int64_t(s) * n + i);
         }
         out[i] = acc;
     }
+}
+
+// Adds the K-slices' partial planes in split order (one slice: nothing to do).
+void fold_partials(b200_ctx* ctx, float* out, const float* partial, int64_t n, int splits) {
+    if (splits <= 1) return;
+    ProfScope scope(ctx, "matmul.fold");
+    const bool quads = n % 4 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0 && reinterpret_cast<uintptr_t>(partial) % 16 == 0;
+    launch_kernel(ctx, fold_partials_kernel, grid_for(quads ? n / 4 : n, 256), 256, 0, out, partial, n, splits, quads ? 1 : 0);
+    ctx->count_launch();
+    check_last_launch("matmul (fold)");
 }
 
 // ---------------------------------------------------------------------------
@@ -1579,7 +1550,7 @@ void gemm_stream(b200_ctx* ctx, const GemmProblem& p, bool three_pass, const Str
     const int64_t tiles = tiles_m * tiles_n * batch_groups;
     const int sms = ctx->prop.multiProcessorCount;
     int64_t splits = 1;
-    if (tiles < sms && k_blocks >= 16 && tiles * 4 <= kStreamCounters) {
+    if (tiles < sms && k_blocks >= 16) {
         splits = std::min<int64_t>(sms / tiles, k_blocks / 8);
         splits = std::max<int64_t>(1, std::min<int64_t>(splits, 64));
     }
@@ -1634,7 +1605,6 @@ void gemm_stream(b200_ctx* ctx, const GemmProblem& p, bool three_pass, const Str
 
     StreamArgs g{};
     g.out = splits > 1 ? partial : p.out;
-    g.folded = p.out;
     g.m = p.m;
     g.n = p.n;
     g.batches = batches;
@@ -1649,7 +1619,6 @@ void gemm_stream(b200_ctx* ctx, const GemmProblem& p, bool three_pass, const Str
     g.bpt = sp.bpt;
     g.batch_groups = batch_groups;
     g.status = ctx->d_status;
-    g.counters = ctx->d_counters + kStreamCounterBase;
     const int grid = static_cast<int>(std::min<int64_t>(tiles * splits, sms));
     {
         ProfScope scope(ctx, three_pass ? "matmul.tcgen05_3xtf32_stream" : "matmul.tcgen05_tf32_stream");
@@ -1661,7 +1630,50 @@ void gemm_stream(b200_ctx* ctx, const GemmProblem& p, bool three_pass, const Str
     }
     ctx->count_launch();
     check_last_launch("matmul (tcgen05, streamed operand)");
+    fold_partials(ctx, p.out, partial, out_elems, static_cast<int>(splits));
     release_use(ctx, ow);
+}
+
+// The plane kernel's tile width and K-slices.
+struct TcPlan {
+    int bn;
+    int64_t tiles_m, tiles_n, k_blocks, splits, kb_per_split;
+};
+
+TcPlan plan_planes(const b200_ctx* ctx, const GemmProblem& p) {
+    const int64_t batches = p.b0 * p.b1;
+    // Tile width: 128x256 tiles are the most efficient per tile (measured 5.5 % better than two
+    // 128x128 tiles), but the persistent grid runs whole waves of 148 tiles, so the narrower
+    // tile wins whenever it wastes less of the last wave (M=2048, N=8192: 4 waves of 256-wide
+    // tiles against 7 half-cost waves of 128-wide ones).
+    int bn = 64;
+    if (p.n > 64) bn = 128;
+    if (p.n > 128 && p.m * p.n * batches >= int64_t(128) * 256 * sm_count()) {
+        const int64_t tm = ceil_div(p.m, BM);
+        const double cost256 = double(ceil_div(tm * ceil_div(p.n, 256) * batches, sm_count()));
+        const double cost128 = double(ceil_div(tm * ceil_div(p.n, 128) * batches, sm_count())) * 0.5275;
+        bn = cost128 < cost256 ? 128 : 256;
+    }
+    if (ctx->gemm_bn_override == 64 || ctx->gemm_bn_override == 128 || ctx->gemm_bn_override == 256) {
+        bn = ctx->gemm_bn_override;
+    }
+    const int64_t tiles_m = ceil_div(p.m, BM);
+    const int64_t tiles_n = ceil_div(p.n, bn);
+    const int64_t tiles = tiles_m * tiles_n * batches;
+    const int64_t k_blocks = ceil_div(p.k, BK);
+
+    // split K when the tiles alone cannot fill the machine
+    int64_t splits = 1;
+    if (tiles < sm_count() && k_blocks >= 16) {
+        // as many K-slices as keep every unit in ONE wave of the persistent grid: rounding up
+        // instead (32 tiles x 5 slices = 160 units on 148 SMs) runs a second, nearly empty wave
+        splits = std::min<int64_t>(sm_count() / tiles, k_blocks / 8);
+        splits = std::max<int64_t>(1, std::min<int64_t>(splits, 64));
+    }
+    int64_t kb_per_split = ceil_div(k_blocks, splits);
+    splits = ceil_div(k_blocks, kb_per_split);
+
+    return TcPlan{bn, tiles_m, tiles_n, k_blocks, splits, kb_per_split};
 }
 
 }  // namespace
@@ -1685,6 +1697,8 @@ bool gemm_tc_eligible(const b200_ctx* ctx, const GemmProblem& p) {
     }
     return true;
 }
+
+int64_t gemm_tc_chain(const b200_ctx* ctx, const GemmProblem& p) { return plan_planes(ctx, p).kb_per_split * BK; }
 
 bool gemm_tc_streams(const b200_ctx* ctx, const GemmProblem& p) { return plan_stream(ctx, p).ok; }
 
@@ -1713,41 +1727,13 @@ void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass) {
         return;
     }
     const int64_t batches = p.b0 * p.b1;
-    const int64_t kp = align_up(p.k, BK);
     const bool a_bcast = (p.a_s[0] == 0 || p.b0 == 1) && (p.a_s[1] == 0 || p.b1 == 1);
     const bool b_bcast = (p.b_s[0] == 0 || p.b0 == 1) && (p.b_s[1] == 0 || p.b1 == 1);
 
-    // Tile width: 128x256 tiles are the most efficient per tile (measured 5.5 % better than two
-    // 128x128 tiles), but the persistent grid runs whole waves of 148 tiles, so the narrower
-    // tile wins whenever it wastes less of the last wave (M=2048, N=8192: 4 waves of 256-wide
-    // tiles against 7 half-cost waves of 128-wide ones).
-    int bn = 64;
-    if (p.n > 64) bn = 128;
-    if (p.n > 128 && p.m * p.n * batches >= int64_t(128) * 256 * sm_count()) {
-        const int64_t tm = ceil_div(p.m, BM);
-        const double cost256 = double(ceil_div(tm * ceil_div(p.n, 256) * batches, sm_count()));
-        const double cost128 = double(ceil_div(tm * ceil_div(p.n, 128) * batches, sm_count())) * 0.5275;
-        bn = cost128 < cost256 ? 128 : 256;
-    }
-    if (ctx->gemm_bn_override == 64 || ctx->gemm_bn_override == 128 || ctx->gemm_bn_override == 256) {
-        bn = ctx->gemm_bn_override;
-    }
-    const int64_t tiles_m = ceil_div(p.m, BM);
-    const int64_t tiles_n = ceil_div(p.n, bn);
-    const int64_t tiles = tiles_m * tiles_n * batches;
-    const int64_t k_blocks = kp / BK;
-
-    // split K when the tiles alone cannot fill the machine
-    int64_t splits = 1;
-    if (tiles < sm_count() && k_blocks >= 16) {
-        // as many K-slices as keep every unit in ONE wave of the persistent grid: rounding up
-        // instead (32 tiles x 5 slices = 160 units on 148 SMs) runs a second, nearly empty wave
-        splits = std::min<int64_t>(sm_count() / tiles, k_blocks / 8);
-        splits = std::max<int64_t>(1, std::min<int64_t>(splits, 64));
-    }
-    int64_t kb_per_split = ceil_div(k_blocks, splits);
-    splits = ceil_div(k_blocks, kb_per_split);
-
+    const TcPlan plan = plan_planes(ctx, p);
+    const int bn = plan.bn;
+    const int64_t tiles_m = plan.tiles_m, tiles_n = plan.tiles_n, tiles = tiles_m * tiles_n * batches;
+    const int64_t k_blocks = plan.k_blocks, splits = plan.splits, kb_per_split = plan.kb_per_split;
     const int64_t out_elems = batches * p.m * p.n;
     const size_t partial_bytes = splits > 1 ? static_cast<size_t>(align_up(out_elems * splits * 4, 1024)) : 0;
     Operand oa = plan_operand(p.a, p.a_s[0], p.a_s[1], p.a_s[2], p.a_s[3], p.m, p.k, a_bcast, p);
@@ -1800,13 +1786,7 @@ void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass) {
         }
         ctx->count_launch();
         check_last_launch("matmul (tcgen05, direct operands)");
-        if (splits > 1) {
-            ProfScope scope(ctx, "matmul.fold");
-            launch_kernel(ctx, fold_partials_kernel, grid_for(out_elems, 256), 256, 0, p.out, partial, out_elems,
-                                                                                  static_cast<int>(splits));
-            ctx->count_launch();
-            check_last_launch("matmul (fold)");
-        }
+        fold_partials(ctx, p.out, partial, out_elems, static_cast<int>(splits));
         return;
     }
 
@@ -1916,13 +1896,7 @@ void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass) {
     ctx->count_launch();
     check_last_launch("matmul (tcgen05)");
 
-    if (splits > 1) {
-        ProfScope scope(ctx, "matmul.fold");
-        launch_kernel(ctx, fold_partials_kernel, grid_for(out_elems, 256), 256, 0, p.out, partial, out_elems,
-                                                                              static_cast<int>(splits));
-        ctx->count_launch();
-        check_last_launch("matmul (fold)");
-    }
+    fold_partials(ctx, p.out, partial, out_elems, static_cast<int>(splits));
     // the stream is in order: a plane released here is only reused by later work
     release_use(ctx, oa);
     release_use(ctx, ob);
