@@ -300,17 +300,18 @@ def run_b200(args, rank, local_rank, world):
         avg_ms = sum(by_label[main_label]) / len(by_label[main_label])
         achieved = flops_per_step / (avg_ms * 1e-3) / 1e12
         passes = 3 if args.precision == "3xtf32" else 1
-        # TF32 issues at half the bf16 rate; MEASURED_PEAKS.json has no TF32 entry, so the
-        # denominator is half the measured bf16 burst figure.
-        peak = pk["bf16_tflops"] / 2.0
+        # half terms run at the bf16 rate; TF32 issues at half of it (MEASURED_PEAKS.json has no TF32
+        # entry, so its denominator is half the measured bf16 burst figure)
+        half_terms = "f16" in main_label
+        peak = pk["bf16_tflops"] / (1.0 if half_terms else 2.0)
         roofline = {"bound": "tensor", "kernel": main_label, "achieved": achieved, "peak": peak,
                     "unit": "TFLOP/s", "frac": achieved / peak,
-                    "traffic": TRAFFIC_BYTES_PER_LAUNCH if (size == 8192 and args.precision == "3xtf32") else None,
-                    "traffic_source": "quoted from one ncu capture of this kernel at this size; not measured in this run",
+                    "traffic": TRAFFIC_BYTES_PER_LAUNCH if (size == 8192 and args.precision == "3xtf32" and not half_terms) else None,
+                    "traffic_source": "quoted from one ncu capture of the TF32 kernel at this size; none for half terms",
                     "avg_launch_ms": avg_ms, "launches_timed": len(by_label[main_label]),
                     "tensor_pipe_tflops": achieved * passes, "tensor_pipe_frac": achieved * passes / peak,
-                    "peak_source": f"{pk['source']}: bf16_tflops/2 (TF32 runs at half the bf16 rate)",
-                    "note": "achieved counts the algorithmic 2*M*N*K once; 3xTF32 issues it three times on "
+                    "peak_source": f"{pk['source']}: bf16_tflops" + (" (half terms)" if half_terms else "/2 (TF32 runs at half the bf16 rate)"),
+                    "note": "achieved counts the algorithmic 2*M*N*K once; two terms per operand issue it three times on "
                             "the tensor pipe (tensor_pipe_*), so frac cannot exceed 1/3"}
         if args.precision == "fp32":
             roofline["bound"] = "fp32-simt"
@@ -370,7 +371,7 @@ def run_b200(args, rank, local_rank, world):
             "metric": "fp32_gemm_tflops", "value": value, "unit": "TFLOP/s", "n_gpus": world, "steps": args.steps,
             "warmup": max(args.warmup, 3), "ms_per_step": ms / args.steps, "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None,
-            "dtype": {"3xtf32": "f32 (3xTF32 split on tcgen05, fp32 accumulate)", "tf32": "tf32",
+            "dtype": {"3xtf32": "f32 (two 11-bit terms per operand on tcgen05, three products, fp32 accumulate)", "tf32": "tf32",
                       "fp32": "f32"}[args.precision],
             "data": "synthetic",
             "config": gemm_config(size, args.precision, world),
