@@ -94,17 +94,19 @@ __global__ void __launch_bounds__(256) range_kernel(MatrixPair pair) {
     const MatrixArgs& a = pair.m[blockIdx.y];
     const int64_t per_row = (a.cols + 7) / 8;
     const int64_t total = per_row * a.rows * a.n_batches;
-    const int64_t stride = max(int64_t(1), total / kSampleGroups);  // of the pieces, one in so many
-    const int64_t groups = (total + stride - 1) / stride;
-    const int64_t step = int64_t(gridDim.x) * blockDim.x;
+    const uint32_t stride = static_cast<uint32_t>(max(int64_t(1), total / kSampleGroups));  // of the pieces, one in so many
+    const uint32_t groups = static_cast<uint32_t>((total + stride - 1) / stride);           // (at most 2 * kSampleGroups)
+    const bool small = total < (int64_t(1) << 31);
     uint32_t top = 0;
-    for (int64_t j = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < groups; j += step) {
-        const int64_t piece = j / kPiece;
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < groups; j += gridDim.x * blockDim.x) {
+        // (64-bit divisions for every group were most of this kernel's time on small matrices)
+        const uint32_t piece = j / kPiece;
         // (a piece's place inside its stretch varies, so that no column pattern of the matrix is in step with it)
-        const int64_t i = min(total - 1, (piece * stride + (piece * 7919) % stride) * kPiece + j % kPiece);
+        const uint32_t shift = stride == 1 ? 0u : (piece * 7919u) % stride;
+        const int64_t i = min(total - 1, (int64_t(piece) * stride + shift) * kPiece + j % kPiece);
+        const int64_t rb = small ? int64_t(uint32_t(i) / uint32_t(per_row)) : i / per_row;
         float v[8];
         int64_t r;
-        const int64_t rb = row_number(i, per_row, total);
         load8(a, row_of(a, rb, r), (i - rb * per_row) * 8, v);
 #pragma unroll
         for (int q = 0; q < 8; ++q) top = max(top, __float_as_uint(v[q]) & 0x7FFFFFFFu);
@@ -117,6 +119,12 @@ __global__ void __launch_bounds__(256) range_kernel(MatrixPair pair) {
         top = __reduce_max_sync(0xffu, tops[threadIdx.x]);
         if (threadIdx.x == 0 && top != 0) atomicMax(&a.range->max_bits, top);
     }
+}
+
+__global__ void __launch_bounds__(kRangeSlots) clear_ranges_kernel(uint4* slots) {
+    pdl_prologue();
+    static_assert(sizeof(RangeSlot) == sizeof(uint4), "one slot to a thread");
+    slots[threadIdx.x] = make_uint4(0, 0, 0, 0);
 }
 
 // Writes each matrix's two half planes, [batch][row][pitch], in the orientation the matrix has in memory: 4 bytes read, 4 written per element.
@@ -928,7 +936,9 @@ void gemm_h16(b200_ctx* ctx, const GemmProblem& p) {
         return;
     }
     if (ctx->range_next == 0) {
-        B200_CUDA_CHECK(cudaMemsetAsync(ctx->d_ranges, 0, sizeof(RangeSlot) * kRangeSlots, ctx->stream));
+        // (a kernel, not a memset: it overlaps its neighbours' launches, which a memset between them would not let do so either)
+        launch_kernel(ctx, clear_ranges_kernel, 1u, kRangeSlots, 0, static_cast<uint4*>(ctx->d_ranges));
+        ctx->count_launch();
     }
     const size_t cache_limit = std::min<size_t>(size_t(16) << 30, ctx->prop.totalGlobalMem / 8);
     auto place = [&](HalfOperand& o) {

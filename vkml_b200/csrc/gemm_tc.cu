@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(256) split_kernel(SplitArgs a) {
 }
 
 // Both operands of a product in one launch: the planes that stand by for a wide operand.  There is nearly always nothing
-// to do, and then one launch of a few hundred blocks costs less than two full ones.
+// to do, and then one launch of two blocks per SM costs less than two full ones.
 struct SplitPair {
     SplitArgs s[2];
     RangeGuard guard;
@@ -1666,8 +1666,11 @@ TcPlan plan_planes(const b200_ctx* ctx, const GemmProblem& p) {
     int64_t splits = 1;
     if (tiles < sm_count() && k_blocks >= 16) {
         // as many K-slices as keep every unit in ONE wave of the persistent grid: rounding up
-        // instead (32 tiles x 5 slices = 160 units on 148 SMs) runs a second, nearly empty wave
-        splits = std::min<int64_t>(sm_count() / tiles, k_blocks / 8);
+        // instead (32 tiles x 5 slices = 160 units on 148 SMs) runs a second, nearly empty wave.  Slices of eight K-blocks
+        // and more; of three where the tiles fill less than an eighth of the machine (a classifier's few columns: 300 x 900 x 100
+        // took 21 us with three CTAs to a tile), unless the span compares the result, whose bits then stay
+        const int64_t least = tiles * 8 <= sm_count() && ctx->compared.count(p.out) == 0 ? 3 : 8;
+        splits = std::min<int64_t>(sm_count() / tiles, k_blocks / least);
         splits = std::max<int64_t>(1, std::min<int64_t>(splits, 64));
     }
     int64_t kb_per_split = ceil_div(k_blocks, splits);
@@ -1926,7 +1929,7 @@ void gemm_tc_if_wide(b200_ctx* ctx, const GemmProblem& p, const RangeGuard& guar
     }
     {
         ProfScope scope(ctx, "matmul.if_wide");
-        launch_kernel(ctx, split_pair_kernel, dim3(ctx->prop.multiProcessorCount * 2, 2), 256, 0, pair);
+        launch_kernel(ctx, split_pair_kernel, dim3(ctx->prop.multiProcessorCount, 2), 256, 0, pair);
     }
     ctx->count_launch();
     constexpr int bn = 128;
