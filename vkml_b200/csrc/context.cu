@@ -328,10 +328,10 @@ void note_compared_products(b200_ctx* ctx, const b200_node* nodes, size_t n_node
 // that a matrix used twice (a weight in forward and backward, an activation in forward and in
 // the weight gradient) is split into its TF32 planes only once.
 void count_matmul_operands(b200_ctx* ctx, const b200_node* nodes, size_t n_nodes) {
-    if (ctx->gemm_precision == B200_GEMM_FP32 || !ctx->share_planes) return;
     size_t matmuls = 0;
     for (size_t i = 0; i < n_nodes; ++i) matmuls += nodes[i].op == B200_OP_MATMUL ? 1 : 0;
-    if (matmuls < 2) return;
+    ctx->lone_matmul = matmuls < 2;
+    if (matmuls < 2 || ctx->gemm_precision == B200_GEMM_FP32 || !ctx->share_planes) return;
     for (size_t i = 0; i < n_nodes; ++i) {
         const b200_node& node = nodes[i];
         if (node.op != B200_OP_MATMUL || node.out.data == nullptr || node.n_src < 2 ||

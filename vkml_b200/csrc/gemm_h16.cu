@@ -164,25 +164,6 @@ __global__ void __launch_bounds__(256) split_half_kernel(MatrixPair pair) {
     if (over) a.range->spoiled = 1;
 }
 
-// A half matrix that TMA cannot read as it lies (odd pitch, misaligned base, two strided axes): a dense copy.
-__global__ void __launch_bounds__(256) pack_half_kernel(const __half* __restrict__ src, __half* __restrict__ dst, int64_t b1,
-                                                        int64_t s_b0, int64_t s_b1, int64_t s_r, int64_t s_c, int64_t rows,
-                                                        int64_t cols, int64_t pitch, int64_t batches) {
-    pdl_prologue();
-    const int64_t per_row = pitch / 8;
-    const int64_t total = per_row * rows * batches;
-    const int64_t step = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += step) {
-        const int64_t rb = i / per_row, c = (i - rb * per_row) * 8;
-        const int64_t b = rb / rows, r = rb - b * rows;
-        const __half* row = src + (b / b1) * s_b0 + (b % b1) * s_b1 + r * s_r;
-        __half v[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = c + j < cols ? row[(c + j) * s_c] : __half(0.0F);
-        *reinterpret_cast<uint4*>(dst + rb * pitch + c) = *reinterpret_cast<const uint4*>(v);
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Main kernel
 // ---------------------------------------------------------------------------
@@ -243,8 +224,9 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
 }
 
 __device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    // (not the aligned forms: one lane of a producer or MMA warp may come from its loop later than the others)
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
 
 template <int CG>
@@ -288,6 +270,7 @@ __device__ __forceinline__ void commit_all(uint32_t bar) {
 
 template <int CG>
 __device__ __forceinline__ void tmem_get(uint32_t dst_smem, uint32_t cols) {
+    __syncwarp();
     if constexpr (CG == 2) {
         asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(cols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -298,6 +281,7 @@ __device__ __forceinline__ void tmem_get(uint32_t dst_smem, uint32_t cols) {
 
 template <int CG>
 __device__ __forceinline__ void tmem_put(uint32_t taddr, uint32_t cols) {
+    __syncwarp();
     if constexpr (CG == 2) {
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
     } else {
@@ -433,6 +417,11 @@ gemm_h16_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_const
                         load(stage + 2 * T::kABytes + T::kBBytes, &map_b_lo, B_MN, BN / CG, n0, b2, b3);
                     }
                 }
+            }
+            // every stage's last release has arrived (from the even CTA's commits) before this CTA's memory becomes another's
+            for (uint32_t i = 0; i < static_cast<uint32_t>(STAGES) && i < it && ok; ++i) {
+                const uint32_t last = it - 1 - i;
+                ok = mbar_wait(empty_bar(last % STAGES), (last / STAGES) & 1, abort_p, g.status);
             }
         }
     } else if (warp == 1) {
@@ -627,6 +616,7 @@ gemm_h16_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_const
         }
     }
 
+    __syncwarp();
     __syncthreads();
     if (abort_flag != 0) {
         for (int i = 0; i < 200; ++i) __nanosleep(1000);  // copies in flight land before the CTA retires
@@ -706,7 +696,7 @@ struct HalfOperand {
     bool mn = false, bcast = false;
     int64_t rows = 0, cols = 0, nb = 1, b1 = 1, s_b0 = 0, s_b1 = 0, s_r = 0, s_c = 0, pitch = 0;
     const void* src = nullptr;
-    const __half* hi = nullptr;  // (one pass: the operand itself, or its packed copy)
+    const __half* hi = nullptr;  // (one pass: the operand itself)
     const __half* lo = nullptr;
     int64_t map_b1 = 1, map_s_b1 = 0, map_b0 = 1, map_s_b0 = 0;
     RangeSlot* range = nullptr;
@@ -741,7 +731,7 @@ HalfOperand half_operand(const void* src, const int64_t (&s)[4], int mn_axis, in
 HalfOperand operand_a(const GemmProblem& p) { return half_operand(p.a, p.a_s, 2, 3, p.m, p.k, p); }
 HalfOperand operand_b(const GemmProblem& p) { return half_operand(p.b, p.b_s, 3, 2, p.n, p.k, p); }
 
-// The dense layout of planes and packed copies: [batch][row][pitch].
+// The dense layout of planes: [batch][row][pitch].
 void lay_out_planes(HalfOperand& o) {
     o.pitch = align_up(o.cols, 8);
     o.map_b1 = o.nb;
@@ -794,12 +784,12 @@ TileChoice choose_tile(const GemmProblem& p, int passes, bool b_mn, int sms) {
     // passes over 256 columns leave room for one pair of accumulators, so that tile's epilogue is not hidden; its operand
     // traffic per product is two thirds, which at the power cap is worth 14 % (8192^3: 3.15 -> 2.69 ms sustained).
     static const Form three[] = {{2, 256, 1.65, 6}, {2, 128, 1.0, 2}, {2, 64, 0.56, 2}, {1, 128, 1.08, 2}, {1, 64, 0.6, 2}};
-    static const Form one[] = {{2, 256, 1.75, 2}, {2, 128, 1.0, 2}, {1, 128, 1.08, 2}, {1, 64, 0.6, 2}};
+    static const Form one[] = {{2, 256, 1.75, 2}, {1, 128, 1.08, 2}, {1, 64, 0.6, 2}};
     const Form* forms = passes == 3 ? three : one;
     const int64_t batches = p.b0 * p.b1, k_blocks = ceil_div(p.k, kBlockK);
     TileChoice best{};
     double least = 0;
-    for (int i = 0; i < (passes == 3 ? 5 : 4); ++i) {
+    for (int i = 0; i < (passes == 3 ? 5 : 3); ++i) {
         const Form& f = forms[i];
         if (b_mn && f.bn / f.cg < 64) continue;  // an MN-major atom is 64 wide
         TileChoice c{f.cg, f.bn, ceil_div(p.m, int64_t(f.cg) * kRowsM), ceil_div(p.n, int64_t(f.bn)), 1, k_blocks, 0};
@@ -860,7 +850,6 @@ void run_h16(b200_ctx* ctx, const GemmProblem& p, int passes, const TileChoice& 
         B200_H16_CASE(1, 128, 3)
         B200_H16_CASE(1, 64, 3)
         B200_H16_CASE(2, 256, 1)
-        B200_H16_CASE(2, 128, 1)
         B200_H16_CASE(1, 128, 1)
         B200_H16_CASE(1, 64, 1)
 #undef B200_H16_CASE
@@ -917,7 +906,8 @@ bool gemm_h16_serves(const b200_ctx* ctx, const GemmProblem& p) {
     const double flops = 2.0 * double(p.m) * double(p.n) * double(p.k) * double(p.b0 * p.b1);
     // (A chain of more than 12288 truncating additions moves a TF32 result by about 1e-4 from the exact one, and by as
     // much from half terms; such products keep the results they have always had.)
-    return flops > 2147483648.0 && !gemm_tc_streams(ctx, p) && ctx->compared.count(p.out) == 0 && gemm_tc_chain(ctx, p) <= 12288;
+    return flops > 2147483648.0 && !gemm_tc_streams(ctx, p) && ctx->compared.count(p.out) == 0 && gemm_tc_chain(ctx, p) <= 12288 &&
+           !(ctx->lone_matmul && gemm_tc_reads_directly(ctx, p));
 }
 
 void gemm_h16_note_uses(b200_ctx* ctx, const GemmProblem& p) {
@@ -1040,7 +1030,6 @@ bool gemm_f16_storage(b200_ctx* ctx, const GemmProblem& p, const HalfEpilogue* e
         }
         if (t.splits > 1 || p.n % 64 != 0 || p.b0 * p.b1 != 1) return false;
     }
-    size_t bytes = 2048;
     auto direct = [](HalfOperand& o) {
         const bool ok = o.s_c == 1 && o.s_r % 8 == 0 && o.s_r >= o.cols && reinterpret_cast<uintptr_t>(o.src) % 16 == 0 &&
                         o.s_b0 % 8 == 0 && o.s_b1 % 8 == 0 && (o.nb == 1 || ((o.b1 == 1 || o.s_b1 > 0) && (o.nb == o.b1 || o.s_b0 > 0)));
@@ -1051,28 +1040,15 @@ bool gemm_f16_storage(b200_ctx* ctx, const GemmProblem& p, const HalfEpilogue* e
             o.map_s_b1 = o.s_b1;
             o.map_b0 = o.nb / o.b1;
             o.map_s_b0 = o.s_b0;
-        } else {
-            lay_out_planes(o);
         }
         return ok;
     };
-    const bool da = direct(a), db = direct(b);
-    const int64_t out_elems = p.b0 * p.b1 * p.m * p.n;
-    if (!da) bytes += a.plane_bytes();
-    if (!db) bytes += b.plane_bytes();
-    if (t.splits > 1) bytes += static_cast<size_t>(out_elems * t.splits * 4);
+    // (operands that TMA cannot read as they lie -- odd pitches -- are served through widened copies, dispatch_f16)
+    if (!direct(a) || !direct(b)) return false;
+    size_t bytes = 2048;
+    if (t.splits > 1) bytes += static_cast<size_t>(p.b0 * p.b1 * p.m * p.n * t.splits * 4);
     char* ws = static_cast<char*>(ctx->ensure_workspace(bytes));
     ws = reinterpret_cast<char*>(align_up(reinterpret_cast<int64_t>(ws), 1024));
-    for (HalfOperand* o : {&a, &b}) {
-        if (o == &a ? da : db) continue;
-        o->hi = reinterpret_cast<const __half*>(ws);
-        ws += o->plane_bytes();
-        ProfScope scope(ctx, "matmul.pack");
-        launch_kernel(ctx, pack_half_kernel, grid_for(o->nb * o->rows * (o->pitch / 8), 256), 256, 0,
-                      static_cast<const __half*>(o->src), const_cast<__half*>(o->hi), o->b1, o->s_b0, o->s_b1, o->s_r, o->s_c,
-                      o->rows, o->cols, o->pitch, o->nb);
-        ctx->count_launch();
-    }
     run_h16(ctx, p, 1, t, a, b, reinterpret_cast<float*>(ws), true, epi != nullptr ? "matmul.tcgen05_f16_bias" : "matmul.tcgen05_f16", epi);
     return true;
 }

@@ -1409,6 +1409,11 @@ Operand plan_operand(const float* ptr, int64_t s_b0, int64_t s_b1, int64_t s_mn,
 // against 105; the CNN's head, 19 against 24 us (planes that another product of the span uses too cost each half) --
 // and below 2^28 operations, which take under 2 us either way while a plane pass is one more launch per operand.
 bool direct_pays(const b200_ctx* ctx, const GemmProblem& p, int64_t batches, const Operand& oa, const Operand& ob) {
+    // (the tensor maps over the operands know a whole broadcast, not one of the two batch axes alone)
+    for (const int64_t* st : {p.a_s, p.b_s}) {
+        const bool still0 = p.b0 > 1 && st[0] == 0, still1 = p.b1 > 1 && st[1] == 0;
+        if ((still0 && p.b1 > 1 && !still1) || (still1 && p.b0 > 1 && !still0)) return false;
+    }
     auto share = [&](const Operand& o) {
         const auto it = ctx->plane_uses.find(o.key);
         return it != ctx->plane_uses.end() && it->second >= 2 ? 0.5 : 1.0;
