@@ -318,6 +318,13 @@ inline unsigned grid_for(int64_t work, int threads, int blocks_per_sm = 8) {
     return static_cast<unsigned>(g);
 }
 
+// Every thread of the cluster.  Not the .aligned forms: those count a warp, and a warp that comes from a branch or a loop in two
+// parts would be counted twice.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
 // Programmatic dependent launch.  Every kernel of the library starts with this pair: the first
 // instruction lets the NEXT kernel of the stream be scheduled as soon as all blocks of this one
 // are running (instead of after its last block has retired), the second holds this kernel until

@@ -223,12 +223,6 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
 }
 
-__device__ __forceinline__ void cluster_sync() {
-    // (not the aligned forms: one lane of a producer or MMA warp may come from its loop later than the others)
-    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
-}
-
 template <int CG>
 __device__ __forceinline__ void tma_tile(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2, int c3) {
     if constexpr (CG == 2) {
@@ -418,11 +412,7 @@ gemm_h16_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_const
                     }
                 }
             }
-            // every stage's last release has arrived (from the even CTA's commits) before this CTA's memory becomes another's
-            for (uint32_t i = 0; i < static_cast<uint32_t>(STAGES) && i < it && ok; ++i) {
-                const uint32_t last = it - 1 - i;
-                ok = mbar_wait(empty_bar(last % STAGES), (last / STAGES) & 1, abort_p, g.status);
-            }
+            drain_commits<STAGES>(empty_bar, it, abort_p, g.status);  // (from the even CTA's commits)
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer (the even CTA's) ----------------

@@ -268,8 +268,7 @@ __global__ void __launch_bounds__(256) gemm_small_kernel(SmallArgs g) {
         store(row, col, sum);
     } else {
         *reinterpret_cast<float4*>(&tile_sum[threadIdx.x * 4]) = sum;
-        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        cluster_sync();
         constexpr int kShare = 256 / CS;  // quads of the tile that this CTA adds up
         if (threadIdx.x < kShare) {
             const int q = rank * kShare + threadIdx.x;
@@ -286,8 +285,7 @@ __global__ void __launch_bounds__(256) gemm_small_kernel(SmallArgs g) {
             }
             store(q >> 3, (q & 7) * 4, total);
         }
-        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        cluster_sync();
     }
 }
 

@@ -595,6 +595,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_consta
                 }
                 u = nxt;
             }
+            drain_commits<STAGES>(empty_bar, it, abort_p, g.status);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
@@ -822,6 +823,7 @@ __device__ __forceinline__ void umma_tf32_ts(uint32_t tmem_d, uint32_t tmem_a, u
 }
 
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
+    __syncwarp();
     asm volatile(
         "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
         ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
@@ -987,6 +989,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_const
                     }
                 }
             }
+            drain_commits<STAGES>(empty_bar, it, abort_p, g.status);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
@@ -1171,7 +1174,6 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap map_s, const __grid_const
                         split_tf32_select(v[j], hi[j], lo[j]);  // infinities, NaNs, values that round past the range
                     }
                 }
-                __syncwarp();  // (the rare branch above may have parted the warp: the stores below are one warp's)
                 const uint32_t t_hi = tmem_base + lane_field + kStageCol0 + s * 64 + part * 8;
                 tmem_st8(t_hi, hi);
                 if (THREE_PASS) {

@@ -112,6 +112,16 @@ __device__ __forceinline__ bool mbar_wait_parked(uint32_t bar, uint32_t parity, 
     return true;
 }
 
+// The commits of a ring's last round (`used` stages filled in all) have arrived: nobody waits for them otherwise, and one that came
+// after the CTA had retired would land on a barrier of whatever CTA has its shared memory then.
+template <int STAGES, typename Bar>
+__device__ __forceinline__ void drain_commits(Bar empty_bar, uint32_t used, volatile int* abort_flag, uint32_t* status) {
+    for (uint32_t i = 0; i < static_cast<uint32_t>(STAGES) && i < used; ++i) {
+        const uint32_t last = used - 1 - i;
+        if (!mbar_wait(empty_bar(last % STAGES), (last / STAGES) & 1, abort_flag, status)) return;
+    }
+}
+
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0,
                                             int c1) {
     asm volatile(
@@ -131,7 +141,10 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// (Instructions marked .aligned want the whole warp at once.  Lanes leave a bounded wait, a role's branch or a ragged store
+// each by itself, and nothing makes the compiler bring them together before an asm statement, so every wrapper does.)
 __device__ __forceinline__ void tmem_alloc(uint32_t dst_smem, uint32_t cols) {
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(cols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -159,7 +172,7 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
 }
 
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    __syncwarp();  // (an aligned instruction: lanes that left a wait or a store at different times meet here first)
+    __syncwarp();
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
         "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
