@@ -142,6 +142,28 @@ def test_matmul_tensor_core_both_operand_schemes(oracle, monkeypatch):
         assert np.array_equal(a.view(np.uint32), d.view(np.uint32)), name
 
 
+@pytest.mark.parametrize("operands", ["direct", "auto"])
+@pytest.mark.parametrize("held", [(2, 1), (1, 3)])
+def test_matmul_operand_broadcast_over_one_batch_axis(monkeypatch, operands, held):
+    """An operand that stands still along one of two batch axes is no single tensor map: whatever scheme is asked for,
+    every batch gets its own matrix."""
+    import vkml_b200
+    from vkml_b200 import DeviceTensor, NodeDesc, Op
+    monkeypatch.setenv("VKML_B200_GEMM_OPERANDS", operands)
+    b = vkml_b200.Backend(0)
+    rng = np.random.default_rng(3)
+    x, y = rng.standard_normal(held + (256, 256), dtype=np.float32), rng.standard_normal((2, 3, 256, 192), dtype=np.float32)
+    for left in (True, False):
+        p, q = (x, y) if left else (np.swapaxes(y, 2, 3).copy(), x)
+        dp, dq = (DeviceTensor.from_host(b, t).broadcast_to((2, 3) + t.shape[2:]) for t in (p, q))
+        out = DeviceTensor.empty(b, (2, 3, p.shape[2], q.shape[3]))
+        b.compute([NodeDesc(int(Op.MATMUL), out.desc, [dp.desc, dq.desc])])
+        want = p.astype(np.float64) @ q.astype(np.float64)
+        for i in range(2):
+            for j in range(3):  # (each by itself: a wrong matrix is wrong everywhere)
+                assert np.linalg.norm(out.numpy()[i, j] - want[i, j]) < 1e-5 * np.linalg.norm(want[i, j]), (i, j)
+
+
 def test_matmul_tensor_core_tf32_opt_in(cuda, oracle, backend):
     """Plain TF32 is an explicit opt-in and is only held to TF32-grade error."""
     backend.set_gemm_precision(1)

@@ -1405,6 +1405,16 @@ Operand plan_operand(const float* ptr, int64_t s_b0, int64_t s_b1, int64_t s_mn,
     return o;
 }
 
+// Whether one tensor map each describes the operands as they lie.  It knows a whole broadcast over the batches (one matrix), not one of the
+// two batch axes alone -- which it would read as that axis' first matrix and zeros -- and no axis that stands still or runs backwards.
+bool maps_describe(const GemmProblem& p, const Operand& oa, const Operand& ob) {
+    auto fits = [&](const Operand& o, const int64_t (&st)[4]) {
+        const bool whole = o.nb == 1;
+        return o.dense && o.split.s_r >= o.cols && (whole || ((p.b0 == 1 || st[0] > 0) && (p.b1 == 1 || st[1] > 0)));
+    };
+    return fits(oa, p.a_s) && fits(ob, p.b_s);
+}
+
 // Whether reading the operands directly beats splitting them into planes first.  Measured: the
 // in-kernel split is bound by shared-memory traffic (the converter's loads and stores contend
 // with the tensor core's operand reads) at about 147 TFLOP/s of algorithmic work -- 7.5 ms against
@@ -1414,11 +1424,6 @@ Operand plan_operand(const float* ptr, int64_t s_b0, int64_t s_b1, int64_t s_mn,
 // against 105; the CNN's head, 19 against 24 us (planes that another product of the span uses too cost each half) --
 // and below 2^28 operations, which take under 2 us either way while a plane pass is one more launch per operand.
 bool direct_pays(const b200_ctx* ctx, const GemmProblem& p, int64_t batches, const Operand& oa, const Operand& ob) {
-    // (the tensor maps over the operands know a whole broadcast, not one of the two batch axes alone)
-    for (const int64_t* st : {p.a_s, p.b_s}) {
-        const bool still0 = p.b0 > 1 && st[0] == 0, still1 = p.b1 > 1 && st[1] == 0;
-        if ((still0 && p.b1 > 1 && !still1) || (still1 && p.b0 > 1 && !still0)) return false;
-    }
     auto share = [&](const Operand& o) {
         const auto it = ctx->plane_uses.find(o.key);
         return it != ctx->plane_uses.end() && it->second >= 2 ? 0.5 : 1.0;
@@ -1725,7 +1730,7 @@ bool gemm_tc_reads_directly(const b200_ctx* ctx, const GemmProblem& p) {
     const Operand oa = plan_operand(p.a, p.a_s[0], p.a_s[1], p.a_s[2], p.a_s[3], p.m, p.k, a_bcast, p);
     const Operand ob = plan_operand(p.b, p.b_s[0], p.b_s[1], p.b_s[3], p.b_s[2], p.n, p.k, b_bcast, p);
     const bool want_dynamic = ctx->gemm_schedule == 1;
-    return oa.dense && ob.dense && !want_dynamic && (ctx->gemm_operands == 1 || direct_pays(ctx, p, batches, oa, ob));
+    return maps_describe(p, oa, ob) && !want_dynamic && (ctx->gemm_operands == 1 || direct_pays(ctx, p, batches, oa, ob));
 }
 
 void gemm_tc_wait_probe(b200_ctx* ctx, uint64_t limit_ns) {
@@ -1755,7 +1760,7 @@ void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass) {
 
     // ---- direct operands: no planes at all ----
     const bool want_dynamic = ctx->gemm_schedule == 1 || (ctx->gemm_schedule < 0 && ctx->in_grad_sync_span);
-    if (ctx->gemm_operands != 0 && oa.dense && ob.dense && !want_dynamic &&
+    if (ctx->gemm_operands != 0 && maps_describe(p, oa, ob) && !want_dynamic &&
         (ctx->gemm_operands == 1 || direct_pays(ctx, p, batches, oa, ob))) {
         float* partial = nullptr;
         if (splits > 1) {
