@@ -213,3 +213,28 @@ def test_tape_encoding_round_trips():
                     for k in ("bytes", "buf", "off"):
                         if k in e:
                             assert g[k] == e[k], (k, g, e)
+
+
+@pytest.mark.parametrize("n_src", range(_abi.MAX_SRC + 1))
+def test_packed_nodes_are_the_structures_field_by_field(n_src):
+    """`pack_nodes` gives the bytes of `NodeDesc.to_c`, also once a field has been assigned after a first packing."""
+    def both(nodes):
+        return bytes(graph.pack_nodes(nodes)), b"".join(bytes(n.to_c()) for n in nodes)
+
+    tensors = [TensorDesc.contiguous(4096 * (i + 1), (2, 3 + i)[:i % 3], DType.I64 if i == 1 else DType.F32) for i in range(_abi.MAX_SRC + 1)]
+    nodes = [NodeDesc(int(Op.ADD), tensors[-1], tensors[:n_src], b"\1\2\3"), NodeDesc(int(Op.RELU), tensors[0], [tensors[-1]])]
+    got, want = both(nodes)
+    assert got == want
+    tensors[0].dims, tensors[0].strides, tensors[0].data = (7, 1, 5), (20, 20, 4), 0
+    tensors[-1].dtype = DType.I32
+    again, want = both(nodes)
+    assert again == want and again != got
+
+
+def test_too_many_sources_are_refused():
+    t = TensorDesc.contiguous(4096, (4,), DType.F32)
+    nodes = [NodeDesc(int(Op.ADD), t, [t] * (_abi.MAX_SRC + 1)), NodeDesc(int(Op.RELU), t, [t])]
+    with pytest.raises(IndexError):
+        graph.pack_nodes(nodes)
+    with pytest.raises(IndexError):
+        nodes[0].to_c()

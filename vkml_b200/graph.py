@@ -202,6 +202,8 @@ def pack_nodes(nodes: Sequence[NodeDesc]):
     parts = []
     for n in nodes:
         src = n.src
+        if len(src) > _abi.MAX_SRC:
+            raise IndexError(f"{len(src)} sources exceed {_abi.MAX_SRC}")
         parts.append(_NODE_HEAD.pack(n.op, len(src)))
         parts.append(_tensor_bytes(n.out))
         for s in src:
