@@ -170,9 +170,12 @@ struct RowQuads {
     }
 };
 
-template <bool HEAD>
+// A row's sum of `picked`: the scale where the label is a class, and scale x 0 everywhere else -- nothing, or a NaN where the
+// scale is not finite.
 __device__ __forceinline__ float head_total(const LossArgs& a, float scale, float wanted) {
-    return wanted >= 0.0F && wanted < static_cast<float>(a.cols) ? scale : 0.0F;  // a row of `picked` holds one nonzero
+    const bool hit = wanted >= 0.0F && wanted < static_cast<float>(a.cols);
+    const float off = a.cols > (hit ? 1u : 0u) ? __fmul_rn(scale, 0.0F) : 0.0F;
+    return __fadd_rn(hit ? scale : 0.0F, off);
 }
 
 // A group of threads per row -- a warp up to 1024 classes, a block up to 4096 -- with the row's logits in registers.
@@ -222,7 +225,7 @@ __global__ void __launch_bounds__(256) loss_rows_kernel(LossArgs a) {
 #pragma unroll
             for (int i = 0; i < ITEMS * 4; ++i) denom += expf(v[i] - peak);
             lg = logf(group_sum<GROUP>(denom, red));
-            total = HEAD ? head_total<HEAD>(a, scale, wanted) : group_sum<GROUP>(sum, red);
+            total = HEAD ? head_total(a, scale, wanted) : group_sum<GROUP>(sum, red);
             if (lane == 0) a.total[r] = total;
         }
         if (q.edge < a.cols) {
@@ -324,7 +327,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) loss_long_kernel(LossArgs a, 
             denom += (expf(t[0] - peak) + expf(t[1] - peak)) + (expf(t[2] - peak) + expf(t[3] - peak));
         }
         const float lg = logf(group_sum<kLongThreads>(denom, red));
-        const float total = HEAD ? head_total<HEAD>(a, scale, wanted) : group_sum<kLongThreads>(sum, red);
+        const float total = HEAD ? head_total(a, scale, wanted) : group_sum<kLongThreads>(sum, red);
         if (tid == 0) a.total[r] = total;
         if (q.edge < a.cols) {
             loss_elements<HEAD, BACK, 1, true>(a, base + q.edge, q.edge, scale, wanted, ve, ge, peak, lg, total);
@@ -372,7 +375,7 @@ __global__ void __launch_bounds__(256) loss_any_kernel(LossArgs a) {
                 if (!HEAD) sum += a.g[base + c];
             }
             lg = logf(group_sum<256>(denom, red));
-            total = HEAD ? head_total<HEAD>(a, scale, wanted) : group_sum<256>(sum, red);
+            total = HEAD ? head_total(a, scale, wanted) : group_sum<256>(sum, red);
             if (threadIdx.x == 0) a.total[r] = total;
         }
 #pragma unroll 2
@@ -418,7 +421,7 @@ __global__ void __launch_bounds__(256) loss_tile_kernel(LossArgs a) {
             for (uint32_t c = 0; c < a.cols; ++c) peak = fmaxf(peak, x[c]);
             for (uint32_t c = 0; c < a.cols; ++c) denom += expf(x[c] - peak);
             if constexpr (HEAD) {
-                total = wanted >= 0.0F && wanted < static_cast<float>(a.cols) ? scale : 0.0F;
+                total = head_total(a, scale, wanted);
             } else {
                 for (uint32_t c = 0; c < a.cols; ++c) total += gs[t * a.cols + c];
             }
