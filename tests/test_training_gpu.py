@@ -263,12 +263,47 @@ def test_fused_groups_compute_what_the_separate_kernels_do(monkeypatch, name):
     fused, fused_labels = run(True)
     assert not any(l.startswith("fused.") for l in plain_labels)
     assert "fused.log_softmax_backward" in fused_labels, sorted(set(fused_labels))
-    # the one-hot mask of the loss: a kernel of its own, or part of the single-block chain that serves
-    # the whole prologue when its tensors are tiny
-    assert "fused.one_hot_mul" in fused_labels or "fused.tiny_chain" in fused_labels, sorted(set(fused_labels))
-    assert "fused.tiny_chain" in fused_labels and "fused.scaled_add_group" in fused_labels
+    # the loss's prologue, from its scalar fills to the one-hot mask and its product, is one launch
+    assert "fused.loss_head" in fused_labels and "fused.scaled_add_group" in fused_labels, sorted(set(fused_labels))
     # the bias / mask / relu group appears in whichever form the span holds it
     assert any(l in ("fused.bias_mask_relu", "fused.bias_mask", "fused.bias_relu", "fused.mask") for l in fused_labels)
     assert len(fused_labels) <= len(plain_labels) - 12 * steps, (len(fused_labels), len(plain_labels))
     assert np.all(np.isfinite(plain))
     np.testing.assert_allclose(fused, plain, rtol=1e-6, atol=0)
+
+
+def test_a_run_of_tiny_nodes_is_one_launch(monkeypatch):
+    """The single-block chain, on a run that is no loss's prologue: every node's bits those of its own kernel."""
+    import vkml_b200
+    from vkml_b200 import DeviceTensor, DType, NodeDesc, Op, graph
+    rng = np.random.default_rng(2)
+    x, k = rng.standard_normal((37, 11), dtype=np.float32), rng.integers(-3, 40, 37)
+    x[3, 4], x[5, 6], x[7] = np.inf, np.nan, -0.0
+
+    def run(fuse):
+        monkeypatch.setenv("VKML_B200_FUSE", fuse)
+        b = vkml_b200.Backend(0)
+        dx, dk, nodes, outs = DeviceTensor.from_host(b, x), DeviceTensor.from_host(b, k), [], []
+
+        def node(op, dims, srcs=(), params=b"", dtype=DType.F32):
+            outs.append(DeviceTensor.empty(b, dims, dtype))
+            nodes.append(NodeDesc(int(op), outs[-1].desc, [s.desc for s in srcs], params))
+            return outs[-1]
+
+        wide = node(Op.CAST, (37,), [dk]).reshape((37, 1)).broadcast_to((37, 11))
+        steps = node(Op.ARANGE, (11,), params=graph.arange_params(-0.5, 0.1)).broadcast_to((37, 11))
+        t = node(Op.NEG, (37, 11), [node(Op.MUL, (37, 11), [wide, dx])])
+        t = node(Op.DIV, (37, 11), [t, steps])
+        node(Op.CAST, (37, 11), [node(Op.EQUAL, (37, 11), [t, wide], dtype=DType.BOOL)])
+        node(Op.CONTIGUOUS, (11, 37), [t.transpose(0, 1)])
+        b.set_profiling(True)
+        b.compute(nodes)
+        labels = [l for l, _ in b.last_profile()]
+        b.set_profiling(False)
+        return [o.numpy().view(np.uint8) for o in outs], labels
+
+    plain, plain_labels = run("0")
+    fused, fused_labels = run("1")
+    assert fused_labels == ["fused.tiny_chain"] and len(plain_labels) == 8, (fused_labels, plain_labels)
+    for i, (got, want) in enumerate(zip(fused, plain)):
+        assert np.array_equal(got, want), i

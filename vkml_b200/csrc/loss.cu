@@ -805,8 +805,7 @@ size_t loss_group(b200_ctx* ctx, const b200_node* const* seq, size_t avail, bool
         n = head + back;
         if (n == 0 || !launch) return n;
         if (back > 0) a = both;
-        // (a head by itself, scalars and all, goes by the name of the single-block chain that it takes the place of)
-        ProfScope scope(ctx, back > 0 ? "fused.log_softmax_backward" : a.scalars[0] != nullptr ? "fused.tiny_chain" : "fused.loss_head");
+        ProfScope scope(ctx, back > 0 ? "fused.log_softmax_backward" : "fused.loss_head");
         if (head > 0 && back > 0) launch_rows<true, true>(ctx, a);
         else if (head > 0) launch_rows<true, false>(ctx, a);
         else launch_rows<false, true>(ctx, a);
