@@ -456,6 +456,24 @@ def test_which_kernel_a_product_gets(backend):
         assert "matmul." + want in labels, (want, labels)
 
 
+def test_which_kernel_a_product_gets_does_not_depend_on_the_span_before(backend):
+    """b200_matmul_kernel's answer is about the product by itself, also right after a span that compares its result or
+    holds other products."""
+    from vkml_b200 import DeviceTensor, NodeDesc
+    for lead, m, k, n in (((1, 1), 2048, 1024, 1536), ((1, 64), 512, 1024, 40)):  # half terms; operands read directly
+        a, b = DeviceTensor.empty(backend, lead + (m, k)), DeviceTensor.empty(backend, lead + (k, n))
+        out, other, act = (DeviceTensor.empty(backend, lead + (m, n)) for _ in range(3))
+        node = NodeDesc(Op.MATMUL, out.desc, [a.desc, b.desc])
+        before = backend.matmul_kernel(node)
+        backend.compute([node, NodeDesc(Op.MATMUL, other.desc, [a.desc, b.desc]), NodeDesc(Op.RELU, act.desc, [out.desc])])
+        assert backend.matmul_kernel(node) == before
+        backend.set_profiling(True)
+        backend.compute([node])
+        labels = [l for l, _ in backend.last_profile()]
+        backend.set_profiling(False)
+        assert "matmul." + before[0] in labels, (before, labels)
+
+
 def test_a_span_that_comes_back_is_replayed_as_a_graph_with_fresh_data(oracle, monkeypatch):
     """The same span on the same buffers, seven times with new input data each time: from the third
     submission on it is one CUDA graph launch, and every result is the one the eager path gives

@@ -2012,6 +2012,8 @@ void gemm_tc_end_span(b200_ctx* ctx) {
     ctx->plane_uses.clear();
     ctx->plane_cache_bytes = 0;
     ctx->range_next = 0;
+    ctx->lone_matmul = true;  // (what is asked about between two spans is a product by itself: b200_matmul_kernel)
+    ctx->compared.clear();
 }
 
 }  // namespace b200
