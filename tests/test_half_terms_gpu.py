@@ -93,6 +93,63 @@ def test_ranges(backend, kind):
     assert rows.max() < 2e-5, rows.max()
 
 
+@pytest.fixture(scope="module")
+def tf32_backend():
+    import os
+    import vkml_b200
+    os.environ["VKML_B200_GEMM_HALF_TERMS"] = "0"
+    b = vkml_b200.Backend(0)
+    del os.environ["VKML_B200_GEMM_HALF_TERMS"]
+    yield b
+    b.close()
+
+
+def same_bits(x, y):
+    return np.array_equal(np.ascontiguousarray(x).view(np.uint32), np.ascontiguousarray(y).view(np.uint32))
+
+
+# K-slices where half terms have some and where they have none; 256- and 128-wide tiles; batches, one operand broadcast; odd sizes
+@pytest.mark.parametrize("layout", ["nn", "nt", "tn"])
+@pytest.mark.parametrize("batch,m,k,n", [(1, 512, 16384, 512), (1, 2048, 1024, 2560), (1, 1301, 1333, 1277), (5, 700, 900, 1100), (1, 260, 5000, 2500)])
+def test_a_wide_operand_gets_the_tf32_product(backend, tf32_backend, batch, m, k, n, layout):
+    """One element far above the others: the result is bit for bit that of TF32 terms alone, with the same tiles and K-slices."""
+    rng = np.random.default_rng(batch + k)
+    a, b = rng.standard_normal((m, k), dtype=np.float32), rng.standard_normal((batch, k, n), dtype=np.float32)
+    plain, labels = product(backend, a, b, layout)
+    assert "matmul.tcgen05_3xf16" in labels
+    want, labels = product(tf32_backend, a, b, layout)
+    assert not any("f16" in l for l in labels) and not same_bits(plain, want)
+    for at in ("a", "b"):
+        wide_a, wide_b = a.copy(), b.copy()
+        if at == "a":
+            wide_a[m // 3, k // 2 + 1] = 3e7
+        else:
+            wide_b[batch // 2, k // 3, n - 1] = 3e7
+        got, labels = product(backend, wide_a, wide_b, layout)
+        want, _ = product(tf32_backend, wide_a, wide_b, layout)
+        assert "matmul.tcgen05_3xf16" in labels and same_bits(got, want), at
+
+
+def test_wide_operands_that_a_span_shares(backend, tf32_backend):
+    """A layer's two backward products on a gradient of wide range, and a third on the same activations and weight: planes that stand by
+    are written once and serve every product that needs them, a product of narrow operands none."""
+    rng = np.random.default_rng(8)
+    x, w, g = (rng.standard_normal(s, dtype=np.float32) for s in ((1536, 1024), (1024, 1280), (1536, 1280)))
+    g[:, 5] *= np.exp2(rng.integers(-40, 0, 1536)).astype(np.float32)
+    results = []
+    for b in (backend, tf32_backend):
+        def put(t):
+            return DeviceTensor.from_host(b, t.reshape((1, 1) + t.shape))
+        dx, dw, dg = put(x), put(w), put(g)
+        outs = [DeviceTensor.empty(b, (1, 1) + s) for s in ((1024, 1280), (1536, 1024), (1536, 1280), (1280, 1280))]
+        pairs = [(dx.transpose(2, 3), dg), (dg, dw.transpose(2, 3)), (dx, dw), (dg.transpose(2, 3), dg)]
+        b.compute([NodeDesc(int(Op.MATMUL), o.desc, [p.desc, q.desc]) for o, (p, q) in zip(outs, pairs)])
+        results.append([o.numpy() for o in outs])
+    got, want = results
+    assert [same_bits(p, q) for p, q in zip(got, want)] == [True, True, False, True]
+    assert rel(got[2], x, w) < 6e-6
+
+
 @pytest.mark.parametrize("layout", ["nn", "nt", "tn", "tt"])
 @pytest.mark.parametrize("m,k,n", [(256, 256, 256), (264, 520, 264), (104, 336, 776), (64, 4096, 512), (40, 1024, 1000)])
 def test_f16_storage_products(backend, m, k, n, layout):

@@ -84,7 +84,8 @@ struct PlaneEntry {
     int uses_left;
     const char* src_begin;
     const char* src_end;
-    void* range = nullptr;  // half planes: the matrix's RangeSlot
+    void* range = nullptr;  // half planes: the matrix's RangeSlot, and the TF32 planes that stand by for it
+    float* tf32 = nullptr;
 };
 
 // Ranges of the matrices that one span's half-term products split (gemm_h16.cu).

@@ -19,12 +19,15 @@ struct GemmProblem {
 };
 
 // The range of one operand matrix, found on the device (gemm_h16.cu): the bits of the largest magnitude in
-// a sample of it, how many nonzero elements are too small beside that for the half split, and whether one is too large.
-struct RangeSlot {
+// a sample of it, how many nonzero elements are too small beside that for the half split, whether one is too large, and
+// whether the TF32 planes that stand by for it have been written.
+struct __align__(16) RangeSlot {
     uint32_t max_bits;
     uint32_t strays;
     uint32_t spoiled;
     uint32_t unused;
+    uint32_t tf32;
+    uint32_t pad[3];
 };
 
 // Launches carrying a guard run only if one of the two matrices is wide (see gemm_h16.cu); a == null: always.
@@ -34,15 +37,26 @@ struct RangeGuard {
     uint32_t limit_a, limit_b;
 };
 
+// TF32 planes (hi, then lo) standing by for one operand of a half-term product; `done`: where it is noted that they have
+// been written, for an operand that several products of the span share (null: this product alone uses them).
+struct StandbyPlanes {
+    float* planes;
+    uint32_t* done;
+};
+
 // fp32 FMA on the CUDA cores; any strides, any size. gemm_simt.cu
 void gemm_simt(b200_ctx* ctx, const GemmProblem& p);
 
 // tcgen05 tensor-core path (3xTF32 or single-pass TF32). gemm_tc.cu
 bool gemm_tc_eligible(const b200_ctx* ctx, const GemmProblem& p);
 void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass);
-// The TF32 planes for the case that an operand turns out wide on the device: queued behind gemm_h16's kernel.
-void gemm_tc_if_wide(b200_ctx* ctx, const GemmProblem& p, const RangeGuard& guard, void* planes);
-size_t gemm_tc_plane_bytes(const GemmProblem& p);  // bytes that gemm_tc_if_wide wants at `planes`
+// The product from TF32 planes for the case that an operand turns out wide on the device, queued behind gemm_h16's kernel: the tiles
+// and K-slices that gemm_tc gives the product, so that its results are gemm_tc's bit for bit.  With slices the partial
+// planes are left at `partial` for the caller's fold.
+void gemm_tc_if_wide(b200_ctx* ctx, const GemmProblem& p, const RangeGuard& guard, const StandbyPlanes& a, const StandbyPlanes& b,
+                     float* partial);
+int gemm_tc_slices(const b200_ctx* ctx, const GemmProblem& p);
+size_t gemm_tc_plane_bytes(const GemmProblem& p, bool left);  // of one operand's two planes
 
 // tcgen05 kind::f16: F32 products from two half terms per operand, F16 products directly. gemm_h16.cu
 bool gemm_h16_serves(const b200_ctx* ctx, const GemmProblem& p);

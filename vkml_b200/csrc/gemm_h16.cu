@@ -123,8 +123,8 @@ __global__ void __launch_bounds__(256) range_kernel(MatrixPair pair) {
 
 __global__ void __launch_bounds__(kRangeSlots) clear_ranges_kernel(uint4* slots) {
     pdl_prologue();
-    static_assert(sizeof(RangeSlot) == sizeof(uint4), "one slot to a thread");
-    slots[threadIdx.x] = make_uint4(0, 0, 0, 0);
+    static_assert(sizeof(RangeSlot) == 2 * sizeof(uint4), "one slot to a thread");
+    slots[threadIdx.x] = slots[kRangeSlots + threadIdx.x] = make_uint4(0, 0, 0, 0);
 }
 
 // Writes each matrix's two half planes, [batch][row][pitch], in the orientation the matrix has in memory: 4 bytes read, 4 written per element.
@@ -620,12 +620,14 @@ gemm_h16_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_const
     }
 }
 
-// Sums the K-slices' partial planes in split order.
+// Sums the K-slices' partial planes in split order: `splits` of this product, or `wide_splits` from the TF32 planes that stood
+// by for a wide operand (one slice: the product went straight to `out`).
 template <typename Out>
 __global__ void __launch_bounds__(256) fold_kernel(Out* __restrict__ out, const float* __restrict__ part, int64_t n, int splits,
-                                                   H16Args g, int passes) {
+                                                   RangeGuard guard, int wide_splits) {
     pdl_prologue();
-    if (passes == 3 && (range_wide(g.range_a, g.limit_a) || range_wide(g.range_b, g.limit_b))) return;
+    if (guard.a != nullptr && !guard_idle(guard)) splits = wide_splits;
+    if (splits <= 1) return;
     const int64_t step = int64_t(gridDim.x) * blockDim.x;
     if (n % 4 == 0) {
         for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n / 4; i += step) {
@@ -692,6 +694,7 @@ struct HalfOperand {
     RangeSlot* range = nullptr;
     PlaneKey key{};
     bool cached = false, fresh = false;
+    StandbyPlanes standby{};
 
     int64_t numel() const { return nb * rows * cols; }
     size_t plane_bytes() const { return static_cast<size_t>(align_up(nb * rows * pitch * 2, 1024)); }
@@ -845,18 +848,17 @@ void run_h16(b200_ctx* ctx, const GemmProblem& p, int passes, const TileChoice& 
 #undef B200_H16_CASE
     }
     check_last_launch("matmul (tcgen05, half terms)");
-    if (t.splits > 1) {
-        ProfScope scope(ctx, "matmul.fold");
-        const int blocks = grid_for(ceil_div(out_elems, 4), 256);
-        if (out_half) {
-            launch_kernel(ctx, fold_kernel<__half>, blocks, 256, 0, reinterpret_cast<__half*>(p.out), partial, out_elems,
-                          static_cast<int>(t.splits), g, passes);
-        } else {
-            launch_kernel(ctx, fold_kernel<float>, blocks, 256, 0, p.out, partial, out_elems, static_cast<int>(t.splits), g, passes);
-        }
-        ctx->count_launch();
-        check_last_launch("matmul (fold)");
-    }
+}
+
+template <typename Out>
+void run_fold(b200_ctx* ctx, const GemmProblem& p, const float* partial, int splits, const RangeGuard& guard = {}, int wide_splits = 1) {
+    if (splits <= 1 && wide_splits <= 1) return;
+    ProfScope scope(ctx, "matmul.fold");
+    const int64_t out_elems = p.b0 * p.b1 * p.m * p.n;
+    launch_kernel(ctx, fold_kernel<Out>, grid_for(ceil_div(out_elems, 4), 256), 256, 0, reinterpret_cast<Out*>(p.out), partial, out_elems,
+                  splits, guard, wide_splits);
+    ctx->count_launch();
+    check_last_launch("matmul (fold)");
 }
 
 bool fits_tma(const GemmProblem& p) {
@@ -921,12 +923,13 @@ void gemm_h16(b200_ctx* ctx, const GemmProblem& p) {
         ctx->count_launch();
     }
     const size_t cache_limit = std::min<size_t>(size_t(16) << 30, ctx->prop.totalGlobalMem / 8);
-    auto place = [&](HalfOperand& o) {
+    auto place = [&](HalfOperand& o, size_t tf32_bytes) {
         lay_out_planes(o);
         if (auto it = ctx->plane_cache.find(o.key); it != ctx->plane_cache.end()) {
             o.hi = reinterpret_cast<const __half*>(it->second.hi);
             o.lo = reinterpret_cast<const __half*>(it->second.lo);
             o.range = static_cast<RangeSlot*>(it->second.range);
+            o.standby = {it->second.tf32, &o.range->tf32};
             o.cached = true;
             ++ctx->plane_hits;
             return;
@@ -934,40 +937,43 @@ void gemm_h16(b200_ctx* ctx, const GemmProblem& p) {
         o.fresh = true;
         o.range = static_cast<RangeSlot*>(ctx->d_ranges) + ctx->range_next++;
         const auto uses = ctx->plane_uses.find(o.key);
-        const size_t bytes = 2 * o.plane_bytes();
+        const size_t bytes = 2 * o.plane_bytes() + tf32_bytes;
         if (uses != ctx->plane_uses.end() && uses->second >= 2 && ctx->plane_cache_bytes + bytes <= cache_limit) {
             char* block = static_cast<char*>(ctx->scratch.allocate(bytes));
             o.hi = reinterpret_cast<const __half*>(block);
             o.lo = reinterpret_cast<const __half*>(block + o.plane_bytes());
+            o.standby = {reinterpret_cast<float*>(block + 2 * o.plane_bytes()), &o.range->tf32};
             const char* begin = static_cast<const char*>(o.src);
             auto mag = [](int64_t v) { return v < 0 ? -v : v; };
             const int64_t span = (o.nb / o.b1 - 1) * mag(o.s_b0) + (o.b1 - 1) * mag(o.s_b1) + (o.rows - 1) * mag(o.s_r) +
                                  (o.cols - 1) * mag(o.s_c) + 1;
             ctx->plane_cache[o.key] = PlaneEntry{reinterpret_cast<float*>(block), reinterpret_cast<float*>(block + o.plane_bytes()),
-                                                 bytes, uses->second, begin, begin + span * 4, o.range};
+                                                 bytes, uses->second, begin, begin + span * 4, o.range, o.standby.planes};
             ctx->plane_cache_bytes += bytes;
             o.cached = true;
         }
     };
-    place(a);
-    place(b);  // (B may be the very matrix A just put there)
+    const size_t a_tf32 = gemm_tc_plane_bytes(p, true), b_tf32 = gemm_tc_plane_bytes(p, false);
+    place(a, a_tf32);
+    place(b, b_tf32);  // (B may be the very matrix A just put there)
 
     const int64_t out_elems = p.b0 * p.b1 * p.m * p.n;
-    const size_t partial_bytes = t.splits > 1 ? static_cast<size_t>(align_up(out_elems * t.splits * 4, 1024)) : 0;
-    const size_t tf32_bytes = gemm_tc_plane_bytes(p);
-    size_t bytes = partial_bytes + tf32_bytes + 1024;
-    if (!a.cached) bytes += 2 * a.plane_bytes();
-    if (!b.cached) bytes += 2 * b.plane_bytes();
+    const int wide_splits = gemm_tc_slices(ctx, p);
+    const int64_t slices = std::max<int64_t>(t.splits, wide_splits);
+    const size_t partial_bytes = slices > 1 ? static_cast<size_t>(align_up(out_elems * slices * 4, 1024)) : 0;
+    size_t bytes = partial_bytes + 1024;
+    if (!a.cached) bytes += 2 * a.plane_bytes() + a_tf32;
+    if (!b.cached) bytes += 2 * b.plane_bytes() + b_tf32;
     char* ws = static_cast<char*>(ctx->ensure_workspace(bytes));
     ws = reinterpret_cast<char*>(align_up(reinterpret_cast<int64_t>(ws), 1024));
     for (HalfOperand* o : {&a, &b}) {
         if (o->cached) continue;
         o->hi = reinterpret_cast<const __half*>(ws);
         o->lo = reinterpret_cast<const __half*>(ws + o->plane_bytes());
-        ws += 2 * o->plane_bytes();
+        o->standby.planes = reinterpret_cast<float*>(ws + 2 * o->plane_bytes());
+        ws += 2 * o->plane_bytes() + (o == &a ? a_tf32 : b_tf32);
     }
     float* partial = reinterpret_cast<float*>(ws);
-    ws += partial_bytes;
 
     MatrixPair pair{};
     int fresh = 0;
@@ -991,7 +997,9 @@ void gemm_h16(b200_ctx* ctx, const GemmProblem& p) {
         check_last_launch("matmul (operand range and split)");
     }
     run_h16(ctx, p, 3, t, a, b, partial, false, "matmul.tcgen05_3xf16");
-    gemm_tc_if_wide(ctx, p, RangeGuard{a.range, b.range, a.limit(), b.limit()}, ws);
+    const RangeGuard guard{a.range, b.range, a.limit(), b.limit()};
+    gemm_tc_if_wide(ctx, p, guard, a.standby, b.standby, partial);
+    run_fold<float>(ctx, p, partial, static_cast<int>(t.splits), guard, wide_splits);
     for (HalfOperand* o : {&a, &b}) {
         if (!o->cached) continue;
         const auto it = ctx->plane_cache.find(o->key);
@@ -1040,6 +1048,7 @@ bool gemm_f16_storage(b200_ctx* ctx, const GemmProblem& p, const HalfEpilogue* e
     char* ws = static_cast<char*>(ctx->ensure_workspace(bytes));
     ws = reinterpret_cast<char*>(align_up(reinterpret_cast<int64_t>(ws), 1024));
     run_h16(ctx, p, 1, t, a, b, reinterpret_cast<float*>(ws), true, epi != nullptr ? "matmul.tcgen05_f16_bias" : "matmul.tcgen05_f16", epi);
+    run_fold<__half>(ctx, p, reinterpret_cast<const float*>(ws), static_cast<int>(t.splits));
     return true;
 }
 

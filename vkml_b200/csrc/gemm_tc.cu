@@ -277,12 +277,13 @@ __global__ void __launch_bounds__(256) split_kernel(SplitArgs a) {
 // to do, and then one launch of two blocks per SM costs less than two full ones.
 struct SplitPair {
     SplitArgs s[2];
+    const uint32_t* done[2];
     RangeGuard guard;
 };
 
 __global__ void __launch_bounds__(256) split_pair_kernel(SplitPair p) {
     pdl_prologue();
-    if (guard_idle(p.guard)) return;
+    if (guard_idle(p.guard) || (p.done[blockIdx.y] != nullptr && __ldcg(p.done[blockIdx.y]) != 0)) return;
     const SplitArgs& a = p.s[blockIdx.y];
     if (a.unit) split_rows(a);
     else split_tiles(a);
@@ -322,6 +323,7 @@ struct TcArgs {
     // or shares its SM with another kernel (an all-reduce) simply takes fewer tiles.
     unsigned int* sched;
     RangeGuard guard;
+    uint32_t* done[2];  // (guarded: set once the planes before this launch are known to be written)
 };
 
 // Direct-operand variant: TMA brings the fp32 operand tiles themselves into the `hi` slots of a
@@ -408,6 +410,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_consta
 
     const int64_t tiles_per_batch = g.tiles_m * g.tiles_n;
     const int64_t n_units = guard_idle(g.guard) ? 0 : tiles_per_batch * g.batches * g.splits;
+    if (n_units > 0 && blockIdx.x == 0 && threadIdx.x < 2 && g.done[threadIdx.x] != nullptr) *g.done[threadIdx.x] = 1;
 
     // unit -> (split, batch, m tile, n tile); M-tiles walked in groups of kGroupM
     auto decode = [&](int64_t u, int& split, int64_t& batch, int64_t& tm, int64_t& tn) {
@@ -1920,58 +1923,68 @@ void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass) {
     release_use(ctx, ob);
 }
 
-size_t gemm_tc_plane_bytes(const GemmProblem& p) {
-    const bool a_bcast = (p.a_s[0] == 0 || p.b0 == 1) && (p.a_s[1] == 0 || p.b1 == 1);
-    const bool b_bcast = (p.b_s[0] == 0 || p.b0 == 1) && (p.b_s[1] == 0 || p.b1 == 1);
-    return 2 * plan_operand(p.a, p.a_s[0], p.a_s[1], p.a_s[2], p.a_s[3], p.m, p.k, a_bcast, p).plane_bytes +
-           2 * plan_operand(p.b, p.b_s[0], p.b_s[1], p.b_s[3], p.b_s[2], p.n, p.k, b_bcast, p).plane_bytes;
+int gemm_tc_slices(const b200_ctx* ctx, const GemmProblem& p) { return static_cast<int>(plan_planes(ctx, p).splits); }
+
+size_t gemm_tc_plane_bytes(const GemmProblem& p, bool left) {
+    const int64_t* s = left ? p.a_s : p.b_s;
+    const bool bcast = (s[0] == 0 || p.b0 == 1) && (s[1] == 0 || p.b1 == 1);
+    return 2 * plan_operand(left ? p.a : p.b, s[0], s[1], left ? s[2] : s[3], left ? s[3] : s[2], left ? p.m : p.n, p.k, bcast, p).plane_bytes;
 }
 
-void gemm_tc_if_wide(b200_ctx* ctx, const GemmProblem& p, const RangeGuard& guard, void* planes) {
+void gemm_tc_if_wide(b200_ctx* ctx, const GemmProblem& p, const RangeGuard& guard, const StandbyPlanes& a, const StandbyPlanes& b,
+                     float* partial) {
     const bool a_bcast = (p.a_s[0] == 0 || p.b0 == 1) && (p.a_s[1] == 0 || p.b1 == 1);
     const bool b_bcast = (p.b_s[0] == 0 || p.b0 == 1) && (p.b_s[1] == 0 || p.b1 == 1);
+    const TcPlan plan = plan_planes(ctx, p);
     Operand oa = plan_operand(p.a, p.a_s[0], p.a_s[1], p.a_s[2], p.a_s[3], p.m, p.k, a_bcast, p);
     Operand ob = plan_operand(p.b, p.b_s[0], p.b_s[1], p.b_s[3], p.b_s[2], p.n, p.k, b_bcast, p);
-    char* ws = static_cast<char*>(planes);
     SplitPair pair{};
     pair.guard = guard;
-    int i = 0;
-    for (Operand* o : {&oa, &ob}) {
-        o->split.hi = o->hi = reinterpret_cast<float*>(ws);
-        o->split.lo = o->lo = reinterpret_cast<float*>(ws + o->plane_bytes);
-        ws += 2 * o->plane_bytes;
-        pair.s[i++] = o->split;
+    Operand* const operands[2] = {&oa, &ob};
+    const StandbyPlanes* const at[2] = {&a, &b};
+    for (int i = 0; i < 2; ++i) {
+        Operand& o = *operands[i];
+        o.split.hi = o.hi = at[i]->planes;
+        o.split.lo = o.lo = at[i]->planes + o.plane_bytes / sizeof(float);
+        pair.s[i] = o.split;
+        pair.done[i] = at[i]->done;
     }
     {
         ProfScope scope(ctx, "matmul.if_wide");
         launch_kernel(ctx, split_pair_kernel, dim3(ctx->prop.multiProcessorCount, 2), 256, 0, pair);
     }
     ctx->count_launch();
-    constexpr int bn = 128;
     auto map_of = [&](float* plane, const Operand& o, int tile) {
         return o.mn ? make_map(plane, o.nb * o.rows_pad, o.cols_pad, BK, true)
                     : make_map(plane, o.nb * o.rows_pad, o.cols_pad, tile, false);
     };
     TcArgs g{};
-    g.out = p.out;
+    g.batches = p.b0 * p.b1;
+    g.splits = static_cast<int>(plan.splits);
+    g.split_stride = g.batches * p.m * p.n;
+    g.out = plan.splits > 1 ? partial : p.out;
     g.m = p.m;
     g.n = p.n;
-    g.batches = p.b0 * p.b1;
     g.a_batch_rows = a_bcast ? 0 : oa.rows_pad;
     g.b_batch_rows = b_bcast ? 0 : ob.rows_pad;
-    g.k_blocks = ceil_div(p.k, BK);
-    g.kb_per_split = g.k_blocks;  // (no K-slices: what is queued here almost never runs)
-    g.splits = 1;
-    g.tiles_m = ceil_div(p.m, BM);
-    g.tiles_n = ceil_div(p.n, bn);
-    g.group_m = kGroupM;
+    g.k_blocks = plan.k_blocks;
+    g.kb_per_split = plan.kb_per_split;
+    g.tiles_m = plan.tiles_m;
+    g.tiles_n = plan.tiles_n;
+    g.group_m = ctx->gemm_group_m > 0 ? ctx->gemm_group_m : kGroupM;
     g.status = ctx->d_status;
     g.guard = guard;
-    const int grid = static_cast<int>(std::min<int64_t>(g.tiles_m * g.tiles_n * g.batches, ctx->prop.multiProcessorCount));
+    g.done[0] = a.done;
+    g.done[1] = b.done;
+    int sms = ctx->prop.multiProcessorCount;
+    if (ctx->in_grad_sync_span && ctx->comm_pending) sms = std::max(sms - ctx->comm_sms, sms / 2);
+    const int grid = static_cast<int>(std::min<int64_t>(plan.tiles_m * plan.tiles_n * g.batches * plan.splits, sms));
+    const CUtensorMap ah = map_of(oa.hi, oa, BM), al = map_of(oa.lo, oa, BM), bh = map_of(ob.hi, ob, plan.bn), bl = map_of(ob.lo, ob, plan.bn);
     {
         ProfScope scope(ctx, "matmul.if_wide");
-        launch_main<bn, 3>(ctx, true, oa.mn, ob.mn, map_of(oa.hi, oa, BM), map_of(oa.lo, oa, BM), map_of(ob.hi, ob, bn),
-                           map_of(ob.lo, ob, bn), g, grid);
+        if (plan.bn == 256) launch_main<256, 2>(ctx, true, oa.mn, ob.mn, ah, al, bh, bl, g, grid);
+        else if (plan.bn == 128) launch_main<128, 3>(ctx, true, oa.mn, ob.mn, ah, al, bh, bl, g, grid);
+        else launch_main<64, 4>(ctx, true, oa.mn, ob.mn, ah, al, bh, bl, g, grid);
     }
     ctx->count_launch();
     check_last_launch("matmul (TF32 planes of a wide operand)");
