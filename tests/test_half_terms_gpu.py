@@ -130,6 +130,16 @@ def test_a_wide_operand_gets_the_tf32_product(backend, tf32_backend, batch, m, k
         assert "matmul.tcgen05_3xf16" in labels and same_bits(got, want), at
 
 
+@pytest.mark.parametrize("row", range(600, 608))
+def test_small_elements_in_one_place(backend, tf32_backend, row):
+    """More small elements than a matrix may have, all inside one piece of the sample's raster: seen in the sample or only
+    by the split, the product is that of TF32 terms."""
+    rng = np.random.default_rng(row)
+    a, b = rng.standard_normal((2048, 2048), dtype=np.float32), rng.standard_normal((2048, 1024), dtype=np.float32)
+    a[row, :100] *= np.float32(1e-12)
+    assert same_bits(product(backend, a, b, "nn")[0], product(tf32_backend, a, b, "nn")[0])
+
+
 def test_wide_operands_that_a_span_shares(backend, tf32_backend):
     """A layer's two backward products on a gradient of wide range, and a third on the same activations and weight: planes that stand by
     are written once and serve every product that needs them, a product of narrow operands none."""

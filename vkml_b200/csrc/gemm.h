@@ -19,13 +19,13 @@ struct GemmProblem {
 };
 
 // The range of one operand matrix, found on the device (gemm_h16.cu): the bits of the largest magnitude in
-// a sample of it, how many nonzero elements are too small beside that for the half split, whether one is too large, and
-// whether the TF32 planes that stand by for it have been written.
+// a sample of it, how many nonzero elements are too small beside that for the half split, whether one is too large, how many
+// of the sample's own elements are too small, and whether the TF32 planes that stand by for it have been written.
 struct __align__(16) RangeSlot {
     uint32_t max_bits;
     uint32_t strays;
     uint32_t spoiled;
-    uint32_t unused;
+    uint32_t early;
     uint32_t tf32;
     uint32_t pad[3];
 };

@@ -20,7 +20,12 @@
 // ends.  A matrix that overflows, that holds an infinity or a NaN, or in which more than a few elements
 // lie below the lower end (kStrayFloor plus one in 2^21: N(0,1) data has one in 7e6) is WIDE, and a product
 // with a wide operand is computed by the TF32 planes queued behind this kernel instead (gemm_tc_if_wide;
-// its launches return at once otherwise).  No host synchronisation decides this.
+// its launches return at once otherwise).  No host synchronisation decides this.  The gradient of a classifier that has
+// learned something is wide -- probabilities of 1e-9 beside a label's 1 -- and shows it in the sample already: such a
+// matrix gets no half planes, nor does an operand that only its product would read, so that what is left over the TF32 product
+// is the range pass and two idle launches.  (8192x2048 . 2048x1000 on the gradient of logits of deviation 3: 229 us with TF32
+// terms alone, 431 with half planes split first and thrown away and a standby split of one small block per SM, 234 now;
+// x.W^T, g.W and x^T.g in one span 550, 765 and 532.  An outlier that the sample misses, 4096^3: 637, 800, 680.)
 #include "gemm.h"
 #include "tcgen05.cuh"
 
@@ -51,6 +56,9 @@ struct MatrixArgs {
     int64_t s_b0, s_b1, s_r, s_c;     // element strides
     int64_t rows, cols, pitch;        // pitch: halves per plane row (a multiple of 8)
     int vec;                          // rows start on 16 bytes and columns are dense
+    // The other operand, where its being wide makes this one's planes useless: no other product of the span reads them.
+    const RangeSlot* partner;
+    uint32_t partner_limit;
 };
 
 struct MatrixPair {
@@ -80,10 +88,10 @@ __device__ __forceinline__ void load8(const MatrixArgs& a, const float* row, int
 }
 
 // The largest magnitude in a sample of each matrix, as the bits of its absolute value (infinities and
-// NaNs included: they compare above every finite value).  Looking at all of both operands took 98 us at
-// 8192^3 and 53 us at 512 x 65536 x 512; one piece in `stride` takes a few.
+// NaNs included: they compare above every finite value), and how much of the sample is too small beside it.  Looking at all of both
+// operands took 98 us at 8192^3 and 53 us at 512 x 65536 x 512; one piece in `stride`, a group to a thread, takes a few.
 constexpr int kPiece = 16;  // consecutive groups of eight columns that are looked at together
-constexpr int64_t kSampleGroups = int64_t(1) << 17;
+constexpr int64_t kSampleGroups = int64_t(1) << 16;
 
 __device__ __forceinline__ int64_t row_number(int64_t i, int64_t per_row, int64_t total) {
     return total < (int64_t(1) << 31) ? int64_t(uint32_t(i) / uint32_t(per_row)) : i / per_row;
@@ -97,28 +105,35 @@ __global__ void __launch_bounds__(256) range_kernel(MatrixPair pair) {
     const uint32_t stride = static_cast<uint32_t>(max(int64_t(1), total / kSampleGroups));  // of the pieces, one in so many
     const uint32_t groups = static_cast<uint32_t>((total + stride - 1) / stride);           // (at most 2 * kSampleGroups)
     const bool small = total < (int64_t(1) << 31);
-    uint32_t top = 0;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < groups; j += gridDim.x * blockDim.x) {
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    float v[8] = {};
+    if (j < groups) {
         // (64-bit divisions for every group were most of this kernel's time on small matrices)
         const uint32_t piece = j / kPiece;
         // (a piece's place inside its stretch varies, so that no column pattern of the matrix is in step with it)
         const uint32_t shift = stride == 1 ? 0u : (piece * 7919u) % stride;
         const int64_t i = min(total - 1, (int64_t(piece) * stride + shift) * kPiece + j % kPiece);
         const int64_t rb = small ? int64_t(uint32_t(i) / uint32_t(per_row)) : i / per_row;
-        float v[8];
         int64_t r;
         load8(a, row_of(a, rb, r), (i - rb * per_row) * 8, v);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) top = max(top, __float_as_uint(v[q]) & 0x7FFFFFFFu);
     }
+    uint32_t top = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) top = max(top, __float_as_uint(v[q]) & 0x7FFFFFFFu);
     top = __reduce_max_sync(0xffffffffu, top);
     __shared__ uint32_t tops[8];
     if ((threadIdx.x & 31) == 0) tops[threadIdx.x >> 5] = top;
     __syncthreads();
-    if (threadIdx.x < 8) {
-        top = __reduce_max_sync(0xffu, tops[threadIdx.x]);
-        if (threadIdx.x == 0 && top != 0) atomicMax(&a.range->max_bits, top);
-    }
+#pragma unroll
+    for (int w = 0; w < 8; ++w) top = max(top, tops[w]);
+    if (threadIdx.x == 0 && top != 0) atomicMax(&a.range->max_bits, top);
+    // what is too small beside the largest of this block's share of the sample is too small beside the matrix' largest
+    const float low = __uint_as_float(top) * 0x1p-25F;
+    uint32_t early = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) early += fabsf(v[q]) < low && v[q] != 0.0F;
+    early = __reduce_add_sync(0xffffffffu, early);
+    if ((threadIdx.x & 31) == 0 && early != 0) atomicAdd(&a.range->early, early);
 }
 
 __global__ void __launch_bounds__(kRangeSlots) clear_ranges_kernel(uint4* slots) {
@@ -131,21 +146,33 @@ __global__ void __launch_bounds__(kRangeSlots) clear_ranges_kernel(uint4* slots)
 __global__ void __launch_bounds__(256) split_half_kernel(MatrixPair pair) {
     pdl_prologue();
     const MatrixArgs& a = pair.m[blockIdx.y];
-    const uint32_t top = __ldcg(&a.range->max_bits);
-    if (top >= 0x7F800000u) return;  // the planes will not be read
-    const int up = range_shift(top);
-    const float s1 = exp2_int(up / 2), s2 = exp2_int(up - up / 2);
     const int64_t per_row = a.pitch / 8;
     const int64_t total = per_row * a.rows * a.n_batches;
     const int64_t step = int64_t(gridDim.x) * blockDim.x;
+    int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, rb = 0, c = 0;
+    float v[8];
+    auto fetch = [&] {
+        int64_t r;
+        rb = row_number(i, per_row, total);
+        c = (i - rb * per_row) * 8;
+        load8(a, row_of(a, rb, r), c, v);
+    };
+    if (i < total) fetch();  // (before the range is known: the two latencies overlap)
+    __shared__ uint32_t largest;
+    bool unread = false;
+    if (threadIdx.x == 0) {
+        const uint4 s = __ldcg(reinterpret_cast<const uint4*>(a.range));
+        largest = s.x;
+        unread = s.x >= 0x7F800000u || s.w > kStrayFloor;
+    } else if (threadIdx.x == 1 && a.partner != nullptr) {
+        unread = range_wide(a.partner, a.partner_limit);  // (its strays may still be counted beside this: what is seen only grows)
+    }
+    if (__syncthreads_or(unread)) return;
+    const int up = range_shift(largest);
+    const float s1 = exp2_int(up / 2), s2 = exp2_int(up - up / 2);
     uint32_t strays = 0;
     bool over = false;
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += step) {
-        float v[8];
-        int64_t r;
-        const int64_t rb = row_number(i, per_row, total);
-        const int64_t c = (i - rb * per_row) * 8;
-        load8(a, row_of(a, rb, r), c, v);
+    while (i < total) {
         __half2 hi[4], lo[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -158,6 +185,8 @@ __global__ void __launch_bounds__(256) split_half_kernel(MatrixPair pair) {
         }
         *reinterpret_cast<uint4*>(a.hi + rb * a.pitch + c) = *reinterpret_cast<const uint4*>(hi);
         *reinterpret_cast<uint4*>(a.lo + rb * a.pitch + c) = *reinterpret_cast<const uint4*>(lo);
+        i += step;
+        if (i < total) fetch();
     }
     strays = __reduce_add_sync(0xffffffffu, strays);
     if ((threadIdx.x & 31) == 0 && strays != 0) atomicAdd(&a.range->strays, strays);
@@ -351,8 +380,11 @@ gemm_h16_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_const
     pdl_prologue();
 
     int64_t n_units = g.tiles_m * g.tiles_n * g.batches * g.splits;
-    if (PASSES == 3 && (range_wide(g.range_a, g.limit_a) || range_wide(g.range_b, g.limit_b))) {
-        n_units = 0;  // the TF32 planes behind this kernel serve the product
+    __shared__ int range_shifts[2];
+    if (PASSES == 3) {
+        if (threadIdx.x < 2) range_shifts[threadIdx.x] = range_shift(__ldcg(&(threadIdx.x == 0 ? g.range_a : g.range_b)->max_bits));
+        // (the TF32 planes behind this kernel serve a wide operand's product)
+        if (block_wide(RangeGuard{g.range_a, g.range_b, g.limit_a, g.limit_b})) n_units = 0;
     }
     const int64_t unit0 = blockIdx.x / CG, unit_step = gridDim.x / CG;
     auto decode = [&](int64_t u, int& split, int64_t& batch, int64_t& tm, int64_t& tn) {
@@ -461,7 +493,7 @@ gemm_h16_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_const
         const int quarter = warp & 3;
         float f1 = 1.0F, f2 = 1.0F, f3 = 1.0F;  // 2^-(shift_a + shift_b) in factors that stay in range
         if (PASSES == 3 && n_units > 0) {
-            const int e = -range_shift(__ldcg(&g.range_a->max_bits)) - range_shift(__ldcg(&g.range_b->max_bits));
+            const int e = -(range_shifts[0] + range_shifts[1]);
             const int e1 = max(-126, min(126, e));
             const int e2 = max(-126, min(126, e - e1));
             f1 = exp2_int(e1);
@@ -626,7 +658,7 @@ template <typename Out>
 __global__ void __launch_bounds__(256) fold_kernel(Out* __restrict__ out, const float* __restrict__ part, int64_t n, int splits,
                                                    RangeGuard guard, int wide_splits) {
     pdl_prologue();
-    if (guard.a != nullptr && !guard_idle(guard)) splits = wide_splits;
+    if (guard.a != nullptr && block_wide(guard)) splits = wide_splits;
     if (splits <= 1) return;
     const int64_t step = int64_t(gridDim.x) * blockDim.x;
     if (n % 4 == 0) {
@@ -980,14 +1012,20 @@ void gemm_h16(b200_ctx* ctx, const GemmProblem& p) {
     int64_t largest = 0;
     for (HalfOperand* o : {&a, &b}) {
         if (!o->fresh) continue;
-        pair.m[fresh++] = matrix_args(*o);
+        pair.m[fresh] = matrix_args(*o);
+        if (!o->cached) {
+            const HalfOperand& other = o == &a ? b : a;
+            pair.m[fresh].partner = other.range;
+            pair.m[fresh].partner_limit = other.limit();
+        }
+        ++fresh;
         largest = std::max(largest, o->nb * o->rows * (o->pitch / 8));
     }
     if (fresh > 0) {
         const dim3 grid(grid_for(largest, 256), static_cast<unsigned>(fresh));
         {
             ProfScope scope(ctx, "matmul.range");
-            launch_kernel(ctx, range_kernel, dim3(grid_for(std::min(largest, kSampleGroups), 256), grid.y), 256, 0, pair);
+            launch_kernel(ctx, range_kernel, dim3(static_cast<unsigned>(ceil_div(std::min(largest, 2 * kSampleGroups), 256)), grid.y), 256, 0, pair);
         }
         {
             ProfScope scope(ctx, "matmul.split");

@@ -211,8 +211,10 @@ __device__ __forceinline__ void split_rows(const SplitArgs& a) {
 // thread in flight in each phase.
 constexpr int kSplitTile = 64;
 
+template <int THREADS>
 __device__ __forceinline__ void split_tiles(const SplitArgs& a) {
     __shared__ float tile[kSplitTile][kSplitTile + 1];  // [row][k]
+    constexpr int kLines = THREADS / kSplitTile;  // of the tile per step
     const int fast = threadIdx.x & 63, slow = threadIdx.x >> 6;
     const int64_t tiles_k = a.kp / kSplitTile + (a.kp % kSplitTile != 0);
     const int64_t tiles_r = (a.rows + kSplitTile - 1) / kSplitTile;
@@ -227,31 +229,31 @@ __device__ __forceinline__ void split_tiles(const SplitArgs& a) {
         const bool full = r0 + kSplitTile <= a.rows && k0 + kSplitTile <= a.k;
         if (k_fast) {
             const float* p = src + (r0 + slow) * a.s_r + (k0 + fast) * a.s_k;
-            const int64_t step = 4 * a.s_r;
+            const int64_t step = kLines * a.s_r;
 #pragma unroll
-            for (int j = 0; j < kSplitTile / 4; ++j) {
-                const bool ok = full || (r0 + slow + 4 * j < a.rows && k0 + fast < a.k);
-                tile[slow + 4 * j][fast] = ok ? p[j * step] : 0.0F;
+            for (int j = 0; j < kSplitTile / kLines; ++j) {
+                const bool ok = full || (r0 + slow + kLines * j < a.rows && k0 + fast < a.k);
+                tile[slow + kLines * j][fast] = ok ? p[j * step] : 0.0F;
             }
         } else {
             const float* p = src + (r0 + fast) * a.s_r + (k0 + slow) * a.s_k;
-            const int64_t step = 4 * a.s_k;
+            const int64_t step = kLines * a.s_k;
 #pragma unroll
-            for (int j = 0; j < kSplitTile / 4; ++j) {
-                const bool ok = full || (r0 + fast < a.rows && k0 + slow + 4 * j < a.k);
-                tile[fast][slow + 4 * j] = ok ? p[j * step] : 0.0F;
+            for (int j = 0; j < kSplitTile / kLines; ++j) {
+                const bool ok = full || (r0 + fast < a.rows && k0 + slow + kLines * j < a.k);
+                tile[fast][slow + kLines * j] = ok ? p[j * step] : 0.0F;
             }
         }
         __syncthreads();
         if (k0 + fast < a.kp) {
             float* hi = a.hi + (b * a.rows + r0 + slow) * a.kp + k0 + fast;
             float* lo = a.lo != nullptr ? a.lo + (b * a.rows + r0 + slow) * a.kp + k0 + fast : nullptr;
-            const int64_t ostep = 4 * a.kp;
+            const int64_t ostep = kLines * a.kp;
 #pragma unroll
-            for (int j = 0; j < kSplitTile / 4; ++j) {
-                if (full || r0 + slow + 4 * j < a.rows) {
+            for (int j = 0; j < kSplitTile / kLines; ++j) {
+                if (full || r0 + slow + kLines * j < a.rows) {
                     float h, l;
-                    split_tf32(tile[slow + 4 * j][fast], h, l);
+                    split_tf32(tile[slow + kLines * j][fast], h, l);
                     hi[j * ostep] = h;
                     if (lo != nullptr) {
                         lo[j * ostep] = l;
@@ -270,23 +272,25 @@ __global__ void __launch_bounds__(256) split_rows_kernel(SplitArgs a) {
 
 __global__ void __launch_bounds__(256) split_kernel(SplitArgs a) {
     pdl_prologue();
-    split_tiles(a);
+    split_tiles<256>(a);
 }
 
-// Both operands of a product in one launch: the planes that stand by for a wide operand.  There is nearly always nothing
-// to do, and then one launch of two blocks per SM costs less than two full ones.
+// Both operands of a product in one launch: the planes that stand by for a wide operand.  There is nearly always nothing to do, and then
+// few large blocks cost least; where there is, they keep as many loads in flight as many small ones.
+constexpr int kPairThreads = 1024;
+
 struct SplitPair {
     SplitArgs s[2];
     const uint32_t* done[2];
     RangeGuard guard;
 };
 
-__global__ void __launch_bounds__(256) split_pair_kernel(SplitPair p) {
+__global__ void __launch_bounds__(kPairThreads) split_pair_kernel(SplitPair p) {
     pdl_prologue();
-    if (guard_idle(p.guard) || (p.done[blockIdx.y] != nullptr && __ldcg(p.done[blockIdx.y]) != 0)) return;
+    if (!block_wide(p.guard) || (p.done[blockIdx.y] != nullptr && __ldcg(p.done[blockIdx.y]) != 0)) return;
     const SplitArgs& a = p.s[blockIdx.y];
     if (a.unit) split_rows(a);
-    else split_tiles(a);
+    else split_tiles<kPairThreads>(a);
 }
 
 int64_t split_blocks(const SplitArgs& s) {
@@ -409,7 +413,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a_hi, const __grid_consta
     pdl_prologue();
 
     const int64_t tiles_per_batch = g.tiles_m * g.tiles_n;
-    const int64_t n_units = guard_idle(g.guard) ? 0 : tiles_per_batch * g.batches * g.splits;
+    const bool idle = g.guard.a != nullptr && !block_wide(g.guard);
+    const int64_t n_units = idle ? 0 : tiles_per_batch * g.batches * g.splits;
     if (n_units > 0 && blockIdx.x == 0 && threadIdx.x < 2 && g.done[threadIdx.x] != nullptr) *g.done[threadIdx.x] = 1;
 
     // unit -> (split, batch, m tile, n tile); M-tiles walked in groups of kGroupM
@@ -1951,7 +1956,7 @@ void gemm_tc_if_wide(b200_ctx* ctx, const GemmProblem& p, const RangeGuard& guar
     }
     {
         ProfScope scope(ctx, "matmul.if_wide");
-        launch_kernel(ctx, split_pair_kernel, dim3(ctx->prop.multiProcessorCount, 2), 256, 0, pair);
+        launch_kernel(ctx, split_pair_kernel, dim3(2 * ctx->prop.multiProcessorCount, 2), kPairThreads, 0, pair);
     }
     ctx->count_launch();
     auto map_of = [&](float* plane, const Operand& o, int tile) {

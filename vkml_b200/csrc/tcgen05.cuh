@@ -235,12 +235,13 @@ __device__ __forceinline__ int range_shift(uint32_t max_bits) {
 
 __device__ __forceinline__ bool range_wide(const RangeSlot* s, uint32_t limit) {
     const uint4 v = __ldcg(reinterpret_cast<const uint4*>(s));
-    return v.x >= 0x7F800000u || v.y > limit || v.z != 0;
+    return v.x >= 0x7F800000u || v.y > limit || v.z != 0 || v.w > kStrayFloor;
 }
 
-// Whether a guarded launch has nothing to do.
-__device__ __forceinline__ bool guard_idle(const RangeGuard& g) {
-    return g.a != nullptr && !range_wide(g.a, g.limit_a) && !range_wide(g.b, g.limit_b);
+// Whether one of the guard's matrices is wide; every thread of the block calls it.  Two of them ask: all warps of a large grid reading the
+// same few words took 4 to 6 us.
+__device__ __forceinline__ bool block_wide(const RangeGuard& g) {
+    return __syncthreads_or(threadIdx.x < 2 && range_wide(threadIdx.x == 0 ? g.a : g.b, threadIdx.x == 0 ? g.limit_a : g.limit_b)) != 0;
 }
 
 }  // namespace
