@@ -130,6 +130,27 @@ def test_a_wide_operand_gets_the_tf32_product(backend, tf32_backend, batch, m, k
         assert "matmul.tcgen05_3xf16" in labels and same_bits(got, want), at
 
 
+# K-slices and none; batches with one operand broadcast; odd sizes
+@pytest.mark.parametrize("layout", ["nn", "nt", "tn", "tt"])
+@pytest.mark.parametrize("batch,m,k,n", [(1, 1536, 1280, 1280), (1, 512, 16384, 512), (5, 700, 901, 1100), (1, 1301, 1333, 1277)])
+def test_strays_keep_their_share(backend, tf32_backend, batch, m, k, n, layout):
+    """A few elements far below the rest, alone in their rows and columns, beside others, at one K in both operands: every
+    element of the product is right beside the terms it is the sum of, from half terms."""
+    rng = np.random.default_rng(m + n)
+    a, b = rng.standard_normal((m, k), dtype=np.float32), rng.standard_normal((batch, k, n), dtype=np.float32)
+    a[5], a[6], a[m - 1] = 0, 0, 0
+    b[:, :, 9], b[batch - 1, :, n - 1] = 0, 0
+    tiny = np.float32(3.7e-9)
+    a[5, k - 1], a[6, 3], a[6, 100], a[m - 1, 0], a[20, 3], a[20, 4] = tiny, -tiny, 2 * tiny, tiny / 1024, tiny, 1e-30
+    b[:, 3, 9], b[:, 100, 9], b[batch - 1, k - 1, n - 1], b[0, 4, 33] = tiny, tiny, tiny, -tiny
+    got, labels = product(backend, a, b, layout)
+    assert "matmul.tcgen05_3xf16" in labels and not same_bits(got, product(tf32_backend, a, b, layout)[0])
+    got = got.reshape(batch, m, n).astype(np.float64)
+    a, b = a.astype(np.float64), b.astype(np.float64)
+    # (an accumulator of truncating additions is off by up to K / 16 of them; both operands keep 22 bits)
+    assert np.all(np.abs(got - a @ b) <= (k / 16 / 4 * 2.0 ** -23 + 2.0 ** -20) * (np.abs(a) @ np.abs(b)) + 1e-45)
+
+
 @pytest.mark.parametrize("row", range(600, 608))
 def test_small_elements_in_one_place(backend, tf32_backend, row):
     """More small elements than a matrix may have, all inside one piece of the sample's raster: seen in the sample or only

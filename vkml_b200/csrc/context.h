@@ -84,8 +84,9 @@ struct PlaneEntry {
     int uses_left;
     const char* src_begin;
     const char* src_end;
-    void* range = nullptr;  // half planes: the matrix's RangeSlot, and the TF32 planes that stand by for it
+    void* range = nullptr;  // half planes: the matrix's RangeSlot, the TF32 planes that stand by for it and the strays left out
     float* tf32 = nullptr;
+    int64_t* strays = nullptr;
 };
 
 // Ranges of the matrices that one span's half-term products split (gemm_h16.cu).

@@ -37,12 +37,15 @@ struct RangeGuard {
     uint32_t limit_a, limit_b;
 };
 
-// TF32 planes (hi, then lo) standing by for one operand of a half-term product; `done`: where it is noted that they have
-// been written, for an operand that several products of the span share (null: this product alone uses them).
-struct StandbyPlanes {
+// What stands by for one operand of a half-term product.  `planes`: its TF32 planes (hi, then lo); `done`: where it is noted that they have
+// been written, for an operand that several products of the span share (null: this product alone uses them).  `strays`: the
+// positions, in the order of the matrix in memory, of the elements that its half planes leave out.
+struct Standby {
     float* planes;
     uint32_t* done;
+    const int64_t* strays;
 };
+constexpr uint32_t kMaxStrays = 512;  // of one matrix; with more it is wide
 
 // fp32 FMA on the CUDA cores; any strides, any size. gemm_simt.cu
 void gemm_simt(b200_ctx* ctx, const GemmProblem& p);
@@ -50,11 +53,12 @@ void gemm_simt(b200_ctx* ctx, const GemmProblem& p);
 // tcgen05 tensor-core path (3xTF32 or single-pass TF32). gemm_tc.cu
 bool gemm_tc_eligible(const b200_ctx* ctx, const GemmProblem& p);
 void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass);
-// The product from TF32 planes for the case that an operand turns out wide on the device, queued behind gemm_h16's kernel: the tiles
+// What is queued behind gemm_h16's kernel.  Its strays' share of the product is added to `target`, the result or its first partial plane;
+// and for the case that an operand turns out wide on the device, the product from TF32 planes: the tiles
 // and K-slices that gemm_tc gives the product, so that its results are gemm_tc's bit for bit.  With slices the partial
 // planes are left at `partial` for the caller's fold.
-void gemm_tc_if_wide(b200_ctx* ctx, const GemmProblem& p, const RangeGuard& guard, const StandbyPlanes& a, const StandbyPlanes& b,
-                     float* partial);
+void gemm_tc_stand_by(b200_ctx* ctx, const GemmProblem& p, const RangeGuard& guard, const Standby& a, const Standby& b, float* target,
+                      float* partial);
 int gemm_tc_slices(const b200_ctx* ctx, const GemmProblem& p);
 size_t gemm_tc_plane_bytes(const GemmProblem& p, bool left);  // of one operand's two planes
 

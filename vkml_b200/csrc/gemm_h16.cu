@@ -15,11 +15,12 @@
 //
 // Half has five exponent bits, so s has to suit the matrix.  A first pass looks for the largest magnitude
 // in a sample -- 128-element pieces spread over the whole matrix, all of it where it is small -- and s puts
-// that into [2^11, 2^12): room for elements sixteen times larger, and all 22 bits for elements down to
-// 2^-24 of it (below, an absolute error of at most 2^-36/s).  The split checks every element against both
-// ends.  A matrix that overflows, that holds an infinity or a NaN, or in which more than a few elements
-// lie below the lower end (kStrayFloor plus one in 2^21: N(0,1) data has one in 7e6) is WIDE, and a product
-// with a wide operand is computed by the TF32 planes queued behind this kernel instead (gemm_tc_if_wide;
+// that into [2^13, 2^14): room for elements four times larger, and all 22 bits for elements down to
+// 2^-26 of it.  The split checks every element against both ends.  The few that lie below the lower end, STRAYS (N(0,1) data has
+// one in 3e7), are left out of the planes and noted, and their share of the product is added in fp32 behind this kernel (add_strays,
+// gemm_tc.cu; 3 to 8 us where there are any): wherever they stand, each term keeps 22 bits, as with TF32 terms.  A matrix that overflows,
+// that holds an infinity or a NaN, or that has more strays than kStrayFloor plus one in 2^21, is WIDE, and a product
+// with a wide operand is computed by the TF32 planes queued behind this kernel instead (gemm_tc_stand_by;
 // its launches return at once otherwise).  No host synchronisation decides this.  The gradient of a classifier that has
 // learned something is wide -- probabilities of 1e-9 beside a label's 1 -- and shows it in the sample already: such a
 // matrix gets no half planes, nor does an operand that only its product would read, so that what is left over the TF32 product
@@ -59,6 +60,8 @@ struct MatrixArgs {
     // The other operand, where its being wide makes this one's planes useless: no other product of the span reads them.
     const RangeSlot* partner;
     uint32_t partner_limit;
+    int64_t* strays;                  // positions of the elements left out, the first `limit` of them
+    uint32_t limit;
 };
 
 struct MatrixPair {
@@ -128,7 +131,7 @@ __global__ void __launch_bounds__(256) range_kernel(MatrixPair pair) {
     for (int w = 0; w < 8; ++w) top = max(top, tops[w]);
     if (threadIdx.x == 0 && top != 0) atomicMax(&a.range->max_bits, top);
     // what is too small beside the largest of this block's share of the sample is too small beside the matrix' largest
-    const float low = __uint_as_float(top) * 0x1p-25F;
+    const float low = __uint_as_float(top) * 0x1p-27F;
     uint32_t early = 0;
 #pragma unroll
     for (int q = 0; q < 8; ++q) early += fabsf(v[q]) < low && v[q] != 0.0F;
@@ -170,14 +173,17 @@ __global__ void __launch_bounds__(256) split_half_kernel(MatrixPair pair) {
     if (__syncthreads_or(unread)) return;
     const int up = range_shift(largest);
     const float s1 = exp2_int(up / 2), s2 = exp2_int(up - up / 2);
-    uint32_t strays = 0;
     bool over = false;
     while (i < total) {
         __half2 hi[4], lo[4];
+        uint32_t few = 0;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const float x = v[2 * j] * s1 * s2, y = v[2 * j + 1] * s1 * s2;  // exact: powers of two
-            strays += (fabsf(x) < kStrayBelow && v[2 * j] != 0.0F) + (fabsf(y) < kStrayBelow && v[2 * j + 1] != 0.0F);
+            float x = v[2 * j] * s1 * s2, y = v[2 * j + 1] * s1 * s2;  // exact: powers of two
+            const bool stray_x = fabsf(x) < kStrayBelow && v[2 * j] != 0.0F, stray_y = fabsf(y) < kStrayBelow && v[2 * j + 1] != 0.0F;
+            few |= (stray_x ? 1u : 0u) << (2 * j) | (stray_y ? 2u : 0u) << (2 * j);
+            x = stray_x ? 0.0F : x;
+            y = stray_y ? 0.0F : y;
             over = over || !(fmaxf(fabsf(x), fabsf(y)) < 65504.0F) || x != x || y != y;
             hi[j] = __floats2half2_rn(x, y);
             const float2 h = __half22float2(hi[j]);
@@ -185,11 +191,13 @@ __global__ void __launch_bounds__(256) split_half_kernel(MatrixPair pair) {
         }
         *reinterpret_cast<uint4*>(a.hi + rb * a.pitch + c) = *reinterpret_cast<const uint4*>(hi);
         *reinterpret_cast<uint4*>(a.lo + rb * a.pitch + c) = *reinterpret_cast<const uint4*>(lo);
+        if (few != 0) {
+            uint32_t at = atomicAdd(&a.range->strays, static_cast<uint32_t>(__popc(few)));
+            for (; few != 0 && at < a.limit; few &= few - 1) a.strays[at++] = rb * a.cols + c + (__ffs(few) - 1);
+        }
         i += step;
         if (i < total) fetch();
     }
-    strays = __reduce_add_sync(0xffffffffu, strays);
-    if ((threadIdx.x & 31) == 0 && strays != 0) atomicAdd(&a.range->strays, strays);
     if (over) a.range->spoiled = 1;
 }
 
@@ -726,11 +734,12 @@ struct HalfOperand {
     RangeSlot* range = nullptr;
     PlaneKey key{};
     bool cached = false, fresh = false;
-    StandbyPlanes standby{};
+    Standby standby{};
 
     int64_t numel() const { return nb * rows * cols; }
     size_t plane_bytes() const { return static_cast<size_t>(align_up(nb * rows * pitch * 2, 1024)); }
-    uint32_t limit() const { return kStrayFloor + static_cast<uint32_t>(std::min<int64_t>(numel() >> 21, 1 << 30)); }
+    uint32_t limit() const { return std::min(kMaxStrays, kStrayFloor + static_cast<uint32_t>(std::min<int64_t>(numel() >> 21, kMaxStrays))); }
+    size_t stray_bytes() const { return static_cast<size_t>(align_up(int64_t(limit()) * 8, 1024)); }
     CUtensorMap map(const __half* plane, int tile) const {
         return half_map(plane, cols, rows, pitch, map_b1, map_s_b1, map_b0, map_s_b0, mn ? kBlockK : tile);
     }
@@ -961,7 +970,7 @@ void gemm_h16(b200_ctx* ctx, const GemmProblem& p) {
             o.hi = reinterpret_cast<const __half*>(it->second.hi);
             o.lo = reinterpret_cast<const __half*>(it->second.lo);
             o.range = static_cast<RangeSlot*>(it->second.range);
-            o.standby = {it->second.tf32, &o.range->tf32};
+            o.standby = {it->second.tf32, &o.range->tf32, it->second.strays};
             o.cached = true;
             ++ctx->plane_hits;
             return;
@@ -969,18 +978,19 @@ void gemm_h16(b200_ctx* ctx, const GemmProblem& p) {
         o.fresh = true;
         o.range = static_cast<RangeSlot*>(ctx->d_ranges) + ctx->range_next++;
         const auto uses = ctx->plane_uses.find(o.key);
-        const size_t bytes = 2 * o.plane_bytes() + tf32_bytes;
+        const size_t bytes = 2 * o.plane_bytes() + tf32_bytes + o.stray_bytes();
         if (uses != ctx->plane_uses.end() && uses->second >= 2 && ctx->plane_cache_bytes + bytes <= cache_limit) {
             char* block = static_cast<char*>(ctx->scratch.allocate(bytes));
             o.hi = reinterpret_cast<const __half*>(block);
             o.lo = reinterpret_cast<const __half*>(block + o.plane_bytes());
-            o.standby = {reinterpret_cast<float*>(block + 2 * o.plane_bytes()), &o.range->tf32};
+            int64_t* strays = reinterpret_cast<int64_t*>(block + 2 * o.plane_bytes() + tf32_bytes);
+            o.standby = {reinterpret_cast<float*>(block + 2 * o.plane_bytes()), &o.range->tf32, strays};
             const char* begin = static_cast<const char*>(o.src);
             auto mag = [](int64_t v) { return v < 0 ? -v : v; };
             const int64_t span = (o.nb / o.b1 - 1) * mag(o.s_b0) + (o.b1 - 1) * mag(o.s_b1) + (o.rows - 1) * mag(o.s_r) +
                                  (o.cols - 1) * mag(o.s_c) + 1;
             ctx->plane_cache[o.key] = PlaneEntry{reinterpret_cast<float*>(block), reinterpret_cast<float*>(block + o.plane_bytes()),
-                                                 bytes, uses->second, begin, begin + span * 4, o.range, o.standby.planes};
+                                                 bytes, uses->second, begin, begin + span * 4, o.range, o.standby.planes, strays};
             ctx->plane_cache_bytes += bytes;
             o.cached = true;
         }
@@ -994,8 +1004,8 @@ void gemm_h16(b200_ctx* ctx, const GemmProblem& p) {
     const int64_t slices = std::max<int64_t>(t.splits, wide_splits);
     const size_t partial_bytes = slices > 1 ? static_cast<size_t>(align_up(out_elems * slices * 4, 1024)) : 0;
     size_t bytes = partial_bytes + 1024;
-    if (!a.cached) bytes += 2 * a.plane_bytes() + a_tf32;
-    if (!b.cached) bytes += 2 * b.plane_bytes() + b_tf32;
+    if (!a.cached) bytes += 2 * a.plane_bytes() + a_tf32 + a.stray_bytes();
+    if (!b.cached) bytes += 2 * b.plane_bytes() + b_tf32 + b.stray_bytes();
     char* ws = static_cast<char*>(ctx->ensure_workspace(bytes));
     ws = reinterpret_cast<char*>(align_up(reinterpret_cast<int64_t>(ws), 1024));
     for (HalfOperand* o : {&a, &b}) {
@@ -1004,6 +1014,8 @@ void gemm_h16(b200_ctx* ctx, const GemmProblem& p) {
         o->lo = reinterpret_cast<const __half*>(ws + o->plane_bytes());
         o->standby.planes = reinterpret_cast<float*>(ws + 2 * o->plane_bytes());
         ws += 2 * o->plane_bytes() + (o == &a ? a_tf32 : b_tf32);
+        o->standby.strays = reinterpret_cast<int64_t*>(ws);
+        ws += o->stray_bytes();
     }
     float* partial = reinterpret_cast<float*>(ws);
 
@@ -1013,6 +1025,8 @@ void gemm_h16(b200_ctx* ctx, const GemmProblem& p) {
     for (HalfOperand* o : {&a, &b}) {
         if (!o->fresh) continue;
         pair.m[fresh] = matrix_args(*o);
+        pair.m[fresh].strays = const_cast<int64_t*>(o->standby.strays);
+        pair.m[fresh].limit = o->limit();
         if (!o->cached) {
             const HalfOperand& other = o == &a ? b : a;
             pair.m[fresh].partner = other.range;
@@ -1036,7 +1050,7 @@ void gemm_h16(b200_ctx* ctx, const GemmProblem& p) {
     }
     run_h16(ctx, p, 3, t, a, b, partial, false, "matmul.tcgen05_3xf16");
     const RangeGuard guard{a.range, b.range, a.limit(), b.limit()};
-    gemm_tc_if_wide(ctx, p, guard, a.standby, b.standby, partial);
+    gemm_tc_stand_by(ctx, p, guard, a.standby, b.standby, t.splits > 1 ? partial : p.out, partial);
     run_fold<float>(ctx, p, partial, static_cast<int>(t.splits), guard, wide_splits);
     for (HalfOperand* o : {&a, &b}) {
         if (!o->cached) continue;

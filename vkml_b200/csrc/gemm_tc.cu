@@ -212,8 +212,7 @@ __device__ __forceinline__ void split_rows(const SplitArgs& a) {
 constexpr int kSplitTile = 64;
 
 template <int THREADS>
-__device__ __forceinline__ void split_tiles(const SplitArgs& a) {
-    __shared__ float tile[kSplitTile][kSplitTile + 1];  // [row][k]
+__device__ __forceinline__ void split_tiles(const SplitArgs& a, float (&tile)[kSplitTile][kSplitTile + 1]) {  // tile: [row][k]
     constexpr int kLines = THREADS / kSplitTile;  // of the tile per step
     const int fast = threadIdx.x & 63, slow = threadIdx.x >> 6;
     const int64_t tiles_k = a.kp / kSplitTile + (a.kp % kSplitTile != 0);
@@ -272,25 +271,130 @@ __global__ void __launch_bounds__(256) split_rows_kernel(SplitArgs a) {
 
 __global__ void __launch_bounds__(256) split_kernel(SplitArgs a) {
     pdl_prologue();
-    split_tiles<256>(a);
+    __shared__ float tile[kSplitTile][kSplitTile + 1];
+    split_tiles<256>(a, tile);
 }
 
-// Both operands of a product in one launch: the planes that stand by for a wide operand.  There is nearly always nothing to do, and then
-// few large blocks cost least; where there is, they keep as many loads in flight as many small ones.
+// Behind a half-term product, in one launch: its operands' strays, or the planes of both for a wide one.  There is mostly little or nothing
+// to do, and then few large blocks cost least; for planes they keep as many loads in flight as many small ones.
 constexpr int kPairThreads = 1024;
 
 struct SplitPair {
     SplitArgs s[2];
     const uint32_t* done[2];
     RangeGuard guard;
+    // the narrow case: strays of both operands
+    GemmProblem p;
+    const int64_t* strays[2];
+    int mn[2];      // the matrix in memory has K rows
+    int bcast[2];   // one matrix for every batch
+    float* target;
 };
 
-__global__ void __launch_bounds__(kPairThreads) split_pair_kernel(SplitPair p) {
+// The elements that the half planes leave out (gemm_h16.cu), a few dozen in a large matrix: a row of the product gets the share of its strays
+// in A, a column that of its strays in B, in fp32.  Every element of the product is added to by one thread, in the
+// order of K: a row with strays takes along what its columns have, and columns leave such rows out.  A block's unit of work is 1024
+// elements of one line, so the handful of strays that two N(0,1) matrices of 8192^2 have is one round of the grid.
+struct Stray {
+    int batch, line, k;  // line: the row of A, the column of B
+};
+
+struct StrayLists {
+    Stray at[2][kMaxStrays];
+    int64_t raw[2][kMaxStrays];
+};
+static_assert(kPairThreads == 2 * kMaxStrays, "a thread to a stray");
+
+__device__ __forceinline__ int64_t quotient(int64_t a, int64_t b) {
+    return ((a | b) >> 32) != 0 ? a / b : int64_t(uint32_t(a) / uint32_t(b));
+}
+
+__device__ void add_strays(const SplitPair& w, StrayLists& lists, const uint32_t (&counts)[2]) {
+    const GemmProblem& p = w.p;
+    const int64_t batches = p.b0 * p.b1;
+    const uint32_t tid = threadIdx.x;
+    {
+        // both lists into the order of the matrix in memory, in which K ascends along a line: half of the block each
+        const int o = tid < kMaxStrays ? 0 : 1;
+        const uint32_t i = tid - o * kMaxStrays, n = counts[o];
+        const int64_t at = i < n ? w.strays[o][i] : 0;
+        if (i < n) lists.raw[o][i] = at;
+        const int64_t rows = w.s[o].rows, cols = w.s[o].k, rb = quotient(at, cols), c = at - rb * cols;
+        const int64_t b = w.s[o].n_batches == 1 ? 0 : quotient(rb, rows), r = rb - b * rows;
+        __syncthreads();
+        if (i < n) {
+            uint32_t rank = 0;
+#pragma unroll 1
+            for (uint32_t j = 0; j < n; ++j) rank += lists.raw[o][j] < at;
+            lists.at[o][rank] = Stray{static_cast<int>(b), static_cast<int>(w.mn[o] ? c : r), static_cast<int>(w.mn[o] ? r : c)};
+        }
+        __syncthreads();
+    }
+    const int64_t extent[2] = {p.n, p.m};  // along a line of the product with strays in A, in B
+    int64_t tasks[2], chunks[2];
+    for (int o = 0; o < 2; ++o) {
+        chunks[o] = (extent[o] + kPairThreads - 1) / kPairThreads;
+        tasks[o] = chunks[o] * counts[o] * (w.bcast[o] ? batches : 1);
+    }
+#pragma unroll 1
+    for (int64_t t = blockIdx.y * gridDim.x + blockIdx.x; t < tasks[0] + tasks[1]; t += gridDim.x * gridDim.y) {
+        const int o = t < tasks[0] ? 0 : 1;
+        const int64_t in = o == 0 ? t : t - tasks[0], u = quotient(in, chunks[o]), pos = (in - u * chunks[o]) * kPairThreads + tid;
+        const int64_t repeat = quotient(u, counts[o]);
+        const uint32_t e = static_cast<uint32_t>(u - repeat * counts[o]);
+        const Stray s = lists.at[o][e];
+        // the first stray of a line serves the line
+        if (__syncthreads_or(tid < e && lists.at[o][tid].line == s.line && lists.at[o][tid].batch == s.batch)) continue;
+        if (pos >= extent[o]) continue;
+        const int64_t b = w.bcast[o] ? repeat : s.batch, bo = batches == 1 ? 0 : quotient(b, p.b1), bi = b - bo * p.b1;
+        const int64_t m = o == 0 ? s.line : pos, n = o == 0 ? pos : s.line;
+        const float* a_row = p.a + bo * p.a_s[0] + bi * p.a_s[1] + m * p.a_s[2];
+        const float* b_col = p.b + bo * p.b_s[0] + bi * p.b_s[1] + n * p.b_s[3];
+        const int a_batch = w.bcast[0] ? 0 : static_cast<int>(b), b_batch = w.bcast[1] ? 0 : static_cast<int>(b);
+        auto in_a = [&](int k) {  // whether A has a stray in row m, at k (k < 0: anywhere)
+#pragma unroll 1
+            for (uint32_t i = 0; i < counts[0]; ++i) {
+                const Stray& q = lists.at[0][i];
+                if (q.line == m && q.batch == a_batch && (k < 0 || q.k == k)) return true;
+            }
+            return false;
+        };
+        if (o == 1 && in_a(-1)) continue;
+        float* to = w.target + (b * p.m + m) * p.n + n;
+        float sum = *to;
+        auto term = [&](int k) { sum = fmaf(__ldg(a_row + k * p.a_s[3]), __ldg(b_col + k * p.b_s[2]), sum); };
+        if (o == 0) {
+#pragma unroll 1
+            for (uint32_t i = e; i < counts[0]; ++i) {
+                if (lists.at[0][i].line == m && lists.at[0][i].batch == a_batch) term(lists.at[0][i].k);
+            }
+        }
+#pragma unroll 1
+        for (uint32_t i = 0; i < counts[1]; ++i) {
+            const Stray& q = lists.at[1][i];
+            if (q.line == n && q.batch == b_batch && (o == 1 || !in_a(q.k))) term(q.k);
+        }
+        *to = sum;
+    }
+}
+
+__global__ void __launch_bounds__(kPairThreads, 2) split_pair_kernel(const __grid_constant__ SplitPair p) {
     pdl_prologue();
-    if (!block_wide(p.guard) || (p.done[blockIdx.y] != nullptr && __ldcg(p.done[blockIdx.y]) != 0)) return;
+    __shared__ union {
+        StrayLists lists;
+        float tile[kSplitTile][kSplitTile + 1];
+    } sm;
+    __shared__ uint32_t counted[2];
+    if (threadIdx.x < 2) counted[threadIdx.x] = __ldcg(&(threadIdx.x == 0 ? p.guard.a : p.guard.b)->strays);
+    if (!block_wide(p.guard)) {
+        const uint32_t counts[2] = {counted[0], counted[1]};
+        if (counts[0] + counts[1] != 0) add_strays(p, sm.lists, counts);
+        return;
+    }
+    if (p.done[blockIdx.y] != nullptr && __ldcg(p.done[blockIdx.y]) != 0) return;
     const SplitArgs& a = p.s[blockIdx.y];
     if (a.unit) split_rows(a);
-    else split_tiles<kPairThreads>(a);
+    else split_tiles<kPairThreads>(a, sm.tile);
 }
 
 int64_t split_blocks(const SplitArgs& s) {
@@ -1936,8 +2040,8 @@ size_t gemm_tc_plane_bytes(const GemmProblem& p, bool left) {
     return 2 * plan_operand(left ? p.a : p.b, s[0], s[1], left ? s[2] : s[3], left ? s[3] : s[2], left ? p.m : p.n, p.k, bcast, p).plane_bytes;
 }
 
-void gemm_tc_if_wide(b200_ctx* ctx, const GemmProblem& p, const RangeGuard& guard, const StandbyPlanes& a, const StandbyPlanes& b,
-                     float* partial) {
+void gemm_tc_stand_by(b200_ctx* ctx, const GemmProblem& p, const RangeGuard& guard, const Standby& a, const Standby& b, float* target,
+                      float* partial) {
     const bool a_bcast = (p.a_s[0] == 0 || p.b0 == 1) && (p.a_s[1] == 0 || p.b1 == 1);
     const bool b_bcast = (p.b_s[0] == 0 || p.b0 == 1) && (p.b_s[1] == 0 || p.b1 == 1);
     const TcPlan plan = plan_planes(ctx, p);
@@ -1945,14 +2049,20 @@ void gemm_tc_if_wide(b200_ctx* ctx, const GemmProblem& p, const RangeGuard& guar
     Operand ob = plan_operand(p.b, p.b_s[0], p.b_s[1], p.b_s[3], p.b_s[2], p.n, p.k, b_bcast, p);
     SplitPair pair{};
     pair.guard = guard;
+    pair.p = p;
+    pair.target = target;
+    pair.bcast[0] = a_bcast ? 1 : 0;
+    pair.bcast[1] = b_bcast ? 1 : 0;
     Operand* const operands[2] = {&oa, &ob};
-    const StandbyPlanes* const at[2] = {&a, &b};
+    const Standby* const at[2] = {&a, &b};
     for (int i = 0; i < 2; ++i) {
         Operand& o = *operands[i];
         o.split.hi = o.hi = at[i]->planes;
         o.split.lo = o.lo = at[i]->planes + o.plane_bytes / sizeof(float);
         pair.s[i] = o.split;
         pair.done[i] = at[i]->done;
+        pair.strays[i] = at[i]->strays;
+        pair.mn[i] = o.mn ? 1 : 0;
     }
     {
         ProfScope scope(ctx, "matmul.if_wide");

@@ -226,11 +226,11 @@ constexpr uint32_t kStrayFloor = 32;      // as many such elements as any matrix
 // 2^e for -126 <= e <= 127
 __device__ __forceinline__ float exp2_int(int e) { return __uint_as_float(static_cast<uint32_t>(e + 127) << 23); }
 
-// The power of two that takes the largest magnitude of a matrix's sample (its bits, finite) into [2^11, 2^12).
+// The power of two that takes the largest magnitude of a matrix's sample (its bits, finite) into [2^13, 2^14).
 __device__ __forceinline__ int range_shift(uint32_t max_bits) {
     if (max_bits == 0) return 0;
     const int e = max_bits >= 0x00800000u ? static_cast<int>(max_bits >> 23) - 127 : -118 - __clz(max_bits);
-    return 11 - e;
+    return 13 - e;
 }
 
 __device__ __forceinline__ bool range_wide(const RangeSlot* s, uint32_t limit) {
