@@ -939,7 +939,7 @@ bool gemm_h16_serves(const b200_ctx* ctx, const GemmProblem& p) {
     const double flops = 2.0 * double(p.m) * double(p.n) * double(p.k) * double(p.b0 * p.b1);
     // (A chain of more than 12288 truncating additions moves a TF32 result by about 1e-4 from the exact one, and by as
     // much from half terms; such products keep the results they have always had.)
-    return flops > 2147483648.0 && !gemm_tc_streams(ctx, p) && ctx->compared.count(p.out) == 0 && gemm_tc_chain(ctx, p) <= 12288 &&
+    return flops > 2147483648.0 && !gemm_tc_streams(ctx, p) && gemm_tc_chain(ctx, p) <= 12288 &&
            !(ctx->lone_matmul && gemm_tc_reads_directly(ctx, p));
 }
 
