@@ -49,6 +49,8 @@ constexpr uint32_t kMaxStrays = 512;  // of one matrix; with more it is wide
 
 // fp32 FMA on the CUDA cores; any strides, any size. gemm_simt.cu
 void gemm_simt(b200_ctx* ctx, const GemmProblem& p);
+// Whether its single-launch kernel beats the tensor cores, which could serve `p` too (`streams`: from a streamed operand).
+bool gemm_small_pays(const GemmProblem& p, bool streams);
 
 // tcgen05 tensor-core path (3xTF32 or single-pass TF32). gemm_tc.cu
 bool gemm_tc_eligible(const b200_ctx* ctx, const GemmProblem& p);

@@ -133,8 +133,8 @@ split_fold_kernel(float* __restrict__ out, const float* __restrict__ partial, in
 // eight CTAs, each of which takes an equal stretch of K, brings it into shared memory in as few rounds of loads as
 // its length allows (128 of K per round, every load of a round in flight at once) and lets its eight warps take
 // every eighth k; the partial tiles are added warp by warp in shared memory, then rank by rank through the cluster's shared
-// memory -- a fixed order, no partial planes, no fold kernel.  64x784 . 784x128 (8 tiles): 11 us with the
-// tiled kernel and its fold, SMALL here; 784x64 . 64x128: 9 -> SMALLB; 256^3: 13.1 (operand split and tensor cores) -> SMALLC.
+// memory -- a fixed order, no partial planes, no fold kernel.  64x784 . 784x256: 15.0 us on the
+// tensor cores, 10.8 here; 128x128 . 128x1024: 9.6 -> 5.6; 256^3: 12.6 -> 7.5.
 constexpr int kTile = 32, kRound = 128, kPitch = 36;
 
 // rows x kRound elements of an operand into As[k][row]; `along_k`: k is the axis with unit stride.
@@ -295,18 +295,27 @@ bool quad_operand(const float* base, int64_t unit_extent, int64_t s_other, int64
     return reinterpret_cast<uintptr_t>(base) % 16 == 0 && unit_extent % 4 == 0 && s_other % 4 == 0 && s_b0 % 4 == 0 && s_b1 % 4 == 0;
 }
 
+struct SmallPlan {
+    int64_t tiles;
+    int cs;  // CTAs that share a tile's K: one round of loads each, as long as the SMs are not all busy with tiles
+};
+
+SmallPlan small_plan(const GemmProblem& p) {
+    SmallPlan s{p.b0 * p.b1 * ceil_div(p.m, kTile) * ceil_div(p.n, kTile), 1};
+    while (s.cs < 8 && p.k > kRound * s.cs && s.tiles * s.cs * 2 <= 2 * sm_count()) s.cs *= 2;
+    return s;
+}
+
 bool gemm_small(b200_ctx* ctx, const GemmProblem& p) {
     const int64_t batches = p.b0 * p.b1;
     // (what takes longer than a few microseconds is better off with larger tiles and less traffic per product)
-    if (2.0 * double(p.m) * double(p.n) * double(p.k) * double(batches) > double(1 << 26)) return false;
+    if (2.0 * double(p.m) * double(p.n) * double(p.k) * double(batches) > double(1 << 26) && !gemm_small_pays(p, false)) return false;
     SmallArgs g{};
     g.p = p;
     g.tiles_m = ceil_div(p.m, kTile);
     g.tiles_n = ceil_div(p.n, kTile);
-    const int64_t tiles = batches * g.tiles_m * g.tiles_n;
+    const auto [tiles, cs] = small_plan(p);
     if (tiles > (int64_t(1) << 28)) return false;
-    int cs = 1;  // CTAs that share a tile's K: one round of loads each, as long as the SMs are not all busy with tiles
-    while (cs < 8 && p.k > kRound * cs && tiles * cs * 2 <= 2 * sm_count()) cs *= 2;
     g.k_chunk = ceil_div(ceil_div(p.k, cs), 4) * 4;
     const bool a_k = p.a_s[3] == 1 || p.a_s[2] != 1, b_k = p.b_s[2] == 1 && p.b_s[3] != 1;
     g.a_quads = a_k ? p.a_s[3] == 1 && quad_operand(p.a, p.k, p.a_s[2], p.a_s[0], p.a_s[1]) : quad_operand(p.a, p.m, p.a_s[3], p.a_s[0], p.a_s[1]);
@@ -324,6 +333,22 @@ bool gemm_small(b200_ctx* ctx, const GemmProblem& p) {
 }
 
 }  // namespace
+
+// Products of 2^24 to 2^27 operations: this kernel or the tensor cores?  Measured over 55 shapes in three layouts.  It wins while all CTAs are
+// resident at once, two to an SM -- with clusters of eight, of which an odd GPC holds fewer, 28 tiles: 96x784x256 11.1 against 15.4 us,
+// 128x784x256 (32 tiles) 15.8 against 15.8, 64x1024x512 17.4 against 14.5 -- and loses with more of them: 32 x 128x32x128 11.9 against
+// 8.1, 700x33x700 13.8 against 8.5, 64x64x8192 13.8 against 8.2.  Above 2^25 it wins against operands read directly or through planes while a CTA
+// has two rounds of K and the tensor cores no K-slices, which they have from sixteen K-blocks on: 264^3 12.5 against 17.2, 275x376x276 14.1
+// against 21.1, 384^3 15.6 against 21.2, 2048x136x68 10.5 against 12.3; but 300x900x100 15.4 against 13.4, 400^3 (four rounds) 20.8
+// against 22.4.  Streamed operands and batches stay on the tensor cores there (64x1024x512 above; 2 x 300x300x100 would take 13.3 for 18.5).
+bool gemm_small_pays(const GemmProblem& p, bool streams) {
+    const double flops = 2.0 * double(p.m) * double(p.n) * double(p.k) * double(p.b0 * p.b1);
+    if (flops <= double(1 << 24)) return true;
+    if (flops > double(1 << 27)) return false;
+    const SmallPlan s = small_plan(p);
+    if (s.tiles * s.cs > 2 * sm_count() || (s.cs == 8 && s.tiles > 28)) return false;
+    return flops <= double(1 << 25) || (!streams && p.b0 * p.b1 == 1 && ceil_div(p.k, s.cs) <= 2 * kRound && p.k <= 480);
+}
 
 void gemm_simt(b200_ctx* ctx, const GemmProblem& p) {
     const int64_t batches = p.b0 * p.b1;

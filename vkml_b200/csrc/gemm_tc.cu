@@ -1816,9 +1816,8 @@ bool gemm_tc_eligible(const b200_ctx* ctx, const GemmProblem& p) {
     if (p.m < 32 || p.n < 16 || p.k < 16 || batches < 1) {  // K is zero-padded to the 32-wide K-block
         return false;
     }
-    const double flops = 2.0 * double(p.m) * double(p.n) * double(p.k) * double(batches);
-    if (flops <= double(1 << 25)) {
-        return false;  // launch-bound either way: the single CUDA-core kernel is cheaper than split + GEMM
+    if (gemm_small_pays(p, plan_stream(ctx, p).ok)) {
+        return false;  // one launch on the CUDA cores is cheaper
     }
     // TMA coordinates are 32-bit
     const int64_t kp = align_up(p.k, BK);
