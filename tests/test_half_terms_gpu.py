@@ -63,6 +63,14 @@ def test_a_product_does_not_depend_on_what_reads_it(backend, m, k, n):
     assert same_bits(y.numpy().reshape(alone.shape), alone) and same_bits(h.numpy(), np.maximum(y.numpy() + bias, 0))
 
 
+@pytest.mark.parametrize("m,k,n,half", [(1024, 1024, 1024, False), (2048, 1024, 1023, False), (2048, 1024, 1024, True), (2048, 1025, 1024, True)])
+def test_from_which_size_on(backend, m, k, n, half):
+    rng = np.random.default_rng(m + n)
+    a, b = rng.standard_normal((m, k), dtype=np.float32), rng.standard_normal((k, n), dtype=np.float32)
+    got, labels = product(backend, a, b, "nn")
+    assert ("matmul.tcgen05_3xf16" in labels) == half and rel(got, a, b) < 1e-5, labels
+
+
 def test_batches_and_a_broadcast_operand(backend):
     rng = np.random.default_rng(5)
     a, b = rng.standard_normal((9, 500, 516), dtype=np.float32), rng.standard_normal((516, 1030), dtype=np.float32)
@@ -178,14 +186,14 @@ def test_wide_operands_that_a_span_shares(backend, tf32_backend):
     """A layer's two backward products on a gradient of wide range, and a third on the same activations and weight: planes that stand by
     are written once and serve every product that needs them, a product of narrow operands none."""
     rng = np.random.default_rng(8)
-    x, w, g = (rng.standard_normal(s, dtype=np.float32) for s in ((1536, 1024), (1024, 1280), (1536, 1280)))
+    x, w, g = (rng.standard_normal(s, dtype=np.float32) for s in ((1536, 1152), (1152, 1280), (1536, 1280)))
     g[:, 5] *= np.exp2(rng.integers(-40, 0, 1536)).astype(np.float32)
     results = []
     for b in (backend, tf32_backend):
         def put(t):
             return DeviceTensor.from_host(b, t.reshape((1, 1) + t.shape))
         dx, dw, dg = put(x), put(w), put(g)
-        outs = [DeviceTensor.empty(b, (1, 1) + s) for s in ((1024, 1280), (1536, 1024), (1536, 1280), (1280, 1280))]
+        outs = [DeviceTensor.empty(b, (1, 1) + s) for s in ((1152, 1280), (1536, 1152), (1536, 1280), (1280, 1280))]
         pairs = [(dx.transpose(2, 3), dg), (dg, dw.transpose(2, 3)), (dx, dw), (dg.transpose(2, 3), dg)]
         b.compute([NodeDesc(int(Op.MATMUL), o.desc, [p.desc, q.desc]) for o, (p, q) in zip(outs, pairs)])
         results.append([o.numpy() for o in outs])

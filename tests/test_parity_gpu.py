@@ -460,7 +460,7 @@ def test_which_kernel_a_product_gets_does_not_depend_on_the_span_before(backend)
     """b200_matmul_kernel's answer is about the product by itself, also right after a span that compares its result or
     holds other products."""
     from vkml_b200 import DeviceTensor, NodeDesc
-    for lead, m, k, n in (((1, 1), 2048, 1024, 1536), ((1, 64), 512, 1024, 40)):  # half terms; operands read directly
+    for lead, m, k, n in (((1, 1), 2048, 1024, 1536), ((1, 128), 512, 1024, 40)):  # half terms; operands read directly
         a, b = DeviceTensor.empty(backend, lead + (m, k)), DeviceTensor.empty(backend, lead + (k, n))
         out, other, act = (DeviceTensor.empty(backend, lead + (m, n)) for _ in range(3))
         node = NodeDesc(Op.MATMUL, out.desc, [a.desc, b.desc])
