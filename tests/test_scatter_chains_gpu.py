@@ -8,8 +8,9 @@ pytestmark = pytest.mark.gpu
 
 
 # rows of single elements and of quads, one piece and several, a ragged last piece; destinations with no, one, 32
-# and 33 sources, and one that takes a third of them
-@pytest.mark.parametrize("count,extent,inner", [(2100, 700, 31), (2100, 700, 129), (2100, 700, 260), (1500, 5000, 516), (700, 90, 256)])
+# and 33 sources, and one that takes a third of them; long lists only, their last stretch one index or a few
+@pytest.mark.parametrize("count,extent,inner", [(2100, 700, 31), (2100, 700, 129), (2100, 700, 260), (1500, 5000, 516), (700, 90, 256),
+                                                (4097, 20, 256), (513, 6, 5000), (767, 12, 2052)])
 def test_sums_in_index_order(backend, count, extent, inner):
     rng = np.random.default_rng(count + inner)
     idx = rng.integers(0, extent - 4, count).astype(np.int64)

@@ -988,7 +988,9 @@ scatter_gather4_kernel(float4* __restrict__ out, const float4* __restrict__ src,
 // ascending order by itself -- up to 32 of them lie one per lane and are ranked by comparing -- or, for a destination
 // with more, finds them in order by reading the index list (at most n / 33 destinations have more, so that all of them
 // together read it a bounded number of times).  The sums and their order are those of the pull form, bit for bit.
-// [8192, 1024] into [50000, 1024]: 152 -> 50 us; 239 MB, nearly all of it the result.
+// [8192, 1024] into [50000, 1024]: 152 -> 50 us; 239 MB, nearly all of it the result.  Long lists, buckets against chains: 16384 indices
+// into 100 rows of 1024, uniform 130 and 92 us, as words of a text are distributed (1/rank) 573 and 445; into 256 of 512 90 and 72, 504 and 381;
+// all into one 3633 and 2594.  (One piece of 32 indices at a time instead of four in flight: 156, 461, 146, 390 and 2797.)
 constexpr int kChainMax = 65536;
 
 __global__ void __launch_bounds__(kThreads)
@@ -1012,8 +1014,9 @@ struct Int {
 };
 
 // One warp per piece of 32*Q*W elements of a destination row, with at most 32 registers of sources in flight: 64 left two
-// blocks on an SM, which took 71 us where this takes 45.
-template <int W, int Q>
+// blocks on an SM, which took 71 us where this takes 45.  LOOK pieces of 32 indices are in flight where a destination's list is long; four
+// of them spill a few registers, which costs 3 % where no list is.
+template <int W, int Q, int LOOK>
 __global__ void __launch_bounds__(kThreads, 4)
 scatter_chain_gather_kernel(float* __restrict__ out, const float* __restrict__ src, const int* __restrict__ count,
                             const int* __restrict__ head, const int* __restrict__ next, const int64_t* __restrict__ idx,
@@ -1082,20 +1085,29 @@ scatter_chain_gather_kernel(float* __restrict__ out, const float* __restrict__ s
             add_few(held, c);
         } else if (c > 32) {
             int have = 0;
-            for (int k0 = 0; k0 < n; k0 += 32) {
-                const int k = k0 + int(lane);
-                const bool hit = k < n && idx[k * idx_stride] == int64_t(j);
-                const uint32_t hits = __ballot_sync(0xffffffffu, hit);
-                if (hit) mine[have + __popc(hits & ((1u << lane) - 1u))] = k;
-                have += __popc(hits);
-                __syncwarp();
-                if (have >= 32) {
-                    add_32(mine[lane], 32);
-                    have -= 32;
-                    const int rest = mine[32 + lane];
+            for (int k0 = 0; k0 < n; k0 += 32 * LOOK) {
+                uint32_t here = 0;  // bit u: this lane's index of the u-th 32 leads here
+#pragma unroll
+                for (int u = 0; u < LOOK; ++u) {
+                    const int k = k0 + 32 * u + int(lane);
+                    here |= (k < n && idx[k * idx_stride] == int64_t(j) ? 1u : 0u) << u;
+                }
+#pragma unroll
+                for (int u = 0; u < LOOK; ++u) {
+                    const bool hit = (here >> u & 1u) != 0;
+                    const uint32_t hits = __ballot_sync(0xffffffffu, hit);
+                    if (hits == 0) continue;
+                    if (hit) mine[have + __popc(hits & ((1u << lane) - 1u))] = k0 + 32 * u + int(lane);
+                    have += __popc(hits);
                     __syncwarp();
-                    mine[lane] = rest;
-                    __syncwarp();
+                    if (have >= 32) {
+                        add_32(mine[lane], 32);
+                        have -= 32;
+                        const int rest = mine[32 + lane];
+                        __syncwarp();
+                        mine[lane] = rest;
+                        __syncwarp();
+                    }
                 }
             }
             add_few(int(lane) < have ? mine[lane] : 0, have);
@@ -1549,8 +1561,14 @@ void launch_movement(b200_ctx* ctx, const b200_node& node) {
                                   static_cast<const int*>(next), ip, istride, n, FastDiv(static_cast<uint32_t>(pieces)),
                                   FastDiv(static_cast<uint32_t>(extent)), static_cast<uint32_t>(inner), static_cast<uint32_t>(tasks));
                 };
-                if (quads) gather(scatter_chain_gather_kernel<4, 2>);
-                else gather(scatter_chain_gather_kernel<1, 4>);
+                // (eight sources to a destination on average: some lists are long)
+                if (n_idx >= 8 * extent) {
+                    if (quads) gather(scatter_chain_gather_kernel<4, 2, 4>);
+                    else gather(scatter_chain_gather_kernel<1, 4, 4>);
+                } else {
+                    if (quads) gather(scatter_chain_gather_kernel<4, 2, 1>);
+                    else gather(scatter_chain_gather_kernel<1, 4, 1>);
+                }
                 break;
             }
             if (n_idx > 0) {
