@@ -392,7 +392,7 @@ def train_section(args, backend, rank, world, dist, barrier, max_over_ranks):
     """Samples/s of a recorded training step (forward, backward, SGD-momentum update, loss
     read-back) replayed through the C ABI; at N > 1 every rank runs the step on its own
     batch and the backward span's gradient sinks are all-reduced over NCCL while the span runs."""
-    from vkml_b200.replay import Replayer, load_program
+    from vkml_b200.replay import load_program, with_resident_inputs
     path = os.path.join(ROOT, "tests", "golden", "programs", args.train + ".json.gz")
     if args.train == "none" or not os.path.exists(path):
         return None
@@ -436,28 +436,29 @@ def train_section(args, backend, rank, world, dist, barrier, max_over_ranks):
         backend.dist_init(rank, world, uid[0])
     # The library's native step tape issues the recorded calls (one foreign call per step), so
     # the host side costs what the framework's C++ executor would, not a Python loop per node.
-    tape = Tape(backend, program, grad_sync=world > 1)
     # steady-state steps as captured CUDA graphs (single GPU; gradient-synchronising steps replay eagerly)
     use_graphs = world == 1 and not args.no_graphs
-    tape.enable_graphs(use_graphs)
-    tape.run_prologue(params)
-    first = [pin_x.ctypes.data, pin_y.ctypes.data]
-    for _ in range(len(program["steps"]) - 1):   # the recorded first steps differ from the steady state
-        tape.step(first)
-    steady = tape.template_for_step(tape.steps_run)
-    with_uploads = tape.upload_ptrs(steady, first)
-    resident = tape.upload_ptrs(steady, [None, None])
     # a graph is captured the second time a step's addresses come up, and the allocator cycles
     # through at most six address sets for these programs: fourteen steps see every set twice
     warm = 14 if use_graphs else 3
-    for _ in range(warm):
-        tape.step_fast(with_uploads)
-    for _ in range(warm):
-        tape.step_fast(resident)
-    backend.synchronize()
-    barrier()
     k = max(3, args.train_steps)
+    first = [pin_x.ctypes.data, pin_y.ctypes.data]
+
+    def started(prog, prologue, step):
+        tape = Tape(backend, prog, grad_sync=world > 1)
+        tape.enable_graphs(use_graphs)
+        tape.run_prologue(prologue)
+        for _ in range(len(prog["steps"]) - 1):   # the recorded first steps differ from the steady state
+            tape.step(step)
+        fast = tape.upload_ptrs(tape.template_for_step(tape.steps_run), step)
+        for _ in range(warm):
+            tape.step_fast(fast)
+        backend.synchronize()
+        barrier()
+        return tape, fast
+
     # end to end: x and labels uploaded from pinned host memory every step, loss read back
+    tape, with_uploads = started(program, params, first)
     l0 = backend.stats()["kernel_launches"]
     t0 = time.perf_counter()
     for _ in range(k):
@@ -465,8 +466,11 @@ def train_section(args, backend, rank, world, dist, barrier, max_over_ranks):
     backend.synchronize()
     e2e_ms = max_over_ranks((time.perf_counter() - t0) * 1e3)
     launches = (backend.stats()["kernel_launches"] - l0) / k
+    comm_bytes = int(backend.stats()["comm_bytes"] / max(1, tape.steps_run))
+    tape.close()
     barrier()
-    # inputs resident: the recorded uploads are skipped (the buffers keep the last batch)
+    # inputs resident: the same steps on a batch that the prologue has uploaded, from the same initial parameters
+    tape, resident = started(with_resident_inputs(program), params + [x, y], [])
     backend.timer_begin()
     for _ in range(k):
         tape.step_fast(resident)
@@ -480,8 +484,6 @@ def train_section(args, backend, rank, world, dist, barrier, max_over_ranks):
     backend.set_profiling(False)
     barrier()
     loss_last = float(tape.downloads[0].view(np.float32)[0]) if tape.downloads else None
-    steps_total = tape.steps_run
-    comm_bytes = int(backend.stats()["comm_bytes"] / max(1, steps_total))
     alone_ms = None
     if world > 1 and comm_bytes:
         # the same bytes all-reduced with nothing else on the GPU: the part of it that the

@@ -238,3 +238,24 @@ def test_too_many_sources_are_refused():
         graph.pack_nodes(nodes)
     with pytest.raises(IndexError):
         nodes[0].to_c()
+
+
+def test_programs_with_resident_inputs():
+    """Every recorded program's uploads move into the prologue: no step uploads, and what read an uploaded buffer reads the prologue's."""
+    import glob
+    from vkml_b200.replay import load_program, with_resident_inputs
+    from vkml_b200.tape import encode
+    paths = glob.glob(os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden", "programs", "*.json.gz"))
+    assert paths
+    for path in paths:
+        program = load_program(path)
+        moved = with_resident_inputs(program)
+        first = sum(e["ev"] == "alloc" for e in program["prologue"])
+        assert [e["bytes"] for e in moved["prologue"][-4:] if e["ev"] == "h2d"] == [e["bytes"] for e in program["steps"][0] if e["ev"] == "h2d"]
+        for before, after in zip(program["steps"], moved["steps"]):
+            ups = [e["buf"] for e in before if e["ev"] == "h2d"]
+            assert len(ups) == 2 and encode(after)[1] == 0 and len(after) == len(before) - 2
+            refs = [[s["buf"] for e in step if e["ev"] == "compute" for n in e["nodes"] for s in n["src"]] for step in (before, after)]
+            assert len(refs[0]) == len(refs[1]) and any(r in ups for r in refs[0])
+            for old, new in zip(*refs):
+                assert new == (["pro", first + ups.index(old)] if old in ups else old) or (old[0] == 1 and new[0] == "pro")

@@ -272,6 +272,29 @@ def test_fused_groups_compute_what_the_separate_kernels_do(monkeypatch, name):
     np.testing.assert_allclose(fused, plain, rtol=1e-6, atol=0)
 
 
+def test_steps_on_resident_inputs_are_the_uploaded_ones():
+    """The program whose inputs lie in the prologue gives the losses of the one that uploads the same batch every step."""
+    import vkml_b200
+    from vkml_b200.replay import load_program, with_resident_inputs
+    from vkml_b200.tape import Tape
+    program = load_program(os.path.join(os.path.dirname(os.path.abspath(__file__)), "golden", "programs", "mlp_784_128_10_b64.json.gz"))
+    meta, rng = program["meta"], np.random.default_rng(6)
+    params = []
+    for fin, fout in zip(meta["widths"][:-1], meta["widths"][1:]):
+        params += [rng.uniform(-1, 1, s).astype(np.float32) / np.float32(np.sqrt(fin)) for s in ((fout, fin), (fout,))]
+    x, y = rng.random((meta["batch"], meta["widths"][0]), dtype=np.float32), rng.integers(0, meta["widths"][-1], meta["batch"]).astype(np.int64)
+    losses = []
+    for resident in (False, True):
+        tape = Tape(vkml_b200.Backend(0), with_resident_inputs(program) if resident else program)
+        tape.run_prologue(params + ([x, y] if resident else []))
+        losses.append([])
+        for _ in range(8):
+            tape.step([] if resident else [x, y])
+            losses[-1].append(tape.downloads[0].view(np.float32)[0].copy())
+        tape.close()
+    assert np.array_equal(np.array(losses[0]).view(np.uint32), np.array(losses[1]).view(np.uint32)) and losses[0][-1] < losses[0][0]
+
+
 def test_a_run_of_tiny_nodes_is_one_launch(monkeypatch):
     """The single-block chain, on a run that is no loss's prologue: every node's bits those of its own kernel."""
     import vkml_b200

@@ -31,6 +31,47 @@ def load_program(path: str) -> dict:
         return json.load(f)
 
 
+def with_resident_inputs(program: dict) -> dict:
+    """The same program with its steps' uploads moved to the end of the prologue: the buffers that a step uploads into become
+    buffers of the prologue, which every step reads.  (A step that merely skips its uploads reads whatever the
+    block that it was handed held last.)  All steps have to upload the same sizes in the same order."""
+    first = sum(e["ev"] == "alloc" for e in program["prologue"])
+    prologue, steps, held = list(program["prologue"]), [], []
+    for template in program["steps"]:
+        ups = [e for e in template if e["ev"] == "h2d"]
+        if not steps:
+            for i, e in enumerate(ups):
+                prologue.append({"ev": "alloc", "bytes": e["bytes"]})
+                prologue.append(dict(e, buf=["pro", first + i]))
+        sizes = [e["bytes"] for e in ups]
+        if sizes != [e["bytes"] for e in prologue if e["ev"] == "h2d"][-len(ups):] or any(e["buf"][0] != 0 or e["off"] for e in ups):
+            raise ValueError("steps that upload into different buffers")
+        held.append({e["buf"][1]: first + i for i, e in enumerate(ups)})
+    for t, template in enumerate(program["steps"]):
+        def moved(ref):
+            if ref is None or ref[0] == "pro":
+                return ref
+            at = held[max(0, t - ref[0])]  # (the last template follows itself)
+            if ref[0] and t == len(program["steps"]) - 1 and held[t] != held[max(0, t - ref[0])]:
+                raise ValueError("steps that upload into different buffers")
+            return ["pro", at[ref[1]]] if ref[1] in at else ref
+
+        events = []
+        for e in template:
+            if e["ev"] == "h2d":
+                continue
+            if e["ev"] == "compute":
+                e = dict(e, nodes=[dict(n, out=dict(n["out"], buf=moved(n["out"]["buf"])), src=[dict(s, buf=moved(s["buf"])) for s in n["src"]])
+                                   for n in e["nodes"]])
+            elif e["ev"] == "d2d":
+                e = dict(e, copies=[[moved(c[0]), c[1], moved(c[2]), c[3], c[4]] for c in e["copies"]])
+            elif e["ev"] == "d2h":
+                e = dict(e, buf=moved(e["buf"]))
+            events.append(e)
+        steps.append(events)
+    return dict(program, prologue=prologue, steps=steps)
+
+
 class Replayer:
     """Executes a program's prologue once and its step templates on demand.
 
