@@ -71,6 +71,24 @@ def test_from_which_size_on(backend, m, k, n, half):
     assert ("matmul.tcgen05_3xf16" in labels) == half and rel(got, a, b) < 1e-5, labels
 
 
+def test_many_products_of_changing_shapes_in_a_row(backend):
+    """Sequences of odd products that change shape and tile form end, and end without a wait that ran out."""
+    rng = np.random.default_rng(77)
+    pool = DeviceTensor.from_host(backend, rng.standard_normal(1 << 23, dtype=np.float32))
+
+    def matrix(rows, cols):
+        return DeviceTensor(backend, pool.storage, (1, 1, rows, cols), (0, 0, cols * 4, 4), DType.F32, 0)
+
+    for _ in range(60):
+        m, n = (int(2 ** rng.uniform(7, 11.5)) | 1 for _ in range(2))
+        k = min(int(4.4e9 / (2 * m * n)) + 65, (1 << 23) // max(m, n))
+        out = DeviceTensor.empty(backend, (1, 1, m, n))
+        right = matrix(n, k).transpose(2, 3) if rng.random() < 0.5 else matrix(k, n)
+        for _ in range(30):
+            backend.compute([NodeDesc(int(Op.MATMUL), out.desc, [matrix(m, k).desc, right.desc])])
+    backend.synchronize()  # (raises where a bounded wait has run out)
+
+
 def test_batches_and_a_broadcast_operand(backend):
     rng = np.random.default_rng(5)
     a, b = rng.standard_normal((9, 500, 516), dtype=np.float32), rng.standard_normal((516, 1030), dtype=np.float32)

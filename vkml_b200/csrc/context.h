@@ -227,9 +227,9 @@ inline void launch_kernel(b200_ctx* ctx, void (*kernel)(Params...), dim3 grid, d
     (void)cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 
-// The same for a kernel whose blocks work in clusters of `cluster` along x.
+// The same for a kernel whose blocks work in clusters of `cluster` along x; `early`: it may be scheduled before the kernel in front of it is done.
 template <typename... Params, typename... Args>
-inline void launch_kernel_clustered(b200_ctx* ctx, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, int cluster,
+inline void launch_kernel_clustered(b200_ctx* ctx, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, int cluster, bool early,
                                     Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
@@ -244,7 +244,7 @@ inline void launch_kernel_clustered(b200_ctx* ctx, void (*kernel)(Params...), di
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = ctx->pdl ? 2 : 1;
+    cfg.numAttrs = ctx->pdl && early ? 2 : 1;
     (void)cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
 }
 

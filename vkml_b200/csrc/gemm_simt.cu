@@ -324,9 +324,9 @@ bool gemm_small(b200_ctx* ctx, const GemmProblem& p) {
     const unsigned grid = static_cast<unsigned>(tiles * cs);
     ProfScope scope(ctx, "matmul.fp32_simt");
     if (cs == 1) launch_kernel(ctx, gemm_small_kernel<1>, grid, 256, 0, g);
-    else if (cs == 2) launch_kernel_clustered(ctx, gemm_small_kernel<2>, grid, 256, 0, 2, g);
-    else if (cs == 4) launch_kernel_clustered(ctx, gemm_small_kernel<4>, grid, 256, 0, 4, g);
-    else launch_kernel_clustered(ctx, gemm_small_kernel<8>, grid, 256, 0, 8, g);
+    else if (cs == 2) launch_kernel_clustered(ctx, gemm_small_kernel<2>, grid, 256, 0, 2, true, g);
+    else if (cs == 4) launch_kernel_clustered(ctx, gemm_small_kernel<4>, grid, 256, 0, 4, true, g);
+    else launch_kernel_clustered(ctx, gemm_small_kernel<8>, grid, 256, 0, 8, true, g);
     ctx->count_launch();
     check_last_launch("matmul (small)");
     return true;
