@@ -71,6 +71,31 @@ def test_from_which_size_on(backend, m, k, n, half):
     assert ("matmul.tcgen05_3xf16" in labels) == half and rel(got, a, b) < 1e-5, labels
 
 
+# every tile form: whole tiles and odd remainders, units for one wave and several, K-slices and none
+@pytest.mark.parametrize("tile,m,k,n,layout", [
+    ("256x256", 1899, 2034, 1889, "nn"), ("256x256", 2231, 1254, 1556, "tn"), ("256x256", 1000, 9001, 512, "nt"),
+    ("256x128", 1086, 3267, 1052, "nt"), ("256x128", 766, 2993, 2872, "nn"), ("128x128", 3000, 1001, 2999, "nn"),
+    ("128x128", 1301, 1333, 1277, "nt"), ("128x128", 300, 8192, 1000, "tn"), ("128x64", 9001, 4000, 64, "nt"), ("128x64", 317, 2611, 3073, "tn")])
+def test_every_tile_form(backend, tile, m, k, n, layout):
+    rng = np.random.default_rng(m + k)
+    a, b = rng.standard_normal((m, k), dtype=np.float32), rng.standard_normal((k, n), dtype=np.float32)
+    sa, sb = (DeviceTensor.empty(backend, (1, 1) + s) for s in ((m, k), (k, n)))
+    out = DeviceTensor.empty(backend, (1, 1, m, n))
+    name, why = backend.matmul_kernel(NodeDesc(int(Op.MATMUL), out.desc, [sa.desc, sb.desc]))
+    assert name != "tcgen05_3xf16" or why.endswith(" " + tile), (name, why)
+    # (twice in one span: the second one's shared planes keep a thin product from reading its operands directly)
+    da, db = (DeviceTensor.from_host(backend, np.ascontiguousarray(x.T if t == "t" else x).reshape((1, 1) + (x.T if t == "t" else x).shape))
+              for x, t in ((a, layout[0]), (b, layout[1])))
+    da, db = (x.transpose(2, 3) if t == "t" else x for x, t in ((da, layout[0]), (db, layout[1])))
+    again = DeviceTensor.empty(backend, (1, 1, m, n))
+    backend.set_profiling(True)
+    backend.compute([NodeDesc(int(Op.MATMUL), o.desc, [da.desc, db.desc]) for o in (out, again)])
+    labels = [l for l, _ in backend.last_profile()]
+    backend.set_profiling(False)
+    assert labels.count("matmul.tcgen05_3xf16") == 2, labels
+    assert rel(out.numpy(), a, b) < 1e-5 and same_bits(out.numpy(), again.numpy())
+
+
 def test_many_products_of_changing_shapes_in_a_row(backend):
     """Sequences of odd products that change shape and tile form end, and end without a wait that ran out."""
     rng = np.random.default_rng(77)

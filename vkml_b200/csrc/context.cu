@@ -1515,14 +1515,15 @@ int b200_matmul_kernel(b200_ctx* ctx, const b200_node* node, char* name, size_t 
         if (touches_f16(*node)) fail(B200_DTYPE_ERROR, "b200_matmul_kernel: an f32 node is wanted");
         const GemmProblem p = matmul_problem(*node);
         const char* kernel = "fp32_simt";
-        const char* why = "the shape is too small or too ragged for a tensor-core tile";
+        std::string why = "the shape is too small or too ragged for a tensor-core tile";
         if (ctx->gemm_precision == B200_GEMM_FP32) {
             why = "plain fp32 arithmetic was asked for";
         } else if (gemm_tc_eligible(ctx, p)) {
             const bool three = ctx->gemm_precision == B200_GEMM_3XTF32;
             if (gemm_h16_serves(ctx, p)) {
                 kernel = "tcgen05_3xf16";
-                why = "bound by the tensor cores: two half terms per operand (TF32 planes where an operand's range is too wide for them)";
+                why = "bound by the tensor cores: two half terms per operand (TF32 planes where an operand's range is too wide for them), tiles of " +
+                      gemm_h16_tile(ctx, p);
             } else if (gemm_tc_streams(ctx, p)) {
                 kernel = three ? "tcgen05_3xtf32_stream" : "tcgen05_tf32_stream";
                 why = "bound by memory (a small left operand or a short K): the right operand is read as fp32 and split on the way";
@@ -1535,7 +1536,7 @@ int b200_matmul_kernel(b200_ctx* ctx, const b200_node* node, char* name, size_t 
             }
         }
         std::snprintf(name, name_len, "%s", kernel);
-        if (reason != nullptr && reason_len != 0) std::snprintf(reason, reason_len, "%s", why);
+        if (reason != nullptr && reason_len != 0) std::snprintf(reason, reason_len, "%s", why.c_str());
     });
 }
 

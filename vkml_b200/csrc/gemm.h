@@ -68,6 +68,7 @@ size_t gemm_tc_plane_bytes(const GemmProblem& p, bool left);  // of one operand'
 bool gemm_h16_serves(const b200_ctx* ctx, const GemmProblem& p);
 void gemm_h16(b200_ctx* ctx, const GemmProblem& p);
 void gemm_h16_note_uses(b200_ctx* ctx, const GemmProblem& p);
+std::string gemm_h16_tile(const b200_ctx* ctx, const GemmProblem& p);  // "rows x columns" of the tile it gets
 // Half storage: `p`'s pointers are to halves.  False: not a case for this kernel.  With an epilogue the nodes behind the
 // product -- add(y, bias along the rows) and perhaps relu -- are served as well.
 struct HalfEpilogue {

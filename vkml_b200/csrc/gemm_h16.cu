@@ -796,14 +796,10 @@ void launch_tile(b200_ctx* ctx, const HalfOperand& a, const HalfOperand& b, cons
 
 template <int CG, int BN, int PASSES>
 void launch_major(b200_ctx* ctx, const HalfOperand& a, const HalfOperand& b, const H16Args& g, int64_t units) {
-    if constexpr (BN / CG >= 64) {  // (an MN-major atom is 64 wide)
-        if (b.mn) {
-            if (a.mn) launch_tile<CG, BN, PASSES, true, true>(ctx, a, b, g, units);
-            else launch_tile<CG, BN, PASSES, false, true>(ctx, a, b, g, units);
-            return;
-        }
-    }
-    if (a.mn) launch_tile<CG, BN, PASSES, true, false>(ctx, a, b, g, units);
+    static_assert(BN / CG >= 64, "an MN-major atom is 64 wide");
+    if (a.mn && b.mn) launch_tile<CG, BN, PASSES, true, true>(ctx, a, b, g, units);
+    else if (b.mn) launch_tile<CG, BN, PASSES, false, true>(ctx, a, b, g, units);
+    else if (a.mn) launch_tile<CG, BN, PASSES, true, false>(ctx, a, b, g, units);
     else launch_tile<CG, BN, PASSES, false, false>(ctx, a, b, g, units);
 }
 
@@ -815,20 +811,24 @@ struct TileChoice {
 // The tile whose whole waves cost least.  `width` x 128 rows of cg CTAs; a narrower or single-CTA tile moves more
 // operand bytes per product (relative cost per unit of work beside the widest), so it is taken only
 // where the widest one would leave SMs idle: few tiles, or a nearly empty last wave.
-TileChoice choose_tile(const GemmProblem& p, int passes, bool b_mn, int sms) {
+TileChoice choose_tile(const GemmProblem& p, int passes, int sms) {
     struct Form { int cg, bn; double cost, drain; };
     // cost of one K-block of a tile in units of a 256 x 128 tile's, and K-blocks that its fill and drain come to.  Three
     // passes over 256 columns leave room for one pair of accumulators, so that tile's epilogue is not hidden; its operand
-    // traffic per product is two thirds, which at the power cap is worth 14 % (8192^3: 3.15 -> 2.69 ms sustained).
-    static const Form three[] = {{2, 256, 1.65, 6}, {2, 128, 1.0, 2}, {2, 64, 0.56, 2}, {1, 128, 1.08, 2}, {1, 64, 0.6, 2}};
+    // traffic per product is two thirds, which at the power cap is worth 14 % (8192^3: 3.15 -> 2.69 ms sustained).  A 64-wide tile
+    // costs nearly what a 128-wide one does, the instructions being the limit.  Each form forced for 30 products of 2^32 to 2^40 operations: with
+    // these figures the choice is 1 % slower than the best on average and 7 % at most.  us for 256x256, 256x128, 128x128 and 128x64:
+    //   8192^3 2471 2990 3004 4732;  2048x8192x8192 703 796 760 1330;  3000^3 148 169 235 317;  6000x2000x576 77 92 92 107;
+    //   1536^3 47.2 41.6 39.7 51.5;  300x8192x1000 54 54 49 57;  512x8192x512 47 43 42 48;  1200x4000x520 49 48 47 60;  20000x2000x64 139 123 125 121.
+    // (256x64 was slower than one of these on every product: 6000x2000x576 108, 1200x4000x520 62.)
+    static const Form three[] = {{2, 256, 1.65, 6}, {2, 128, 1.0, 2}, {1, 128, 1.03, 1}, {1, 64, 0.85, 2}};
     static const Form one[] = {{2, 256, 1.75, 2}, {1, 128, 1.08, 2}, {1, 64, 0.6, 2}};
     const Form* forms = passes == 3 ? three : one;
     const int64_t batches = p.b0 * p.b1, k_blocks = ceil_div(p.k, kBlockK);
     TileChoice best{};
     double least = 0;
-    for (int i = 0; i < (passes == 3 ? 5 : 3); ++i) {
+    for (int i = 0; i < (passes == 3 ? 4 : 3); ++i) {
         const Form& f = forms[i];
-        if (b_mn && f.bn / f.cg < 64) continue;  // an MN-major atom is 64 wide
         TileChoice c{f.cg, f.bn, ceil_div(p.m, int64_t(f.cg) * kRowsM), ceil_div(p.n, int64_t(f.bn)), 1, k_blocks, 0};
         const int64_t tiles = c.tiles_m * c.tiles_n * batches, slots = sms / f.cg;
         if (tiles < slots && k_blocks >= 8) {
@@ -883,7 +883,6 @@ void run_h16(b200_ctx* ctx, const GemmProblem& p, int passes, const TileChoice& 
     if (t.cg == CG && t.bn == BN && passes == P) launch_major<CG, BN, P>(ctx, a, b, g, t.units);
         B200_H16_CASE(2, 256, 3)
         B200_H16_CASE(2, 128, 3)
-        B200_H16_CASE(2, 64, 3)
         B200_H16_CASE(1, 128, 3)
         B200_H16_CASE(1, 64, 3)
         B200_H16_CASE(2, 256, 1)
@@ -934,8 +933,8 @@ MatrixArgs matrix_args(const HalfOperand& o) {
 // Products of 2^32 operations and more: the range pass (a read of a sample) and the two launches that stand by behind the product cost
 // about 8 us together, which the halved MMA time does not return on smaller ones.  Measured on both sides of the line, TF32 terms
 // against half terms: 1024^3 (half of it) 26.8 and 29.7 us, 1000x1433x777 (half) 34.5 and 38.0, 1024x1536x1024 (0.75) 32.4 and 35.4,
-// 2000x511x2001 (0.95) 35.5 and 36.0; 2048x1024x1024 35.6 and 32.9, 512x8192x512 49.2 and 41.6, 1301x1333x1277 43 and 40, 1536^3 45 and 40.
-// (Products whose TF32 tiles fill little more than one wave cross earlier, 1200^3 at 0.8 with 38.4 and 33.9; 512x2048x2048 later, 41 and 42.6.)
+// 2000x511x2001 (0.95) 35.5 and 36.0; 2048x1024x1024 35.6 and 34.3, 512x8192x512 49.6 and 44.3, 512x2048x2048 41.0 and 40.2, 1301x1333x1277 43 and 41,
+// 1536^3 45 and 41.  (Products whose TF32 tiles fill little more than one wave cross earlier: 1200^3 at 0.8 with 38 and 36.)
 // What the streamed-operand kernel or the direct operands serve stays there.
 bool gemm_h16_serves(const b200_ctx* ctx, const GemmProblem& p) {
     if (ctx->gemm_precision != B200_GEMM_3XTF32 || !ctx->gemm_half_terms || ctx->gemm_operands >= 0 || ctx->gemm_stream > 0 ||
@@ -949,6 +948,11 @@ bool gemm_h16_serves(const b200_ctx* ctx, const GemmProblem& p) {
            !(ctx->lone_matmul && gemm_tc_reads_directly(ctx, p));
 }
 
+std::string gemm_h16_tile(const b200_ctx* ctx, const GemmProblem& p) {
+    const TileChoice t = choose_tile(p, 3, ctx->prop.multiProcessorCount);
+    return std::to_string(t.cg * kRowsM) + "x" + std::to_string(t.bn);
+}
+
 void gemm_h16_note_uses(b200_ctx* ctx, const GemmProblem& p) {
     HalfOperand a = operand_a(p), b = operand_b(p);
     lay_out_planes(a);
@@ -959,7 +963,7 @@ void gemm_h16_note_uses(b200_ctx* ctx, const GemmProblem& p) {
 
 void gemm_h16(b200_ctx* ctx, const GemmProblem& p) {
     HalfOperand a = operand_a(p), b = operand_b(p);
-    const TileChoice t = choose_tile(p, 3, b.mn, ctx->prop.multiProcessorCount);
+    const TileChoice t = choose_tile(p, 3, ctx->prop.multiProcessorCount);
     if (ctx->range_next + 2 > kRangeSlots) {
         gemm_tc(ctx, p, true);
         return;
@@ -1078,7 +1082,7 @@ bool gemm_f16_storage(b200_ctx* ctx, const GemmProblem& p, const HalfEpilogue* e
     }
     if (2.0 * double(p.m) * double(p.n) * double(p.k) * double(p.b0 * p.b1) < double(1 << 25)) return false;
     HalfOperand a = operand_a(p), b = operand_b(p);
-    const TileChoice t = choose_tile(p, 1, b.mn, ctx->prop.multiProcessorCount);
+    const TileChoice t = choose_tile(p, 1, ctx->prop.multiProcessorCount);
     if (epi != nullptr) {
         // the epilogue adds where it stores 64 whole columns: no K-slices, no ragged edge
         for (const void* q : {static_cast<const void*>(p.out), epi->bias, static_cast<const void*>(epi->biased), static_cast<const void*>(epi->rectified)}) {
