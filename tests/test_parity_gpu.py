@@ -424,6 +424,62 @@ def test_device_copies(backend):
     assert z.data == 0 and z.nbytes == 0
 
 
+def test_many_device_copies_in_one_batch(backend):
+    """More ranges than one launch takes, empty, tiny and several tiles long, on any byte."""
+    from vkml_b200 import DeviceTensor, DType
+    rng = np.random.default_rng(12)
+    src = rng.integers(0, 256, 1 << 20, dtype=np.uint8)
+    a, b = DeviceTensor.from_host(backend, src.view(np.int32)), DeviceTensor.from_host(backend, np.zeros(1 << 18, dtype=np.int32))
+    want, batch, at = np.zeros(1 << 20, dtype=np.uint8), [], 0
+    for i in range(101):
+        size = [0, 1, 15, 16, 33, 4096, 16385, 40000][i % 8]
+        to, start = at + int(rng.integers(0, 17)), int(rng.integers(0, (1 << 20) - size))
+        batch.append((b.storage, to, a.storage, start, size))
+        want[to:to + size] = src[start:start + size]
+        at = to + size
+    assert at <= 1 << 20
+    backend.copy_device_to_device(batch)
+    np.testing.assert_array_equal(b.numpy().view(np.uint8), want)
+
+
+def test_device_copies_take_effect_in_order(backend):
+    """A copy that reads an earlier one's target, one that overwrites an earlier one's source, one that overwrites its target."""
+    from vkml_b200 import DeviceTensor
+    n = 1 << 20
+    data = [np.full(n, i, dtype=np.float32) for i in range(4)]
+    a, b, c, d = (DeviceTensor.from_host(backend, x) for x in data)
+    backend.copy_device_to_device([(b.storage, 0, a.storage, 0, 4 * n), (c.storage, 0, b.storage, 0, 4 * n), (a.storage, 0, d.storage, 0, 4 * n),
+                                   (b.storage, 8, d.storage, 0, 4 * n - 8)])
+    want_b = np.full(n, 3, dtype=np.float32)
+    want_b[:2] = 0
+    for t, want in ((a, data[3]), (b, want_b), (c, data[0]), (d, data[3])):
+        np.testing.assert_array_equal(t.numpy(), want)
+
+
+# transposed gradients of whole tiles, odd remainders and single rows and columns beside dense ones, and one too large for the group
+@pytest.mark.parametrize("shapes", [[(64, 64), (65, 130), (1, 7), (128, 784), (10, 1)], [(200, 63), (3, 2), (1024, 1024), (1100, 1000)]])
+def test_optimiser_group_with_transposed_gradients(backend, shapes):
+    from vkml_b200 import DeviceTensor, NodeDesc
+    rng = np.random.default_rng(4)
+    keep, nodes, wants = [], [], []
+    for rows, cols in shapes:
+        for turned in (True, False):
+            p, g = rng.standard_normal((rows, cols), dtype=np.float32), rng.standard_normal((rows, cols), dtype=np.float32)
+            dp = DeviceTensor.from_host(backend, p)
+            dg = DeviceTensor.from_host(backend, np.ascontiguousarray(g.T)).transpose(0, 1) if turned else DeviceTensor.from_host(backend, g)
+            out = DeviceTensor.empty(backend, (rows, cols))
+            keep.append((dp, dg, out))
+            nodes.append(NodeDesc(Op.SCALED_ADD, out.desc, [dp.desc, dg.desc], graph.scaled_add_params(0.9, -0.25)))
+            wants.append(np.float32(0.9) * p + np.float32(-0.25) * g)
+    backend.set_profiling(True)
+    backend.compute(nodes)
+    labels = [l for l, _ in backend.last_profile()]
+    backend.set_profiling(False)
+    assert "fused.scaled_add_group" in labels, labels
+    for (_, _, out), want in zip(keep, wants):
+        assert np.array_equal(out.numpy().view(np.uint32), want.view(np.uint32)), out.dims
+
+
 def test_which_kernel_a_product_gets(backend):
     """b200_matmul_kernel names the kernel a product would get, taken by itself, and the profile of
     the product run by itself agrees: CUDA cores for a tiny product, operand planes for a large

@@ -1671,16 +1671,25 @@ __global__ void __launch_bounds__(kThreads) copy_ranges_kernel(const __grid_cons
 }  // namespace
 
 void launch_copies(b200_ctx* ctx, const b200_copy* copies, size_t n) {
-    for (size_t i0 = 0; i0 < n; i0 += kCopyRanges) {
+    auto meet = [](const char* a, uint64_t na, const char* b, uint64_t nb) { return a < b + nb && b < a + na; };
+    for (size_t i = 0; i < n;) {
         CopyRanges g{};
         uint64_t blocks = 0;
-        for (size_t i = i0; i < n && i < i0 + kCopyRanges; ++i) {
-            const uint64_t need = (copies[i].nbytes + kCopyTile - 1) / kCopyTile;
-            g.dst[g.n] = static_cast<char*>(copies[i].dst);
-            g.src[g.n] = static_cast<const char*>(copies[i].src);
-            g.bytes[g.n] = copies[i].nbytes;
+        for (; i < n && g.n < kCopyRanges; ++i) {
+            char* dst = static_cast<char*>(copies[i].dst);
+            const char* src = static_cast<const char*>(copies[i].src);
+            const uint64_t bytes = copies[i].nbytes;
+            // copies take effect in the order of the list: what meets an earlier one's target, or overwrites its source, waits for the next launch
+            bool later = false;
+            for (int j = 0; j < g.n && !later; ++j) {
+                later = meet(g.dst[j], g.bytes[j], src, bytes) || meet(g.dst[j], g.bytes[j], dst, bytes) || meet(g.src[j], g.bytes[j], dst, bytes);
+            }
+            if (later) break;
+            g.dst[g.n] = dst;
+            g.src[g.n] = src;
+            g.bytes[g.n] = bytes;
             g.first_block[g.n++] = static_cast<uint32_t>(blocks);
-            blocks += need;
+            blocks += (bytes + kCopyTile - 1) / kCopyTile;
         }
         g.first_block[g.n] = static_cast<uint32_t>(blocks);
         launch_kernel(ctx, copy_ranges_kernel, static_cast<unsigned>(blocks), kThreads, 0, g);
