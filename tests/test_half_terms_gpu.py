@@ -282,3 +282,29 @@ def test_f16_linear_layers(backend, m, k, n, relu):
     assert np.array_equal(z.numpy().view(np.uint16), summed.view(np.uint16))
     if relu:
         assert np.array_equal(h.numpy(), np.where(summed <= 0, np.float16(0), summed))
+
+
+def test_f16_linear_layer_keeps_infinities_and_nans(backend):
+    """In the fused epilogue as in separate nodes: a NaN stays one through bias and relu, an infinity keeps its sign."""
+    rng = np.random.default_rng(1)
+    m, k, n = 512, 256, 1024
+    x, w = rng.standard_normal((m, k)).astype(np.float16), rng.standard_normal((n, k)).astype(np.float16)
+    bias = rng.standard_normal(n).astype(np.float16)
+    x[5, 3], x[6, 4], x[7, 200] = np.inf, np.nan, -np.inf
+    bias[9], bias[10], bias[11] = np.inf, np.nan, -np.inf
+    dx, dw = (DeviceTensor.from_host(backend, t.reshape((1, 1) + t.shape)) for t in (x, w))
+    db = DeviceTensor.from_host(backend, bias)
+    y, z, h = (DeviceTensor.empty(backend, (m, n), DType.F16) for _ in range(3))
+    backend.set_profiling(True)
+    backend.compute([NodeDesc(int(Op.MATMUL), y.reshape((1, 1, m, n)).desc, [dx.desc, dw.transpose(2, 3).desc]),
+                     NodeDesc(int(Op.ADD), z.desc, [y.desc, db.broadcast_to((m, n)).desc]), NodeDesc(int(Op.RELU), h.desc, [z.desc])])
+    labels = [l for l, _ in backend.last_profile()]
+    backend.set_profiling(False)
+    assert labels == ["matmul.tcgen05_f16_bias"], labels
+    with np.errstate(invalid="ignore"):
+        exact = x.astype(np.float64) @ w.astype(np.float64).T
+        got = y.numpy()
+        assert np.array_equal(np.isnan(got), np.isnan(exact)) and np.array_equal(got[5:8:2], exact[5:8:2].astype(np.float16), equal_nan=True)
+        summed = (got.astype(np.float32) + bias.astype(np.float32)).astype(np.float16)
+    assert np.array_equal(z.numpy(), summed, equal_nan=True)
+    assert np.array_equal(h.numpy(), np.where(summed <= 0, np.float16(0), summed), equal_nan=True)
