@@ -225,7 +225,8 @@ int b200_get_gemm_precision(b200_ctx* ctx);
  * (vulkan_backend.cpp:2363-2375) so that a run can be tied to the arithmetic that produced it.
  * Names: fp32_simt (CUDA cores), tcgen05_3xtf32 (operand planes), tcgen05_3xtf32_stream (the large
  * operand streamed once through tensor memory), tcgen05_3xtf32_direct (fp32 tiles split inside
- * the kernel), and the tcgen05_tf32* forms under the plain-TF32 precision.  The node is judged by
+ * the kernel), tcgen05_3xf16 (large products, two half terms per operand; the reason ends with the
+ * tile), and the tcgen05_tf32* forms under the plain-TF32 precision.  The node is judged by
  * itself: inside a span, planes shared with another matmul keep a product on the plane scheme. */
 int b200_matmul_kernel(b200_ctx* ctx, const b200_node* node, char* name, size_t name_len, char* reason,
                        size_t reason_len);
