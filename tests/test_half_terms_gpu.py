@@ -50,19 +50,6 @@ def test_f32_products_from_half_terms(backend, m, k, n, layout):
     assert rel(got, a, b) < 6e-6
 
 
-@pytest.mark.parametrize("m,k,n", [(1280, 1536, 1280), (400, 900, 100)])
-def test_a_product_does_not_depend_on_what_reads_it(backend, m, k, n):
-    """The same bits whether a span only stores the product or feeds it to a bias and a ReLU."""
-    rng = np.random.default_rng(m)
-    x, w, bias = (rng.standard_normal(s, dtype=np.float32) for s in ((m, k), (k, n), (n,)))
-    alone, _ = product(backend, x, w, "nn")
-    dx, dw, db = (DeviceTensor.from_host(backend, t) for t in (x.reshape(1, 1, m, k), w.reshape(1, 1, k, n), bias))
-    y, z, h = (DeviceTensor.empty(backend, (m, n)) for _ in range(3))
-    backend.compute([NodeDesc(int(Op.MATMUL), y.reshape((1, 1, m, n)).desc, [dx.desc, dw.desc]),
-                     NodeDesc(int(Op.ADD), z.desc, [y.desc, db.broadcast_to((m, n)).desc]), NodeDesc(int(Op.RELU), h.desc, [z.desc])])
-    assert same_bits(y.numpy().reshape(alone.shape), alone) and same_bits(h.numpy(), np.maximum(y.numpy() + bias, 0))
-
-
 @pytest.mark.parametrize("m,k,n,half", [(1024, 1024, 1024, False), (2048, 1024, 1023, False), (2048, 1024, 1024, True), (2048, 1025, 1024, True)])
 def test_from_which_size_on(backend, m, k, n, half):
     rng = np.random.default_rng(m + n)

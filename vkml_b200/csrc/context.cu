@@ -287,6 +287,43 @@ bool half_linear(const b200_node& mm, const b200_node& add, const b200_node* rel
     return true;
 }
 
+size_t tensor_span_bytes(const b200_tensor& t) {
+    size_t n = dtype_size(t.dtype);
+    for (int d = 0; d < t.ndim; ++d) n *= static_cast<size_t>(t.dims[d]);
+    return n;
+}
+
+// Notes the large products whose result this span compares with something -- a ReLU and its mask, a pooling
+// maximum -- directly or with one bias added.  They keep the TF32 terms bit for bit, so that a program's first forward pass decides its units as it
+// always has: between two arithmetics about one unit in 1e5 switches, and with them the wide MLP's gradients differ by 7e-3 (2-norm)
+// and single ones by up to 0.6 of their rms, more than results are held to from version to version.  It is no matter of accuracy --
+// half terms decide a sixth as many units otherwise than float64 -- and holds until the first update: the backward products take half terms.
+void note_compared_products(b200_ctx* ctx, const b200_node* nodes, size_t n_nodes) {
+    ctx->compared.clear();
+    for (size_t i = 0; i + 1 < n_nodes; ++i) {
+        const b200_node& m = nodes[i];
+        if (m.op != B200_OP_MATMUL || m.out.data == nullptr || m.out.dtype != B200_F32) continue;
+        const char* at[2] = {static_cast<const char*>(m.out.data), nullptr};
+        size_t bytes[2] = {tensor_span_bytes(m.out), 0};
+        for (size_t j = i + 1; j < n_nodes; ++j) {
+            const b200_node& n = nodes[j];
+            bool reads = false;
+            for (uint32_t k = 0; k < n.n_src && k < B200_MAX_SRC; ++k) {
+                const char* p = static_cast<const char*>(n.src[k].data);
+                for (int q = 0; q < 2; ++q) reads = reads || (at[q] != nullptr && p >= at[q] && p < at[q] + bytes[q]);
+            }
+            if (!reads) continue;
+            if (n.op == B200_OP_ADD && at[1] == nullptr) {
+                at[1] = static_cast<const char*>(n.out.data);
+                bytes[1] = tensor_span_bytes(n.out);
+            } else if (n.op == B200_OP_RELU || n.op == B200_OP_MAX_POOL2D || (n.op >= B200_OP_MAXIMUM && n.op <= B200_OP_NOT_EQUAL)) {
+                ctx->compared.insert(m.out.data);
+                break;
+            }
+        }
+    }
+}
+
 // Counts, before a span runs, how often each operand matrix feeds a tensor-core matmul, so
 // that a matrix used twice (a weight in forward and backward, an activation in forward and in
 // the weight gradient) is split into its TF32 planes only once.
@@ -768,6 +805,7 @@ static void compute_span(b200_ctx* ctx, const b200_node* nodes, size_t n_nodes, 
             gemm_tc_end_span(c);
         }
     } span_guard{ctx};
+    note_compared_products(ctx, nodes, n_nodes);
     count_matmul_operands(ctx, nodes, n_nodes);
     std::vector<char> is_sink;
     if (grad_sync && ctx->grads.empty()) {

@@ -142,6 +142,7 @@ struct b200_ctx {
     void* d_ranges = nullptr;  // RangeSlot[kRangeSlots], cleared at a span's first use
     bool lone_matmul = true;   // the current span has one product at most: no planes to share
     int range_next = 0;        // slots taken in the current span
+    std::set<const void*> compared;  // results of the current span's products that keep TF32 terms (note_compared_products)
     int gemm_group_m = 0;      // VKML_B200_GEMM_GROUP_M: M-tiles per L2 group of the tile walk (0: the built-in 16)
     int gemm_bn_override = 0;  // VKML_B200_GEMM_BN: force the N extent of the tensor-core tile (tuning aid)
     // SMs the persistent GEMM kernel leaves free while a span's gradients are being all-reduced,

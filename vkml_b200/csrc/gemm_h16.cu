@@ -944,7 +944,7 @@ bool gemm_h16_serves(const b200_ctx* ctx, const GemmProblem& p) {
     const double flops = 2.0 * double(p.m) * double(p.n) * double(p.k) * double(p.b0 * p.b1);
     // (One accumulator over more than 12288 products leaves a TF32 result about 1e-4 from the exact one -- 4096 x 16384 x 4096: 1.15e-4, from
     // half terms 1.9e-5 -- so the two would differ by more than the 1e-4 that results have kept to from version to version.)
-    return flops >= 4294967296.0 && !gemm_tc_streams(ctx, p) && gemm_tc_chain(ctx, p) <= 12288 &&
+    return flops >= 4294967296.0 && !gemm_tc_streams(ctx, p) && ctx->compared.count(p.out) == 0 && gemm_tc_chain(ctx, p) <= 12288 &&
            !(ctx->lone_matmul && gemm_tc_reads_directly(ctx, p));
 }
 

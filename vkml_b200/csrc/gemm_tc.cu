@@ -1795,8 +1795,8 @@ TcPlan plan_planes(const b200_ctx* ctx, const GemmProblem& p) {
         // as many K-slices as keep every unit in ONE wave of the persistent grid: rounding up
         // instead (32 tiles x 5 slices = 160 units on 148 SMs) runs a second, nearly empty wave.  Slices of eight K-blocks
         // and more; of three where the tiles fill less than an eighth of the machine (a classifier's few columns: 300 x 900 x 100
-        // took 21 us with three CTAs to a tile)
-        const int64_t least = tiles * 8 <= sm_count() ? 3 : 8;
+        // took 21 us with three CTAs to a tile), unless the span compares the result, whose bits then stay
+        const int64_t least = tiles * 8 <= sm_count() && ctx->compared.count(p.out) == 0 ? 3 : 8;
         splits = std::min<int64_t>(sm_count() / tiles, k_blocks / least);
         splits = std::max<int64_t>(1, std::min<int64_t>(splits, 64));
     }
@@ -2140,6 +2140,7 @@ void gemm_tc_end_span(b200_ctx* ctx) {
     ctx->plane_cache_bytes = 0;
     ctx->range_next = 0;
     ctx->lone_matmul = true;  // (what is asked about between two spans is a product by itself: b200_matmul_kernel)
+    ctx->compared.clear();
 }
 
 }  // namespace b200
