@@ -33,7 +33,7 @@ def test_small_products(backend, batch, m, k, n, layout):
 @pytest.mark.parametrize("batch,m,k,n,small", [
     (1, 256, 256, 256, True), (1, 264, 264, 264, True), (1, 275, 376, 276, True), (1, 384, 384, 384, True), (1, 511, 256, 301, True), (1, 511, 256, 300, False),
     (1, 400, 400, 400, False), (1, 300, 484, 300, False), (1, 512, 512, 512, False), (1, 96, 784, 216, True), (1, 100, 784, 256, False),
-    (32, 128, 32, 128, False), (8, 128, 64, 128, True), (1, 700, 33, 700, False)])
+    (32, 128, 32, 128, True), (33, 128, 32, 128, False), (8, 128, 64, 128, True), (1, 700, 33, 700, True), (1, 740, 33, 740, False)])
 def test_which_products_are_small(backend, batch, m, k, n, small):
     rng = np.random.default_rng(m + k + n)
     a, b = rng.standard_normal((1, batch, m, k), dtype=np.float32), rng.standard_normal((1, batch, k, n), dtype=np.float32)

@@ -334,20 +334,19 @@ bool gemm_small(b200_ctx* ctx, const GemmProblem& p) {
 
 }  // namespace
 
-// Products of 2^24 to 2^27 operations: this kernel or the tensor cores?  Measured over 55 shapes in three layouts.  It wins while all CTAs are
-// resident at once, two to an SM -- with clusters of eight, of which an odd GPC holds fewer, 28 tiles: 96x784x256 11.1 against 15.4 us,
-// 128x784x256 (32 tiles) 15.8 against 15.8, 64x1024x512 17.4 against 14.5 -- and loses with more of them: 32 x 128x32x128 11.9 against
-// 8.1, 700x33x700 13.8 against 8.5, 64x64x8192 13.8 against 8.2.  Above 2^25 it wins against operands read directly or through planes while a CTA
-// has two rounds of K and the tensor cores no K-slices, which they have from sixteen K-blocks on: 264^3 12.5 against 17.2, 275x376x276 14.1
-// against 21.1, 384^3 15.6 against 21.2, 2048x136x68 10.5 against 12.3; but 300x900x100 15.4 against 13.4, 400^3 (four rounds) 20.8
-// against 22.4.  Streamed operands and batches stay on the tensor cores there (64x1024x512 above; 2 x 300x300x100 would take 13.3 for 18.5).
+// Products of up to 2^27 operations: this kernel or the tensor cores?  Up to 2^25 it is this one, in full fp32.  (With more CTAs than are
+// resident at once the tensor cores' 22 bits would be had sooner: 32 x 128x32x128 8.1 us against 11.9, 700x33x700 8.5 against 13.8.)
+// Above, measured over 55 shapes in three layouts, it wins against operands read directly or through planes while all CTAs are
+// resident, two to an SM, a CTA has two rounds of K and the tensor cores no K-slices, which they have from sixteen K-blocks on:
+// 264^3 12.5 against 17.2 us, 275x376x276 14.1 against 21.1, 384^3 15.6 against 21.2, 2048x136x68 10.5 against 12.3; but 300x900x100 15.4 against
+// 13.4, 400^3 (four rounds) 20.8 against 22.4, 4096x100x100 (512 CTAs) 15.2 against 11.3.  Streamed operands and batches stay on the tensor cores
+// there (64x1024x512 14.5 against 17.4; 2 x 300x300x100 would take 13.3 for 18.5).
 bool gemm_small_pays(const GemmProblem& p, bool streams) {
     const double flops = 2.0 * double(p.m) * double(p.n) * double(p.k) * double(p.b0 * p.b1);
-    if (flops <= double(1 << 24)) return true;
-    if (flops > double(1 << 27)) return false;
+    if (flops <= double(1 << 25)) return true;
+    if (flops > double(1 << 27) || streams || p.b0 * p.b1 != 1) return false;
     const SmallPlan s = small_plan(p);
-    if (s.tiles * s.cs > 2 * sm_count() || (s.cs == 8 && s.tiles > 28)) return false;
-    return flops <= double(1 << 25) || (!streams && p.b0 * p.b1 == 1 && ceil_div(p.k, s.cs) <= 2 * kRound && p.k <= 480);
+    return s.tiles * s.cs <= 2 * sm_count() && ceil_div(p.k, s.cs) <= 2 * kRound && p.k <= 480;
 }
 
 void gemm_simt(b200_ctx* ctx, const GemmProblem& p) {
