@@ -930,11 +930,12 @@ MatrixArgs matrix_args(const HalfOperand& o) {
 
 }  // namespace
 
-// Products of 2^32 operations and more: the range pass (a read of a sample) and the two launches that stand by behind the product cost
-// about 8 us together, which the halved MMA time does not return on smaller ones.  Measured on both sides of the line, TF32 terms
-// against half terms: 1024^3 (half of it) 26.8 and 29.7 us, 1000x1433x777 (half) 34.5 and 38.0, 1024x1536x1024 (0.75) 32.4 and 35.4,
-// 2000x511x2001 (0.95) 35.5 and 36.0; 2048x1024x1024 35.6 and 34.3, 512x8192x512 49.6 and 44.3, 512x2048x2048 41.0 and 40.2, 1301x1333x1277 43 and 41,
-// 1536^3 45 and 41.  (Products whose TF32 tiles fill little more than one wave cross earlier: 1200^3 at 0.8 with 38 and 36.)
+// Products above 2^31 operations.  The range pass (a read of a sample) and the launches that stand by behind the product cost
+// about 8 us together, which the halved MMA time returns from 2^32 on: 2048x1024x1024 36.2 us with TF32 terms and 34.2 with half
+// terms, 512x8192x512 49.6 and 44.3, 1301x1333x1277 43.2 and 41.2, 1536^3 45 and 41.  Between 2^31 and 2^32 TF32 terms are quicker as a rule --
+// 1000x1433x777 34.6 and 36.6, 1024x1536x1024 33.5 and 34.2, 1536x700x1536 28.7 and 31.0, 511x4097x513 34.5 and 42.5 -- but five times further
+// from the exact product (5e-6 against 9e-7 on those), and what has half terms' error keeps it.  Below, they would be quicker by a
+// third: 768x1024x768 21.3 and 30.4, 1024^3 26.8 and 29.
 // What the streamed-operand kernel or the direct operands serve stays there.
 bool gemm_h16_serves(const b200_ctx* ctx, const GemmProblem& p) {
     if (ctx->gemm_precision != B200_GEMM_3XTF32 || !ctx->gemm_half_terms || ctx->gemm_operands >= 0 || ctx->gemm_stream > 0 ||
@@ -944,7 +945,7 @@ bool gemm_h16_serves(const b200_ctx* ctx, const GemmProblem& p) {
     const double flops = 2.0 * double(p.m) * double(p.n) * double(p.k) * double(p.b0 * p.b1);
     // (One accumulator over more than 12288 products leaves a TF32 result about 1e-4 from the exact one -- 4096 x 16384 x 4096: 1.15e-4, from
     // half terms 1.9e-5 -- so the two would differ by more than the 1e-4 that results have kept to from version to version.)
-    return flops >= 4294967296.0 && !gemm_tc_streams(ctx, p) && ctx->compared.count(p.out) == 0 && gemm_tc_chain(ctx, p) <= 12288 &&
+    return flops > 2147483648.0 && !gemm_tc_streams(ctx, p) && ctx->compared.count(p.out) == 0 && gemm_tc_chain(ctx, p) <= 12288 &&
            !(ctx->lone_matmul && gemm_tc_reads_directly(ctx, p));
 }
 
