@@ -821,7 +821,7 @@ TileChoice choose_tile(const GemmProblem& p, int passes, int sms) {
     //   8192^3 2471 2990 3004 4732;  2048x8192x8192 703 796 760 1330;  3000^3 148 169 235 317;  6000x2000x576 77 92 92 107;
     //   1536^3 47.2 41.6 39.7 51.5;  300x8192x1000 54 54 49 57;  512x8192x512 47 43 42 48;  1200x4000x520 49 48 47 60;  20000x2000x64 139 123 125 121.
     // (256x64 was slower than one of these on every product: 6000x2000x576 108, 1200x4000x520 62.)
-    static const Form three[] = {{2, 256, 1.65, 6}, {2, 128, 1.0, 2}, {1, 128, 1.03, 1}, {1, 64, 0.85, 2}};
+    static const Form three[] = {{2, 256, 1.65, 6}, {2, 128, 1.0, 2}, {1, 128, 1.08, 2}, {1, 64, 0.9, 2}};
     static const Form one[] = {{2, 256, 1.75, 2}, {1, 128, 1.08, 2}, {1, 64, 0.6, 2}};
     const Form* forms = passes == 3 ? three : one;
     const int64_t batches = p.b0 * p.b1, k_blocks = ceil_div(p.k, kBlockK);
