@@ -812,8 +812,9 @@ struct TileChoice {
 // operand bytes per product (relative cost per unit of work beside the widest), so it is taken only
 // where the widest one would leave SMs idle: few tiles, or a nearly empty last wave.
 TileChoice choose_tile(const GemmProblem& p, int passes, int sms) {
-    struct Form { int cg, bn; double cost, drain; };
-    // cost of one K-block of a tile in units of a 256 x 128 tile's, and K-blocks that its fill and drain come to.  Three
+    struct Form { int cg, bn; double cost, alone, drain; };
+    // cost of one K-block of a tile in units of a 256 x 128 tile's, the same where one wave serves the product (a CTA by itself starts and
+    // ends sooner than a pair, but fetches B for half as many rows), and K-blocks that its fill and drain come to.  Three
     // passes over 256 columns leave room for one pair of accumulators, so that tile's epilogue is not hidden; its operand
     // traffic per product is two thirds, which at the power cap is worth 14 % (8192^3: 3.15 -> 2.69 ms sustained).  A 64-wide tile
     // costs nearly what a 128-wide one does, the instructions being the limit.  Each form forced for 30 products of 2^32 to 2^40 operations: with
@@ -821,8 +822,8 @@ TileChoice choose_tile(const GemmProblem& p, int passes, int sms) {
     //   8192^3 2471 2990 3004 4732;  2048x8192x8192 703 796 760 1330;  3000^3 148 169 235 317;  6000x2000x576 77 92 92 107;
     //   1536^3 47.2 41.6 39.7 51.5;  300x8192x1000 54 54 49 57;  512x8192x512 47 43 42 48;  1200x4000x520 49 48 47 60;  20000x2000x64 139 123 125 121.
     // (256x64 was slower than one of these on every product: 6000x2000x576 108, 1200x4000x520 62.)
-    static const Form three[] = {{2, 256, 1.65, 6}, {2, 128, 1.0, 2}, {1, 128, 1.08, 2}, {1, 64, 0.9, 2}};
-    static const Form one[] = {{2, 256, 1.75, 2}, {1, 128, 1.08, 2}, {1, 64, 0.6, 2}};
+    static const Form three[] = {{2, 256, 1.65, 1.65, 6}, {2, 128, 1.0, 1.0, 2}, {1, 128, 1.08, 1.02, 1}, {1, 64, 0.9, 0.9, 2}};
+    static const Form one[] = {{2, 256, 1.75, 1.75, 2}, {1, 128, 1.08, 1.08, 2}, {1, 64, 0.6, 0.6, 2}};
     const Form* forms = passes == 3 ? three : one;
     const int64_t batches = p.b0 * p.b1, k_blocks = ceil_div(p.k, kBlockK);
     TileChoice best{};
@@ -840,7 +841,7 @@ TileChoice choose_tile(const GemmProblem& p, int passes, int sms) {
         c.units = tiles * c.splits;
         const double waves = double(ceil_div(c.units, slots));
         // (slices write and fold partial planes)
-        const double cost = waves * f.cost * (double(c.kb_per_split) + f.drain) + (c.splits > 1 ? 4.0 : 0.0);
+        const double cost = waves * (waves > 1 ? f.cost : f.alone) * (double(c.kb_per_split) + f.drain) + (c.splits > 1 ? 4.0 : 0.0);
         if (i == 0 || cost < least) {
             least = cost;
             best = c;
