@@ -245,7 +245,9 @@ GemmProblem matmul_problem(const b200_node& node) {
 
 void dispatch_matmul(b200_ctx* ctx, const b200_node& node) {
     const GemmProblem p = matmul_problem(node);
-    if (gemm_h16_serves(ctx, p) && gemm_tc_eligible(ctx, p)) {
+    if (gemm_inline_serves(ctx, p)) {
+        gemm_inline(ctx, p);
+    } else if (gemm_h16_serves(ctx, p) && gemm_tc_eligible(ctx, p)) {
         gemm_h16(ctx, p);
     } else if (ctx->gemm_precision != B200_GEMM_FP32 && gemm_tc_eligible(ctx, p)) {
         gemm_tc(ctx, p, ctx->gemm_precision == B200_GEMM_3XTF32);
@@ -648,6 +650,10 @@ int b200_create(int cuda_ordinal, b200_ctx** out) {
         }
         if (const char* e = std::getenv("VKML_B200_GEMM_HALF_TERMS")) {
             ctx->gemm_half_terms = std::string(e) != "0";
+        }
+        if (const char* e = std::getenv("VKML_B200_GEMM_INLINE")) {
+            const std::string v = e;
+            if (v != "auto") ctx->gemm_inline = std::atoi(e);
         }
         if (const char* e = std::getenv("VKML_B200_GEMM_BN")) {
             ctx->gemm_bn_override = std::atoi(e);
@@ -1558,7 +1564,11 @@ int b200_matmul_kernel(b200_ctx* ctx, const b200_node* node, char* name, size_t 
             why = "plain fp32 arithmetic was asked for";
         } else if (gemm_tc_eligible(ctx, p)) {
             const bool three = ctx->gemm_precision == B200_GEMM_3XTF32;
-            if (gemm_h16_serves(ctx, p)) {
+            if (gemm_inline_serves(ctx, p)) {
+                kernel = "tcgen05_3xf16";
+                why = "bound by reading its operands: two half terms per operand, split inside the kernel (TF32 planes where an operand's range is too "
+                      "wide for them), tiles of " + gemm_inline_tile(ctx, p);
+            } else if (gemm_h16_serves(ctx, p)) {
                 kernel = "tcgen05_3xf16";
                 why = "bound by the tensor cores: two half terms per operand (TF32 planes where an operand's range is too wide for them), tiles of " +
                       gemm_h16_tile(ctx, p);

@@ -139,6 +139,9 @@ struct b200_ctx {
     // VKML_B200_GEMM_HALF_TERMS: large F32 products from two half terms per operand where their range allows
     // it (gemm_h16.cu); 0: TF32 terms everywhere (A/B runs).
     bool gemm_half_terms = true;
+    // VKML_B200_GEMM_INLINE: products that are split inside their kernel (gemm_inline.cu).  auto (-1): where that is quicker; 0: never;
+    // 1: every product it can serve, whatever its size (A/B runs).
+    int gemm_inline = -1;
     void* d_ranges = nullptr;  // RangeSlot[kRangeSlots], cleared at a span's first use
     bool lone_matmul = true;   // the current span has one product at most: no planes to share
     int range_next = 0;        // slots taken in the current span

@@ -69,6 +69,17 @@ bool gemm_h16_serves(const b200_ctx* ctx, const GemmProblem& p);
 void gemm_h16(b200_ctx* ctx, const GemmProblem& p);
 void gemm_h16_note_uses(b200_ctx* ctx, const GemmProblem& p);
 std::string gemm_h16_tile(const b200_ctx* ctx, const GemmProblem& p);  // "rows x columns" of the tile it gets
+// Ranges of `n` matrices, cleared at a span's first use (null: the span has used them up); and the sum of the K-slices' partial planes.
+RangeSlot* gemm_h16_slots(b200_ctx* ctx, int n);
+void gemm_h16_fold(b200_ctx* ctx, const GemmProblem& p, const float* partial, int splits, const RangeGuard& guard, int wide_splits);
+// The same terms, split inside the product's kernel. gemm_inline.cu
+bool gemm_inline_serves(const b200_ctx* ctx, const GemmProblem& p);
+bool gemm_inline_fits(const GemmProblem& p);
+std::string gemm_inline_tile(const b200_ctx* ctx, const GemmProblem& p);
+bool gemm_h16_would_serve(const b200_ctx* ctx, const GemmProblem& p);  // (whatever else reads the operands without planes)
+bool gemm_h16_shares(const b200_ctx* ctx, const GemmProblem& p);       // another product of the span reads the planes of an operand
+double gemm_h16_time(const b200_ctx* ctx, const GemmProblem& p);       // estimate in us, its planes included
+void gemm_inline(b200_ctx* ctx, const GemmProblem& p);
 // Half storage: `p`'s pointers are to halves.  False: not a case for this kernel.  With an epilogue the nodes behind the
 // product -- add(y, bias along the rows) and perhaps relu -- are served as well.
 struct HalfEpilogue {

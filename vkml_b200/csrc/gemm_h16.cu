@@ -243,23 +243,6 @@ struct H16Tile {
     static constexpr int kTotal = kBars + 256 + 1024;
 };
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-
-// The address, in the cluster's shared window, of the even CTA's copy of a shared-memory location.
-__device__ __forceinline__ uint32_t lead_addr(uint32_t addr) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
-    return r;
-}
-
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
-}
-
 template <int CG>
 __device__ __forceinline__ void tma_tile(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1, int c2, int c3) {
     if constexpr (CG == 2) {
@@ -270,70 +253,6 @@ __device__ __forceinline__ void tma_tile(uint32_t dst, const CUtensorMap* map, u
     } else {
         tma_load_4d(dst, map, bar, c0, c1, c2, c3);
     }
-}
-
-template <int CG>
-__device__ __forceinline__ void umma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
-    if constexpr (CG == 2) {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-            ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
-    } else {
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-            ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(accumulate) : "memory");
-    }
-}
-
-// Arrives on `bar` of every CTA of the tile once the MMAs issued so far are done.
-template <int CG>
-__device__ __forceinline__ void commit_all(uint32_t bar) {
-    if constexpr (CG == 2) {
-        asm volatile(
-            "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-            ::"r"(bar), "h"(static_cast<uint16_t>(3)) : "memory");
-    } else {
-        umma_commit(bar);
-    }
-}
-
-template <int CG>
-__device__ __forceinline__ void tmem_get(uint32_t dst_smem, uint32_t cols) {
-    __syncwarp();
-    if constexpr (CG == 2) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(dst_smem), "r"(cols) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    } else {
-        tmem_alloc(dst_smem, cols);
-    }
-}
-
-template <int CG>
-__device__ __forceinline__ void tmem_put(uint32_t taddr, uint32_t cols) {
-    __syncwarp();
-    if constexpr (CG == 2) {
-        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
-    } else {
-        tmem_dealloc(taddr, cols);
-    }
-}
-
-// D = f32, A = B = f16.
-__host__ __device__ constexpr uint32_t h16_idesc(int m, int n, bool a_mn, bool b_mn) {
-    return (1u << 4) | (a_mn ? (1u << 15) : 0u) | (b_mn ? (1u << 16) : 0u) | (static_cast<uint32_t>(n >> 3) << 17) |
-           (static_cast<uint32_t>(m >> 4) << 24);
-}
-
-// Tiles of 16-bit elements, 128-byte swizzle.  K-major: rows of 64 halves, 8-row groups 1024 bytes apart,
-// one K-step is 32 bytes further.  MN-major: atoms of 64 K-rows x 128 bytes (64 elements along MN), 8-row
-// groups again 1024 bytes apart, the next atom along MN 8192 bytes further, one K-step 16 rows further.
-constexpr uint32_t kAtomBytes = kBlockK * 128;
-
-template <bool MN>
-__device__ __forceinline__ uint64_t h16_desc(uint32_t addr) {
-    return smem_desc(addr, MN ? kAtomBytes : 0, 1024, 2);
 }
 
 // Bounded by the tensor cores for the large products.  Layout of the roles as in gemm_tc_kernel: warp 0 TMA,
@@ -806,6 +725,7 @@ void launch_major(b200_ctx* ctx, const HalfOperand& a, const HalfOperand& b, con
 struct TileChoice {
     int cg, bn;
     int64_t tiles_m, tiles_n, splits, kb_per_split, units;
+    double cost;
 };
 
 // The tile whose whole waves cost least.  `width` x 128 rows of cg CTAs; a narrower or single-CTA tile moves more
@@ -845,6 +765,7 @@ TileChoice choose_tile(const GemmProblem& p, int passes, int sms) {
         if (i == 0 || cost < least) {
             least = cost;
             best = c;
+            best.cost = cost;
         }
     }
     return best;
@@ -939,6 +860,10 @@ MatrixArgs matrix_args(const HalfOperand& o) {
 // third: 768x1024x768 21.3 and 30.4, 1024^3 26.8 and 29.
 // What the streamed-operand kernel or the direct operands serve stays there.
 bool gemm_h16_serves(const b200_ctx* ctx, const GemmProblem& p) {
+    return gemm_h16_would_serve(ctx, p) && !(ctx->lone_matmul && gemm_tc_reads_directly(ctx, p));
+}
+
+bool gemm_h16_would_serve(const b200_ctx* ctx, const GemmProblem& p) {
     if (ctx->gemm_precision != B200_GEMM_3XTF32 || !ctx->gemm_half_terms || ctx->gemm_operands >= 0 || ctx->gemm_stream > 0 ||
         ctx->gemm_schedule == 1 || ctx->gemm_bn_override != 0 || !fits_tma(p)) {
         return false;
@@ -946,8 +871,22 @@ bool gemm_h16_serves(const b200_ctx* ctx, const GemmProblem& p) {
     const double flops = 2.0 * double(p.m) * double(p.n) * double(p.k) * double(p.b0 * p.b1);
     // (One accumulator over more than 12288 products leaves a TF32 result about 1e-4 from the exact one -- 4096 x 16384 x 4096: 1.15e-4, from
     // half terms 1.9e-5 -- so the two would differ by more than the 1e-4 that results have kept to from version to version.)
-    return flops > 2147483648.0 && !gemm_tc_streams(ctx, p) && ctx->compared.count(p.out) == 0 && gemm_tc_chain(ctx, p) <= 12288 &&
-           !(ctx->lone_matmul && gemm_tc_reads_directly(ctx, p));
+    return flops > 2147483648.0 && !gemm_tc_streams(ctx, p) && ctx->compared.count(p.out) == 0 && gemm_tc_chain(ctx, p) <= 12288;
+}
+
+bool gemm_h16_shares(const b200_ctx* ctx, const GemmProblem& p) {
+    for (HalfOperand o : {operand_a(p), operand_b(p)}) {
+        lay_out_planes(o);
+        const auto it = ctx->plane_uses.find(o.key);
+        if (it != ctx->plane_uses.end() && it->second >= 2) return true;
+    }
+    return false;
+}
+
+// The planes' bytes at the rate their pass runs at, the tiles (a K-block of the 256 x 128 tile takes 0.66 us) and the launches around them.
+double gemm_h16_time(const b200_ctx* ctx, const GemmProblem& p) {
+    const HalfOperand a = operand_a(p), b = operand_b(p);
+    return 8.0 * double(a.numel() + b.numel()) / 5.8e6 + 0.66 * choose_tile(p, 3, ctx->prop.multiProcessorCount).cost + 7.0;
 }
 
 std::string gemm_h16_tile(const b200_ctx* ctx, const GemmProblem& p) {
@@ -961,6 +900,21 @@ void gemm_h16_note_uses(b200_ctx* ctx, const GemmProblem& p) {
     lay_out_planes(b);
     ++ctx->plane_uses[a.key];
     ++ctx->plane_uses[b.key];
+}
+
+RangeSlot* gemm_h16_slots(b200_ctx* ctx, int n) {
+    if (ctx->range_next + n > kRangeSlots) return nullptr;
+    if (ctx->range_next == 0) {
+        // (a kernel, not a memset: it overlaps its neighbours' launches, which a memset between them would not let do so either)
+        launch_kernel(ctx, clear_ranges_kernel, 1u, kRangeSlots, 0, static_cast<uint4*>(ctx->d_ranges));
+        ctx->count_launch();
+    }
+    ctx->range_next += n;
+    return static_cast<RangeSlot*>(ctx->d_ranges) + (ctx->range_next - n);
+}
+
+void gemm_h16_fold(b200_ctx* ctx, const GemmProblem& p, const float* partial, int splits, const RangeGuard& guard, int wide_splits) {
+    run_fold<float>(ctx, p, partial, splits, guard, wide_splits);
 }
 
 void gemm_h16(b200_ctx* ctx, const GemmProblem& p) {

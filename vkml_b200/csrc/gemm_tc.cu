@@ -69,32 +69,6 @@ __global__ void wait_probe_kernel(uint32_t* status, uint64_t limit_ns) {
     }
 }
 
-// Shared-memory matrix descriptors, 128-byte swizzle, 32-bit elements.
-//
-// K-major tile ([rows][32 floats], one swizzle row per matrix row): 8-row groups are 1024
-// bytes apart (stride-dimension offset); the leading-dimension offset is unused because the
-// K extent of one instruction (8 floats = 32 bytes) lies inside the swizzle row.  One K step
-// advances the start address by 32 bytes.
-//
-// MN-major tile (the operand is stored with its M or N axis contiguous, as a row-major
-// [K][N] matrix is for B): the tile is a row of "atoms", each 32 K-rows of 128 bytes (32
-// floats along MN).  32-bit operands must use the 128-byte swizzle with 32-byte atomicity
-// here (layout type 1, TMA mode SWIZZLE_128B_ATOM_32B): the pattern repeats every 4 K-rows,
-// so the stride-dimension offset is 512 bytes; the next atom along MN starts kMnAtomBytes
-// later (leading-dimension offset).  One K step (8 K-rows) advances the start by 1024 bytes.
-constexpr uint32_t kMnAtomBytes = BK * 128;  // 32 K-rows x 128 bytes
-
-template <bool MN_MAJOR>
-__device__ __forceinline__ uint64_t operand_desc(uint32_t smem_addr) {
-    return MN_MAJOR ? smem_desc(smem_addr, kMnAtomBytes, 512, 1) : smem_desc(smem_addr, 0, 1024, 2);
-}
-
-// Instruction descriptor: D = f32, A = B = tf32, M x N tile, operand majors as given.
-__host__ __device__ constexpr uint32_t make_idesc(int m, int n, bool a_mn, bool b_mn) {
-    return (1u << 4) | (2u << 7) | (2u << 10) | (a_mn ? (1u << 15) : 0u) | (b_mn ? (1u << 16) : 0u) |
-           (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
-}
-
 // ---------------------------------------------------------------------------
 // Operand split pre-pass
 // ---------------------------------------------------------------------------
@@ -133,27 +107,6 @@ __device__ __forceinline__ void split_tf32_fast(float x, float& hi, float& lo) {
     const uint32_t r = __float_as_uint(x - fh);  // exact
     hi = fh;
     lo = __uint_as_float((r + 0x1000u) & 0xFFFFE000u);
-}
-
-// The same split without a branch, for the converter warps of the streamed-operand kernel: two
-// warps per scheduler cannot hide a taken-or-not decision per element, and sixteen independent
-// elements interleave only if they are one basic block.  hi on the integer pipe (add half a TF32
-// ulp, clear 13 bits; where that reaches the infinity exponent -- x is infinite, NaN, or finite
-// but rounds past the largest TF32 -- truncate instead, keeping a NaN a NaN), lo = tf32(x - hi)
-// on the conversion pipe, forced to zero for a non-finite x.  Same values as split_tf32.
-__device__ __forceinline__ void split_tf32_select(float x, uint32_t& hi, uint32_t& lo) {
-    const uint32_t b = __float_as_uint(x);
-    uint32_t h = (b + 0x1000u) & 0xFFFFE000u;
-    const bool nonfinite = (b & 0x7F800000u) == 0x7F800000u;
-    const bool over = nonfinite || (h & 0x7F800000u) == 0x7F800000u;  // (a NaN's carry can leave the exponent)
-    const bool is_nan = nonfinite && (b & 0x007FFFFFu) != 0u;
-    h = over ? (b & 0xFFFFE000u) : h;
-    h = is_nan ? (h | 0x00400000u) : h;
-    const float rest = x - __uint_as_float(h);  // exact for a finite x
-    uint32_t l;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(l) : "f"(rest));
-    hi = h;
-    lo = nonfinite ? 0u : l;
 }
 
 struct SplitArgs {
