@@ -37,6 +37,7 @@ namespace {
 
 constexpr int kRowsP = 128;  // accumulator lanes
 constexpr int kBlockK = 64;  // halves per K-block: one 128-byte swizzle row
+constexpr int kBlockTf32 = 32;  // floats of one
 constexpr int kStepK = 16;
 constexpr int kQuads = 8;    // float4 per converter thread and K-block
 constexpr int kGroup = 4;    // ... that are asked for and converted together
@@ -139,14 +140,15 @@ __device__ __forceinline__ int64_t batch_offset(const InlineSide& s, int64_t b1,
     return int64_t(bo) * s.s_b0 + int64_t(batch - bo * static_cast<uint32_t>(b1)) * s.s_b1;
 }
 
-// What one converter thread reads of its operand's tile and where it puts it: eight quads along the unit-stride axis.
-// K-major: 16 quads to a row of 64 K.  MN-major: ROWS / 4 quads to a K-row, K-rows 8 apart.
+// What one converter thread reads of its operand's tile and where it puts it: eight quads (TF32 terms: four) along the unit-stride axis.
+// K-major: 16 (8) quads to a row of 64 (32) K.  MN-major: ROWS / 4 quads to a K-row, K-rows 8 apart.
 // Past the matrix' last line or its last K the last one is read again: what a line too many gives lies outside C, and what a K too many gives is
 // cleared behind the conversion.  So no load needs a predicate.
 // QUAD: the unit-stride axis is whole quads, each on 16 bytes.
-template <bool MN, int ROWS, bool QUAD>
+template <bool MN, int ROWS, bool QUAD, bool TF32 = false>
 struct Feed {
-    static constexpr int kBlock = kBlockK;
+    static constexpr bool kMn = MN;
+    static constexpr int kBlock = TF32 ? kBlockTf32 : kBlockK;
     static constexpr int kQuads = kBlock / 8;
     static constexpr int kLanes = MN ? ROWS / 4 : kBlock / 4;
     static constexpr int kRowStep = 2 * ROWS / kLanes;
@@ -162,8 +164,12 @@ struct Feed {
         const int c = t % kLanes;
         along = 4 * c;
         row = t / kLanes;
-        offset = MN ? (c >> 4) * kAtomBytes + row * 128 + ((((c & 15) >> 1) ^ (row & 7)) << 4) + (c & 1) * 8
-                    : row * 128 + ((((c >> 1) ^ (row & 7))) << 4) + (c & 1) * 8;
+        if (TF32) {
+            offset = MN ? (c >> 3) * kMnAtomBytes + row * 128 + ((((c & 7) >> 1) ^ (row & 3)) << 5) + (c & 1) * 16 : row * 128 + ((c ^ (row & 7)) << 4);
+        } else {
+            offset = MN ? (c >> 4) * kAtomBytes + row * 128 + ((((c & 15) >> 1) ^ (row & 7)) << 4) + (c & 1) * 8
+                        : row * 128 + ((((c >> 1) ^ (row & 7))) << 4) + (c & 1) * 8;
+        }
         rows_apart = static_cast<int>(kRowStep * (MN ? s.s_k : s.s_mn) * 4);
     }
     __device__ __forceinline__ void place(int64_t b1, uint32_t batch, uint32_t tile, uint32_t kb, int K) {
@@ -187,6 +193,59 @@ struct Feed {
         const char* p = at + int64_t(min(i, last_row)) * rows_apart;
         if constexpr (QUAD) return load_quad(p);
         return make_float4(load_one(p), load_one(p + step[0]), load_one(p + step[1]), load_one(p + step[2]));
+    }
+    // (TF32 terms: of the sixteen elements, four to a quad)
+    __device__ __forceinline__ uint32_t word(int e) const { return offset + (e >> 2) * (kRowStep * 128) + (e & 3) * 4; }
+    __device__ __forceinline__ int k_of(int e) const { return MN ? row + kRowStep * (e >> 2) : along + (e & 3); }
+    __device__ __forceinline__ void put(uint8_t* to, int i, const uint32_t (&v)[4]) const {
+        *reinterpret_cast<uint4*>(to + word(4 * i)) = make_uint4(v[0], v[1], v[2], v[3]);
+    }
+};
+
+// The same for TF32 terms where rows do not lie on 16 bytes: a warp reads 32 neighbours along the unit axis at a time -- a row of the stage
+// (K-major), an atom's K-row (MN-major) -- and stores them one word to a lane.  (As four loads of a quad each, sixteen bytes from lane to lane,
+// every load touched as many lines as a quad's: 1166x129x4131 33.6 us, 172x1615x2684 39.8.)
+template <bool MN, int ROWS>
+struct LaneFeed {
+    static constexpr bool kMn = MN;
+    static constexpr int kQuads = 4;  // sixteen elements, four at a time
+    static constexpr int kWarps = ROWS / 16, kAtoms = ROWS / 32;
+    static constexpr int kStep = MN ? 2 : kWarps;  // rows between its elements
+    const InlineSide& s;
+    int lane, row, atom;   // of its first element
+    uint32_t even, odd;    // where its elements go: their swizzle alternates
+    const char* at;
+    int rows_apart, last_row;
+
+    __device__ __forceinline__ LaneFeed(const InlineSide& side, int t) : s(side) {
+        const int w = t >> 5;
+        lane = t & 31;
+        row = MN ? w / kAtoms : w;
+        atom = MN ? w % kAtoms : 0;
+        auto place_of = [&](int r) {
+            return static_cast<uint32_t>(MN ? atom * kMnAtomBytes + r * 128 + (((lane >> 3) ^ (r & 3)) << 5) + (lane & 7) * 4
+                                            : r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
+        };
+        even = place_of(row);
+        odd = place_of(row + kStep);
+        rows_apart = static_cast<int>(kStep * (MN ? s.s_k : s.s_mn) * 4);
+    }
+    __device__ __forceinline__ void place(int64_t b1, uint32_t batch, uint32_t tile, uint32_t kb, int K) {
+        const int line0 = static_cast<int>(tile * ROWS), k0 = static_cast<int>(kb * kBlockTf32);
+        const int lines = static_cast<int>(s.mn) - line0 - 1, ks = K - k0 - 1;  // behind the tile's first
+        const int first = min(MN ? 32 * atom + lane : lane, MN ? lines : ks), top = min(row, MN ? ks : lines);
+        const float* base = s.base + batch_offset(s, b1, batch);
+        at = reinterpret_cast<const char*>(base + int64_t(line0 + (MN ? first : top)) * s.s_mn + int64_t(k0 + (MN ? top : first)) * s.s_k);
+        last_row = min(15, ((MN ? ks : lines) - top) / kStep);
+    }
+    __device__ __forceinline__ void next() { at += kBlockTf32 * s.s_k * 4; }
+    __device__ __forceinline__ float one(int e) const { return load_one(at + int64_t(min(e, last_row)) * rows_apart); }
+    __device__ __forceinline__ float4 load(int i) const { return make_float4(one(4 * i), one(4 * i + 1), one(4 * i + 2), one(4 * i + 3)); }
+    __device__ __forceinline__ uint32_t word(int e) const { return (e & 1 ? odd : even) + (e >> 1) * (2 * kStep * 128); }
+    __device__ __forceinline__ int k_of(int e) const { return MN ? row + kStep * e : lane; }
+    __device__ __forceinline__ void put(uint8_t* to, int i, const uint32_t (&v)[4]) const {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) *reinterpret_cast<uint32_t*>(to + word(4 * i + j)) = v[j];
     }
 };
 
@@ -603,6 +662,269 @@ __global__ void __launch_bounds__(InlineTile<CG, BN>::kThreads, 1) gemm_inline_k
 }
 
 // ---------------------------------------------------------------------------
+// TF32 terms
+// ---------------------------------------------------------------------------
+
+// The same for products that take TF32 terms (gemm_tc.cu): hi and lo of each float as the planes would hold them, the same three MMAs per K-step, the
+// same K-slices, so the result is that of the planes bit for bit -- from one launch instead of two splits and a product, and with no
+// plane to write and read.  Neither range nor strays to look for.  One CTA to a 128 x BN tile.
+template <int BN>
+struct InlineTf32Tile {
+    static constexpr int kConverters = (kRowsP + BN) / 16;  // warps
+    static constexpr int kThreads = (kFirstConverter + kConverters) * 32;
+    static constexpr int kPBytes = kRowsP * kBlockTf32 * 4;
+    static constexpr int kQBytes = BN * kBlockTf32 * 4;
+    static constexpr int kStageBytes = 2 * (kPBytes + kQBytes);
+    static constexpr int kStages = 192 * 1024 / kStageBytes;
+    static constexpr int kTmemCols = 2 * BN;  // two accumulators
+    static constexpr int kConverterRegs = BN == 128 ? 96 : 112;
+    static constexpr int kBars = kStages * kStageBytes;
+    static constexpr int kTotal = kBars + 256 + 1024;
+};
+
+template <int BN, bool P_MN, bool Q_MN>
+__global__ void __launch_bounds__(InlineTf32Tile<BN>::kThreads, 1) gemm_inline_tf32_kernel(const __grid_constant__ InlineArgs g) {
+    using T = InlineTf32Tile<BN>;
+    constexpr int STAGES = T::kStages;
+    constexpr uint32_t kIdesc = make_idesc(kRowsP, BN, P_MN, Q_MN);
+    constexpr int kPitch = 36;
+    static_assert(8 * (2 * STAGES + 4) <= 256, "barrier block");
+
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
+    const uint32_t bars = base + T::kBars;
+    auto full_bar = [&](int s) { return bars + 8u * s; };               // a stage is converted
+    auto empty_bar = [&](int s) { return bars + 8u * (STAGES + s); };   // its MMAs are done
+    auto acc_full = [&](int a) { return bars + 8u * (2 * STAGES + a); };
+    auto acc_empty = [&](int a) { return bars + 8u * (2 * STAGES + 2 + a); };
+    __shared__ uint32_t tmem_base_slot;
+    __shared__ int abort_flag;
+    __shared__ __align__(16) float epi_patch[4][32][kPitch];
+
+    const int warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        abort_flag = 0;
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(full_bar(s), T::kConverters);
+            mbar_init(empty_bar(s), 1);
+        }
+        for (int a = 0; a < 2; ++a) {
+            mbar_init(acc_full(a), 1);
+            mbar_init(acc_empty(a), 4);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 4) {
+        tmem_alloc(smem_u32(&tmem_base_slot), T::kTmemCols);
+        tc_fence_before();
+    }
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = tmem_base_slot;
+    volatile int* abort_p = &abort_flag;
+    pdl_prologue();
+
+    // Registers: a launch of 768 threads has 80 each, one of 640 has 96; 512 x 96 (384 x 112) + 128 x 64 + 128 x 24 are fewer.
+    if (warp >= kFirstConverter) {
+        // ---------------- converters ----------------
+        set_registers<true, T::kConverterRegs>();
+        auto convert = [&](auto feed, const int index, const uint32_t tile_at, const uint32_t plane_bytes) {
+            using F = decltype(feed);
+            const int K = static_cast<int>(g.k);
+            // where the loads are, two stages ahead of the conversion; what is left of K there
+            uint32_t next_u = blockIdx.x, next_kb = 0, next_end = 0;
+            auto place = [&](const Unit& x, uint32_t kb) { feed.place(g.b1, x.batch, index == 0 ? x.tp : x.tq, kb, K); };
+            auto enter = [&] {
+                const Unit x = unit_of(g, next_u);
+                next_kb = x.kb0;
+                next_end = x.kb1;
+                place(x, x.kb0);
+            };
+            auto request = [&](float4 (&to)[F::kQuads], int& left) {
+                left = -1;  // nothing more to convert
+                if (next_u >= g.n_units) return;
+                left = K - static_cast<int>(next_kb) * kBlockTf32;
+#pragma unroll
+                for (int i = 0; i < F::kQuads; ++i) to[i] = feed.load(i);
+                if (++next_kb < next_end) {
+                    if (static_cast<int>(next_kb + 1) * kBlockTf32 <= K) feed.next();
+                    else place(unit_of(g, next_u), next_kb);
+                } else if ((next_u += gridDim.x) < g.n_units) {
+                    enter();
+                }
+            };
+            float4 v0[F::kQuads], v1[F::kQuads];
+            int left0, left1;
+            enter();
+            request(v0, left0);
+            request(v1, left1);
+            uint32_t it = 0;
+            auto step = [&](float4 (&q)[F::kQuads], int& left) {
+                const int s = it % STAGES;
+                if (!mbar_wait(empty_bar(s), ((it / STAGES) & 1) ^ 1, abort_p, g.status)) return false;
+                uint8_t* to = base_ptr + s * T::kStageBytes + tile_at;
+                uint32_t top = 0;
+#pragma unroll
+                for (int i = 0; i < F::kQuads; ++i) {
+                    for (float x : {q[i].x, q[i].y, q[i].z, q[i].w}) top = max(top, __float_as_uint(x) << 1);
+                }
+                if (top < 0xFEFFE000u) {
+                    // every value is finite and rounds inside the TF32 range: add half a TF32 ulp, clear 13 bits, lo = tf32(x - hi)
+#pragma unroll
+                    for (int i = 0; i < F::kQuads; ++i) {
+                        uint32_t hi[4], lo[4];
+                        const float x[4] = {q[i].x, q[i].y, q[i].z, q[i].w};
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            hi[j] = (__float_as_uint(x[j]) + 0x1000u) & 0xFFFFE000u;
+                            const float rest = x[j] - __uint_as_float(hi[j]);
+                            asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo[j]) : "f"(rest));
+                        }
+                        feed.put(to, i, hi);
+                        feed.put(to + plane_bytes, i, lo);
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < F::kQuads; ++i) {
+                        uint32_t hi[4], lo[4];
+                        const float x[4] = {q[i].x, q[i].y, q[i].z, q[i].w};
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) split_tf32_select(x[j], hi[j], lo[j]);
+                        feed.put(to, i, hi);
+                        feed.put(to + plane_bytes, i, lo);
+                    }
+                }
+                if (left < kBlockTf32) {
+                    // K past the matrix' end
+#pragma unroll 1
+                    for (int e = 0; e < 4 * F::kQuads; ++e) {
+                        if (feed.k_of(e) < left) continue;
+                        *reinterpret_cast<uint32_t*>(to + feed.word(e)) = 0;
+                        *reinterpret_cast<uint32_t*>(to + feed.word(e) + plane_bytes) = 0;
+                    }
+                }
+                request(q, left);
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(full_bar(s));
+                ++it;
+                return true;
+            };
+            while (left0 > 0 && step(v0, left0) && left1 > 0 && step(v1, left1)) {
+            }
+            if (threadIdx.x == kFirstConverter * 32) drain_commits<STAGES>(empty_bar, it, abort_p, g.status);
+        };
+        constexpr int kPWarps = kRowsP / 16;
+        const int t = threadIdx.x - kFirstConverter * 32;
+        if (warp < kFirstConverter + kPWarps) {
+            if (g.p.quads) convert(Feed<P_MN, kRowsP, true, true>(g.p, t), 0, 0, T::kPBytes);
+            else convert(LaneFeed<P_MN, kRowsP>(g.p, t), 0, 0, T::kPBytes);
+        } else {
+            if (g.q.quads) convert(Feed<Q_MN, BN, true, true>(g.q, t - kPWarps * 32), 1, 2 * T::kPBytes, T::kQBytes);
+            else convert(LaneFeed<Q_MN, BN>(g.q, t - kPWarps * 32), 1, 2 * T::kPBytes, T::kQBytes);
+        }
+    } else if (warp >= 4) {
+        // ---------------- MMA issuer ----------------
+        set_registers<false, 24>();
+        if (warp == 4 && lane == 0) {
+            uint32_t it = 0, tile_it = 0;
+            bool ok = true;
+            for (uint32_t u = blockIdx.x; u < g.n_units && ok; u += gridDim.x, ++tile_it) {
+                const Unit r = unit_of(g, u);
+                const int acc = tile_it & 1;
+                if (!mbar_wait(acc_empty(acc), ((tile_it >> 1) & 1) ^ 1, abort_p, g.status)) break;
+                tc_fence_after();
+                const uint32_t d = tmem_base + acc * BN;
+                for (uint32_t kb = r.kb0; kb < r.kb1; ++kb, ++it) {
+                    const int s = it % STAGES;
+                    if (!mbar_wait(full_bar(s), (it / STAGES) & 1, abort_p, g.status)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t stage = base + s * T::kStageBytes;
+                    const uint64_t p_hi = operand_desc<P_MN>(stage);
+                    const uint64_t p_lo = operand_desc<P_MN>(stage + T::kPBytes);
+                    const uint64_t q_hi = operand_desc<Q_MN>(stage + 2 * T::kPBytes);
+                    const uint64_t q_lo = operand_desc<Q_MN>(stage + 2 * T::kPBytes + T::kQBytes);
+#pragma unroll
+                    for (int kk = 0; kk < kBlockTf32 / 8; ++kk) {
+                        const uint64_t adv_p = static_cast<uint64_t>((P_MN ? kk * 1024 : kk * 32) >> 4);
+                        const uint64_t adv_q = static_cast<uint64_t>((Q_MN ? kk * 1024 : kk * 32) >> 4);
+                        const uint32_t first = (kb == r.kb0 && kk == 0) ? 0u : 1u;
+                        umma_tf32(d, p_lo + adv_p, q_hi + adv_q, kIdesc, first);
+                        umma_tf32(d, p_hi + adv_p, q_lo + adv_q, kIdesc, 1u);
+                        umma_tf32(d, p_hi + adv_p, q_hi + adv_q, kIdesc, 1u);
+                    }
+                    umma_commit(empty_bar(s));
+                }
+                if (ok) umma_commit(acc_full(acc));
+            }
+        }
+    } else {
+        // ---------------- epilogue ----------------
+        set_registers<false, 64>();
+        const bool vec = g.n % 4 == 0 && g.split_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(g.out) & 15) == 0;
+        uint32_t tile_it = 0;
+        for (uint32_t u = blockIdx.x; u < g.n_units; u += gridDim.x, ++tile_it) {
+            const Unit r = unit_of(g, u);
+            const int acc = tile_it & 1;
+            if (!mbar_wait_parked(acc_full(acc), (tile_it >> 1) & 1, abort_p, g.status)) break;
+            tc_fence_after();
+            const uint32_t t_acc = tmem_base + (static_cast<uint32_t>(warp * 32) << 16) + acc * BN;
+            const int64_t p0 = int64_t(r.tp) * kRowsP + warp * 32, q0 = int64_t(r.tq) * BN;
+            const int64_t p_left = g.m - p0;
+            float* out = g.out + int64_t(r.split) * g.split_stride + (int64_t(r.batch) * g.m + p0) * g.n + q0;
+            float* patch = &epi_patch[warp][0][0];
+#pragma unroll 1
+            for (int c = 0; c < BN; c += 32) {
+                const int64_t q_left = g.n - (q0 + c);
+                if (q_left <= 0 || p_left <= 0) break;  // uniform across the warp
+                uint32_t v[32];
+                tmem_ld32(t_acc + c, v);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    *reinterpret_cast<uint4*>(patch + lane * kPitch + 4 * j) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+                }
+                __syncwarp();
+                if (vec && q_left >= 32) {
+                    const int sub = lane >> 3, seg = lane & 7;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int rl = i * 4 + sub;
+                        if (rl < p_left) {
+                            *reinterpret_cast<float4*>(out + int64_t(rl) * g.n + c + seg * 4) = *reinterpret_cast<const float4*>(patch + rl * kPitch + seg * 4);
+                        }
+                    }
+                } else if (lane < q_left) {
+                    // a ragged right edge, or rows that do not begin on 16 bytes: a row's 32 columns per store
+                    const int rows = static_cast<int>(min(int64_t(32), p_left));
+#pragma unroll 4
+                    for (int rl = 0; rl < rows; ++rl) out[int64_t(rl) * g.n + c + lane] = patch[rl * kPitch + lane];
+                }
+                __syncwarp();
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_empty(acc));
+        }
+    }
+
+    __syncwarp();
+    __syncthreads();
+    if (abort_flag != 0) {
+        for (int i = 0; i < 200; ++i) __nanosleep(1000);  // MMAs in flight end before their memory is given up
+        __syncthreads();
+    }
+    if (warp == 4) {
+        tc_fence_after();
+        tmem_dealloc(tmem_base, T::kTmemCols);
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------
 
@@ -788,6 +1110,54 @@ void gemm_inline(b200_ctx* ctx, const GemmProblem& p) {
     const RangeGuard guard{side[0].range, side[1].range, side[0].limit, side[1].limit};
     gemm_tc_stand_by(ctx, p, guard, standby[0], standby[1], t.splits > 1 ? partial : p.out, partial);
     gemm_h16_fold(ctx, p, partial, static_cast<int>(t.splits), guard, wide_splits);
+}
+
+// TF32 terms split in the kernel: for products that would get TF32 planes, with their K-slices.
+void gemm_inline_tf32(b200_ctx* ctx, const GemmProblem& p, float* partial, int64_t splits, int64_t kb_per_split, const char* label) {
+    bool mn[2];
+    InlineArgs g{};
+    g.p = side_of(p.a, p.a_s, 2, 3, p.m, p, mn[0]);
+    g.q = side_of(p.b, p.b_s, 3, 2, p.n, p, mn[1]);
+    const int bn = p.n > 64 ? 128 : 64;
+    g.k = p.k;
+    g.b1 = p.b1;
+    g.out = splits > 1 ? partial : p.out;
+    g.m = p.m;
+    g.n = p.n;
+    g.tiles_p = static_cast<uint32_t>(ceil_div(p.m, int64_t(kRowsP)));
+    g.tiles_q = static_cast<uint32_t>(ceil_div(p.n, int64_t(bn)));
+    g.n_units = static_cast<uint32_t>(int64_t(g.tiles_p) * g.tiles_q * p.b0 * p.b1 * splits);
+    g.group_p = std::min<uint32_t>(g.tiles_p, 16);
+    g.k_blocks = static_cast<uint32_t>(ceil_div(p.k, int64_t(kBlockTf32)));
+    g.kb_per_split = static_cast<uint32_t>(kb_per_split);
+    g.by_splits = FastDiv(static_cast<uint32_t>(splits));
+    g.by_batch = FastDiv(g.tiles_p * g.tiles_q);
+    g.by_group = FastDiv(g.group_p * g.tiles_q);
+    g.split_stride = p.b0 * p.b1 * p.m * p.n;
+    g.status = ctx->d_status;
+    int sms = ctx->prop.multiProcessorCount;
+    if (ctx->in_grad_sync_span && ctx->comm_pending) sms = std::max(sms - ctx->comm_sms, sms / 2);
+    const int grid = static_cast<int>(std::min<int64_t>(g.n_units, sms));
+    auto launch = [&](auto tile, auto kernel) {
+        using T = decltype(tile);
+        B200_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kTotal));
+        launch_kernel(ctx, kernel, grid, T::kThreads, T::kTotal, g);
+    };
+    auto majors = [&](auto width) {
+        constexpr int BN = decltype(width)::value;
+        using T = InlineTf32Tile<BN>;
+        if (mn[0] && mn[1]) launch(T{}, gemm_inline_tf32_kernel<BN, true, true>);
+        else if (mn[0]) launch(T{}, gemm_inline_tf32_kernel<BN, true, false>);
+        else if (mn[1]) launch(T{}, gemm_inline_tf32_kernel<BN, false, true>);
+        else launch(T{}, gemm_inline_tf32_kernel<BN, false, false>);
+    };
+    {
+        ProfScope scope(ctx, label);
+        if (bn == 128) majors(std::integral_constant<int, 128>());
+        else majors(std::integral_constant<int, 64>());
+    }
+    ctx->count_launch();
+    check_last_launch("matmul (tcgen05, TF32 terms split in the kernel)");
 }
 
 bool gemm_inline_fits(const GemmProblem& p) {

@@ -1498,6 +1498,37 @@ bool direct_pays(const b200_ctx* ctx, const GemmProblem& p, int64_t batches, con
     return flops / 147e12 < 4.0 * (double(oa.plane_bytes) * share(oa) + double(ob.plane_bytes) * share(ob)) / 6.5e12;
 }
 
+// The plane kernel's tile width and K-slices.
+struct TcPlan {
+    int bn;
+    int64_t tiles_m, tiles_n, k_blocks, splits, kb_per_split;
+};
+
+// Whether the product is better off with operands split inside its kernel (gemm_inline.cu): where it is the only one of its span, and one wave
+// serves it.  Where fp32 tiles by TMA would be taken otherwise, always: the converters hold the operands in registers, not in a stage that the tensor
+// cores read (2816x1536x128 21.2 us -> 17.8, 704x1664x64 11.7 -> 10.4, 568x6746x228 32.2 -> 25.5).  Instead of planes, while K is not too long: a
+// K-block takes 1 us for 0.6 from planes, but there are no passes over the operands in front (512^3 16.8 -> 11.5, 1024^3 26.8 -> 23.3; rows that do
+// not lie on 16 bytes 637x947x201 19.0 -> 13.6, 37x8191x1999 79.5 -> 44.1, 681x1026x1021 29.1 -> 25.7; with three waves 1166x129x4131 26.2 -> 31.4;
+// 1540x41875x910 935 -> 1535).  A training step's products stay as they were: a CTA here takes an SM's registers whole, so neither this
+// kernel nor the one behind it is scheduled ahead, which costs such a step more than the passes (MLP 248-2451x3-56 545 us -> 562, two products of the
+// CNN 12 us).  A compared product of 2^28 operations, up to which fp32 tiles would serve it, keeps its planes.
+bool inline_pays(const b200_ctx* ctx, const GemmProblem& p, const Operand& oa, const Operand& ob, const TcPlan& plan, bool direct) {
+    if (ctx->gemm_inline == 0 || ctx->gemm_operands >= 0 || ctx->gemm_stream > 0 || ctx->gemm_bn_override != 0 || ctx->gemm_schedule == 1 ||
+        (ctx->gemm_schedule < 0 && ctx->in_grad_sync_span) || !gemm_inline_fits(p)) {
+        return false;
+    }
+    if (ctx->gemm_inline >= 8) return true;
+    if (!ctx->lone_matmul) return false;
+    const int64_t batches = p.b0 * p.b1, bn = p.n > 64 ? 128 : 64;
+    if (ceil_div(p.m, int64_t(BM)) * ceil_div(p.n, bn) * batches * plan.splits > sm_count()) return false;
+    if (direct) return true;
+    // us: K-blocks, what is around them, and the passes over the operands (12 bytes per element)
+    const double inline_us = double(plan.kb_per_split) + 7.0;
+    const double planes_us = 0.6 * double(plan.kb_per_split) + 12.0 * double(oa.plane_bytes + ob.plane_bytes) / 4 / 5.8e6 + 11.0;
+    const double flops = 2.0 * double(p.m) * double(p.n) * double(p.k) * double(batches);
+    return inline_us <= planes_us && (flops > double(1 << 28) || ctx->compared.count(p.out) == 0 || !maps_describe(p, oa, ob));
+}
+
 size_t plane_cache_limit(const b200_ctx* ctx) {
     return std::min<size_t>(size_t(16) << 30, ctx->prop.totalGlobalMem / 8);
 }
@@ -1714,12 +1745,6 @@ void gemm_stream(b200_ctx* ctx, const GemmProblem& p, bool three_pass, const Str
     release_use(ctx, ow);
 }
 
-// The plane kernel's tile width and K-slices.
-struct TcPlan {
-    int bn;
-    int64_t tiles_m, tiles_n, k_blocks, splits, kb_per_split;
-};
-
 TcPlan plan_planes(const b200_ctx* ctx, const GemmProblem& p) {
     const int64_t batches = p.b0 * p.b1;
     // Tile width: 128x256 tiles are the most efficient per tile (measured 5.5 % better than two
@@ -1822,10 +1847,22 @@ void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass) {
     Operand ob = plan_operand(p.b, p.b_s[0], p.b_s[1], p.b_s[3], p.b_s[2], p.n, p.k, b_bcast, p);
     const bool a_mn = oa.mn, b_mn = ob.mn;
 
-    // ---- direct operands: no planes at all ----
     const bool want_dynamic = ctx->gemm_schedule == 1 || (ctx->gemm_schedule < 0 && ctx->in_grad_sync_span);
-    if (ctx->gemm_operands != 0 && maps_describe(p, oa, ob) && !want_dynamic &&
-        (ctx->gemm_operands == 1 || direct_pays(ctx, p, batches, oa, ob))) {
+    const bool direct = ctx->gemm_operands != 0 && maps_describe(p, oa, ob) && !want_dynamic &&
+                        (ctx->gemm_operands == 1 || direct_pays(ctx, p, batches, oa, ob));
+    if (three_pass && inline_pays(ctx, p, oa, ob, plan, direct)) {
+        float* partial = nullptr;
+        if (splits > 1) {
+            char* ws = static_cast<char*>(ctx->ensure_workspace(partial_bytes + 2048));
+            partial = reinterpret_cast<float*>(align_up(reinterpret_cast<int64_t>(ws), 1024));
+        }
+        gemm_inline_tf32(ctx, p, partial, splits, kb_per_split, direct ? "matmul.tcgen05_3xtf32_direct" : "matmul.tcgen05_3xtf32");
+        fold_partials(ctx, p.out, partial, out_elems, static_cast<int>(splits));
+        return;
+    }
+
+    // ---- direct operands: no planes at all ----
+    if (direct) {
         float* partial = nullptr;
         if (splits > 1) {
             char* ws = static_cast<char*>(ctx->ensure_workspace(partial_bytes + 2048));
