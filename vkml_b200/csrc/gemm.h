@@ -89,6 +89,7 @@ struct HalfEpilogue {
     void* rectified;  // may be null
 };
 bool gemm_f16_storage(b200_ctx* ctx, const GemmProblem& p, const HalfEpilogue* epilogue = nullptr);
+bool gemm_f16_any(b200_ctx* ctx, const GemmProblem& p, const HalfEpilogue* epilogue);  // (operands that TMA cannot read, gemm_f16_any.cu)
 // True when gemm_tc would serve `p` with the streamed-operand kernel (a small left operand, the
 // right operand read once from HBM) rather than from operand planes.
 bool gemm_tc_streams(const b200_ctx* ctx, const GemmProblem& p);

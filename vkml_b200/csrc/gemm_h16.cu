@@ -1039,13 +1039,6 @@ bool gemm_f16_storage(b200_ctx* ctx, const GemmProblem& p, const HalfEpilogue* e
     if (2.0 * double(p.m) * double(p.n) * double(p.k) * double(p.b0 * p.b1) < double(1 << 25)) return false;
     HalfOperand a = operand_a(p), b = operand_b(p);
     const TileChoice t = choose_tile(p, 1, ctx->prop.multiProcessorCount);
-    if (epi != nullptr) {
-        // the epilogue adds where it stores 64 whole columns: no K-slices, no ragged edge
-        for (const void* q : {static_cast<const void*>(p.out), epi->bias, static_cast<const void*>(epi->biased), static_cast<const void*>(epi->rectified)}) {
-            if (reinterpret_cast<uintptr_t>(q) % 16 != 0) return false;
-        }
-        if (t.splits > 1 || p.n % 64 != 0 || p.b0 * p.b1 != 1) return false;
-    }
     auto direct = [](HalfOperand& o) {
         const bool ok = o.s_c == 1 && o.s_r % 8 == 0 && o.s_r >= o.cols && reinterpret_cast<uintptr_t>(o.src) % 16 == 0 &&
                         o.s_b0 % 8 == 0 && o.s_b1 % 8 == 0 && (o.nb == 1 || ((o.b1 == 1 || o.s_b1 > 0) && (o.nb == o.b1 || o.s_b0 > 0)));
@@ -1059,8 +1052,15 @@ bool gemm_f16_storage(b200_ctx* ctx, const GemmProblem& p, const HalfEpilogue* e
         }
         return ok;
     };
-    // (operands that TMA cannot read as they lie -- odd pitches -- are served through widened copies, dispatch_f16)
-    if (!direct(a) || !direct(b)) return false;
+    const bool readable = direct(a) && direct(b);
+    if (!readable) return gemm_f16_any(ctx, p, epi);
+    if (epi != nullptr) {
+        // the epilogue adds where it stores 64 whole columns: no K-slices, no ragged edge
+        for (const void* q : {static_cast<const void*>(p.out), epi->bias, static_cast<const void*>(epi->biased), static_cast<const void*>(epi->rectified)}) {
+            if (reinterpret_cast<uintptr_t>(q) % 16 != 0) return false;
+        }
+        if (t.splits > 1 || p.n % 64 != 0 || p.b0 * p.b1 != 1) return false;
+    }
     size_t bytes = 2048;
     if (t.splits > 1) bytes += static_cast<size_t>(p.b0 * p.b1 * p.m * p.n * t.splits * 4);
     char* ws = static_cast<char*>(ctx->ensure_workspace(bytes));

@@ -25,12 +25,13 @@
 // What bounds it: a ring of three stages of 64 K.  With the MMAs, the loads or both left out a K-block of the pair's tile takes 2375, 2560 and 1900
 // cycles for 3250: converting, handing over and multiplying add up around the ring.  512x65536x512: 182 us with planes, 119 here.
 #include "gemm.h"
-#include "tcgen05.cuh"
 
 #include <algorithm>
 #include <type_traits>
 
 #include <cuda_fp16.h>
+
+#include "gemm_inline.cuh"
 
 namespace b200 {
 namespace {
@@ -69,30 +70,10 @@ struct InlineArgs {
     float* out;       // C, or the partial planes when splits > 1
     int64_t m, n;     // of C
     int swap;         // q holds C's rows
-    uint32_t n_units, tiles_p, tiles_q, group_p, k_blocks, kb_per_split;
-    FastDiv by_splits, by_batch, by_group;  // K-slices; tiles of a batch; tiles of a group of P-tiles
+    UnitPlan units;
     int64_t split_stride;
     uint32_t* status;
 };
-
-// A tile and a K-slice of one batch.
-struct Unit {
-    uint32_t split, batch, tp, tq, kb0, kb1;
-};
-
-__device__ __forceinline__ Unit unit_of(const InlineArgs& g, uint32_t u) {
-    Unit r;
-    uint32_t t, in_batch, group, in_group;
-    g.by_splits.divmod(u, t, r.split);
-    g.by_batch.divmod(t, r.batch, in_batch);
-    g.by_group.divmod(in_batch, group, in_group);
-    const uint32_t first = group * g.group_p, rows = min(g.group_p, g.tiles_p - first);
-    r.tq = in_group / rows;
-    r.tp = first + (in_group - r.tq * rows);
-    r.kb0 = r.split * g.kb_per_split;
-    r.kb1 = min(r.kb0 + g.kb_per_split, g.k_blocks);
-    return r;
-}
 
 // CG CTAs share a tile of CG * 128 x BN: each holds its 128 rows of P and BN / CG of Q.
 template <int CG, int BN>
@@ -301,14 +282,6 @@ __device__ __forceinline__ void half_terms(uint64_t x, uint32_t& hi, uint32_t& l
     lo = *reinterpret_cast<const uint32_t*>(&l);
 }
 
-// The calling warps' register count from here on; their group of four warps calls it.
-template <bool MORE, int N>
-__device__ __forceinline__ void set_registers() {
-    __syncwarp();
-    if constexpr (MORE) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
-    else asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
-}
-
 // This warp's share of the sample, and the largest magnitude in it.
 __device__ __forceinline__ uint32_t take_sample(const InlineSide& s, int first, int apart, float (&v)[4 * kSamplePieces]) {
     const int lane = threadIdx.x & 31;
@@ -378,7 +351,7 @@ __global__ void __launch_bounds__(InlineTile<CG, BN>::kThreads, 1) gemm_inline_k
     volatile int* abort_p = &abort_flag;
     pdl_prologue();
 
-    auto decode = [&](uint32_t u) { return unit_of(g, u); };
+    auto decode = [&](uint32_t u) { return unit_of(g.units, u); };
     // whether the sample has shown that an operand is wide: nothing is computed then
     auto verdict = [&]() {
         return mbar_wait(verdict_bar, 0, abort_p, g.status) && ((volatile uint32_t*)sample_small)[0] <= kEarlyStrays &&
@@ -428,7 +401,7 @@ __global__ void __launch_bounds__(InlineTile<CG, BN>::kThreads, 1) gemm_inline_k
             const uint64_t s1 = pair_of(scale.s1, scale.s1);
             const bool two = scale.s2 != 1.0F;
             uint32_t it = 0;
-            for (; ok && u < g.n_units; u += unit_step) {
+            for (; ok && u < g.units.n_units; u += unit_step) {
                 const Unit now = at;
                 for (uint32_t kb = now.kb0; kb < now.kb1; ++kb, ++it) {
                     const int s = it % STAGES;
@@ -437,7 +410,7 @@ __global__ void __launch_bounds__(InlineTile<CG, BN>::kThreads, 1) gemm_inline_k
                     if (kb + 1 < now.kb1) {
                         if (static_cast<int>(kb + 2) * kBlockK <= K) feed.next();
                         else place(now, kb + 1);
-                    } else if (u + unit_step < g.n_units) {
+                    } else if (u + unit_step < g.units.n_units) {
                         at = decode(u + unit_step);
                         place(at, at.kb0);
                     } else {
@@ -542,7 +515,7 @@ __global__ void __launch_bounds__(InlineTile<CG, BN>::kThreads, 1) gemm_inline_k
         float finite = 0.0F;
         uint32_t it = 0, tile_it = 0;
         bool ok = any;
-        for (uint32_t u = unit0; ok && u < g.n_units; u += unit_step, ++tile_it) {
+        for (uint32_t u = unit0; ok && u < g.units.n_units; u += unit_step, ++tile_it) {
             const Unit r = decode(u);
             const int acc = tile_it % T::kAccs;
             if (warp == 4 && lane == 0 && rank == 0) {
@@ -737,21 +710,21 @@ __global__ void __launch_bounds__(InlineTf32Tile<BN>::kThreads, 1) gemm_inline_t
             uint32_t next_u = blockIdx.x, next_kb = 0, next_end = 0;
             auto place = [&](const Unit& x, uint32_t kb) { feed.place(g.b1, x.batch, index == 0 ? x.tp : x.tq, kb, K); };
             auto enter = [&] {
-                const Unit x = unit_of(g, next_u);
+                const Unit x = unit_of(g.units, next_u);
                 next_kb = x.kb0;
                 next_end = x.kb1;
                 place(x, x.kb0);
             };
             auto request = [&](float4 (&to)[F::kQuads], int& left) {
                 left = -1;  // nothing more to convert
-                if (next_u >= g.n_units) return;
+                if (next_u >= g.units.n_units) return;
                 left = K - static_cast<int>(next_kb) * kBlockTf32;
 #pragma unroll
                 for (int i = 0; i < F::kQuads; ++i) to[i] = feed.load(i);
                 if (++next_kb < next_end) {
                     if (static_cast<int>(next_kb + 1) * kBlockTf32 <= K) feed.next();
-                    else place(unit_of(g, next_u), next_kb);
-                } else if ((next_u += gridDim.x) < g.n_units) {
+                    else place(unit_of(g.units, next_u), next_kb);
+                } else if ((next_u += gridDim.x) < g.units.n_units) {
                     enter();
                 }
             };
@@ -831,8 +804,8 @@ __global__ void __launch_bounds__(InlineTf32Tile<BN>::kThreads, 1) gemm_inline_t
         if (warp == 4 && lane == 0) {
             uint32_t it = 0, tile_it = 0;
             bool ok = true;
-            for (uint32_t u = blockIdx.x; u < g.n_units && ok; u += gridDim.x, ++tile_it) {
-                const Unit r = unit_of(g, u);
+            for (uint32_t u = blockIdx.x; u < g.units.n_units && ok; u += gridDim.x, ++tile_it) {
+                const Unit r = unit_of(g.units, u);
                 const int acc = tile_it & 1;
                 if (!mbar_wait(acc_empty(acc), ((tile_it >> 1) & 1) ^ 1, abort_p, g.status)) break;
                 tc_fence_after();
@@ -868,8 +841,8 @@ __global__ void __launch_bounds__(InlineTf32Tile<BN>::kThreads, 1) gemm_inline_t
         set_registers<false, 64>();
         const bool vec = g.n % 4 == 0 && g.split_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(g.out) & 15) == 0;
         uint32_t tile_it = 0;
-        for (uint32_t u = blockIdx.x; u < g.n_units; u += gridDim.x, ++tile_it) {
-            const Unit r = unit_of(g, u);
+        for (uint32_t u = blockIdx.x; u < g.units.n_units; u += gridDim.x, ++tile_it) {
+            const Unit r = unit_of(g.units, u);
             const int acc = tile_it & 1;
             if (!mbar_wait_parked(acc_full(acc), (tile_it >> 1) & 1, abort_p, g.status)) break;
             tc_fence_after();
@@ -1085,15 +1058,7 @@ void gemm_inline(b200_ctx* ctx, const GemmProblem& p) {
     g.m = p.m;
     g.n = p.n;
     g.swap = t.swap ? 1 : 0;
-    g.n_units = static_cast<uint32_t>(t.units);
-    g.tiles_p = static_cast<uint32_t>(t.tiles_p);
-    g.tiles_q = static_cast<uint32_t>(t.tiles_q);
-    g.group_p = static_cast<uint32_t>(std::min<int64_t>(t.tiles_p, 8));
-    g.k_blocks = static_cast<uint32_t>(t.k_blocks);
-    g.kb_per_split = static_cast<uint32_t>(t.kb_per_split);
-    g.by_splits = FastDiv(static_cast<uint32_t>(t.splits));
-    g.by_batch = FastDiv(static_cast<uint32_t>(t.tiles_p * t.tiles_q));
-    g.by_group = FastDiv(g.group_p * g.tiles_q);
+    g.units = unit_plan(t.tiles_p, t.tiles_q, p.b0 * p.b1, t.splits, t.k_blocks, t.kb_per_split, 8);
     g.split_stride = out_elems;
     g.status = ctx->d_status;
     int sms = ctx->prop.multiProcessorCount;
@@ -1124,20 +1089,12 @@ void gemm_inline_tf32(b200_ctx* ctx, const GemmProblem& p, float* partial, int64
     g.out = splits > 1 ? partial : p.out;
     g.m = p.m;
     g.n = p.n;
-    g.tiles_p = static_cast<uint32_t>(ceil_div(p.m, int64_t(kRowsP)));
-    g.tiles_q = static_cast<uint32_t>(ceil_div(p.n, int64_t(bn)));
-    g.n_units = static_cast<uint32_t>(int64_t(g.tiles_p) * g.tiles_q * p.b0 * p.b1 * splits);
-    g.group_p = std::min<uint32_t>(g.tiles_p, 16);
-    g.k_blocks = static_cast<uint32_t>(ceil_div(p.k, int64_t(kBlockTf32)));
-    g.kb_per_split = static_cast<uint32_t>(kb_per_split);
-    g.by_splits = FastDiv(static_cast<uint32_t>(splits));
-    g.by_batch = FastDiv(g.tiles_p * g.tiles_q);
-    g.by_group = FastDiv(g.group_p * g.tiles_q);
+    g.units = unit_plan(ceil_div(p.m, int64_t(kRowsP)), ceil_div(p.n, int64_t(bn)), p.b0 * p.b1, splits, ceil_div(p.k, int64_t(kBlockTf32)), kb_per_split, 16);
     g.split_stride = p.b0 * p.b1 * p.m * p.n;
     g.status = ctx->d_status;
     int sms = ctx->prop.multiProcessorCount;
     if (ctx->in_grad_sync_span && ctx->comm_pending) sms = std::max(sms - ctx->comm_sms, sms / 2);
-    const int grid = static_cast<int>(std::min<int64_t>(g.n_units, sms));
+    const int grid = static_cast<int>(std::min<int64_t>(g.units.n_units, sms));
     auto launch = [&](auto tile, auto kernel) {
         using T = decltype(tile);
         B200_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kTotal));
