@@ -2,12 +2,11 @@
 //
 // They used to run on widened copies: two conversions, the F32 product with its own passes over the operands, a narrowing, and a bias and a relu of
 // their own -- 6 to 11 launches, 116 us for a 969x1327x3468 layer whose operations take 5.5.  Here warps of the product's kernel
-// bring the halves into shared memory themselves: a warp reads 64 neighbours along the unit-stride axis -- a word to a lane where
-// rows begin on 4 bytes, two halves to a lane where they do not -- and stores them in the 128-byte swizzle that TMA would give the
-// tile.  The arithmetic is gemm_h16.cu's one pass: exact products, fp32 accumulators, one narrowing; a Linear layer's bias and relu are added
+// bring the halves into shared memory themselves: a warp reads 64 neighbours along the unit-stride axis, a word to a lane,
+// and stores them in the 128-byte swizzle that TMA would give the tile.  The arithmetic is gemm_h16.cu's one pass: exact products, fp32 accumulators, one narrowing; a Linear layer's bias and relu are added
 // behind it, each narrowing its own result.
 //
-// 128 x 128 by one CTA, or 256 x 256 by a pair where there are tiles enough for a wave of pairs.  Roles as in gemm_inline.cu: warps 0-3 epilogue,
+// 128 x 128 by one CTA, or 256 x 256 by a pair, whichever takes less time in whole waves (2808x7147x621 138 us by single CTAs, 91 by pairs).  Roles as in gemm_inline.cu: warps 0-3 epilogue,
 // 4 MMA (in the odd CTA of a pair it passes on that a stage has been filled), 8-23 fill the stages.
 #include "gemm.h"
 
@@ -23,15 +22,16 @@ namespace {
 constexpr int kRowsP = 128;   // accumulator lanes
 constexpr int kRowsQ = 128;   // of Q, in one CTA
 constexpr int kBlockK = 64;   // halves: one 128-byte swizzle row
+constexpr int kStageK = 2 * kBlockK;  // of a stage: a handover every other block (2808x7148x621 87 -> 78 us)
 constexpr int kStepK = 16;
 constexpr int kRows = 16;     // a filling warp's rows of a stage
-constexpr int kGroup = 8;     // ... that are asked for and stored together
 constexpr int kFirstFiller = 8;
 constexpr int kFillers = (kRowsP + kRowsQ) / kRows;
 constexpr int kThreads = (kFirstFiller + kFillers) * 32;
 constexpr int kTileBytes = kRowsP * kBlockK * 2;
-constexpr int kStageBytes = 2 * kTileBytes;
-constexpr int kStages = 6;
+constexpr int kBlockBytes = 2 * kTileBytes;
+constexpr int kStageBytes = 2 * kBlockBytes;
+constexpr int kStages = 3;
 constexpr int kPitch = 36;    // floats: 32 columns of the epilogue's patch
 constexpr int kBars = kStages * kStageBytes;
 constexpr int kTotal = kBars + 256 + 1024;
@@ -60,63 +60,85 @@ struct F16Args {
 
 __device__ __forceinline__ uint32_t load_word(const void* p) {
     uint32_t v;
-    asm volatile("ld.global.nc.L1::no_allocate.b32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ uint16_t load_half(const void* p) {
-    uint16_t v;
-    asm volatile("ld.global.nc.b16 %0, [%1];" : "=h"(v) : "l"(p));
+    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
 
 // What one lane of a filling warp reads: a pair of halves along the unit-stride axis, sixteen rows across it.  K-major: 64 K of a row, rows eight
-// apart.  MN-major: 64 elements of a K-row (an atom), K-rows four apart.  Past the matrix' end the last one is read again: what a line too many gives lies
-// outside C, and K's end is cleared behind the stores.
+// apart.  MN-major: 64 elements of a K-row (an atom), K-rows four apart.  Either way a warp's rows all begin on 4 bytes or all beside them; where they begin
+// beside them a lane's word is the second half of its neighbour's pair and the first of its own, and one more word ends the row.  (Pairs put together
+// by shuffles instead of two stores of a half: 2808x7147x621 116 -> 111 us.)  A word is only read if it holds an element of the row, so it lies in
+// the row's allocation.  Past the matrix' end the last word or row is read again: what a line too many gives lies outside C, and K's end is cleared behind the
+// stores.
 template <bool MN, bool WORDS>
 struct PairFeed {
     static constexpr int kStep = MN ? 4 : 8;
+    struct Block {
+        uint32_t v[kRows], end;  // lane i of `end`: the word behind row i
+        bool beside;
+        int left;                // of K, from the block on
+    };
     const HalfSide& s;
     int lane, row, atom;
     uint32_t even, odd;  // where the pairs go: their swizzle alternates
-    const char* at;
-    int rows_apart, second, last_row;  // bytes between its rows, to the pair's other half; the last of the rows that exists
+    uint32_t before_even, before_odd, end_at;  // where the second half of the neighbour's pair goes, and of the row's last
+    const char* at;      // this lane's word of the first row
+    int rows_apart, to_end, last_row;  // bytes between its rows, from its word to the one behind the row; the last of the rows that exists
+    bool beside;
 
     __device__ __forceinline__ PairFeed(const HalfSide& side, int t) : s(side) {
         const int w = t >> 5;
         lane = t & 31;
         row = MN ? w >> 1 : w;
         atom = MN ? w & 1 : 0;
-        auto place_of = [&](int r) { return static_cast<uint32_t>(atom * kAtomBytes + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4); };
-        even = place_of(row);
-        odd = place_of(row + kStep);
+        auto place_of = [&](int r, int l) { return static_cast<uint32_t>(atom * kAtomBytes + r * 128 + (((l >> 2) ^ (r & 7)) << 4) + (l & 3) * 4); };
+        even = place_of(row, lane);
+        odd = place_of(row + kStep, lane);
+        before_even = place_of(row, lane - 1) + 2;
+        before_odd = place_of(row + kStep, lane - 1) + 2;
+        end_at = place_of(row + kStep * (lane & (kRows - 1)), 31) + 2;
         rows_apart = static_cast<int>(kStep * (MN ? s.s_k : s.s_mn) * 2);
     }
     __device__ __forceinline__ void place(int64_t b1, uint32_t batch, uint32_t tile, uint32_t kb, int K) {
         // (the odd CTA's rows may all lie behind the last line)
-        const int line0 = min(static_cast<int>(tile * kRowsP), static_cast<int>(s.mn - 1) & ~1), k0 = static_cast<int>(kb * kBlockK);
+        const int line0 = min(static_cast<int>(tile * kRowsP), static_cast<int>(s.mn - 1) & ~1);
+        const int k0 = min(static_cast<int>(kb * kBlockK), (K - 1) & ~(kBlockK - 1));  // (a stage's second block may lie behind K)
         const int lines = static_cast<int>(s.mn) - line0 - 1, ks = K - k0 - 1;  // behind the tile's first
-        const int left = MN ? lines : ks, down = MN ? ks : lines;
-        const int first = min((MN ? 64 * atom : 0) + 2 * lane, WORDS ? left & ~1 : left), top = min(row, down);
+        const int left = MN ? lines : ks, down = MN ? ks : lines, top = min(row, down);
         int64_t offset = 0;
         if (s.n_batches != 1) {
             const uint32_t bo = batch / static_cast<uint32_t>(b1);
             offset = int64_t(bo) * s.s_b0 + int64_t(batch - bo * static_cast<uint32_t>(b1)) * s.s_b1;
         }
-        at = reinterpret_cast<const char*>(s.base + offset + int64_t(line0 + (MN ? first : top)) * s.s_mn + int64_t(k0 + (MN ? top : first)) * s.s_k);
-        second = min(1, left - first) * 2;
+        const uintptr_t start = reinterpret_cast<uintptr_t>(s.base + offset + int64_t(line0 + (MN ? 0 : top)) * s.s_mn + int64_t(k0 + (MN ? top : 0)) * s.s_k);
+        beside = !WORDS && (start & 2) != 0;
+        const int last = (left + (beside ? 1 : 0)) >> 1, mine = min(32 * atom + lane, last);  // words of the row
+        at = reinterpret_cast<const char*>(start & ~uintptr_t(3)) + 4 * mine;
+        to_end = (min(32 * atom + 32, last) - mine) * 4;
         last_row = min(kRows - 1, (down - top) / kStep);
     }
     __device__ __forceinline__ void next() { at += kBlockK * s.s_k * 2; }  // (not onto a K-block that reaches past K)
-    __device__ __forceinline__ void load(int i, uint32_t& v, uint16_t& w) const {
-        const char* p = at + int64_t(min(i, last_row)) * rows_apart;
-        if constexpr (WORDS) {
-            v = load_word(p);
-        } else {
-            v = load_half(p);
-            w = load_half(p + second);
-        }
+    __device__ __forceinline__ void load(Block& b) const {
+        b.beside = beside;
+#pragma unroll
+        for (int i = 0; i < kRows; ++i) b.v[i] = load_word(at + int64_t(min(i, last_row)) * rows_apart);
+        if (!WORDS && beside) b.end = load_word(at + int64_t(min(lane & (kRows - 1), last_row)) * rows_apart + to_end);
     }
     __device__ __forceinline__ uint32_t word(int i) const { return (i & 1 ? odd : even) + (i >> 1) * (2 * kStep * 128); }
+    __device__ __forceinline__ void store(uint8_t* to, const Block& b) const {
+        if (!WORDS && b.beside) {  // (the same for the whole warp)
+            // a word holds elements 2 lane - 1 and 2 lane of the row, and the one behind it element 63
+#pragma unroll
+            for (int i = 0; i < kRows; ++i) {
+                *reinterpret_cast<uint16_t*>(to + word(i)) = static_cast<uint16_t>(b.v[i] >> 16);
+                if (lane > 0) *reinterpret_cast<uint16_t*>(to + (i & 1 ? before_odd : before_even) + (i >> 1) * (2 * kStep * 128)) = static_cast<uint16_t>(b.v[i]);
+            }
+            if (lane < kRows) *reinterpret_cast<uint16_t*>(to + end_at) = static_cast<uint16_t>(b.end);
+        } else {
+#pragma unroll
+            for (int i = 0; i < kRows; ++i) *reinterpret_cast<uint32_t*>(to + word(i)) = b.v[i];
+        }
+    }
 };
 
 template <int CG, bool P_MN, bool Q_MN>
@@ -174,60 +196,60 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f16_any_kernel(const __grid_
     if (warp >= kFirstFiller) {
         // ---------------- fillers ----------------
         set_registers<true, 88>();
-        auto fill = [&](auto feed, const int index, const uint32_t tile_at, auto mn_tag, auto words_tag) {
-            constexpr bool MN = decltype(mn_tag)::value, WORDS = decltype(words_tag)::value;
+        auto fill = [&](auto feed, const int index, const uint32_t tile_at, auto mn_tag) {
+            constexpr bool MN = decltype(mn_tag)::value;
+            using Block = typename decltype(feed)::Block;
             const int K = static_cast<int>(g.k);
-            uint32_t u = unit0;
-            Unit at = unit_of(g.units, u);
-            auto place = [&](const Unit& x, uint32_t kb) { feed.place(g.b1, x.batch, (index == 0 ? x.tp : x.tq) * CG + rank, kb, K); };
-            uint32_t v[kRows];
-            uint16_t w[WORDS ? 1 : kRows];
-            auto load = [&](int i) { feed.load(i, v[i], w[WORDS ? 0 : i]); };
-            place(at, at.kb0);
-#pragma unroll
-            for (int i = 0; i < kRows; ++i) load(i);
+            // where the loads are, a stage ahead of the stores
+            uint32_t next_u = unit0, next_block = 0, next_end = 0;
+            auto place = [&](const Unit& x, uint32_t block) { feed.place(g.b1, x.batch, (index == 0 ? x.tp : x.tq) * CG + rank, block, K); };
+            auto enter = [&] {
+                const Unit x = unit_of(g.units, next_u);
+                next_block = 2 * x.kb0;
+                next_end = 2 * x.kb1;
+                place(x, next_block);
+            };
+            auto request = [&](Block& b) {
+                if (next_u >= g.units.n_units) return;
+                b.left = K - static_cast<int>(next_block) * kBlockK;
+                feed.load(b);
+                if (++next_block < next_end) {
+                    if (static_cast<int>(next_block + 1) * kBlockK <= K) feed.next();
+                    else place(unit_of(g.units, next_u), next_block);
+                } else if ((next_u += unit_step) < g.units.n_units) {
+                    enter();
+                }
+            };
+            auto store = [&](uint8_t* to, const Block& b) {
+                if (b.left <= 0) return;  // (nor is it multiplied)
+                feed.store(to, b);
+                if (b.left < kBlockK) {
+                    // K past the matrix' end (a pair's second half may be another lane's store)
+                    __syncwarp();
+#pragma unroll 1
+                    for (int e = 0; e < 2 * kRows; ++e) {
+                        if ((MN ? feed.row + feed.kStep * (e >> 1) : 2 * lane + (e & 1)) < b.left) continue;
+                        *reinterpret_cast<uint16_t*>(to + feed.word(e >> 1) + 2 * (e & 1)) = 0;
+                    }
+                }
+            };
+            Block b0, b1;
+            enter();
+            request(b0);
+            request(b1);
             uint32_t it = 0;
             bool ok = true;
-            for (; ok && u < g.units.n_units; u += unit_step) {
-                const Unit now = at;
+            for (uint32_t u = unit0; ok && u < g.units.n_units; u += unit_step) {
+                const Unit now = unit_of(g.units, u);
                 for (uint32_t kb = now.kb0; kb < now.kb1; ++kb, ++it) {
                     const int s = it % STAGES;
-                    const int left = K - static_cast<int>(kb) * kBlockK;
-                    bool more = true;
-                    if (kb + 1 < now.kb1) {
-                        if (static_cast<int>(kb + 2) * kBlockK <= K) feed.next();
-                        else place(now, kb + 1);
-                    } else if (u + unit_step < g.units.n_units) {
-                        at = unit_of(g.units, u + unit_step);
-                        place(at, at.kb0);
-                    } else {
-                        more = false;
-                    }
-                    if (!mbar_wait_parked(empty_bar(s), ((it / STAGES) & 1) ^ 1, abort_p, g.status)) {
-                        ok = false;
-                        break;
-                    }
+                    ok = mbar_wait(empty_bar(s), ((it / STAGES) & 1) ^ 1, abort_p, g.status);
+                    if (!ok) break;
                     uint8_t* to = base_ptr + s * kStageBytes + tile_at;
-#pragma unroll
-                    for (int from = 0; from < kRows; from += kGroup) {
-#pragma unroll
-                        for (int i = from; i < from + kGroup; ++i) {
-                            const uint32_t bits = WORDS ? v[i] : __byte_perm(v[i], w[WORDS ? 0 : i], 0x5410);
-                            *reinterpret_cast<uint32_t*>(to + feed.word(i)) = bits;
-                        }
-                        if (more) {
-#pragma unroll
-                            for (int i = from; i < from + kGroup; ++i) load(i);
-                        }
-                    }
-                    if (left < kBlockK) {
-                        // K past the matrix' end
-#pragma unroll 1
-                        for (int e = 0; e < 2 * kRows; ++e) {
-                            if ((MN ? feed.row + feed.kStep * (e >> 1) : 2 * lane + (e & 1)) < left) continue;
-                            *reinterpret_cast<uint16_t*>(to + feed.word(e >> 1) + 2 * (e & 1)) = 0;
-                        }
-                    }
+                    store(to, b0);
+                    request(b0);
+                    store(to + kBlockBytes, b1);
+                    request(b1);
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     __syncwarp();
                     if (lane == 0) mbar_arrive(full_bar(s));
@@ -236,16 +258,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f16_any_kernel(const __grid_
             if (threadIdx.x == kFirstFiller * 32) drain_commits<STAGES>(empty_bar, it, abort_p, g.status);
         };
         const int t = threadIdx.x - kFirstFiller * 32;
-        using Yes = std::true_type;
-        using No = std::false_type;
         using PMn = std::integral_constant<bool, P_MN>;
         using QMn = std::integral_constant<bool, Q_MN>;
         if (t < kThreads / 3) {
-            if (g.p.words) fill(PairFeed<P_MN, true>(g.p, t), 0, 0, PMn(), Yes());
-            else fill(PairFeed<P_MN, false>(g.p, t), 0, 0, PMn(), No());
+            if (g.p.words) fill(PairFeed<P_MN, true>(g.p, t), 0, 0, PMn());
+            else fill(PairFeed<P_MN, false>(g.p, t), 0, 0, PMn());
         } else {
-            if (g.q.words) fill(PairFeed<Q_MN, true>(g.q, t - kThreads / 3), 1, kTileBytes, QMn(), Yes());
-            else fill(PairFeed<Q_MN, false>(g.q, t - kThreads / 3), 1, kTileBytes, QMn(), No());
+            if (g.q.words) fill(PairFeed<Q_MN, true>(g.q, t - kThreads / 3), 1, kTileBytes, QMn());
+            else fill(PairFeed<Q_MN, false>(g.q, t - kThreads / 3), 1, kTileBytes, QMn());
         }
     } else if (warp >= 4) {
         // ---------------- MMA issuer (the even CTA's) ----------------
@@ -273,12 +293,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f16_any_kernel(const __grid_
                     if (CG == 2) ok = ok && mbar_wait_cluster(peer_bar(s), (it / STAGES) & 1, abort_p, g.status);
                     if (!ok) break;
                     tc_fence_after();
-                    const uint64_t a = h16_desc<P_MN>(base + s * kStageBytes), b = h16_desc<Q_MN>(base + s * kStageBytes + kTileBytes);
 #pragma unroll
-                    for (int kk = 0; kk < kBlockK / kStepK; ++kk) {
-                        const uint64_t adv_a = static_cast<uint64_t>((P_MN ? kk * kStepK * 128 : kk * kStepK * 2) >> 4);
-                        const uint64_t adv_b = static_cast<uint64_t>((Q_MN ? kk * kStepK * 128 : kk * kStepK * 2) >> 4);
-                        umma_f16<CG>(d, a + adv_a, b + adv_b, kIdesc, (kb == r.kb0 && kk == 0) ? 0u : 1u);
+                    for (int j = 0; j < kStageK / kBlockK; ++j) {
+                        if (j > 0 && int64_t(kb) * kStageK + j * kBlockK >= g.k) break;
+                        const uint32_t at = base + s * kStageBytes + j * kBlockBytes;
+                        const uint64_t a = h16_desc<P_MN>(at), b = h16_desc<Q_MN>(at + kTileBytes);
+#pragma unroll
+                        for (int kk = 0; kk < kBlockK / kStepK; ++kk) {
+                            const uint64_t adv_a = static_cast<uint64_t>((P_MN ? kk * kStepK * 128 : kk * kStepK * 2) >> 4);
+                            const uint64_t adv_b = static_cast<uint64_t>((Q_MN ? kk * kStepK * 128 : kk * kStepK * 2) >> 4);
+                            umma_f16<CG>(d, a + adv_a, b + adv_b, kIdesc, (kb == r.kb0 && j == 0 && kk == 0) ? 0u : 1u);
+                        }
                     }
                     commit_all<CG>(empty_bar(s));
                 }
@@ -405,16 +430,31 @@ bool gemm_f16_any(b200_ctx* ctx, const GemmProblem& p, const HalfEpilogue* epi) 
         const HalfSide& s = i == 0 ? g.p : g.q;
         if ((mn[i] ? s.s_mn : s.s_k) != 1 || std::abs(mn[i] ? s.s_k : s.s_mn) >= (int64_t(1) << 26) || reinterpret_cast<uintptr_t>(s.base) % 2 != 0) return false;
     }
-    const int64_t batches = p.b0 * p.b1, lim = int64_t(1) << 30, k_blocks = ceil_div(p.k, int64_t(kBlockK)), out_elems = batches * p.m * p.n;
+    const int64_t batches = p.b0 * p.b1, lim = int64_t(1) << 30, k_blocks = ceil_div(p.k, int64_t(kStageK)), out_elems = batches * p.m * p.n;
     if (p.m >= lim || p.n >= lim || p.k >= lim || batches >= lim || out_elems >= (int64_t(1) << 31) || (epi != nullptr && batches != 1)) return false;
     const int sms = ctx->prop.multiProcessorCount;
-    const int64_t pairs = ceil_div(p.m, int64_t(2 * kRowsP)) * ceil_div(p.n, int64_t(2 * kRowsQ)) * batches;
-    const int cg = pairs * 4 >= sms ? 2 : 1;
-    const int64_t tiles_p = ceil_div(p.m, int64_t(cg * kRowsP)), tiles_q = ceil_div(p.n, int64_t(cg * kRowsQ)), tiles = tiles_p * tiles_q * batches;
-    int64_t splits = 1;
-    if (tiles < sms / cg && k_blocks >= 8) splits = std::max<int64_t>(1, std::min({int64_t(sms / cg) / tiles, k_blocks / 4, int64_t(64)}));
-    const int64_t kb_per_split = ceil_div(k_blocks, splits);
-    splits = ceil_div(k_blocks, kb_per_split);
+    // One CTA or a pair, and K-slices: the least time of whole waves.  (us: a stage takes 1.8 in either, for twice the work per CTA in a pair; a pair
+    // is not scheduled ahead of the kernel in front of it; slices are written, read and folded.)
+    int cg = 0;
+    int64_t tiles_p = 0, tiles_q = 0, tiles = 0, splits = 0, kb_per_split = 0;
+    double least = 0;
+    for (int c = 1; c <= 2; ++c) {
+        const int64_t tp = ceil_div(p.m, int64_t(c * kRowsP)), tq = ceil_div(p.n, int64_t(c * kRowsQ)), slots = sms / c;
+        int64_t n = 1;
+        if (tp * tq * batches < slots && k_blocks >= 4) n = std::max<int64_t>(1, std::min({slots / (tp * tq * batches), k_blocks / 2, int64_t(64)}));
+        const int64_t each = ceil_div(k_blocks, n);
+        n = ceil_div(k_blocks, each);
+        const double us = double(ceil_div(tp * tq * batches * n, slots)) * (1.8 * double(each) + 2.0) + (c == 2 ? 2.0 : 0.0) +
+                          (n > 1 ? 3.0 + 1.4e-6 * double(n) * double(out_elems) : 0.0);
+        if (cg != 0 && us >= least) continue;
+        least = us;
+        cg = c;
+        tiles_p = tp;
+        tiles_q = tq;
+        tiles = tp * tq * batches;
+        splits = n;
+        kb_per_split = each;
+    }
     if (tiles * splits >= lim) return false;
     float* partial = nullptr;
     if (splits > 1) {
