@@ -685,6 +685,11 @@ max_pool2d_backward_tiled_kernel(float* __restrict__ out, const float* __restric
 // index_select / scatter_add
 // ---------------------------------------------------------------------------
 
+template <int N>
+struct Int {
+    static constexpr int value = N;
+};
+
 // out[outer, k, rest] = a[outer, idx[k], rest]  (kernels_movement.cpp:339-369).
 // An out-of-range index is recorded in the status word and clamped; the host
 // reports it as an index error at the next synchronize.
@@ -752,6 +757,37 @@ index_select_rows_kernel(uint4* __restrict__ out, const uint4* __restrict__ a, c
             if (live[u]) {
                 out[base + u * stride] = v[u];
             }
+        }
+    }
+}
+
+// Dense source rows that begin or end anywhere: a warp copies a piece of 32 * Q elements of a row, all of a lane's loads in flight.  Bound by the chain
+// of index, row and store where rows are short, by HBM where they are long ([2643, 483] at 12872 indices, 50 MB: 39 us with an index and a
+// division chain per element, 8 here).
+template <typename T, int Q>
+__global__ void __launch_bounds__(kThreads)
+index_select_pieces_kernel(T* __restrict__ out, const T* __restrict__ a, const int64_t* __restrict__ idx, int64_t idx_stride, FastDiv by_pieces,
+                           FastDiv by_extent, uint32_t inner, int64_t a_extent, uint32_t tasks, uint32_t* status) {
+    pdl_prologue();
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t task = (blockIdx.x * kThreads + threadIdx.x) >> 5; task < tasks; task += (gridDim.x * kThreads) >> 5) {
+        uint32_t row, piece, outer, k;
+        by_pieces.divmod(task, row, piece);
+        by_extent.divmod(row, outer, k);
+        int64_t j = idx[int64_t(k) * idx_stride];
+        if (j < 0 || j >= a_extent) {
+            if (lane == 0) atomicOr(status, kStatusIndexOutOfRange);
+            j = j < 0 ? 0 : a_extent - 1;
+        }
+        const uint32_t c0 = piece * (32 * Q) + lane;
+        const T* from = a + (int64_t(outer) * a_extent + j) * inner;
+        T* to = out + int64_t(row) * inner + c0;
+        T v[Q];
+#pragma unroll
+        for (int q = 0; q < Q; ++q) v[q] = __ldg(from + min(c0 + 32 * q, inner - 1));
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            if (c0 + 32 * q < inner) to[32 * q] = v[q];
         }
     }
 }
@@ -988,10 +1024,35 @@ scatter_gather4_kernel(float4* __restrict__ out, const float4* __restrict__ src,
 // ascending order by itself -- up to 32 of them lie one per lane and are ranked by comparing -- or, for a destination
 // with more, finds them in order by reading the index list (at most n / 33 destinations have more, so that all of them
 // together read it a bounded number of times).  The sums and their order are those of the pull form, bit for bit.
-// [8192, 1024] into [50000, 1024]: 152 -> 50 us; 239 MB, nearly all of it the result.  Long lists, buckets against chains: 16384 indices
+// [8192, 1024] into [50000, 1024]: 152 -> 50 us; 239 MB, nearly all of it the result.  Rows that are no quads, 7548 of 898 into 4760: 40 -> 17 us since
+// no load stands under a condition (each then waited for the one before it).  Long lists, buckets against chains: 16384 indices
 // into 100 rows of 1024, uniform 130 and 92 us, as words of a text are distributed (1/rank) 573 and 445; into 256 of 512 90 and 72, 504 and 381;
 // all into one 3633 and 2594.  (One piece of 32 indices at a time instead of four in flight: 156, 461, 146, 390 and 2797.)
 constexpr int kChainMax = 65536;
+// While the destinations are not too many for it, the sources lie side by side in a line of 32 per destination instead of a chain: a warp has them with one load
+// where it followed one after the other.
+constexpr int64_t kLineExtent = int64_t(1) << 18;  // 32 MB of lines
+
+__global__ void __launch_bounds__(kThreads) scatter_clear_kernel(int* __restrict__ count, int64_t n) {
+    pdl_prologue();  // (a kernel, not a memset: its neighbours' launches overlap)
+    const int64_t i = int64_t(blockIdx.x) * kThreads + threadIdx.x;
+    if (i < n) count[i] = 0;
+}
+
+__global__ void __launch_bounds__(kThreads)
+scatter_lines_kernel(int* __restrict__ count, int* __restrict__ lines, const int64_t* __restrict__ idx, int64_t idx_stride, int n, int64_t extent,
+                     uint32_t* status) {
+    pdl_prologue();
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const int64_t t = idx[k * idx_stride];
+    if (t < 0 || t >= extent) {
+        atomicOr(status, kStatusIndexOutOfRange);  // no destination: left out
+        return;
+    }
+    const int at = atomicAdd(count + t, 1);
+    if (at < 32) lines[t * 32 + at] = k;
+}
 
 __global__ void __launch_bounds__(kThreads)
 scatter_chain_kernel(int* __restrict__ count, int* __restrict__ head, int* __restrict__ next, const int64_t* __restrict__ idx,
@@ -1007,11 +1068,6 @@ scatter_chain_kernel(int* __restrict__ count, int* __restrict__ head, int* __res
     next[k] = atomicExch(head + t, k);
     atomicAdd(count + t, 1);
 }
-
-template <int N>
-struct Int {
-    static constexpr int value = N;
-};
 
 // One warp per piece of 32*Q*W elements of a destination row, with at most 32 registers of sources in flight: 64 left two
 // blocks on an SM, which took 71 us where this takes 45.  LOOK pieces of 32 indices are in flight where a destination's list is long; four
@@ -1039,16 +1095,17 @@ scatter_chain_gather_kernel(float* __restrict__ out, const float* __restrict__ s
                 float v[F][C][W];
 #pragma unroll
                 for (int i = 0; i < F; ++i) {
-                    const int k = __shfl_sync(0xffffffffu, held, (i0 + i) & 31);
-                    const float* p = from + int64_t(k) * inner + c0 + q0 * 32 * W;
+                    // (past the list the last source is read again, past the row its last columns: a load under a condition waits for the one before it)
+                    const int k = __shfl_sync(0xffffffffu, held, min(i0 + i, m - 1));
+                    const float* p = from + int64_t(k) * inner;
 #pragma unroll
                     for (int q = 0; q < C; ++q) {
-                        const bool in = i0 + i < m && c0 + (q0 + q) * 32 * W < inner;
+                        const uint32_t c = min(c0 + (q0 + q) * 32 * W, inner - W);
                         if constexpr (W == 4) {
-                            const float4 t = in ? __ldg(reinterpret_cast<const float4*>(p + q * 128)) : make_float4(0.0F, 0.0F, 0.0F, 0.0F);
+                            const float4 t = __ldg(reinterpret_cast<const float4*>(p + c));
                             v[i][q][0] = t.x; v[i][q][1] = t.y; v[i][q][2] = t.z; v[i][q][3] = t.w;
                         } else {
-                            v[i][q][0] = in ? __ldg(p + q * 32) : 0.0F;
+                            v[i][q][0] = __ldg(p + c);
                         }
                     }
                 }
@@ -1070,11 +1127,18 @@ scatter_chain_gather_kernel(float* __restrict__ out, const float* __restrict__ s
             add(held, m, Int<8>{}, Int<Q / 2>{}, Int<Q / 2>{});
         };
         const int c = count[j];
-        if (c > 0 && c <= 32) {
-            int k = head[j], held = 0x7fffffff;
-            for (int i = 0; i < c; ++i) {
-                if (int(lane) == i) held = k;
-                if (i + 1 < c) k = next[k];
+        if (c == 1) {  // (most lists, where destinations are many)
+            add(head[next == nullptr ? int64_t(j) * 32 : int64_t(j)], 1, Int<1>{}, Int<Q>{}, Int<0>{});
+        } else if (c > 1 && c <= 32) {
+            int held = 0x7fffffff;
+            if (next == nullptr) {
+                if (int(lane) < c) held = head[int64_t(j) * 32 + lane];  // (a line per destination)
+            } else {
+                int k = head[j];
+                for (int i = 0; i < c; ++i) {
+                    if (int(lane) == i) held = k;
+                    if (i + 1 < c) k = next[k];
+                }
             }
             int rank = 0;
             for (int i = 0; i < c; ++i) rank += __shfl_sync(0xffffffffu, held, i) < held;
@@ -1507,6 +1571,25 @@ void launch_movement(b200_ctx* ctx, const b200_node& node) {
                               static_cast<unsigned>(total16), ctx->d_status);
                 break;
             }
+            if (a.contiguous && small && (esz == 4 || esz == 8)) {
+                auto pieces = [&](auto* o, const auto* from, auto width) {
+                    using T = std::remove_pointer_t<decltype(o)>;
+                    constexpr int Q = decltype(width)::value;
+                    const int64_t per_row = ceil_div(inner, int64_t(32 * Q)), tasks = total / inner * per_row;
+                    launch_kernel(ctx, index_select_pieces_kernel<T, Q>, grid_for(tasks * 32, kThreads), kThreads, 0, o, from, ip, istride,
+                                  FastDiv(static_cast<uint32_t>(per_row)), FastDiv(static_cast<uint32_t>(out.dim[axis])), static_cast<uint32_t>(inner),
+                                  a.dim[axis], static_cast<uint32_t>(tasks), ctx->d_status);
+                };
+                auto widths = [&](auto* o, const auto* from) {  // (as many elements to a lane as the row has, eight at most)
+                    if (inner <= 32) pieces(o, from, Int<1>{});
+                    else if (inner <= 64) pieces(o, from, Int<2>{});
+                    else if (inner <= 128) pieces(o, from, Int<4>{});
+                    else pieces(o, from, Int<8>{});
+                };
+                if (esz == 4) widths(reinterpret_cast<uint32_t*>(out.data), reinterpret_cast<const uint32_t*>(a.data));
+                else widths(reinterpret_cast<unsigned long long*>(out.data), reinterpret_cast<const unsigned long long*>(a.data));
+                break;
+            }
             const unsigned grid = grid_for(total, kThreads);
 #define B200_INDEX_SELECT(T, I)                                                                              \
     launch_kernel(ctx, index_select_kernel<T, I>, grid, kThreads, 0, \
@@ -1546,27 +1629,34 @@ void launch_movement(b200_ctx* ctx, const b200_node& node) {
                 const int n = static_cast<int>(n_idx);
                 const int64_t extent = out.dim[axis];
                 const float* sp = reinterpret_cast<const float*>(src.data);
-                int* count = static_cast<int*>(ctx->ensure_workspace(static_cast<size_t>(2 * extent + n_idx) * sizeof(int)));
-                int* head = count + extent;
-                int* next = head + extent;
-                B200_CUDA_CHECK(cudaMemsetAsync(count, 0, static_cast<size_t>(extent) * sizeof(int), ctx->stream));
-                launch_kernel(ctx, scatter_chain_kernel, static_cast<unsigned>(ceil_div(n_idx, kThreads)), kThreads, 0, count, head, next, ip,
-                              istride, n, extent, ctx->d_status);
-                ctx->count_launch();
+                const bool lines = extent <= kLineExtent;
+                const int64_t counts = ceil_div(extent, int64_t(32)) * 32;  // (lines begin on 128 bytes)
+                int* count = static_cast<int*>(ctx->ensure_workspace(static_cast<size_t>(lines ? counts + 32 * extent : counts + extent + n_idx) * sizeof(int)));
+                int* head = count + counts;
+                int* next = lines ? nullptr : head + extent;
+                const unsigned blocks = static_cast<unsigned>(ceil_div(n_idx, kThreads));
+                launch_kernel(ctx, scatter_clear_kernel, static_cast<unsigned>(ceil_div(extent, int64_t(kThreads))), kThreads, 0, count, extent);
+                if (lines) launch_kernel(ctx, scatter_lines_kernel, blocks, kThreads, 0, count, head, ip, istride, n, extent, ctx->d_status);
+                else launch_kernel(ctx, scatter_chain_kernel, blocks, kThreads, 0, count, head, next, ip, istride, n, extent, ctx->d_status);
+                ctx->count_launch(2);
                 const bool quads = inner % 4 == 0 && reinterpret_cast<uintptr_t>(sp) % 16 == 0 && reinterpret_cast<uintptr_t>(o) % 16 == 0;
-                const int64_t pieces = ceil_div(inner, quads ? 256 : 128), tasks = total / inner * pieces;
+                const bool long_lists = n_idx >= 8 * extent;  // (eight sources to a destination on average)
+                // (rows that are no quads: as many single elements to a lane as are in flight with quads, half of it for short rows and for long lists,
+                // where more tasks are worth more: 16384 indices into 100 rows of 1023, distributed as 1/rank, 663 us, 1133 with 256 to a task)
+                const bool wide = quads || (inner > 128 && !long_lists);
+                const int64_t pieces = ceil_div(inner, wide ? 256 : 128), tasks = total / inner * pieces;
                 const unsigned grid = grid_for(tasks * 32, kThreads);
                 auto gather = [&](auto kernel) {
                     launch_kernel(ctx, kernel, grid, kThreads, 0, o, sp, static_cast<const int*>(count), static_cast<const int*>(head),
                                   static_cast<const int*>(next), ip, istride, n, FastDiv(static_cast<uint32_t>(pieces)),
                                   FastDiv(static_cast<uint32_t>(extent)), static_cast<uint32_t>(inner), static_cast<uint32_t>(tasks));
                 };
-                // (eight sources to a destination on average: some lists are long)
-                if (n_idx >= 8 * extent) {
+                if (long_lists) {
                     if (quads) gather(scatter_chain_gather_kernel<4, 2, 4>);
                     else gather(scatter_chain_gather_kernel<1, 4, 4>);
                 } else {
                     if (quads) gather(scatter_chain_gather_kernel<4, 2, 1>);
+                    else if (wide) gather(scatter_chain_gather_kernel<1, 8, 1>);
                     else gather(scatter_chain_gather_kernel<1, 4, 1>);
                 }
                 break;
