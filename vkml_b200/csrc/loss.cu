@@ -248,12 +248,15 @@ __global__ void __launch_bounds__(256) loss_rows_kernel(LossArgs a) {
 // brings the next row in behind it, chunk by chunk as this one's are written, so that reading the
 // logits never stops the writing.  (Rows re-read from L2 by three smaller blocks per SM took 245 us at [1024, 32000]
 // -- 1024 rows make 2.3 waves of those -- against 218 here.)
+// Rows of up to 16384 and 8192 classes leave room for more and smaller blocks, so that one block's rows are written while another reduces
+// its own ([689, 6337]: 53 us with one block of 1024 threads, 32 with six of 256; [4000, 4500] 222 and 119).  A row's head planes do not depend on
+// its logits and are written first: they drain while the row is reduced.
 constexpr int kLongThreads = 1024;
 constexpr int kLongChunks = 8;
 constexpr uint32_t kLongMax = 51200;  // classes: 200 KB of shared memory
 
-template <bool HEAD, bool BACK>
-__global__ void __launch_bounds__(kLongThreads, 1) loss_long_kernel(LossArgs a, uint32_t* status) {
+template <bool HEAD, bool BACK, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1536 / THREADS) loss_long_kernel(LossArgs a, uint32_t* status) {
     extern __shared__ __align__(16) float row[];
     __shared__ uint64_t landed[kLongChunks];
     __shared__ int abort_flag;
@@ -268,7 +271,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) loss_long_kernel(LossArgs a, 
     __syncthreads();
     pdl_prologue();
     if (HEAD) {
-        for (int64_t c = int64_t(blockIdx.x) * kLongThreads + tid; c < a.cols; c += int64_t(gridDim.x) * kLongThreads) {
+        for (int64_t c = int64_t(blockIdx.x) * THREADS + tid; c < a.cols; c += int64_t(gridDim.x) * THREADS) {
             a.index[c] = static_cast<float>(c);
         }
     }
@@ -296,7 +299,15 @@ __global__ void __launch_bounds__(kLongThreads, 1) loss_long_kernel(LossArgs a, 
         const int64_t base = r * a.cols;
         const RowQuads q(base, a.cols, tid);
         float scale = 0.0F, wanted = -1.0F, peak, sum = 0.0F, ve[1] = {-INFINITY}, ge[1] = {0.0F};
-        if constexpr (HEAD) head_row(a, r, tid == 0, scale, wanted);
+        if constexpr (HEAD) {
+            head_row(a, r, tid == 0, scale, wanted);
+            const float none[4] = {}, one[1] = {};
+            if (q.edge < a.cols) loss_elements<true, false, 1, true>(a, base + q.edge, q.edge, scale, wanted, one, one, 0.0F, 0.0F, 0.0F);
+            for (uint32_t u = tid; u < q.quads; u += THREADS) {
+                const uint32_t col = q.head + u * 4;
+                loss_elements<true, false, 4, true>(a, base + col, col, scale, wanted, none, none, 0.0F, 0.0F, 0.0F);
+            }
+        }
         if (q.edge < a.cols) {
             get<1>(a.x + base + q.edge, ve);
             if constexpr (!HEAD) get<1>(a.g + base + q.edge, ge);
@@ -308,7 +319,7 @@ __global__ void __launch_bounds__(kLongThreads, 1) loss_long_kernel(LossArgs a, 
             ok = mbar_wait_parked(smem_u32(&landed[c]), phase, &abort_flag, status);
             uint32_t q0, q1;
             chunk(q.quads, c, q0, q1);
-            for (uint32_t u = q0 + tid; u < q1; u += kLongThreads) {
+            for (uint32_t u = q0 + tid; u < q1; u += THREADS) {
                 float t[4];
                 get<4>(row + u * 4, t);
                 peak = fmaxf(fmaxf(fmaxf(peak, t[0]), fmaxf(t[1], t[2])), t[3]);
@@ -319,28 +330,33 @@ __global__ void __launch_bounds__(kLongThreads, 1) loss_long_kernel(LossArgs a, 
             }
         }
         if (__syncthreads_or(!ok)) break;
-        peak = group_max<kLongThreads>(peak, red);
+        peak = group_max<THREADS>(peak, red);
         float denom = expf(ve[0] - peak);
-        for (uint32_t u = tid; u < q.quads; u += kLongThreads) {
+        for (uint32_t u = tid; u < q.quads; u += THREADS) {
             float t[4];
             get<4>(row + u * 4, t);
             denom += (expf(t[0] - peak) + expf(t[1] - peak)) + (expf(t[2] - peak) + expf(t[3] - peak));
         }
-        const float lg = logf(group_sum<kLongThreads>(denom, red));
-        const float total = HEAD ? head_total(a, scale, wanted) : group_sum<kLongThreads>(sum, red);
+        const float lg = logf(group_sum<THREADS>(denom, red));
+        const float total = HEAD ? head_total(a, scale, wanted) : group_sum<THREADS>(sum, red);
         if (tid == 0) a.total[r] = total;
         if (q.edge < a.cols) {
-            loss_elements<HEAD, BACK, 1, true>(a, base + q.edge, q.edge, scale, wanted, ve, ge, peak, lg, total);
+            if constexpr (HEAD) ge[0] = __fmul_rn(scale, wanted == static_cast<float>(q.edge) ? 1.0F : 0.0F);
+            loss_elements<false, BACK, 1, true>(a, base + q.edge, q.edge, scale, wanted, ve, ge, peak, lg, total);
         }
         for (int c = 0; c < kLongChunks; ++c) {
             uint32_t q0, q1;
             chunk(q.quads, c, q0, q1);
-            for (uint32_t u = q0 + tid; u < q1; u += kLongThreads) {
+            for (uint32_t u = q0 + tid; u < q1; u += THREADS) {
                 const uint32_t col = q.head + u * 4;
                 float t[4], h[4] = {};
                 get<4>(row + u * 4, t);
                 if constexpr (!HEAD) get<4>(a.g + base + col, h);
-                loss_elements<HEAD, BACK, 4, true>(a, base + col, col, scale, wanted, t, h, peak, lg, total);
+                if constexpr (HEAD) {
+#pragma unroll
+                    for (int w = 0; w < 4; ++w) h[w] = __fmul_rn(scale, wanted == static_cast<float>(col + w) ? 1.0F : 0.0F);
+                }
+                loss_elements<false, BACK, 4, true>(a, base + col, col, scale, wanted, t, h, peak, lg, total);
             }
             __syncthreads();
             if (tid == 0 && r + gridDim.x < a.rows) fetch(r + gridDim.x, c);
@@ -733,8 +749,13 @@ void launch_rows(b200_ctx* ctx, LossArgs a) {
     else if (a.cols <= 4096) B200_LOSS(256, 4, blocks);
     else if constexpr (BACK) {
         const size_t smem = (a.cols + 3) / 4 * 16;
-        B200_CUDA_CHECK(cudaFuncSetAttribute(loss_long_kernel<HEAD, BACK>, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kLongMax));
-        launch_kernel(ctx, loss_long_kernel<HEAD, BACK>, static_cast<unsigned>(std::min<int64_t>(a.rows, sm_count())), kLongThreads, smem, a, ctx->d_status);
+        auto launch = [&](auto kernel, int threads, int blocks) {
+            B200_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kLongMax));
+            launch_kernel(ctx, kernel, static_cast<unsigned>(std::min<int64_t>(a.rows, int64_t(sm_count()) * blocks)), threads, smem, a, ctx->d_status);
+        };
+        if (a.cols <= 8192) launch(loss_long_kernel<HEAD, BACK, 256>, 256, 6);
+        else if (a.cols <= 16384) launch(loss_long_kernel<HEAD, BACK, 512>, 512, 3);
+        else launch(loss_long_kernel<HEAD, BACK, kLongThreads>, kLongThreads, 1);
     }
 #undef B200_LOSS
 }
