@@ -130,7 +130,7 @@ __device__ __forceinline__ void loss_elements(const LossArgs& a, int64_t at, uin
 template <int GROUP>
 __device__ __forceinline__ float group_max(float v, float* red) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    for (int o = GROUP < 32 ? GROUP / 2 : 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
     if constexpr (GROUP > 32) {
         if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
         __syncthreads();
@@ -145,7 +145,7 @@ __device__ __forceinline__ float group_max(float v, float* red) {
 template <int GROUP>
 __device__ __forceinline__ float group_sum(float v, float* red) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    for (int o = GROUP < 32 ? GROUP / 2 : 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if constexpr (GROUP > 32) {
         if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
         __syncthreads();
@@ -178,7 +178,10 @@ __device__ __forceinline__ float head_total(const LossArgs& a, float scale, floa
     return __fadd_rn(hit ? scale : 0.0F, off);
 }
 
-// A group of threads per row -- a warp up to 1024 classes, a block up to 4096 -- with the row's logits in registers.
+// A group of threads per row -- a warp up to 1024 classes, a block up to 4096 -- with the row's logits in registers.  Up to 128 classes, where the
+// machine's warps would take more than one row each, eight threads: a warp to a row of 47 leaves most of its lanes idle ([17795, 47] 24.7 us with the
+// loss's value, 17.1 with eight; [60000, 33] 59.5 and 32.9; but 278 rows of 107 9.8 and 14.4).
+constexpr int64_t kManyRows = 64;  // per SM: eight blocks of eight warps
 template <bool HEAD, bool BACK, int GROUP, int ITEMS>
 __global__ void __launch_bounds__(256) loss_rows_kernel(LossArgs a) {
     pdl_prologue();
@@ -190,7 +193,11 @@ __global__ void __launch_bounds__(256) loss_rows_kernel(LossArgs a) {
             a.index[c] = static_cast<float>(c);
         }
     }
-    for (int64_t r = int64_t(blockIdx.x) * kRows + threadIdx.x / GROUP; r < a.rows; r += int64_t(gridDim.x) * kRows) {
+    constexpr int kInWarp = GROUP < 32 ? 32 / GROUP : 1;  // rows that a warp has at a time: it goes through them together, past the end over the last one again
+    const uint32_t in_warp = GROUP < 32 ? (threadIdx.x & 31) / GROUP : 0;
+    for (int64_t first = int64_t(blockIdx.x) * kRows + threadIdx.x / (GROUP * kInWarp) * kInWarp; first < a.rows; first += int64_t(gridDim.x) * kRows) {
+        const int64_t r = min(first + in_warp, a.rows - 1);
+        const bool live = GROUP >= 32 || first + in_warp < a.rows;
         const int64_t base = r * a.cols;
         const RowQuads q(base, a.cols, lane);
         float scale = 0.0F, wanted = -1.0F, peak = -INFINITY, lg = 0.0F, total = 0.0F;
@@ -228,6 +235,7 @@ __global__ void __launch_bounds__(256) loss_rows_kernel(LossArgs a) {
             total = HEAD ? head_total(a, scale, wanted) : group_sum<GROUP>(sum, red);
             if (lane == 0) a.total[r] = total;
         }
+        if (!live) continue;
         if (q.edge < a.cols) {
             loss_elements<HEAD, BACK, 1, false>(a, base + q.edge, q.edge, scale, wanted, ve, ge, peak, lg, total);
         }
@@ -410,8 +418,10 @@ constexpr uint32_t kTileCols = 32;
 template <bool HEAD, bool BACK>
 __global__ void __launch_bounds__(256) loss_tile_kernel(LossArgs a) {
     pdl_prologue();
-    __shared__ float xs[BACK ? kTileRows * kTileCols : 1];
-    __shared__ float gs[BACK && !HEAD ? kTileRows * kTileCols : 1];
+    // (rows lie an odd number of words apart: a thread to a row of 32 met 31 others on its bank)
+    __shared__ float xs[BACK ? kTileRows * (kTileCols + 1) : 1];
+    __shared__ float gs[BACK && !HEAD ? kTileRows * (kTileCols + 1) : 1];
+    const uint32_t pitch = a.cols | 1u;
     __shared__ float row_scale[kTileRows], row_wanted[kTileRows], row_peak[kTileRows], row_lg[kTileRows], row_total[kTileRows];
     const int64_t r0 = int64_t(blockIdx.x) * kTileRows;
     const int rows = static_cast<int>(min(int64_t(kTileRows), a.rows - r0));
@@ -420,8 +430,10 @@ __global__ void __launch_bounds__(256) loss_tile_kernel(LossArgs a) {
     if (HEAD && blockIdx.x == 0 && threadIdx.x < a.cols) a.index[threadIdx.x] = static_cast<float>(threadIdx.x);
     if constexpr (BACK) {
         for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-            xs[i] = a.x[base + i];
-            if constexpr (!HEAD) gs[i] = a.g[base + i];
+            uint32_t r, c;
+            a.by_cols.divmod(i, r, c);
+            xs[r * pitch + c] = a.x[base + i];
+            if constexpr (!HEAD) gs[r * pitch + c] = a.g[base + i];
         }
         __syncthreads();
     }
@@ -432,14 +444,14 @@ __global__ void __launch_bounds__(256) loss_tile_kernel(LossArgs a) {
         row_scale[t] = scale;
         row_wanted[t] = wanted;
         if constexpr (BACK) {
-            const float* x = xs + t * a.cols;
+            const float* x = xs + t * pitch;
             float peak = -INFINITY, denom = 0.0F, total = 0.0F;
             for (uint32_t c = 0; c < a.cols; ++c) peak = fmaxf(peak, x[c]);
             for (uint32_t c = 0; c < a.cols; ++c) denom += expf(x[c] - peak);
             if constexpr (HEAD) {
                 total = head_total(a, scale, wanted);
             } else {
-                for (uint32_t c = 0; c < a.cols; ++c) total += gs[t * a.cols + c];
+                for (uint32_t c = 0; c < a.cols; ++c) total += gs[t * pitch + c];
             }
             row_peak[t] = peak;
             row_lg[t] = logf(denom);
@@ -451,7 +463,7 @@ __global__ void __launch_bounds__(256) loss_tile_kernel(LossArgs a) {
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
         uint32_t r, c;
         a.by_cols.divmod(i, r, c);
-        const float x[1] = {BACK ? xs[i] : 0.0F}, g[1] = {BACK && !HEAD ? gs[i] : 0.0F};
+        const float x[1] = {BACK ? xs[r * pitch + c] : 0.0F}, g[1] = {BACK && !HEAD ? gs[r * pitch + c] : 0.0F};
         loss_elements<HEAD, BACK, 1, false>(a, base + i, c, row_scale[r], row_wanted[r], x, g, BACK ? row_peak[r] : 0.0F,
                                             BACK ? row_lg[r] : 0.0F, BACK ? row_total[r] : 0.0F);
     }
@@ -499,7 +511,11 @@ __global__ void __launch_bounds__(256) loss_value_kernel(ValueArgs v) {
     __shared__ float red[32];
     const uint32_t lane = threadIdx.x % GROUP;
     float mean = 0.0F;  // of the rows this group's first thread has seen
-    for (int64_t r = int64_t(blockIdx.x) * kRows + threadIdx.x / GROUP; r < v.rows; r += int64_t(gridDim.x) * kRows) {
+    constexpr int kInWarp = GROUP < 32 ? 32 / GROUP : 1;  // (as in loss_rows_kernel)
+    const uint32_t in_warp = GROUP < 32 ? (threadIdx.x & 31) / GROUP : 0;
+    for (int64_t first = int64_t(blockIdx.x) * kRows + threadIdx.x / (GROUP * kInWarp) * kInWarp; first < v.rows; first += int64_t(gridDim.x) * kRows) {
+        const int64_t r = min(first + in_warp, v.rows - 1);
+        const bool live = GROUP >= 32 || first + in_warp < v.rows;
         const int64_t base = r * v.cols;
         float s = 0.0F;
         auto single = [&](uint32_t c) {
@@ -526,7 +542,7 @@ __global__ void __launch_bounds__(256) loss_value_kernel(ValueArgs v) {
             for (uint32_t c = lane; c < v.cols; c += GROUP) single(c);
         }
         s = group_sum<GROUP>(s, red);
-        if (lane == 0) {
+        if (lane == 0 && live) {
             v.sum[r] = s;
             v.negated[r] = -s;
             mean += -s;
@@ -542,20 +558,24 @@ __global__ void __launch_bounds__(256) loss_value_kernel(ValueArgs v) {
 
 __global__ void __launch_bounds__(256) loss_value_tile_kernel(ValueArgs v) {
     pdl_prologue();
-    __shared__ float p[kTileRows * kTileCols];
+    __shared__ float p[kTileRows * (kTileCols + 1)];
+    const uint32_t pitch = v.cols | 1u;
     __shared__ float red[32];
     const int64_t r0 = int64_t(blockIdx.x) * kTileRows;
     const int rows = static_cast<int>(min(int64_t(kTileRows), v.rows - r0));
     const uint32_t n = rows * v.cols;
     const int64_t base = r0 * v.cols;
     for (uint32_t i = threadIdx.x; i < n; i += 256) {
-        p[i] = __fmul_rn(v.a[base + i], v.b[base + i]);
-        v.product[base + i] = p[i];
+        uint32_t r, c;
+        v.by_cols.divmod(i, r, c);
+        const float t = __fmul_rn(v.a[base + i], v.b[base + i]);
+        p[r * pitch + c] = t;
+        v.product[base + i] = t;
     }
     __syncthreads();
     float s = 0.0F;
     if (threadIdx.x < rows) {
-        for (uint32_t c = 0; c < v.cols; ++c) s += p[threadIdx.x * v.cols + c];
+        for (uint32_t c = 0; c < v.cols; ++c) s += p[threadIdx.x * pitch + c];
         v.sum[r0 + threadIdx.x] = s;
         v.negated[r0 + threadIdx.x] = -s;
     }
@@ -738,13 +758,15 @@ void launch_rows(b200_ctx* ctx, LossArgs a) {
     }
     const bool quads_ok = quads && reinterpret_cast<uintptr_t>(a.equal) % 4 == 0;
     const unsigned warps = static_cast<unsigned>(std::min<int64_t>(ceil_div(a.rows, 8), int64_t(sm_count()) * 8));
+    const unsigned eights = static_cast<unsigned>(std::min<int64_t>(ceil_div(a.rows, 32), int64_t(sm_count()) * 8));
     const unsigned blocks = static_cast<unsigned>(std::min<int64_t>(a.rows, int64_t(sm_count()) * 8));
     if (!quads_ok || (BACK ? a.cols > kLongMax : a.cols > 4096)) {
         launch_kernel(ctx, loss_any_kernel<HEAD, BACK>, blocks, 256, 0, a);
         return;
     }
 #define B200_LOSS(GROUP, ITEMS, GRID) launch_kernel(ctx, loss_rows_kernel<HEAD, BACK, GROUP, ITEMS>, GRID, 256, 0, a)
-    if (a.cols <= 256) B200_LOSS(32, 2, warps);
+    if (a.cols <= 128 && a.rows > kManyRows * sm_count()) B200_LOSS(8, 4, eights);
+    else if (a.cols <= 256) B200_LOSS(32, 2, warps);
     else if (a.cols <= 1024) B200_LOSS(32, 8, warps);
     else if (a.cols <= 4096) B200_LOSS(256, 4, blocks);
     else if constexpr (BACK) {
@@ -791,13 +813,15 @@ size_t match_value(const b200_node* const* seq, size_t avail, ValueArgs& v) {
 
 void launch_value(b200_ctx* ctx, ValueArgs v) {
     const bool quads = aligned16(v.a) && aligned16(v.b) && aligned16(v.product);
-    const bool tile = v.cols <= kTileCols, warp = v.cols <= 1024;
+    const bool tile = v.cols <= kTileCols, eight = v.cols <= 128 && v.rows > kManyRows * sm_count(), warp = v.cols <= 1024;
     const unsigned grid = tile ? static_cast<unsigned>(ceil_div(v.rows, kTileRows))
-                               : static_cast<unsigned>(std::min<int64_t>(warp ? ceil_div(v.rows, 8) : v.rows, int64_t(sm_count()) * 8));
+                               : static_cast<unsigned>(std::min<int64_t>(eight ? ceil_div(v.rows, 32) : warp ? ceil_div(v.rows, 8) : v.rows, int64_t(sm_count()) * 8));
     v.by_cols = FastDiv(v.cols);
     v.partial = static_cast<float*>(ctx->ensure_workspace(sizeof(float) * grid));
     v.arrived = ctx->d_counters + kLossCounter;
     if (tile) launch_kernel(ctx, loss_value_tile_kernel, grid, 256, 0, v);
+    else if (eight && quads) launch_kernel(ctx, loss_value_kernel<8, true>, grid, 256, 0, v);
+    else if (eight) launch_kernel(ctx, loss_value_kernel<8, false>, grid, 256, 0, v);
     else if (warp && quads) launch_kernel(ctx, loss_value_kernel<32, true>, grid, 256, 0, v);
     else if (warp) launch_kernel(ctx, loss_value_kernel<32, false>, grid, 256, 0, v);
     else if (quads) launch_kernel(ctx, loss_value_kernel<256, true>, grid, 256, 0, v);
