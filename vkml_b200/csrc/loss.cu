@@ -45,6 +45,7 @@ struct LossArgs {
     float* total;
     float* share;
     float* grad;
+    int quads;               // every plane begins on 16 bytes
 };
 
 // The row's values of the head's vectors; every thread of the row's group calls it, `first` writes them.
@@ -428,13 +429,23 @@ __global__ void __launch_bounds__(256) loss_tile_kernel(LossArgs a) {
     const uint32_t n = rows * a.cols;
     const int64_t base = r0 * a.cols;
     if (HEAD && blockIdx.x == 0 && threadIdx.x < a.cols) a.index[threadIdx.x] = static_cast<float>(threadIdx.x);
+    // (the block's run of memory begins on 16 bytes; what is no whole quad at its end, or all of it where a plane does not, goes by elements)
+    const uint32_t quads = a.quads != 0 ? n / 4 : 0;
     if constexpr (BACK) {
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        auto keep = [&](uint32_t i, float x, float g) {
             uint32_t r, c;
             a.by_cols.divmod(i, r, c);
-            xs[r * pitch + c] = a.x[base + i];
-            if constexpr (!HEAD) gs[r * pitch + c] = a.g[base + i];
+            xs[r * pitch + c] = x;
+            if constexpr (!HEAD) gs[r * pitch + c] = g;
+        };
+        for (uint32_t u = threadIdx.x; u < quads; u += blockDim.x) {
+            float x[4], g[4] = {};
+            get<4>(a.x + base + 4 * u, x);
+            if constexpr (!HEAD) get<4>(a.g + base + 4 * u, g);
+#pragma unroll
+            for (int w = 0; w < 4; ++w) keep(4 * u + w, x[w], g[w]);
         }
+        for (uint32_t i = 4 * quads + threadIdx.x; i < n; i += blockDim.x) keep(i, a.x[base + i], HEAD ? 0.0F : a.g[base + i]);
         __syncthreads();
     }
     if (threadIdx.x < rows) {
@@ -460,7 +471,45 @@ __global__ void __launch_bounds__(256) loss_tile_kernel(LossArgs a) {
         }
     }
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+    for (uint32_t u = threadIdx.x; u < quads; u += blockDim.x) {
+        // (four elements of one or more rows: the values of loss_elements, element by element)
+        float plane[4], hot[4], g[4], l[4], e[4], sh[4], d[4];
+        uint32_t bits = 0;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            uint32_t r, c;
+            a.by_cols.divmod(4 * u + w, r, c);
+            if constexpr (HEAD) {
+                const bool hit = row_wanted[r] == static_cast<float>(c);
+                bits |= (hit ? 1u : 0u) << (8 * w);
+                plane[w] = row_scale[r];
+                hot[w] = hit ? 1.0F : 0.0F;
+                g[w] = __fmul_rn(plane[w], hot[w]);
+            } else {
+                g[w] = gs[r * pitch + c];
+            }
+            if constexpr (BACK) {
+                l[w] = (xs[r * pitch + c] - row_peak[r]) - row_lg[r];
+                e[w] = expf(l[w]);
+                sh[w] = __fmul_rn(e[w], row_total[r]);
+                d[w] = __fsub_rn(g[w], sh[w]);
+            }
+        }
+        const int64_t at = base + 4 * u;
+        if constexpr (HEAD) {
+            put<4, false>(a.plane + at, plane);
+            put<4, false>(a.onehot + at, hot);
+            put<4, false>(a.picked + at, g);
+            *reinterpret_cast<uint32_t*>(a.equal + at) = bits;
+        }
+        if constexpr (BACK) {
+            put<4, false>(a.logp + at, l);
+            put<4, false>(a.prob + at, e);
+            put<4, false>(a.share + at, sh);
+            put<4, false>(a.grad + at, d);
+        }
+    }
+    for (uint32_t i = 4 * quads + threadIdx.x; i < n; i += blockDim.x) {
         uint32_t r, c;
         a.by_cols.divmod(i, r, c);
         const float x[1] = {BACK ? xs[r * pitch + c] : 0.0F}, g[1] = {BACK && !HEAD ? gs[r * pitch + c] : 0.0F};
@@ -481,6 +530,7 @@ struct ValueArgs {
     float* sum;
     float* negated;
     float* mean;
+    int quads;           // a, b and product begin on 16 bytes
     float* partial;      // one word per block
     unsigned* arrived;   // counts the blocks; wraps to zero by itself
 };
@@ -565,11 +615,26 @@ __global__ void __launch_bounds__(256) loss_value_tile_kernel(ValueArgs v) {
     const int rows = static_cast<int>(min(int64_t(kTileRows), v.rows - r0));
     const uint32_t n = rows * v.cols;
     const int64_t base = r0 * v.cols;
-    for (uint32_t i = threadIdx.x; i < n; i += 256) {
+    auto keep = [&](uint32_t i, float t) {
         uint32_t r, c;
         v.by_cols.divmod(i, r, c);
-        const float t = __fmul_rn(v.a[base + i], v.b[base + i]);
         p[r * pitch + c] = t;
+    };
+    const uint32_t quads = v.quads != 0 ? n / 4 : 0;
+    for (uint32_t u = threadIdx.x; u < quads; u += 256) {
+        float x[4], y[4];
+        get<4>(v.a + base + 4 * u, x);
+        get<4>(v.b + base + 4 * u, y);
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            x[w] = __fmul_rn(x[w], y[w]);
+            keep(4 * u + w, x[w]);
+        }
+        put<4, false>(v.product + base + 4 * u, x);
+    }
+    for (uint32_t i = 4 * quads + threadIdx.x; i < n; i += 256) {
+        const float t = __fmul_rn(v.a[base + i], v.b[base + i]);
+        keep(i, t);
         v.product[base + i] = t;
     }
     __syncthreads();
@@ -745,11 +810,6 @@ size_t match_backward(const b200_node* const* seq, size_t avail, LossArgs& a) {
 
 template <bool HEAD, bool BACK>
 void launch_rows(b200_ctx* ctx, LossArgs a) {
-    if (a.cols <= kTileCols) {
-        a.by_cols = FastDiv(a.cols);
-        launch_kernel(ctx, loss_tile_kernel<HEAD, BACK>, static_cast<unsigned>(ceil_div(a.rows, kTileRows)), 256, 0, a);
-        return;
-    }
     bool quads = true;
     for (const void* p : {static_cast<const void*>(a.plane), static_cast<const void*>(a.onehot), static_cast<const void*>(a.picked),
                           static_cast<const void*>(a.x), static_cast<const void*>(BACK ? a.g : nullptr), static_cast<const void*>(a.logp),
@@ -757,6 +817,12 @@ void launch_rows(b200_ctx* ctx, LossArgs a) {
         quads = quads && aligned16(p);
     }
     const bool quads_ok = quads && reinterpret_cast<uintptr_t>(a.equal) % 4 == 0;
+    a.quads = quads_ok ? 1 : 0;
+    if (a.cols <= kTileCols) {
+        a.by_cols = FastDiv(a.cols);
+        launch_kernel(ctx, loss_tile_kernel<HEAD, BACK>, static_cast<unsigned>(ceil_div(a.rows, kTileRows)), 256, 0, a);
+        return;
+    }
     const unsigned warps = static_cast<unsigned>(std::min<int64_t>(ceil_div(a.rows, 8), int64_t(sm_count()) * 8));
     const unsigned eights = static_cast<unsigned>(std::min<int64_t>(ceil_div(a.rows, 32), int64_t(sm_count()) * 8));
     const unsigned blocks = static_cast<unsigned>(std::min<int64_t>(a.rows, int64_t(sm_count()) * 8));
@@ -817,6 +883,7 @@ void launch_value(b200_ctx* ctx, ValueArgs v) {
     const unsigned grid = tile ? static_cast<unsigned>(ceil_div(v.rows, kTileRows))
                                : static_cast<unsigned>(std::min<int64_t>(eight ? ceil_div(v.rows, 32) : warp ? ceil_div(v.rows, 8) : v.rows, int64_t(sm_count()) * 8));
     v.by_cols = FastDiv(v.cols);
+    v.quads = quads ? 1 : 0;
     v.partial = static_cast<float*>(ctx->ensure_workspace(sizeof(float) * grid));
     v.arrived = ctx->d_counters + kLossCounter;
     if (tile) launch_kernel(ctx, loss_value_tile_kernel, grid, 256, 0, v);
