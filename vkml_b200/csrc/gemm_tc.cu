@@ -123,19 +123,17 @@ struct SplitArgs {
 
 // Source rows dense along K: one thread per four K-elements, 128-bit stores and, where every row lies on 16
 // bytes, 128-bit loads; no shared memory.
-__device__ __forceinline__ void split_rows(const SplitArgs& a) {
-    const int64_t kp4 = a.kp / 4;
-    const int64_t total = kp4 * a.out_rows * a.n_batches;
-    const int64_t step = int64_t(gridDim.x) * blockDim.x;
-    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += step) {
-        const int64_t k4 = i % kp4;
-        const int64_t rb = i / kp4;
-        const int64_t r = rb % a.out_rows;
-        const int64_t b = rb / a.out_rows;
-        const int64_t k = k4 * 4;
+template <typename I>
+__device__ __forceinline__ void split_rows_as(const SplitArgs& a, I total) {
+    const I kp4 = static_cast<I>(a.kp / 4), out_rows = static_cast<I>(a.out_rows), b1 = static_cast<I>(a.b1);
+    const I step = static_cast<I>(gridDim.x) * blockDim.x;
+    for (I i = static_cast<I>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += step) {
+        const I rb = i / kp4, b = rb / out_rows;
+        const int64_t k = int64_t(i - rb * kp4) * 4, r = rb - b * out_rows;
         float4 v = make_float4(0.0F, 0.0F, 0.0F, 0.0F);
         if (r < a.rows) {
-            const float* src = a.src + (b / a.b1) * a.s_b0 + (b % a.b1) * a.s_b1 + r * a.s_r;
+            const I bo = b / b1;
+            const float* src = a.src + int64_t(bo) * a.s_b0 + int64_t(b - bo * b1) * a.s_b1 + r * a.s_r;
             if (a.vec && k + 3 < a.k) {
                 v = *reinterpret_cast<const float4*>(src + k);
             } else {
@@ -150,12 +148,19 @@ __device__ __forceinline__ void split_rows(const SplitArgs& a) {
         split_tf32(v.y, h.y, l.y);
         split_tf32(v.z, h.z, l.z);
         split_tf32(v.w, h.w, l.w);
-        const int64_t o = rb * a.kp + k;
+        const int64_t o = int64_t(rb) * a.kp + k;
         *reinterpret_cast<float4*>(a.hi + o) = h;
         if (a.lo != nullptr) {
             *reinterpret_cast<float4*>(a.lo + o) = l;
         }
     }
+}
+
+__device__ __forceinline__ void split_rows(const SplitArgs& a) {
+    const int64_t total = a.kp / 4 * a.out_rows * a.n_batches;
+    // (divisions of 64 bits are most of a small matrix' time; the counter runs past the total by less than a grid)
+    if (total < (int64_t(1) << 31)) split_rows_as<uint32_t>(a, static_cast<uint32_t>(total));
+    else split_rows_as<int64_t>(a, total);
 }
 
 // General layouts, 64x64 (rows x k) tiles through shared memory: global reads follow
@@ -226,6 +231,19 @@ __global__ void __launch_bounds__(256) split_kernel(SplitArgs a) {
     pdl_prologue();
     __shared__ float tile[kSplitTile][kSplitTile + 1];
     split_tiles<256>(a, tile);
+}
+
+struct SplitTwo {
+    SplitArgs s[2];
+};
+
+// Both operands of a product side by side.
+__global__ void __launch_bounds__(256) split_two_kernel(const __grid_constant__ SplitTwo p) {
+    pdl_prologue();
+    __shared__ float tile[kSplitTile][kSplitTile + 1];
+    const SplitArgs& a = p.s[blockIdx.y];
+    if (a.unit) split_rows(a);
+    else split_tiles<256>(a, tile);
 }
 
 // Behind a half-term product, in one launch: its operands' strays, or the planes of both for a wide one.  There is mostly little or nothing
@@ -1959,8 +1977,16 @@ void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass) {
     oa.split.lo = oa.lo;
     ob.split.hi = ob.hi;
     ob.split.lo = ob.lo;
-    if (!a_hit) launch_split(ctx, oa.split, "matmul.split_a");
-    if (!b_hit) launch_split(ctx, ob.split, "matmul.split_b");
+    if (!a_hit && !b_hit && ctx->gemm_operands < 0 && !ctx->lone_matmul) {
+        // (among a step's launches one less: 315 rows through an MLP 160-83-32 77 us a step, 64 now; 93 through 284-1130x3-201 233 and 222)
+        ProfScope scope(ctx, "matmul.split");
+        SplitTwo two{{oa.split, ob.split}};
+        launch_kernel(ctx, split_two_kernel, dim3(static_cast<unsigned>(std::max(split_blocks(oa.split), split_blocks(ob.split))), 2), 256, 0, two);
+        ctx->count_launch();
+    } else {
+        if (!a_hit) launch_split(ctx, oa.split, "matmul.split_a");
+        if (!b_hit) launch_split(ctx, ob.split, "matmul.split_b");
+    }
     if (!a_hit || !b_hit) {
         check_last_launch("matmul (operand split)");
     }
