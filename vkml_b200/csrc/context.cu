@@ -243,16 +243,26 @@ GemmProblem matmul_problem(const b200_node& node) {
     return p;
 }
 
-void dispatch_matmul(b200_ctx* ctx, const b200_node& node) {
+// Whether the kernel that writes the product's last sum can write an epilogue as well.
+// A launch inside a step costs 6 to 8 us whatever it does, and these nodes are such launches: an MLP's training step has 13 in place of 15
+// (784-128-10, batch 64: 51.0 us, 50.4 now; 315 rows through 160-83-32 63.9 and 61.5) or 35 in place of 41 (93 rows through 284-1130x3-201
+// 222.6 and 214.7).  Behind a small product the group with ReLU's mask stays the launch of its own that a step's profile shows.
+bool takes_epilogue(b200_ctx* ctx, const GemmProblem& p, const ProductEpilogue& e) {
+    if (p.b0 * p.b1 != 1 || p.m * p.n * p.k == 0) return false;
+    if (ctx->gemm_precision == B200_GEMM_FP32 || !gemm_tc_eligible(ctx, p)) return e.full_a == nullptr && gemm_small_serves(p);
+    return !gemm_inline_serves(ctx, p) && !gemm_h16_serves(ctx, p) && gemm_tc_folds(ctx, p);
+}
+
+void dispatch_matmul(b200_ctx* ctx, const b200_node& node, const ProductEpilogue* epilogue = nullptr) {
     const GemmProblem p = matmul_problem(node);
-    if (gemm_inline_serves(ctx, p)) {
+    if (epilogue == nullptr && gemm_inline_serves(ctx, p)) {
         gemm_inline(ctx, p);
-    } else if (gemm_h16_serves(ctx, p) && gemm_tc_eligible(ctx, p)) {
+    } else if (epilogue == nullptr && gemm_h16_serves(ctx, p) && gemm_tc_eligible(ctx, p)) {
         gemm_h16(ctx, p);
     } else if (ctx->gemm_precision != B200_GEMM_FP32 && gemm_tc_eligible(ctx, p)) {
-        gemm_tc(ctx, p, ctx->gemm_precision == B200_GEMM_3XTF32);
+        gemm_tc(ctx, p, ctx->gemm_precision == B200_GEMM_3XTF32, epilogue);
     } else {
-        gemm_simt(ctx, p);
+        gemm_simt(ctx, p, epilogue);
     }
 }
 
@@ -1041,6 +1051,48 @@ static void compute_span(b200_ctx* ctx, const b200_node* nodes, size_t n_nodes, 
                     p += taken;
                     continue;
                 }
+            }
+        }
+        if (ctx->fuse && node.op == B200_OP_MATMUL && node.out.dtype == B200_F32 && node.out.data != nullptr && p + 1 < exec.size() && is_sink.empty() &&
+            !grad_sync && !touches_f16(node)) {
+            // what follows a product element by element, by the launch that writes the product
+            constexpr size_t kLater = 20;
+            const b200_node* seq[kLater];
+            size_t later = 0;
+            while (later < kLater && p + 1 + later < exec.size() && !done[p + 1 + later] && nodes[exec[p + 1 + later]].out.data != nullptr) {
+                seq[later] = &nodes[exec[p + 1 + later]];
+                ++later;
+            }
+            size_t early = 0;
+            ProductEpilogue e{};
+            const size_t taken = match_product_epilogue(node, seq, std::min<size_t>(later, 5), later, &early, e);
+            bool served = false;
+            if (taken > 0) {
+                prepare(i);  // (checks the operands before they are looked at)
+                if (takes_epilogue(ctx, matmul_problem(node), e)) {
+                    for (size_t k = 0; k < later; ++k) {
+                        if (k < taken || (early > 0 && k == early)) prepare(exec[p + 1 + k]);
+                    }
+                    ctx->current_op = node.op;
+                    dispatch_matmul(ctx, node, &e);
+                    served = true;
+                }
+            }
+            if (served) {
+                constants.erase(node.out.data);
+                finish(i);
+                if (early > 0) {
+                    constants.erase(seq[early]->out.data);
+                    finish(exec[p + 1 + early]);
+                    done[p + 1 + early] = 1;
+                }
+                for (size_t k = 0; k < taken; ++k) {
+                    if (seq[k]->op == B200_OP_FULL && seq[k]->out.dtype == B200_F32) constants[seq[k]->out.data] = tensor_bytes(seq[k]->out);
+                    else constants.erase(seq[k]->out.data);
+                    finish(exec[p + 1 + k]);
+                }
+                p += 1 + taken;
+                continue;
             }
         }
         if (ctx->fuse && exec.size() - p >= 2 &&

@@ -26,6 +26,7 @@
 // layout the kernel reads (dense outputs, a bias that is one contiguous vector), and none of its
 // members is a gradient that a data-parallel span all-reduces.  VKML_B200_FUSE=0 turns it off.
 #include "context.h"
+#include "gemm.h"
 
 namespace b200 {
 namespace {
@@ -155,6 +156,21 @@ __global__ void __launch_bounds__(kThreads) bias_relu_group_kernel(BiasGroup g) 
     }
 }
 
+bool overlaps(const void* p, size_t pn, const void* q, size_t qn) {
+    const char* a = static_cast<const char*>(p);
+    const char* b = static_cast<const char*>(q);
+    return a < b + qn && b < a + pn;
+}
+
+// The span of addresses that the tensor can touch (strided views included).
+size_t bytes_of(const b200_tensor& t) {
+    int64_t hi = static_cast<int64_t>(dtype_size(t.dtype));
+    for (int d = 0; d < t.ndim; ++d) {
+        if (t.dims[d] > 1) hi += (t.dims[d] - 1) * std::abs(t.strides[d]);
+    }
+    return static_cast<size_t>(hi);
+}
+
 // The bias operand of `add`: a broadcast view of ONE contiguous vector, i.e. exactly one axis
 // with extent > 1 carries a stride, and that stride is one element.
 bool bias_layout(const b200_tensor& b, int64_t& inner, int64_t& count) {
@@ -177,8 +193,7 @@ bool bias_layout(const b200_tensor& b, int64_t& inner, int64_t& count) {
 // convolution, whose mask nodes come with the backward pass) and the mask alone.
 // A relu(y) that comes only after other nodes (the layer before the loss, whose relu follows the loss's head) is served
 // here all the same, if it is among `later`: nothing but y is read for it.  `early` then tells its place there.
-size_t fuse_bias_group(b200_ctx* ctx, const b200_node* const* seq, size_t avail, size_t later, size_t* early) {
-    BiasGroup g{};
+size_t match_bias_group(const b200_node* const* seq, size_t avail, size_t later, size_t* early, BiasGroup& g) {
     size_t at = 0;
     const b200_tensor* y = nullptr;  // what the mask compares and the relu reads
     if (seq[0]->op == B200_OP_ADD) {
@@ -241,11 +256,17 @@ size_t fuse_bias_group(b200_ctx* ctx, const b200_node* const* seq, size_t avail,
             }
         }
     }
-    if (at < 2) return 0;  // a lone add: nothing to fuse
     const int64_t n = numel_of(*y);
     if (n == 0) return 0;
     g.n4 = n / 4;
     g.rest = static_cast<int>(n % 4);
+    return at;
+}
+
+size_t fuse_bias_group(b200_ctx* ctx, const b200_node* const* seq, size_t avail, size_t later, size_t* early) {
+    BiasGroup g{};
+    const size_t at = match_bias_group(seq, avail, later, early, g);
+    if (at < 2) return 0;  // a lone add: nothing to fuse
     const char* label = g.bias != nullptr ? (g.full_a != nullptr ? (g.relu != nullptr ? "fused.bias_mask_relu" : "fused.bias_mask")
                                                                  : "fused.bias_relu")
                                           : "fused.mask";
@@ -510,12 +531,6 @@ __global__ void __launch_bounds__(kThreads) scaled_add_group_kernel(const __grid
     }
 }
 
-bool overlaps(const void* p, size_t pn, const void* q, size_t qn) {
-    const char* a = static_cast<const char*>(p);
-    const char* b = static_cast<const char*>(q);
-    return a < b + qn && b < a + pn;
-}
-
 }  // namespace
 
 // `seq`: the next nodes of a span in execution order, the first a scaled_add.  Picks the scaled_add
@@ -528,14 +543,6 @@ size_t launch_scaled_add_group(b200_ctx* ctx, const b200_node* const* seq, size_
     uint64_t blocks = 0;
     size_t n = 0;
     constexpr int64_t kTurnedElements = 1 << 20;
-    auto bytes_of = [](const b200_tensor& t) {
-        // the span of addresses the tensor can touch (strided views included)
-        int64_t hi = static_cast<int64_t>(dtype_size(t.dtype));
-        for (int d = 0; d < t.ndim; ++d) {
-            if (t.dims[d] > 1) hi += (t.dims[d] - 1) * std::abs(t.strides[d]);
-        }
-        return static_cast<size_t>(hi);
-    };
     auto independent = [&](const b200_node& x, const b200_node& y) {
         // x and y may run in either order: neither writes what the other reads or writes
         for (uint32_t s = 0; s < y.n_src && s < B200_MAX_SRC; ++s) {
@@ -604,6 +611,64 @@ size_t launch_scaled_add_group(b200_ctx* ctx, const b200_node* const* seq, size_
 // order); returns how many nodes one fused launch served, or 0.
 // `later` >= avail nodes of `seq` may be looked at for one that a group can serve ahead of its turn; `early` is its
 // place in `seq` then (0: none).
+// Whether `x` writes nothing that the product reads: its blocks may still be reading when others write their results.
+static bool apart(const b200_node& product, const b200_node& x) {
+    for (uint32_t s = 0; s < 2; ++s) {
+        if (product.src[s].data != nullptr && overlaps(x.out.data, bytes_of(x.out), product.src[s].data, bytes_of(product.src[s]))) return false;
+    }
+    // nor the product's result's bytes in another order than its own
+    return x.out.data == product.out.data ? x.out.dtype == B200_F32 : !overlaps(x.out.data, bytes_of(x.out), product.out.data, bytes_of(product.out));
+}
+
+size_t match_product_epilogue(const b200_node& product, const b200_node* const* seq, size_t avail, size_t later, size_t* early, ProductEpilogue& e) {
+    *early = 0;
+    e = ProductEpilogue{};
+    const int64_t n = numel_of(product.out), cols = product.out.dims[product.out.ndim - 1];
+    if (avail == 0 || n == 0 || n >= (int64_t(1) << 31) || n != product.out.dims[product.out.ndim - 2] * cols || !dense_tensor(product.out)) return 0;
+    auto whole = [&](const b200_tensor& t, int dtype) { return t.dtype == dtype && t.data != nullptr && numel_of(t) == n && dense_tensor(t); };
+    const b200_node& first = *seq[0];
+    if (first.op == B200_OP_WHERE) {
+        if (first.n_src != 3 || !whole(first.src[0], B200_BOOL) || !whole(first.src[1], B200_F32) || !whole(first.src[2], B200_F32) ||
+            first.src[2].data != product.out.data || first.src[1].data == product.out.data || !whole(first.out, B200_F32)) {
+            return 0;
+        }
+        if (!apart(product, first) || overlaps(first.out.data, bytes_of(first.out), first.src[0].data, bytes_of(first.src[0]))) return 0;
+        for (int k = 0; k < 2; ++k) {  // (nor does the product overwrite what is chosen from, or its choice)
+            if (overlaps(product.out.data, bytes_of(product.out), first.src[k].data, bytes_of(first.src[k]))) return 0;
+        }
+        e.cond = static_cast<const uint8_t*>(first.src[0].data);
+        e.other = static_cast<const float*>(first.src[1].data);
+        e.chosen = static_cast<float*>(first.out.data);
+        return 1;
+    }
+    if (first.op != B200_OP_ADD || first.n_src != 2 || !whole(first.src[0], B200_F32) || first.src[0].data != product.out.data || !whole(first.out, B200_F32)) {
+        return 0;
+    }
+    BiasGroup g{};
+    const size_t at = match_bias_group(seq, avail, later, early, g);
+    if (at == 0 || g.bias == nullptr || g.x != product.out.data || g.by_inner.d != 1 || int64_t(g.count) != cols) {
+        *early = 0;
+        return 0;
+    }
+    for (size_t k = 0; k < later; ++k) {
+        if ((k < at || (*early > 0 && k == *early)) &&
+            (!apart(product, *seq[k]) || overlaps(seq[k]->out.data, bytes_of(seq[k]->out), g.bias, size_t(cols) * 4) ||
+             overlaps(product.out.data, bytes_of(product.out), g.bias, size_t(cols) * 4))) {
+            *early = 0;
+            return 0;
+        }
+    }
+    e.bias = g.bias;
+    e.add = g.add;
+    e.full_a = g.full_a;
+    e.mask = g.mask;
+    e.full_b = g.full_b;
+    e.value_a = g.value_a;
+    e.value_b = g.value_b;
+    e.relu = g.relu;
+    return at;
+}
+
 size_t launch_fused(b200_ctx* ctx, const b200_node* const* seq, size_t avail, size_t later, size_t* early) {
     *early = 0;
     if (size_t n = fuse_bias_group(ctx, seq, avail, later, early)) return n;

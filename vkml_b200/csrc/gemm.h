@@ -47,14 +47,49 @@ struct Standby {
 };
 constexpr uint32_t kMaxStrays = 512;  // of one matrix; with more it is wide
 
+// What the nodes behind a product make of it, element by element, where the kernel that writes the product can write that too: a bias along the
+// columns with ReLU's mask and a ReLU, or where(cond, other, product).  The values are those of the nodes' own kernels.
+struct ProductEpilogue {
+    const float* bias;  // null: the other form
+    float* add;
+    float* full_a;      // null: no mask
+    uint8_t* mask;
+    float* full_b;
+    float value_a, value_b;
+    float* relu;        // null: none
+    const uint8_t* cond;
+    const float* other;
+    float* chosen;
+};
+#ifdef __CUDACC__
+__device__ __forceinline__ void write_epilogue(const ProductEpilogue& e, int64_t i, int64_t col, float v) {
+    if (e.bias == nullptr) {
+        e.chosen[i] = e.cond[i] != 0 ? e.other[i] : v;
+        return;
+    }
+    const float y = __fadd_rn(v, e.bias[col]);
+    e.add[i] = y;
+    if (e.full_a != nullptr) {
+        e.full_a[i] = e.value_a;
+        e.full_b[i] = e.value_b;
+        e.mask[i] = y <= e.value_a ? 1 : 0;  // false for NaN, as the CPU's comparison
+    }
+    if (e.relu != nullptr) e.relu[i] = y <= 0.0F ? 0.0F : y;
+}
+#endif
+
 // fp32 FMA on the CUDA cores; any strides, any size. gemm_simt.cu
-void gemm_simt(b200_ctx* ctx, const GemmProblem& p);
+void gemm_simt(b200_ctx* ctx, const GemmProblem& p, const ProductEpilogue* epilogue = nullptr);
+// fuse.cu: how many of the nodes `seq` behind `product` one epilogue serves, and which (`early`: a relu further on, as in launch_fused)
+size_t match_product_epilogue(const b200_node& product, const b200_node* const* seq, size_t avail, size_t later, size_t* early, ProductEpilogue& e);
+bool gemm_small_serves(const GemmProblem& p);  // its single-launch kernel, which can write an epilogue
 // Whether its single-launch kernel beats the tensor cores, which could serve `p` too (`streams`: from a streamed operand).
 bool gemm_small_pays(const GemmProblem& p, bool streams);
 
 // tcgen05 tensor-core path (3xTF32 or single-pass TF32). gemm_tc.cu
 bool gemm_tc_eligible(const b200_ctx* ctx, const GemmProblem& p);
-void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass);
+void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass, const ProductEpilogue* epilogue = nullptr);
+bool gemm_tc_folds(const b200_ctx* ctx, const GemmProblem& p);  // in K-slices, whose fold can write an epilogue
 // What is queued behind gemm_h16's kernel.  Its strays' share of the product is added to `target`, the result or its first partial plane;
 // and for the case that an operand turns out wide on the device, the product from TF32 planes: the tiles
 // and K-slices that gemm_tc gives the product, so that its results are gemm_tc's bit for bit.  With slices the partial

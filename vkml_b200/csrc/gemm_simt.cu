@@ -192,6 +192,8 @@ struct SmallArgs {
     int64_t k_chunk;       // of K per CTA of a cluster
     int a_quads, b_quads;  // operands that can be read 16 bytes at a time along their unit-stride axis
     int c_quads;
+    int with;              // an epilogue
+    ProductEpilogue e;
 };
 
 template <int CS>
@@ -263,6 +265,14 @@ __global__ void __launch_bounds__(256) gemm_small_kernel(SmallArgs g) {
             if (n0 + c + 2 < p.n) dst[2] = v.z;
             if (n0 + c + 3 < p.n) dst[3] = v.w;
         }
+        if (g.with != 0) {
+            const int64_t i = dst - p.out;
+            const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (n0 + c + j < p.n) write_epilogue(g.e, i + j, n0 + c + j, e[j]);
+            }
+        }
     };
     if constexpr (CS == 1) {
         store(row, col, sum);
@@ -306,16 +316,15 @@ SmallPlan small_plan(const GemmProblem& p) {
     return s;
 }
 
-bool gemm_small(b200_ctx* ctx, const GemmProblem& p) {
-    const int64_t batches = p.b0 * p.b1;
-    // (what takes longer than a few microseconds is better off with larger tiles and less traffic per product)
-    if (2.0 * double(p.m) * double(p.n) * double(p.k) * double(batches) > double(1 << 26) && !gemm_small_pays(p, false)) return false;
+bool gemm_small(b200_ctx* ctx, const GemmProblem& p, const ProductEpilogue* epilogue) {
+    if (!gemm_small_serves(p)) return false;
     SmallArgs g{};
     g.p = p;
     g.tiles_m = ceil_div(p.m, kTile);
     g.tiles_n = ceil_div(p.n, kTile);
     const auto [tiles, cs] = small_plan(p);
-    if (tiles > (int64_t(1) << 28)) return false;
+    g.with = epilogue != nullptr ? 1 : 0;
+    if (epilogue != nullptr) g.e = *epilogue;
     g.k_chunk = ceil_div(ceil_div(p.k, cs), 4) * 4;
     const bool a_k = p.a_s[3] == 1 || p.a_s[2] != 1, b_k = p.b_s[2] == 1 && p.b_s[3] != 1;
     g.a_quads = a_k ? p.a_s[3] == 1 && quad_operand(p.a, p.k, p.a_s[2], p.a_s[0], p.a_s[1]) : quad_operand(p.a, p.m, p.a_s[3], p.a_s[0], p.a_s[1]);
@@ -349,7 +358,13 @@ bool gemm_small_pays(const GemmProblem& p, bool streams) {
     return s.tiles * s.cs <= 2 * sm_count() && ceil_div(p.k, s.cs) <= 2 * kRound && p.k <= 480;
 }
 
-void gemm_simt(b200_ctx* ctx, const GemmProblem& p) {
+bool gemm_small_serves(const GemmProblem& p) {
+    // (what takes longer than a few microseconds is better off with larger tiles and less traffic per product)
+    const double flops = 2.0 * double(p.m) * double(p.n) * double(p.k) * double(p.b0 * p.b1);
+    return flops > 0 && (flops <= double(1 << 26) || gemm_small_pays(p, false)) && small_plan(p).tiles <= (int64_t(1) << 28);
+}
+
+void gemm_simt(b200_ctx* ctx, const GemmProblem& p, const ProductEpilogue* epilogue) {
     const int64_t batches = p.b0 * p.b1;
     const int64_t out_elems = batches * p.m * p.n;
     if (out_elems == 0) {
@@ -359,7 +374,7 @@ void gemm_simt(b200_ctx* ctx, const GemmProblem& p) {
         B200_CUDA_CHECK(cudaMemsetAsync(p.out, 0, sizeof(float) * out_elems, ctx->stream));
         return;
     }
-    if (gemm_small(ctx, p)) {
+    if (gemm_small(ctx, p, epilogue)) {
         return;
     }
     const int64_t tiles = batches * ceil_div(p.m, BM) * ceil_div(p.n, BN);

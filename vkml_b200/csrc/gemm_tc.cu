@@ -1315,9 +1315,32 @@ fold_partials_kernel(float* __restrict__ out, const float* __restrict__ partial,
     }
 }
 
+// The same with what the nodes behind the product make of it: bound by its latency at the sizes that are folded, so an element to a thread,
+// whose epilogue needs no alignment, and the nodes' results cost no pass over the sum (6.4 us in a step, with the group's launch behind it 12.9 before).
+__global__ void __launch_bounds__(256) fold_epilogue_kernel(float* __restrict__ out, const float* __restrict__ partial, uint32_t n, int splits,
+                                                            FastDiv by_cols, const __grid_constant__ ProductEpilogue e) {
+    pdl_prologue();
+    const uint32_t stride = gridDim.x * blockDim.x;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        float acc = __ldcg(partial + i);
+#pragma unroll 4
+        for (int s = 1; s < splits; ++s) acc += __ldcg(partial + int64_t(s) * n + i);
+        out[i] = acc;
+        write_epilogue(e, i, i - by_cols.div(i) * by_cols.d, acc);
+    }
+}
+
 // Adds the K-slices' partial planes in split order (one slice: nothing to do).
-void fold_partials(b200_ctx* ctx, float* out, const float* partial, int64_t n, int splits) {
+void fold_partials(b200_ctx* ctx, float* out, const float* partial, int64_t n, int splits, const ProductEpilogue* e = nullptr, int64_t cols = 0) {
     if (splits <= 1) return;
+    if (e != nullptr) {
+        ProfScope scope(ctx, "matmul.fold");
+        launch_kernel(ctx, fold_epilogue_kernel, grid_for(n, 256), 256, 0, out, partial, static_cast<uint32_t>(n), splits,
+                      FastDiv(static_cast<uint32_t>(cols)), *e);
+        ctx->count_launch();
+        check_last_launch("matmul (fold and epilogue)");
+        return;
+    }
     ProfScope scope(ctx, "matmul.fold");
     // four elements to a thread where that still fills the machine: a small result with many slices is bound by the loads in
     // flight (384 x 128 x 2 with 24 slices: the product 43.5 us with quads, 42 without)
@@ -1668,7 +1691,15 @@ void launch_stream(b200_ctx* ctx, bool three_pass, bool w_mn, bool s_km, const C
 #undef B200_STREAM_CASE
 }
 
-void gemm_stream(b200_ctx* ctx, const GemmProblem& p, bool three_pass, const StreamPlan& sp) {
+int64_t stream_slices(const b200_ctx* ctx, const GemmProblem& p, const StreamPlan& sp) {
+    const int64_t tiles = ceil_div(p.m, sp.bnw) * (sp.bpt > 1 ? 1 : ceil_div(p.n, 128)) * ceil_div(p.b0 * p.b1, sp.bpt), sms = ctx->prop.multiProcessorCount;
+    const int64_t k_blocks = align_up(p.k, BK) / BK;
+    int64_t splits = 1;
+    if (tiles < sms && k_blocks >= 16) splits = std::max<int64_t>(1, std::min<int64_t>(std::min(sms / tiles, k_blocks / 8), 64));
+    return ceil_div(k_blocks, ceil_div(k_blocks, splits));
+}
+
+void gemm_stream(b200_ctx* ctx, const GemmProblem& p, bool three_pass, const StreamPlan& sp, const ProductEpilogue* epilogue) {
     const int64_t batches = p.b0 * p.b1;
     const bool a_bcast = (p.a_s[0] == 0 || p.b0 == 1) && (p.a_s[1] == 0 || p.b1 == 1);
     Operand ow = plan_operand(p.a, p.a_s[0], p.a_s[1], p.a_s[2], p.a_s[3], p.m, p.k, a_bcast, p);
@@ -1678,13 +1709,7 @@ void gemm_stream(b200_ctx* ctx, const GemmProblem& p, bool three_pass, const Str
     const int64_t batch_groups = ceil_div(batches, sp.bpt);
     const int64_t tiles = tiles_m * tiles_n * batch_groups;
     const int sms = ctx->prop.multiProcessorCount;
-    int64_t splits = 1;
-    if (tiles < sms && k_blocks >= 16) {
-        splits = std::min<int64_t>(sms / tiles, k_blocks / 8);
-        splits = std::max<int64_t>(1, std::min<int64_t>(splits, 64));
-    }
-    const int64_t kb_per_split = ceil_div(k_blocks, splits);
-    splits = ceil_div(k_blocks, kb_per_split);
+    const int64_t kb_per_split = ceil_div(k_blocks, stream_slices(ctx, p, sp)), splits = ceil_div(k_blocks, kb_per_split);
     const int64_t out_elems = batches * p.m * p.n;
     const size_t partial_bytes = splits > 1 ? static_cast<size_t>(align_up(out_elems * splits * 4, 1024)) : 0;
 
@@ -1759,7 +1784,7 @@ void gemm_stream(b200_ctx* ctx, const GemmProblem& p, bool three_pass, const Str
     }
     ctx->count_launch();
     check_last_launch("matmul (tcgen05, streamed operand)");
-    fold_partials(ctx, p.out, partial, out_elems, static_cast<int>(splits));
+    fold_partials(ctx, p.out, partial, out_elems, static_cast<int>(splits), epilogue, p.n);
     release_use(ctx, ow);
 }
 
@@ -1846,9 +1871,14 @@ void gemm_tc_wait_probe(b200_ctx* ctx, uint64_t limit_ns) {
     check_last_launch("wait probe");
 }
 
-void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass) {
+bool gemm_tc_folds(const b200_ctx* ctx, const GemmProblem& p) {
+    const StreamPlan sp = plan_stream(ctx, p);
+    return (sp.ok ? stream_slices(ctx, p, sp) : plan_planes(ctx, p).splits) > 1;
+}
+
+void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass, const ProductEpilogue* epilogue) {
     if (const StreamPlan sp = plan_stream(ctx, p); sp.ok) {
-        gemm_stream(ctx, p, three_pass, sp);
+        gemm_stream(ctx, p, three_pass, sp, epilogue);
         return;
     }
     const int64_t batches = p.b0 * p.b1;
@@ -1875,7 +1905,7 @@ void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass) {
             partial = reinterpret_cast<float*>(align_up(reinterpret_cast<int64_t>(ws), 1024));
         }
         gemm_inline_tf32(ctx, p, partial, splits, kb_per_split, direct ? "matmul.tcgen05_3xtf32_direct" : "matmul.tcgen05_3xtf32");
-        fold_partials(ctx, p.out, partial, out_elems, static_cast<int>(splits));
+        fold_partials(ctx, p.out, partial, out_elems, static_cast<int>(splits), epilogue, p.n);
         return;
     }
 
@@ -1923,7 +1953,7 @@ void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass) {
         }
         ctx->count_launch();
         check_last_launch("matmul (tcgen05, direct operands)");
-        fold_partials(ctx, p.out, partial, out_elems, static_cast<int>(splits));
+        fold_partials(ctx, p.out, partial, out_elems, static_cast<int>(splits), epilogue, p.n);
         return;
     }
 
@@ -2041,7 +2071,7 @@ void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass) {
     ctx->count_launch();
     check_last_launch("matmul (tcgen05)");
 
-    fold_partials(ctx, p.out, partial, out_elems, static_cast<int>(splits));
+    fold_partials(ctx, p.out, partial, out_elems, static_cast<int>(splits), epilogue, p.n);
     // the stream is in order: a plane released here is only reused by later work
     release_use(ctx, oa);
     release_use(ctx, ob);
