@@ -364,7 +364,8 @@ __global__ void __launch_bounds__(kPairThreads, 2) split_pair_kernel(const __gri
     }
     if (p.done[blockIdx.y] != nullptr && __ldcg(p.done[blockIdx.y]) != 0) return;
     const SplitArgs& a = p.s[blockIdx.y];
-    if (a.unit) split_rows(a);
+    // (one width of index alone: this launch mostly has nothing to do, and with both widths 1000x1433x777 took 36.5 us for 36.2)
+    if (a.unit) split_rows_as<int64_t>(a, a.kp / 4 * a.out_rows * a.n_batches);
     else split_tiles<kPairThreads>(a, sm.tile);
 }
 
