@@ -61,3 +61,24 @@ def test_epilogue_has_the_nodes_bits(monkeypatch, form, m, k, n):
         np.testing.assert_array_equal(got, want)
     if form == "where" or (form == "add" and n > 1):  # (a bias of one element is no vector: its add stays a launch)
         assert len(launches[1]) == len(launches[0]) - 1, launches
+
+
+# a result that lies where the product still reads: the nodes keep their own launches
+@pytest.mark.parametrize("m,k", [(33, 33), (70, 130), (128, 1130)])
+@pytest.mark.parametrize("side", [0, 1])
+def test_results_over_an_operand(monkeypatch, m, k, side):
+    results = []
+    for fuse in ("0", "1"):
+        monkeypatch.setenv("VKML_B200_FUSE", fuse)
+        b = Backend(0)
+        rng = np.random.default_rng(m + k)
+        rows, n = (m, k) if side == 0 else (k, m)  # the result has the shape of the operand that it overwrites
+        shapes = [(1, 1, m, k), (1, 1, k, k)] if side == 0 else [(1, 1, k, k), (1, 1, k, m)]
+        x, w = (DeviceTensor.from_host(b, rng.standard_normal(s, dtype=np.float32)) for s in shapes)
+        prod, bias = DeviceTensor.empty(b, (1, 1, rows, n)), DeviceTensor.from_host(b, rng.standard_normal(n).astype(np.float32))
+        over = (x, w)[side].reshape((rows, n))
+        b.compute([NodeDesc(int(Op.MATMUL), prod.desc, [x.desc, w.desc]),
+                   NodeDesc(int(Op.ADD), over.desc, [prod.reshape((rows, n)).desc, bias.reshape((1, n)).broadcast_to((rows, n)).desc])])
+        results.append((prod.numpy(), over.numpy()))
+    for got, want in zip(results[1], results[0]):
+        np.testing.assert_array_equal(got, want)
