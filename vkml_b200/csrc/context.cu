@@ -246,10 +246,11 @@ GemmProblem matmul_problem(const b200_node& node) {
 // Whether the kernel that writes the product's last sum can write an epilogue as well.
 // A launch inside a step costs 6 to 8 us whatever it does, and these nodes are such launches: an MLP's training step has 13 in place of 15
 // (784-128-10, batch 64: 51.0 us, 50.4 now; 315 rows through 160-83-32 63.9 and 61.5) or 35 in place of 41 (93 rows through 284-1130x3-201
-// 222.6 and 214.7).  Behind a small product the group with ReLU's mask stays the launch of its own that a step's profile shows.
+// 222.6 and 214.7).  A small product writes it word by word, which over many elements takes longer than the launch: 361 rows through 307-2484x3-14,
+// whose where follows a result of 361x2484, 323.7 us a step with it and 316.3 without; 560x455 gains.  Behind a small product the group with ReLU's mask stays the launch of its own that a step's profile shows.
 bool takes_epilogue(b200_ctx* ctx, const GemmProblem& p, const ProductEpilogue& e) {
     if (p.b0 * p.b1 != 1 || p.m * p.n * p.k == 0) return false;
-    if (ctx->gemm_precision == B200_GEMM_FP32 || !gemm_tc_eligible(ctx, p)) return e.full_a == nullptr && gemm_small_serves(p);
+    if (ctx->gemm_precision == B200_GEMM_FP32 || !gemm_tc_eligible(ctx, p)) return e.full_a == nullptr && p.m * p.n <= (int64_t(1) << 18) && gemm_small_serves(p);
     return !gemm_inline_serves(ctx, p) && !gemm_h16_serves(ctx, p) && gemm_tc_folds(ctx, p);
 }
 

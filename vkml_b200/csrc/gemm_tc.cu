@@ -123,16 +123,56 @@ struct SplitArgs {
 
 // Source rows dense along K: one thread per four K-elements, 128-bit stores and, where every row lies on 16
 // bytes, 128-bit loads; no shared memory.
-template <typename I>
-__device__ __forceinline__ void split_rows_as(const SplitArgs& a, I total) {
-    const I kp4 = static_cast<I>(a.kp / 4), out_rows = static_cast<I>(a.out_rows), b1 = static_cast<I>(a.b1);
-    const I step = static_cast<I>(gridDim.x) * blockDim.x;
-    for (I i = static_cast<I>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += step) {
-        const I rb = i / kp4, b = rb / out_rows;
+__device__ __forceinline__ void split_rows(const SplitArgs& a) {
+    const int64_t kp4 = a.kp / 4;
+    const int64_t total = kp4 * a.out_rows * a.n_batches;
+    const int64_t step = int64_t(gridDim.x) * blockDim.x;
+    for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += step) {
+        const int64_t k4 = i % kp4;
+        const int64_t rb = i / kp4;
+        const int64_t r = rb % a.out_rows;
+        const int64_t b = rb / a.out_rows;
+        const int64_t k = k4 * 4;
+        float4 v = make_float4(0.0F, 0.0F, 0.0F, 0.0F);
+        if (r < a.rows) {
+            const float* src = a.src + (b / a.b1) * a.s_b0 + (b % a.b1) * a.s_b1 + r * a.s_r;
+            if (a.vec && k + 3 < a.k) {
+                v = *reinterpret_cast<const float4*>(src + k);
+            } else {
+                if (k < a.k) v.x = src[k];
+                if (k + 1 < a.k) v.y = src[k + 1];
+                if (k + 2 < a.k) v.z = src[k + 2];
+                if (k + 3 < a.k) v.w = src[k + 3];
+            }
+        }
+        float4 h, l;
+        split_tf32(v.x, h.x, l.x);
+        split_tf32(v.y, h.y, l.y);
+        split_tf32(v.z, h.z, l.z);
+        split_tf32(v.w, h.w, l.w);
+        const int64_t o = rb * a.kp + k;
+        *reinterpret_cast<float4*>(a.hi + o) = h;
+        if (a.lo != nullptr) {
+            *reinterpret_cast<float4*>(a.lo + o) = l;
+        }
+    }
+}
+
+// The same with 32-bit indexes, for fewer than kSmallQuads quads: divisions of 64 bits are most of a small matrix' time (64x4096x4096 35.4 us a
+// product with them, 34.9 without).  In kernels of its own: with both widths in one, 1000x1433x777, whose standby launch has nothing to
+// split, took 36.5 us for 36.2; and large planes are the 64-bit loop's (a CNN's at batch 231 82.4 us with it, 88.5 with this one).
+constexpr int64_t kSmallQuads = int64_t(1) << 22;
+
+__device__ __forceinline__ void split_rows_small(const SplitArgs& a) {
+    const uint32_t total = static_cast<uint32_t>(a.kp / 4 * a.out_rows * a.n_batches);
+    const uint32_t kp4 = static_cast<uint32_t>(a.kp / 4), out_rows = static_cast<uint32_t>(a.out_rows), b1 = static_cast<uint32_t>(a.b1);
+    const uint32_t step = static_cast<uint32_t>(gridDim.x) * blockDim.x;
+    for (uint32_t i = static_cast<uint32_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += step) {
+        const uint32_t rb = i / kp4, b = rb / out_rows;
         const int64_t k = int64_t(i - rb * kp4) * 4, r = rb - b * out_rows;
         float4 v = make_float4(0.0F, 0.0F, 0.0F, 0.0F);
         if (r < a.rows) {
-            const I bo = b / b1;
+            const uint32_t bo = b / b1;
             const float* src = a.src + int64_t(bo) * a.s_b0 + int64_t(b - bo * b1) * a.s_b1 + r * a.s_r;
             if (a.vec && k + 3 < a.k) {
                 v = *reinterpret_cast<const float4*>(src + k);
@@ -154,13 +194,6 @@ __device__ __forceinline__ void split_rows_as(const SplitArgs& a, I total) {
             *reinterpret_cast<float4*>(a.lo + o) = l;
         }
     }
-}
-
-__device__ __forceinline__ void split_rows(const SplitArgs& a) {
-    const int64_t total = a.kp / 4 * a.out_rows * a.n_batches;
-    // (divisions of 64 bits are most of a small matrix' time; the counter runs past the total by less than a grid)
-    if (total < (int64_t(1) << 31)) split_rows_as<uint32_t>(a, static_cast<uint32_t>(total));
-    else split_rows_as<int64_t>(a, total);
 }
 
 // General layouts, 64x64 (rows x k) tiles through shared memory: global reads follow
@@ -227,6 +260,11 @@ __global__ void __launch_bounds__(256) split_rows_kernel(SplitArgs a) {
     split_rows(a);
 }
 
+__global__ void __launch_bounds__(256) split_rows_small_kernel(SplitArgs a) {
+    pdl_prologue();
+    split_rows_small(a);
+}
+
 __global__ void __launch_bounds__(256) split_kernel(SplitArgs a) {
     pdl_prologue();
     __shared__ float tile[kSplitTile][kSplitTile + 1];
@@ -242,7 +280,7 @@ __global__ void __launch_bounds__(256) split_two_kernel(const __grid_constant__ 
     pdl_prologue();
     __shared__ float tile[kSplitTile][kSplitTile + 1];
     const SplitArgs& a = p.s[blockIdx.y];
-    if (a.unit) split_rows(a);
+    if (a.unit) split_rows_small(a);
     else split_tiles<256>(a, tile);
 }
 
@@ -364,8 +402,7 @@ __global__ void __launch_bounds__(kPairThreads, 2) split_pair_kernel(const __gri
     }
     if (p.done[blockIdx.y] != nullptr && __ldcg(p.done[blockIdx.y]) != 0) return;
     const SplitArgs& a = p.s[blockIdx.y];
-    // (one width of index alone: this launch mostly has nothing to do, and with both widths 1000x1433x777 took 36.5 us for 36.2)
-    if (a.unit) split_rows_as<int64_t>(a, a.kp / 4 * a.out_rows * a.n_batches);
+    if (a.unit) split_rows(a);
     else split_tiles<kPairThreads>(a, sm.tile);
 }
 
@@ -376,7 +413,8 @@ int64_t split_blocks(const SplitArgs& s) {
 
 void launch_split(b200_ctx* ctx, const SplitArgs& s, const char* label) {
     ProfScope scope(ctx, label);
-    if (s.unit) launch_kernel(ctx, split_rows_kernel, static_cast<unsigned>(split_blocks(s)), 256, 0, s);
+    if (s.unit && s.kp / 4 * s.out_rows * s.n_batches < kSmallQuads) launch_kernel(ctx, split_rows_small_kernel, static_cast<unsigned>(split_blocks(s)), 256, 0, s);
+    else if (s.unit) launch_kernel(ctx, split_rows_kernel, static_cast<unsigned>(split_blocks(s)), 256, 0, s);
     else launch_kernel(ctx, split_kernel, static_cast<unsigned>(split_blocks(s)), 256, 0, s);
     ctx->count_launch();
 }
@@ -2008,7 +2046,10 @@ void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass, const Product
     oa.split.lo = oa.lo;
     ob.split.hi = ob.hi;
     ob.split.lo = ob.lo;
-    if (!a_hit && !b_hit && ctx->gemm_operands < 0 && !ctx->lone_matmul) {
+    auto elements = [](const SplitArgs& s) { return s.kp * s.out_rows * s.n_batches; };
+    if (!a_hit && !b_hit && ctx->gemm_operands < 0 && !ctx->lone_matmul && elements(oa.split) + elements(ob.split) < 4 * kSmallQuads) {
+        // (over more elements the launch saved is no longer seen: an MLP 4096-8192x3-1000 at batch 2048 561 us of splits apart, 565 together; 7 M,
+        // 361x2484 and 2484x2484, 30 apart and 25 together)
         // (among a step's launches one less: 315 rows through an MLP 160-83-32 77 us a step, 64 now; 93 through 284-1130x3-201 233 and 222)
         ProfScope scope(ctx, "matmul.split");
         SplitTwo two{{oa.split, ob.split}};
