@@ -48,6 +48,10 @@ constexpr int kSamplePieces = 4;       // of 128 consecutive elements, per conve
 constexpr int kPieces = 32;             // of one operand
 constexpr uint32_t kEarlyStrays = 4;   // in a sample of 4096: more, and the matrix is taken to be wide without trying
 
+// A thread's rows lie this many apart at most.  Their distance in bytes is held in 32 bits, which bounds the pitches that are served
+// (gemm_inline_fits): 64 bits would cost a multiplication more per load, in warps that wait for nothing but their loads.
+constexpr int max_row_step(bool tf32) { return tf32 ? 32 : 16; }
+
 // One operand as the matrix with `mn` lines along K.
 struct InlineSide {
     const float* base;
@@ -133,6 +137,7 @@ struct Feed {
     static constexpr int kQuads = kBlock / 8;
     static constexpr int kLanes = MN ? ROWS / 4 : kBlock / 4;
     static constexpr int kRowStep = 2 * ROWS / kLanes;
+    static_assert(kRowStep <= max_row_step(TF32), "pitches are bounded by it");
     const InlineSide& s;
     int along, row;   // this thread's first element: offset along the unit axis, row of the tile
     uint32_t offset;  // of its first quad in a tile
@@ -192,6 +197,7 @@ struct LaneFeed {
     static constexpr int kQuads = 4;  // sixteen elements, four at a time
     static constexpr int kWarps = ROWS / 16, kAtoms = ROWS / 32;
     static constexpr int kStep = MN ? 2 : kWarps;  // rows between its elements
+    static_assert(kStep <= max_row_step(true), "pitches are bounded by it");
     const InlineSide& s;
     int lane, row, atom;   // of its first element
     uint32_t even, odd;    // where its elements go: their swizzle alternates
@@ -1001,7 +1007,7 @@ bool gemm_inline_serves(const b200_ctx* ctx, const GemmProblem& p) {
         !gemm_tc_eligible(ctx, p) || gemm_tc_chain(ctx, p) > 12288) {
         return false;
     }
-    if (!gemm_inline_fits(p)) return false;
+    if (!gemm_inline_fits(p, false)) return false;
     const InlinePlan t = plan_inline(ctx, p);
     if (ctx->gemm_inline > 0) return ctx->gemm_inline < 8;
     const bool direct = ctx->lone_matmul && gemm_tc_reads_directly(ctx, p);
@@ -1117,10 +1123,12 @@ void gemm_inline_tf32(b200_ctx* ctx, const GemmProblem& p, float* partial, int64
     check_last_launch("matmul (tcgen05, TF32 terms split in the kernel)");
 }
 
-bool gemm_inline_fits(const GemmProblem& p) {
-    // (a thread's rows are within 32 bits of bytes from one another; units and lines are counted in 31)
+bool gemm_inline_fits(const GemmProblem& p, bool tf32) {
+    // (a thread's neighbouring rows are less than 2^31 bytes apart: pitches below 2^25 floats for half terms, 2^24 for TF32 terms; units and
+    // lines are counted in 31 bits)
+    const int64_t pitch = (int64_t(1) << 31) / (4 * max_row_step(tf32));
     for (int i = 2; i < 4; ++i) {
-        if (std::abs(p.a_s[i]) >= (int64_t(1) << 25) || std::abs(p.b_s[i]) >= (int64_t(1) << 25)) return false;
+        if (std::abs(p.a_s[i]) >= pitch || std::abs(p.b_s[i]) >= pitch) return false;
     }
     const int64_t lim = int64_t(1) << 30;
     return p.m < lim && p.n < lim && p.k < lim && p.b0 * p.b1 < lim &&

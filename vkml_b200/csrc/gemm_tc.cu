@@ -1594,7 +1594,7 @@ struct TcPlan {
 // CNN 12 us).  A compared product of 2^28 operations, up to which fp32 tiles would serve it, keeps its planes.
 bool inline_pays(const b200_ctx* ctx, const GemmProblem& p, const Operand& oa, const Operand& ob, const TcPlan& plan, bool direct) {
     if (ctx->gemm_inline == 0 || ctx->gemm_operands >= 0 || ctx->gemm_stream > 0 || ctx->gemm_bn_override != 0 || ctx->gemm_schedule == 1 ||
-        (ctx->gemm_schedule < 0 && ctx->in_grad_sync_span) || !gemm_inline_fits(p)) {
+        (ctx->gemm_schedule < 0 && ctx->in_grad_sync_span) || !gemm_inline_fits(p, true)) {
         return false;
     }
     if (ctx->gemm_inline >= 8) return true;
