@@ -383,8 +383,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f16_any_kernel(const __grid_
     }
 }
 
-// The K-slices' partial planes in split order, and the layer's bias and relu behind them.
-__global__ void __launch_bounds__(256) fold_f16_kernel(const __grid_constant__ F16Args g, __half* __restrict__ out, const float* __restrict__ part, FastDiv by_n) {
+// The K-slices' partial planes in split order, and the layer's bias and relu behind them, whose results may lie over `out`.
+__global__ void __launch_bounds__(256) fold_f16_kernel(const __grid_constant__ F16Args g, __half* out, const float* __restrict__ part, FastDiv by_n) {
     pdl_prologue();
     const int64_t total = g.split_stride, step = int64_t(gridDim.x) * blockDim.x;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += step) {

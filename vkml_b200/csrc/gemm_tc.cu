@@ -1356,7 +1356,8 @@ fold_partials_kernel(float* __restrict__ out, const float* __restrict__ partial,
 
 // The same with what the nodes behind the product make of it: bound by its latency at the sizes that are folded, so an element to a thread,
 // whose epilogue needs no alignment, and the nodes' results cost no pass over the sum (6.4 us in a step, with the group's launch behind it 12.9 before).
-__global__ void __launch_bounds__(256) fold_epilogue_kernel(float* __restrict__ out, const float* __restrict__ partial, uint32_t n, int splits,
+// (Those results may lie over `out`.)
+__global__ void __launch_bounds__(256) fold_epilogue_kernel(float* out, const float* __restrict__ partial, uint32_t n, int splits,
                                                             FastDiv by_cols, const __grid_constant__ ProductEpilogue e) {
     pdl_prologue();
     const uint32_t stride = gridDim.x * blockDim.x;
