@@ -69,6 +69,22 @@ inline size_t dtype_size(int dt) {
     }
 }
 
+// Whether two tensors have memory in common: from a tensor's first to its last address, whichever way its strides run.
+inline bool overlap(const b200_tensor& x, const b200_tensor& y) {
+    auto first_and_end = [](const b200_tensor& t, const char*& lo, const char*& hi) {
+        lo = static_cast<const char*>(t.data);
+        hi = lo + dtype_size(t.dtype);
+        for (int d = 0; d < t.ndim; ++d) {
+            if (t.dims[d] == 0) return false;
+            const int64_t reach = (t.dims[d] - 1) * t.strides[d];
+            (reach < 0 ? lo : hi) += reach;
+        }
+        return true;
+    };
+    const char *x_lo, *x_hi, *y_lo, *y_hi;
+    return x.data != nullptr && y.data != nullptr && first_and_end(x, x_lo, x_hi) && first_and_end(y, y_lo, y_hi) && x_lo < y_hi && y_lo < x_hi;
+}
+
 // A tensor view with ELEMENT strides, always padded to rank 4 by leading
 // extents of 1 (so linear index decomposition is the same loop everywhere).
 struct View {

@@ -291,10 +291,21 @@ bool half_linear(const b200_node& mm, const b200_node& add, const b200_node* rel
         b.data == nullptr) {
         return false;
     }
+    // The product's blocks still read when others write their results: those lie over neither operand nor bias, and over each other whole or not at all.
+    auto apart = [&](const b200_tensor& out) {
+        for (const b200_tensor* t : {&mm.src[0], &mm.src[1], &b}) {
+            if (overlap(out, *t)) return false;
+        }
+        for (const b200_tensor* t : {&mm.out, &add.out}) {
+            if (out.data != t->data && overlap(out, *t)) return false;
+        }
+        return true;
+    };
+    if (!apart(mm.out) || !apart(add.out)) return false;
     epi.bias = b.data;
     epi.biased = add.out.data;
     if (relu != nullptr && relu->op == B200_OP_RELU && relu->n_src == 1 && half_matrix(relu->out) && half_matrix(relu->src[0]) &&
-        relu->src[0].data == add.out.data) {
+        relu->src[0].data == add.out.data && apart(relu->out)) {
         epi.rectified = relu->out.data;
     }
     return true;
