@@ -78,3 +78,42 @@ def test_half_layers_over_their_operands(backend, side, over, relu):
     for _ in range(3):
         got = half_layer(backend, x, w, bias, over, relu)
         assert np.array_equal(got.view(np.uint16), want.view(np.uint16))
+
+
+# the small kernel; TF32 and half terms split inside the kernel, half terms from planes, the streamed operand; halves that TMA reads and does not
+@pytest.mark.parametrize("dtype,m,k", [("f4", 33, 33), ("f4", 97, 130), ("f4", 512, 512), ("f4", 301, 1003), ("f4", 1400, 1204), ("f4", 4096, 768), ("f4", 64, 4096),
+                                       ("f2", 301, 301), ("f2", 768, 512), ("f2", 40, 1500), ("f2", 2050, 517)])
+@pytest.mark.parametrize("side", [0, 1])
+@pytest.mark.parametrize("turned", [False, True])
+def test_products_over_their_operand(backend, dtype, m, k, side, turned):
+    rng = np.random.default_rng(m + k)
+    shapes = [(m, k), (k, k)] if side == 0 else [(k, k), (k, m)]
+    a, b = (rng.standard_normal(s).astype(dtype) for s in shapes)
+    results = []
+    for over in (False, True, True):
+        put = [DeviceTensor.from_host(backend, t.reshape((1, 1) + t.shape)) for t in (a, b)]
+        if turned:  # the operand that is not written over, stored the other way round
+            t = (a, b)[1 - side]
+            put[1 - side] = DeviceTensor.from_host(backend, np.ascontiguousarray(t.T).reshape((1, 1) + t.T.shape)).transpose(2, 3)
+        out = put[side] if over else DeviceTensor.empty(backend, (1, 1, a.shape[0], b.shape[1]), put[0].dtype)
+        backend.compute([NodeDesc(int(Op.MATMUL), out.desc, [t.desc for t in put])])
+        results.append(out.numpy().astype(np.float64))
+    want, terms = a.astype(np.float64) @ b.astype(np.float64), np.abs(a).astype(np.float64) @ np.abs(b).astype(np.float64)
+    rounding = 2.0 ** -11 * np.abs(want) if dtype == "f2" else 0  # (widened copies add in another order: neighbours may differ)
+    for got in results:
+        assert np.all(np.abs(got.reshape(want.shape) - want) <= (k / 8 / 4 * 2.0 ** -23 + 2.0 ** -20) * terms + rounding)
+    if dtype == "f4":
+        assert np.array_equal(results[0], results[1]) and np.array_equal(results[0], results[2])
+
+
+def test_a_span_reads_what_was_written_over_an_operand(backend):
+    """x . w, x <- x . w, x . w again: the planes of the first x are not those of the second."""
+    rng = np.random.default_rng(5)
+    x, w = rng.standard_normal((1536, 1280), dtype=np.float32), rng.standard_normal((1280, 1280), dtype=np.float32) / np.float32(36)
+    dx, dw = (DeviceTensor.from_host(backend, t.reshape((1, 1) + t.shape)) for t in (x, w))
+    first, last = (DeviceTensor.empty(backend, dx.dims) for _ in range(2))
+    product = lambda out: NodeDesc(int(Op.MATMUL), out.desc, [dx.desc, dw.desc])
+    backend.compute([product(first), product(dx), product(last)])
+    x, w = x.astype(np.float64), w.astype(np.float64)
+    for got, want in ((first, x @ w), (dx, x @ w), (last, x @ w @ w)):
+        assert np.linalg.norm(got.numpy().reshape(want.shape) - want) <= 2e-5 * np.linalg.norm(want)

@@ -249,13 +249,12 @@ GemmProblem matmul_problem(const b200_node& node) {
 // 222.6 and 214.7).  A small product writes it word by word, which over many elements takes longer than the launch: 361 rows through 307-2484x3-14,
 // whose where follows a result of 361x2484, 323.7 us a step with it and 316.3 without; 560x455 gains.  Behind a small product the group with ReLU's mask stays the launch of its own that a step's profile shows.
 bool takes_epilogue(b200_ctx* ctx, const GemmProblem& p, const ProductEpilogue& e) {
-    if (p.b0 * p.b1 != 1 || p.m * p.n * p.k == 0) return false;
+    if (p.b0 * p.b1 != 1 || p.m * p.n * p.k == 0 || result_over_operand(p, sizeof(float))) return false;
     if (ctx->gemm_precision == B200_GEMM_FP32 || !gemm_tc_eligible(ctx, p)) return e.full_a == nullptr && p.m * p.n <= (int64_t(1) << 18) && gemm_small_serves(p);
     return !gemm_inline_serves(ctx, p) && !gemm_h16_serves(ctx, p) && gemm_tc_folds(ctx, p);
 }
 
-void dispatch_matmul(b200_ctx* ctx, const b200_node& node, const ProductEpilogue* epilogue = nullptr) {
-    const GemmProblem p = matmul_problem(node);
+void dispatch_problem(b200_ctx* ctx, const GemmProblem& p, const ProductEpilogue* epilogue) {
     if (epilogue == nullptr && gemm_inline_serves(ctx, p)) {
         gemm_inline(ctx, p);
     } else if (epilogue == nullptr && gemm_h16_serves(ctx, p) && gemm_tc_eligible(ctx, p)) {
@@ -265,6 +264,28 @@ void dispatch_matmul(b200_ctx* ctx, const b200_node& node, const ProductEpilogue
     } else {
         gemm_simt(ctx, p, epilogue);
     }
+}
+
+void dispatch_matmul(b200_ctx* ctx, const b200_node& node, const ProductEpilogue* epilogue = nullptr) {
+    const GemmProblem p = matmul_problem(node);
+    if (p.m * p.n * p.k == 0 || !result_over_operand(p, sizeof(float))) {
+        dispatch_problem(ctx, p, epilogue);
+        return;
+    }
+    // Most kernels read the operands while others of their blocks write results: such a result is put together elsewhere and copied.
+    const size_t bytes = static_cast<size_t>(p.b0 * p.b1 * p.m * p.n) * sizeof(float);
+    struct Release {
+        b200_ctx* c;
+        void* t;
+        ~Release() { c->scratch.release(t); }  // (stream-ordered)
+    } elsewhere{ctx, ctx->scratch.allocate(bytes)};
+    GemmProblem q = p;
+    q.out = static_cast<float*>(elsewhere.t);
+    if (ctx->compared.count(p.out) != 0) ctx->compared.insert(q.out);
+    dispatch_problem(ctx, q, epilogue);
+    ctx->compared.erase(q.out);
+    B200_CUDA_CHECK(cudaMemcpyAsync(p.out, q.out, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+    gemm_tc_invalidate(ctx, p.out, reinterpret_cast<const char*>(p.out) + bytes);  // (planes of what has been written over)
 }
 
 bool touches_f16(const b200_node& n) {
@@ -459,7 +480,11 @@ void dispatch_node(b200_ctx* ctx, const b200_node& node) {
         }
         const bool half_matmul = op == B200_OP_MATMUL && node.n_src >= 2 && node.src[0].dtype == B200_F16 &&
                                  node.src[1].dtype == B200_F16 && node.out.dtype == B200_F16;
-        if (half_matmul && gemm_f16_storage(ctx, matmul_problem(node))) return;
+        // (a result over an operand goes by widened copies)
+        if (half_matmul) {
+            const GemmProblem p = matmul_problem(node);
+            if (!result_over_operand(p, sizeof(uint16_t)) && gemm_f16_storage(ctx, p)) return;
+        }
         if (elementwise && all_half && node.out.dtype != B200_F32) {
             ProfScope scope(ctx, op_label(op));
             launch_elementwise(ctx, node);

@@ -18,6 +18,24 @@ struct GemmProblem {
     int64_t b_s[4];  // element strides of b over (b0, b1, k, n)
 };
 
+// Whether the product's result lies over memory that an operand is read from (`width`: bytes of an element).
+inline bool result_over_operand(const GemmProblem& p, size_t width) {
+    const int64_t outer = p.b0 * p.b1 * p.m * p.n;
+    auto over = [&](const float* at, const int64_t (&s)[4], int64_t rows, int64_t cols) {
+        const int64_t extent[4] = {p.b0, p.b1, rows, cols};
+        int64_t lo = 0, hi = 1;
+        for (int i = 0; i < 4; ++i) {
+            if (extent[i] == 0) return false;
+            const int64_t reach = (extent[i] - 1) * s[i];
+            (reach < 0 ? lo : hi) += reach;
+        }
+        const char *base = reinterpret_cast<const char*>(at), *out = reinterpret_cast<const char*>(p.out);
+        const int64_t w = static_cast<int64_t>(width);
+        return out < base + hi * w && base + lo * w < out + outer * w;
+    };
+    return over(p.a, p.a_s, p.m, p.k) || over(p.b, p.b_s, p.k, p.n);
+}
+
 // The range of one operand matrix, found on the device (gemm_h16.cu): the bits of the largest magnitude in
 // a sample of it, how many nonzero elements are too small beside that for the half split, whether one is too large, how many
 // of the sample's own elements are too small, and whether the TF32 planes that stand by for it have been written.
