@@ -117,3 +117,23 @@ def test_a_span_reads_what_was_written_over_an_operand(backend):
     x, w = x.astype(np.float64), w.astype(np.float64)
     for got, want in ((first, x @ w), (dx, x @ w), (last, x @ w @ w)):
         assert np.linalg.norm(got.numpy().reshape(want.shape) - want) <= 2e-5 * np.linalg.norm(want)
+
+
+# an operand whose rows run backwards, so that its memory lies in front of its first element: the sum that goes there is not the product's launch's
+@pytest.mark.parametrize("m,k", [(33, 33), (70, 130), (128, 1130)])
+def test_results_over_an_operand_that_runs_backwards(backend, m, k):
+    rng = np.random.default_rng(m + k)
+    x, w, bias = rng.standard_normal((m, k), dtype=np.float32), rng.standard_normal((k, k), dtype=np.float32), rng.standard_normal(k).astype(np.float32)
+    results = []
+    for over in (False, True):
+        dx, dw, db = DeviceTensor.from_host(backend, x), DeviceTensor.from_host(backend, w.reshape(1, 1, k, k)), DeviceTensor.from_host(backend, bias)
+        back = DeviceTensor(backend, dx.storage, (1, 1, m, k), (0, 0, -4 * k, 4), dx.dtype, 4 * k * (m - 1))
+        prod = DeviceTensor.empty(backend, (1, 1, m, k))
+        out = dx if over else DeviceTensor.empty(backend, (m, k))
+        backend.compute([NodeDesc(int(Op.MATMUL), prod.desc, [back.desc, dw.desc]),
+                         NodeDesc(int(Op.ADD), out.desc, [prod.reshape((m, k)).desc, db.reshape((1, k)).broadcast_to((m, k)).desc])])
+        results.append(out.numpy())
+    np.testing.assert_array_equal(results[1], results[0])
+    want = x[::-1].astype(np.float64) @ w.astype(np.float64) + bias
+    terms = np.abs(x[::-1]).astype(np.float64) @ np.abs(w).astype(np.float64) + np.abs(bias)
+    assert np.all(np.abs(results[0] - want) <= (k / 8 / 4 * 2.0 ** -23 + 2.0 ** -20) * terms)

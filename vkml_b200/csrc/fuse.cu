@@ -156,21 +156,6 @@ __global__ void __launch_bounds__(kThreads) bias_relu_group_kernel(BiasGroup g) 
     }
 }
 
-bool overlaps(const void* p, size_t pn, const void* q, size_t qn) {
-    const char* a = static_cast<const char*>(p);
-    const char* b = static_cast<const char*>(q);
-    return a < b + qn && b < a + pn;
-}
-
-// The span of addresses that the tensor can touch (strided views included).
-size_t bytes_of(const b200_tensor& t) {
-    int64_t hi = static_cast<int64_t>(dtype_size(t.dtype));
-    for (int d = 0; d < t.ndim; ++d) {
-        if (t.dims[d] > 1) hi += (t.dims[d] - 1) * std::abs(t.strides[d]);
-    }
-    return static_cast<size_t>(hi);
-}
-
 // The bias operand of `add`: a broadcast view of ONE contiguous vector, i.e. exactly one axis
 // with extent > 1 carries a stride, and that stride is one element.
 bool bias_layout(const b200_tensor& b, int64_t& inner, int64_t& count) {
@@ -546,12 +531,12 @@ size_t launch_scaled_add_group(b200_ctx* ctx, const b200_node* const* seq, size_
     auto independent = [&](const b200_node& x, const b200_node& y) {
         // x and y may run in either order: neither writes what the other reads or writes
         for (uint32_t s = 0; s < y.n_src && s < B200_MAX_SRC; ++s) {
-            if (y.src[s].data != nullptr && overlaps(x.out.data, bytes_of(x.out), y.src[s].data, bytes_of(y.src[s]))) return false;
+            if (overlap(x.out, y.src[s])) return false;
         }
         for (uint32_t s = 0; s < x.n_src && s < B200_MAX_SRC; ++s) {
-            if (x.src[s].data != nullptr && overlaps(y.out.data, bytes_of(y.out), x.src[s].data, bytes_of(x.src[s]))) return false;
+            if (overlap(y.out, x.src[s])) return false;
         }
-        return !overlaps(x.out.data, bytes_of(x.out), y.out.data, bytes_of(y.out));
+        return !overlap(x.out, y.out);
     };
     for (size_t k = 0; k < avail; ++k) picked[k] = false;
     for (size_t k = 0; k < avail && n < static_cast<size_t>(kGroupTensors); ++k) {
@@ -607,17 +592,13 @@ size_t launch_scaled_add_group(b200_ctx* ctx, const b200_node* const* seq, size_
     return n;
 }
 
-// Tries every pattern at the head of `seq` (the span's remaining computed nodes, in execution
-// order); returns how many nodes one fused launch served, or 0.
-// `later` >= avail nodes of `seq` may be looked at for one that a group can serve ahead of its turn; `early` is its
-// place in `seq` then (0: none).
 // Whether `x` writes nothing that the product reads: its blocks may still be reading when others write their results.
 static bool apart(const b200_node& product, const b200_node& x) {
     for (uint32_t s = 0; s < 2; ++s) {
-        if (product.src[s].data != nullptr && overlaps(x.out.data, bytes_of(x.out), product.src[s].data, bytes_of(product.src[s]))) return false;
+        if (overlap(x.out, product.src[s])) return false;
     }
     // nor the product's result's bytes in another order than its own
-    return x.out.data == product.out.data ? x.out.dtype == B200_F32 : !overlaps(x.out.data, bytes_of(x.out), product.out.data, bytes_of(product.out));
+    return x.out.data == product.out.data ? x.out.dtype == B200_F32 : !overlap(x.out, product.out);
 }
 
 size_t match_product_epilogue(const b200_node& product, const b200_node* const* seq, size_t avail, size_t later, size_t* early, ProductEpilogue& e) {
@@ -632,9 +613,9 @@ size_t match_product_epilogue(const b200_node& product, const b200_node* const* 
             first.src[2].data != product.out.data || first.src[1].data == product.out.data || !whole(first.out, B200_F32)) {
             return 0;
         }
-        if (!apart(product, first) || overlaps(first.out.data, bytes_of(first.out), first.src[0].data, bytes_of(first.src[0]))) return 0;
+        if (!apart(product, first) || overlap(first.out, first.src[0]) || (first.out.data != first.src[1].data && overlap(first.out, first.src[1]))) return 0;
         for (int k = 0; k < 2; ++k) {  // (nor does the product overwrite what is chosen from, or its choice)
-            if (overlaps(product.out.data, bytes_of(product.out), first.src[k].data, bytes_of(first.src[k]))) return 0;
+            if (overlap(product.out, first.src[k])) return 0;
         }
         e.cond = static_cast<const uint8_t*>(first.src[0].data);
         e.other = static_cast<const float*>(first.src[1].data);
@@ -652,8 +633,7 @@ size_t match_product_epilogue(const b200_node& product, const b200_node* const* 
     }
     for (size_t k = 0; k < later; ++k) {
         if ((k < at || (*early > 0 && k == *early)) &&
-            (!apart(product, *seq[k]) || overlaps(seq[k]->out.data, bytes_of(seq[k]->out), g.bias, size_t(cols) * 4) ||
-             overlaps(product.out.data, bytes_of(product.out), g.bias, size_t(cols) * 4))) {
+            (!apart(product, *seq[k]) || overlap(seq[k]->out, first.src[1]) || overlap(product.out, first.src[1]))) {
             *early = 0;
             return 0;
         }
@@ -669,6 +649,10 @@ size_t match_product_epilogue(const b200_node& product, const b200_node* const* 
     return at;
 }
 
+// Tries every pattern at the head of `seq` (the span's remaining computed nodes, in execution
+// order); returns how many nodes one fused launch served, or 0.
+// `later` >= avail nodes of `seq` may be looked at for one that a group can serve ahead of its turn; `early` is its
+// place in `seq` then (0: none).
 size_t launch_fused(b200_ctx* ctx, const b200_node* const* seq, size_t avail, size_t later, size_t* early) {
     *early = 0;
     if (size_t n = fuse_bias_group(ctx, seq, avail, later, early)) return n;
