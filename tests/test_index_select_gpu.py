@@ -1,0 +1,68 @@
+"""index_select where its kernels change over: the width of a row, index lists with a stride, an index out of range."""
+import numpy as np
+import pytest
+
+from vkml_b200 import DeviceTensor, DType, NodeDesc, Op, graph
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def backend():
+    import vkml_b200
+    b = vkml_b200.Backend(0)
+    yield b
+    b.close()
+
+
+def select(b, table, index, axis):
+    """The node over `index` as every second word of a longer list."""
+    spread = np.full(2 * len(index), -7, np.int64)
+    spread[::2] = index
+    a, i = DeviceTensor.from_host(b, table), DeviceTensor.from_host(b, spread)
+    i = DeviceTensor(b, i.storage, (len(index),), (16,), i.dtype)
+    dims = table.shape[:axis] + (len(index),) + table.shape[axis + 1:]
+    out = DeviceTensor.empty(b, dims, a.dtype)
+    return out, NodeDesc(int(Op.INDEX_SELECT), out.desc, [a.desc, i.desc], graph.axis_params(axis)), (a, i)
+
+
+# from one element to beyond the line between the kernels
+@pytest.mark.parametrize("width", [1, 2, 5, 11, 12, 13, 31, 130])
+@pytest.mark.parametrize("dtype", [np.float32, np.int64])
+@pytest.mark.parametrize("axis", [0, 1])
+def test_widths(backend, width, dtype, axis):
+    rng = np.random.default_rng(width)
+    table = rng.integers(-1000, 1000, (300, width) if axis == 0 else (3, 300, width)).astype(dtype)
+    index = rng.integers(0, 300, 701)
+    out, node, keep = select(backend, table, index, axis)
+    backend.compute([node])
+    assert np.array_equal(out.numpy(), np.take(table, index, axis))
+
+
+@pytest.mark.parametrize("width", [1, 12, 33])
+def test_an_index_out_of_range_is_an_error_and_clamped(backend, width):
+    table = np.arange(20 * width, dtype=np.float32).reshape(20, width)
+    index = np.array([3, 20, -1, 19])
+    out, node, keep = select(backend, table, index, 0)
+    backend.compute([node])
+    with pytest.raises(IndexError):
+        backend.synchronize()
+    assert np.array_equal(out.numpy(), table[[3, 19, 0, 19]])
+
+
+def test_narrow_rows_are_no_warp_each(backend):
+    """Two million floats picked one by one take at most eight times what they take in rows of 16 (a thread to an element: twice and a half to
+    three times; a warp to an element: twenty-six)."""
+    rng = np.random.default_rng(3)
+
+    def us(width):
+        out, node, keep = select(backend, rng.standard_normal((4000, width), dtype=np.float32), rng.integers(0, 4000, 2_000_000 // width), 0)
+        times = []
+        for _ in range(6):
+            backend.synchronize()
+            backend.timer_begin()
+            for _ in range(10):
+                backend.compute([node])
+            times.append(backend.timer_end())
+        return min(times)
+    assert us(1) < 8 * us(16)

@@ -763,7 +763,10 @@ index_select_rows_kernel(uint4* __restrict__ out, const uint4* __restrict__ a, c
 
 // Dense source rows that begin or end anywhere: a warp copies a piece of 32 * Q elements of a row, all of a lane's loads in flight.  Bound by the chain
 // of index, row and store where rows are short, by HBM where they are long ([2643, 483] at 12872 indices, 50 MB: 39 us with an index and a
-// division chain per element, 8 here).
+// division chain per element, 8 here).  Rows of less than twelve elements leave the warp's lanes idle and stay with the kernel above, a thread to an
+// element: 2 million floats in rows of 1, 3, 7 and 9 130, 45, 21 and 16.7 us here and 13.5 there, in rows of 11, 13 and 31 14.2, 12.4 and 6.2; 300
+// columns picked from [4096, 1024] 80 and 9.5.
+constexpr int64_t kPieceElements = 12;
 template <typename T, int Q>
 __global__ void __launch_bounds__(kThreads)
 index_select_pieces_kernel(T* __restrict__ out, const T* __restrict__ a, const int64_t* __restrict__ idx, int64_t idx_stride, FastDiv by_pieces,
@@ -1571,7 +1574,7 @@ void launch_movement(b200_ctx* ctx, const b200_node& node) {
                               static_cast<unsigned>(total16), ctx->d_status);
                 break;
             }
-            if (a.contiguous && small && (esz == 4 || esz == 8)) {
+            if (a.contiguous && small && (esz == 4 || esz == 8) && inner >= kPieceElements) {
                 auto pieces = [&](auto* o, const auto* from, auto width) {
                     using T = std::remove_pointer_t<decltype(o)>;
                     constexpr int Q = decltype(width)::value;
