@@ -66,3 +66,15 @@ def test_narrow_rows_are_no_warp_each(backend):
             times.append(backend.timer_end())
         return min(times)
     assert us(1) < 8 * us(16)
+
+
+@pytest.mark.parametrize("width", [1, 16, 33])
+def test_an_empty_axis_has_no_rows_to_select(backend, width):
+    a, i = DeviceTensor.empty(backend, (0, width)), DeviceTensor.from_host(backend, np.zeros(5, np.int64))
+    out = DeviceTensor.empty(backend, (5, width))
+    with pytest.raises(IndexError):
+        backend.compute([NodeDesc(int(Op.INDEX_SELECT), out.desc, [a.desc, i.desc], graph.axis_params(0))])
+    empty = DeviceTensor.empty(backend, (0, width))
+    none = DeviceTensor.empty(backend, (0,), DType.I64)
+    backend.compute([NodeDesc(int(Op.INDEX_SELECT), empty.desc, [a.desc, none.desc], graph.axis_params(0))])  # (none is asked for)
+    backend.synchronize()

@@ -1556,6 +1556,7 @@ void launch_movement(b200_ctx* ctx, const b200_node& node) {
             if (total == 0) return;
             const int axis = get_params<AxisParams>(node).axis + (kMaxDims - node.out.ndim);
             if (axis < 0 || axis >= kMaxDims) fail(B200_SHAPE_ERROR, "index_select: bad axis");
+            if (a.dim[axis] == 0) fail(B200_INDEX_ERROR, "index_select: an index into an empty axis");  // (nothing to clamp it to)
             int64_t inner = 1;
             for (int i = axis + 1; i < kMaxDims; ++i) inner *= out.dim[i];
             const auto* ip = reinterpret_cast<const int64_t*>(idx.data);
