@@ -1,12 +1,20 @@
 """The bounds within which a product is handed to the kernels that read its operands themselves, against the index arithmetic of those kernels.  No
 GPU is needed: the rules are functions of the sizes and strides alone."""
 import ctypes as C
+import os
+import re
 
 import pytest
 
 from vkml_b200 import _abi
 
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "vkml_b200", "csrc")
 FITS = "_ZN4b20016gemm_inline_fitsERKNS_11GemmProblemEb"  # b200::gemm_inline_fits(const GemmProblem&, bool tf32)
+
+
+def read(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return f.read()
 
 
 class Problem(C.Structure):
@@ -39,3 +47,12 @@ def test_rows_of_a_thread_are_within_32_bits(tf32, sign, side):
             served.append(pitch)
             assert max(row_steps(tf32)) * pitch * 4 < 1 << 31, pitch
     assert max(served) == (1 << (24 if tf32 else 25)) - 1  # and nothing below is given up
+
+
+@pytest.mark.parametrize("name", [f for f in sorted(os.listdir(CSRC)) if f.endswith(".cu") and "= unit_plan(" in read(f)])
+def test_unit_walkers_leave_room_for_a_pending_all_reduce(name):
+    """A kernel whose CTAs stay on their SMs takes none of those that a gradient span's all-reduce has set aside."""
+    launchers = [f for f in re.split(r"\n}\n", read(name)) if "= unit_plan(" in f]
+    assert launchers
+    for f in launchers:
+        assert "in_grad_sync_span && ctx->comm_pending" in f and "comm_sms" in f, f[-300:]

@@ -475,7 +475,9 @@ bool gemm_f16_any(b200_ctx* ctx, const GemmProblem& p, const HalfEpilogue* epi) 
     g.units = unit_plan(tiles_p, tiles_q, batches, splits, k_blocks, kb_per_split, 16 / cg);
     g.split_stride = out_elems;
     g.status = ctx->d_status;
-    const int grid = static_cast<int>(std::min<int64_t>(tiles * splits, sms / cg)) * cg;
+    int free_sms = sms;
+    if (ctx->in_grad_sync_span && ctx->comm_pending) free_sms = std::max(sms - ctx->comm_sms, sms / 2);  // (the others are the all-reduce's)
+    const int grid = static_cast<int>(std::min<int64_t>(tiles * splits, free_sms / cg)) * cg;
     auto launch = [&](auto kernel) {
         B200_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTotal));
         if (cg == 2) launch_kernel_clustered(ctx, kernel, grid, kThreads, kTotal, cg, false, g);
