@@ -115,6 +115,7 @@ bool gemm_tc_folds(const b200_ctx* ctx, const GemmProblem& p);  // in K-slices, 
 void gemm_tc_stand_by(b200_ctx* ctx, const GemmProblem& p, const RangeGuard& guard, const Standby& a, const Standby& b, float* target,
                       float* partial);
 int gemm_tc_slices(const b200_ctx* ctx, const GemmProblem& p);
+size_t gemm_tc_plane_limit(const b200_ctx* ctx);  // bytes of planes that are held beside the operands without need
 size_t gemm_tc_plane_bytes(const GemmProblem& p, bool left);  // of one operand's two planes
 
 // tcgen05 kind::f16: F32 products from two half terms per operand, F16 products directly. gemm_h16.cu

@@ -1012,6 +1012,9 @@ bool gemm_inline_serves(const b200_ctx* ctx, const GemmProblem& p) {
     if (ctx->gemm_inline > 0) return ctx->gemm_inline < 8;
     const bool direct = ctx->lone_matmul && gemm_tc_reads_directly(ctx, p);
     if (!gemm_h16_serves(ctx, p) && !(direct && gemm_h16_would_serve(ctx, p))) return false;
+    // (what is read directly otherwise needs no memory beside its operands, and the planes that stand by take twice theirs: [1048576, 12288] x
+    // 64 columns 103 GB beside 52)
+    if (direct && gemm_tc_plane_bytes(p, true) + gemm_tc_plane_bytes(p, false) > gemm_tc_plane_limit(ctx)) return false;
     return !gemm_h16_shares(ctx, p) && (t.cost + 12.0) * 1.05 < gemm_h16_time(ctx, p);
 }
 
@@ -1043,7 +1046,14 @@ void gemm_inline(b200_ctx* ctx, const GemmProblem& p) {
         place_sample(side[i], p, mn[i]);
         bytes += tf32[i] + kMaxStrays * 8;
     }
-    char* ws = static_cast<char*>(ctx->ensure_workspace(bytes));
+    char* ws = nullptr;
+    try {
+        ws = static_cast<char*>(ctx->ensure_workspace(bytes));
+    } catch (const Error& e) {
+        if (e.status != B200_OUT_OF_MEMORY) throw;
+        gemm_tc(ctx, p, true);  // (a product that is read directly needs none of it)
+        return;
+    }
     ws = reinterpret_cast<char*>(align_up(reinterpret_cast<int64_t>(ws), 1024));
     for (int i = 0; i < 2; ++i) {
         standby[i].planes = reinterpret_cast<float*>(ws);

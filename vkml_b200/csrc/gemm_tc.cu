@@ -2122,6 +2122,8 @@ void gemm_tc(b200_ctx* ctx, const GemmProblem& p, bool three_pass, const Product
 
 int gemm_tc_slices(const b200_ctx* ctx, const GemmProblem& p) { return static_cast<int>(plan_planes(ctx, p).splits); }
 
+size_t gemm_tc_plane_limit(const b200_ctx* ctx) { return plane_cache_limit(ctx); }
+
 size_t gemm_tc_plane_bytes(const GemmProblem& p, bool left) {
     const int64_t* s = left ? p.a_s : p.b_s;
     const bool bcast = (s[0] == 0 || p.b0 == 1) && (s[1] == 0 || p.b1 == 1);
