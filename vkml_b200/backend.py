@@ -122,7 +122,8 @@ class Backend:
 
     def matmul_kernel(self, node: NodeDesc) -> tuple:
         """(kernel, reason) a matmul node would get, taken by itself: fp32_simt, tcgen05_3xtf32 (operand
-        planes), tcgen05_3xtf32_stream (streamed operand) or tcgen05_3xtf32_direct (operands read directly)."""
+        planes, or split inside the kernel), tcgen05_3xtf32_stream (streamed operand), tcgen05_3xtf32_direct
+        (operands read directly) or tcgen05_3xf16 (half terms)."""
         c = node.to_c()
         name, why = C.create_string_buffer(64), C.create_string_buffer(160)
         self._check(self._lib.b200_matmul_kernel(self._ctx, C.byref(c), name, 64, why, 160), "matmul_kernel")

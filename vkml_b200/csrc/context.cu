@@ -1655,8 +1655,8 @@ int b200_matmul_kernel(b200_ctx* ctx, const b200_node* node, char* name, size_t 
             const bool three = ctx->gemm_precision == B200_GEMM_3XTF32;
             if (gemm_inline_serves(ctx, p)) {
                 kernel = "tcgen05_3xf16";
-                why = "bound by reading its operands: two half terms per operand, split inside the kernel (TF32 planes where an operand's range is too "
-                      "wide for them), tiles of " + gemm_inline_tile(ctx, p);
+                why = "bound by reading its operands: two half terms each, split inside the kernel (TF32 planes where a range is too wide), tiles of " +
+                      gemm_inline_tile(ctx, p);
             } else if (gemm_h16_serves(ctx, p)) {
                 kernel = "tcgen05_3xf16";
                 why = "bound by the tensor cores: two half terms per operand (TF32 planes where an operand's range is too wide for them), tiles of " +
@@ -1664,6 +1664,9 @@ int b200_matmul_kernel(b200_ctx* ctx, const b200_node* node, char* name, size_t 
             } else if (gemm_tc_streams(ctx, p)) {
                 kernel = three ? "tcgen05_3xtf32_stream" : "tcgen05_tf32_stream";
                 why = "bound by memory (a small left operand or a short K): the right operand is read as fp32 and split on the way";
+            } else if (gemm_tc_splits_inside(ctx, p)) {
+                kernel = gemm_tc_reads_directly(ctx, p) ? "tcgen05_3xtf32_direct" : "tcgen05_3xtf32";
+                why = "one wave of tiles: the operands are read as fp32 and split into TF32 terms inside the kernel, no planes";
             } else if (gemm_tc_reads_directly(ctx, p)) {
                 kernel = three ? "tcgen05_3xtf32_direct" : "tcgen05_tf32_direct";
                 why = "the plane passes would cost more than the product: fp32 tiles by TMA, split inside the kernel";

@@ -149,6 +149,7 @@ bool gemm_f16_any(b200_ctx* ctx, const GemmProblem& p, const HalfEpilogue* epilo
 bool gemm_tc_streams(const b200_ctx* ctx, const GemmProblem& p);
 int64_t gemm_tc_chain(const b200_ctx* ctx, const GemmProblem& p);  // products that one accumulator of the plane kernel adds up
 bool gemm_tc_reads_directly(const b200_ctx* ctx, const GemmProblem& p);  // (taken by itself: no shared planes)
+bool gemm_tc_splits_inside(const b200_ctx* ctx, const GemmProblem& p);   // ... or split them into TF32 terms in its converters' registers
 // Diagnostic: one block waits `limit_ns` on a barrier nobody arrives on and gives up (gemm_tc.cu).
 void gemm_tc_wait_probe(b200_ctx* ctx, uint64_t limit_ns);
 

@@ -1905,6 +1905,15 @@ bool gemm_tc_reads_directly(const b200_ctx* ctx, const GemmProblem& p) {
     return maps_describe(p, oa, ob) && !want_dynamic && (ctx->gemm_operands == 1 || direct_pays(ctx, p, batches, oa, ob));
 }
 
+bool gemm_tc_splits_inside(const b200_ctx* ctx, const GemmProblem& p) {
+    if (plan_stream(ctx, p).ok || ctx->gemm_precision != B200_GEMM_3XTF32) return false;
+    const bool a_bcast = (p.a_s[0] == 0 || p.b0 == 1) && (p.a_s[1] == 0 || p.b1 == 1);
+    const bool b_bcast = (p.b_s[0] == 0 || p.b0 == 1) && (p.b_s[1] == 0 || p.b1 == 1);
+    const Operand oa = plan_operand(p.a, p.a_s[0], p.a_s[1], p.a_s[2], p.a_s[3], p.m, p.k, a_bcast, p);
+    const Operand ob = plan_operand(p.b, p.b_s[0], p.b_s[1], p.b_s[3], p.b_s[2], p.n, p.k, b_bcast, p);
+    return inline_pays(ctx, p, oa, ob, plan_planes(ctx, p), gemm_tc_reads_directly(ctx, p));
+}
+
 void gemm_tc_wait_probe(b200_ctx* ctx, uint64_t limit_ns) {
     wait_probe_kernel<<<1, 32, 0, ctx->stream>>>(ctx->d_status, limit_ns);
     ctx->count_launch();
