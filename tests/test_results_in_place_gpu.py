@@ -2,7 +2,7 @@
 import numpy as np
 import pytest
 
-from vkml_b200 import DeviceTensor, DType, NodeDesc, Op
+from vkml_b200 import DeviceTensor, DType, NodeDesc, Op, graph
 
 pytestmark = pytest.mark.gpu
 
@@ -59,3 +59,25 @@ def test_half(backend, m, k, n, form, place):
     own = layer(backend, x, w, bias, DType.F16, form, "own")
     got = layer(backend, x, w, bias, DType.F16, form, place)
     assert np.array_equal(got.view(np.uint16), own.view(np.uint16))
+
+
+# what a where chooses from, filled with one value in the span and read as one word, or filled before it and read whole
+@pytest.mark.parametrize("m,k,n", [(33, 127, 31), (64, 784, 128), (300, 1900, 101), (512, 4096, 260)])
+def test_a_filled_choice(backend, m, k, n):
+    rng = np.random.default_rng(m)
+    x, w, c = rng.standard_normal((m, k), dtype=np.float32), rng.standard_normal((k, n), dtype=np.float32), rng.random((m, n)) < 0.5
+    dx, dw, dc = DeviceTensor.from_host(backend, x.reshape(1, 1, m, k)), DeviceTensor.from_host(backend, w.reshape(1, 1, k, n)), DeviceTensor.from_host(backend, c)
+    y = DeviceTensor.empty(backend, (1, 1, m, n))
+    results = []
+    for inside in (True, False):
+        f, z = DeviceTensor.empty(backend, (m, n)), DeviceTensor.empty(backend, (m, n))
+        fill = NodeDesc(int(Op.FULL), f.desc, [], graph.full_params(-0.5))
+        nodes = [NodeDesc(int(Op.MATMUL), y.desc, [dx.desc, dw.desc]), NodeDesc(int(Op.WHERE), z.desc, [dc.desc, f.desc, y.reshape((m, n)).desc])]
+        if inside:
+            backend.compute([fill] + nodes)
+        else:
+            backend.compute([fill])
+            backend.compute(nodes)
+        results.append(z.numpy())
+        assert np.array_equal(results[-1], np.where(c, np.float32(-0.5), y.numpy().reshape(m, n)))
+    assert np.array_equal(*results)

@@ -1106,6 +1106,11 @@ static void compute_span(b200_ctx* ctx, const b200_node* nodes, size_t n_nodes, 
             bool served = false;
             if (taken > 0) {
                 prepare(i);  // (checks the operands before they are looked at)
+                if (e.other != nullptr) {
+                    // (as a node of its own the where would read one word of a buffer that a full has filled)
+                    const auto filled = constants.find(e.other);
+                    if (filled != constants.end() && filled->second == tensor_bytes(seq[0]->src[1])) e.other_step = 0;
+                }
                 if (takes_epilogue(ctx, matmul_problem(node), e)) {
                     for (size_t k = 0; k < later; ++k) {
                         if (k < taken || (early > 0 && k == early)) prepare(exec[p + 1 + k]);

@@ -619,6 +619,7 @@ size_t match_product_epilogue(const b200_node& product, const b200_node* const* 
         }
         e.cond = static_cast<const uint8_t*>(first.src[0].data);
         e.other = static_cast<const float*>(first.src[1].data);
+        e.other_step = 1;
         e.chosen = static_cast<float*>(first.out.data);
         return 1;
     }

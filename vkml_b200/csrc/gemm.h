@@ -77,12 +77,13 @@ struct ProductEpilogue {
     float* relu;        // null: none
     const uint8_t* cond;
     const float* other;
+    int other_step;     // 0: a buffer that is known to hold one value throughout
     float* chosen;
 };
 #ifdef __CUDACC__
 __device__ __forceinline__ void write_epilogue(const ProductEpilogue& e, int64_t i, int64_t col, float v) {
     if (e.bias == nullptr) {
-        e.chosen[i] = e.cond[i] != 0 ? e.other[i] : v;
+        e.chosen[i] = e.cond[i] != 0 ? e.other[i * e.other_step] : v;
         return;
     }
     const float y = __fadd_rn(v, e.bias[col]);
