@@ -243,33 +243,41 @@ GemmProblem matmul_problem(const b200_node& node) {
     return p;
 }
 
+// The kernels that serve a product.  Finding them takes 0.3 to 1 us of the host, so a product is asked about once.
+enum class Route { kNone, kInline, kHalfPlanes, kTc, kSimt };
+
+Route route_of(const b200_ctx* ctx, const GemmProblem& p) {
+    if (gemm_inline_serves(ctx, p)) return Route::kInline;
+    if (!gemm_tc_eligible(ctx, p)) return Route::kSimt;
+    if (gemm_h16_serves(ctx, p)) return Route::kHalfPlanes;
+    return ctx->gemm_precision != B200_GEMM_FP32 ? Route::kTc : Route::kSimt;
+}
+
 // Whether the kernel that writes the product's last sum can write an epilogue as well.
 // A launch inside a step costs 6 to 8 us whatever it does, and these nodes are such launches: an MLP's training step has 13 in place of 15
 // (784-128-10, batch 64: 51.0 us, 50.4 now; 315 rows through 160-83-32 63.9 and 61.5) or 35 in place of 41 (93 rows through 284-1130x3-201
 // 222.6 and 214.7).  A small product writes it word by word, which over many elements takes longer than the launch: 361 rows through 307-2484x3-14,
 // whose where follows a result of 361x2484, 323.7 us a step with it and 316.3 without; 560x455 gains.  Behind a small product the group with ReLU's mask stays the launch of its own that a step's profile shows.
-bool takes_epilogue(b200_ctx* ctx, const GemmProblem& p, const ProductEpilogue& e) {
+bool takes_epilogue(b200_ctx* ctx, const GemmProblem& p, const ProductEpilogue& e, Route& route) {
     if (p.b0 * p.b1 != 1 || p.m * p.n * p.k == 0 || result_over_operand(p, sizeof(float))) return false;
-    if (ctx->gemm_precision == B200_GEMM_FP32 || !gemm_tc_eligible(ctx, p)) return e.full_a == nullptr && p.m * p.n <= (int64_t(1) << 18) && gemm_small_serves(p);
-    return !gemm_inline_serves(ctx, p) && !gemm_h16_serves(ctx, p) && gemm_tc_folds(ctx, p);
+    route = route_of(ctx, p);
+    if (route == Route::kSimt) return e.full_a == nullptr && p.m * p.n <= (int64_t(1) << 18) && gemm_small_serves(p);
+    return route == Route::kTc && gemm_tc_folds(ctx, p);
 }
 
-void dispatch_problem(b200_ctx* ctx, const GemmProblem& p, const ProductEpilogue* epilogue) {
-    if (epilogue == nullptr && gemm_inline_serves(ctx, p)) {
-        gemm_inline(ctx, p);
-    } else if (epilogue == nullptr && gemm_h16_serves(ctx, p) && gemm_tc_eligible(ctx, p)) {
-        gemm_h16(ctx, p);
-    } else if (ctx->gemm_precision != B200_GEMM_FP32 && gemm_tc_eligible(ctx, p)) {
-        gemm_tc(ctx, p, ctx->gemm_precision == B200_GEMM_3XTF32, epilogue);
-    } else {
-        gemm_simt(ctx, p, epilogue);
-    }
+void dispatch_problem(b200_ctx* ctx, const GemmProblem& p, Route route, const ProductEpilogue* epilogue) {
+    if (route == Route::kNone) route = route_of(ctx, p);
+    if (route == Route::kInline) gemm_inline(ctx, p);
+    else if (route == Route::kHalfPlanes) gemm_h16(ctx, p);
+    else if (route == Route::kTc) gemm_tc(ctx, p, ctx->gemm_precision == B200_GEMM_3XTF32, epilogue);
+    else gemm_simt(ctx, p, epilogue);
 }
 
-void dispatch_matmul(b200_ctx* ctx, const b200_node& node, const ProductEpilogue* epilogue = nullptr) {
+// `route`: kNone, or what takes_epilogue found.
+void dispatch_matmul(b200_ctx* ctx, const b200_node& node, Route route = Route::kNone, const ProductEpilogue* epilogue = nullptr) {
     const GemmProblem p = matmul_problem(node);
     if (p.m * p.n * p.k == 0 || !result_over_operand(p, sizeof(float))) {
-        dispatch_problem(ctx, p, epilogue);
+        dispatch_problem(ctx, p, route, epilogue);
         return;
     }
     // Most kernels read the operands while others of their blocks write results: such a result is put together elsewhere and copied.
@@ -282,7 +290,7 @@ void dispatch_matmul(b200_ctx* ctx, const b200_node& node, const ProductEpilogue
     GemmProblem q = p;
     q.out = static_cast<float*>(elsewhere.t);
     if (ctx->compared.count(p.out) != 0) ctx->compared.insert(q.out);
-    dispatch_problem(ctx, q, epilogue);
+    dispatch_problem(ctx, q, Route::kNone, nullptr);
     ctx->compared.erase(q.out);
     B200_CUDA_CHECK(cudaMemcpyAsync(p.out, q.out, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
     gemm_tc_invalidate(ctx, p.out, reinterpret_cast<const char*>(p.out) + bytes);  // (planes of what has been written over)
@@ -1090,6 +1098,7 @@ static void compute_span(b200_ctx* ctx, const b200_node* nodes, size_t n_nodes, 
                 }
             }
         }
+        Route route = Route::kNone;
         if (ctx->fuse && node.op == B200_OP_MATMUL && node.out.dtype == B200_F32 && node.out.data != nullptr && p + 1 < exec.size() && is_sink.empty() &&
             !grad_sync && !touches_f16(node)) {
             // what follows a product element by element, by the launch that writes the product
@@ -1111,12 +1120,12 @@ static void compute_span(b200_ctx* ctx, const b200_node* nodes, size_t n_nodes, 
                     const auto filled = constants.find(e.other);
                     if (filled != constants.end() && filled->second == tensor_bytes(seq[0]->src[1])) e.other_step = 0;
                 }
-                if (takes_epilogue(ctx, matmul_problem(node), e)) {
+                if (takes_epilogue(ctx, matmul_problem(node), e, route)) {
                     for (size_t k = 0; k < later; ++k) {
                         if (k < taken || (early > 0 && k == early)) prepare(exec[p + 1 + k]);
                     }
                     ctx->current_op = node.op;
-                    dispatch_matmul(ctx, node, &e);
+                    dispatch_matmul(ctx, node, route, &e);
                     served = true;
                 }
             }
@@ -1297,6 +1306,9 @@ static void compute_span(b200_ctx* ctx, const b200_node* nodes, size_t n_nodes, 
                 }
             }
             dispatch_node(ctx, changed ? lean : node);
+        } else if (route != Route::kNone) {
+            ctx->current_op = node.op;
+            dispatch_matmul(ctx, node, route);  // (an F32 product whose kernel takes no epilogue)
         } else {
             dispatch_node(ctx, node);
         }

@@ -1003,19 +1003,16 @@ void launch_inline(b200_ctx* ctx, const InlineArgs& g, bool p_mn, bool q_mn, int
 // element at 5.8 TB/s.  Measured, planes / here: 512x65536x512 182 / 119 us, 255x29905x606 105 / 84, 5 x 3335x2687x174 156 / 121,
 // 24 x 366x913x232 59 / 50; but 2048^3 65 / 69, 4096^3 349 / 441, 751x2638x911 45 / 55.)  Planes that another product of the span reads too are kept.
 bool gemm_inline_serves(const b200_ctx* ctx, const GemmProblem& p) {
-    if (ctx->gemm_inline == 0 || ctx->gemm_precision != B200_GEMM_3XTF32 || !ctx->gemm_half_terms || ctx->compared.count(p.out) != 0 ||
-        !gemm_tc_eligible(ctx, p) || gemm_tc_chain(ctx, p) > 12288) {
+    if (ctx->gemm_inline == 0 || ctx->gemm_inline >= 8 || ctx->gemm_precision != B200_GEMM_3XTF32 || !ctx->gemm_half_terms || ctx->compared.count(p.out) != 0) {
         return false;
     }
-    if (!gemm_inline_fits(p, false)) return false;
-    const InlinePlan t = plan_inline(ctx, p);
-    if (ctx->gemm_inline > 0) return ctx->gemm_inline < 8;
-    const bool direct = ctx->lone_matmul && gemm_tc_reads_directly(ctx, p);
-    if (!gemm_h16_serves(ctx, p) && !(direct && gemm_h16_would_serve(ctx, p))) return false;
+    if (ctx->gemm_inline > 0) return gemm_tc_eligible(ctx, p) && gemm_tc_chain(ctx, p) <= 12288 && gemm_inline_fits(p, false);
+    // what takes half terms, and what would if it were not read directly
+    if (!gemm_h16_would_serve(ctx, p) || !gemm_inline_fits(p, false) || gemm_h16_shares(ctx, p)) return false;
     // (what is read directly otherwise needs no memory beside its operands, and the planes that stand by take twice theirs: [1048576, 12288] x
     // 64 columns 103 GB beside 52)
-    if (direct && gemm_tc_plane_bytes(p, true) + gemm_tc_plane_bytes(p, false) > gemm_tc_plane_limit(ctx)) return false;
-    return !gemm_h16_shares(ctx, p) && (t.cost + 12.0) * 1.05 < gemm_h16_time(ctx, p);
+    if (ctx->lone_matmul && gemm_tc_plane_bytes(p, true) + gemm_tc_plane_bytes(p, false) > gemm_tc_plane_limit(ctx) && gemm_tc_reads_directly(ctx, p)) return false;
+    return (plan_inline(ctx, p).cost + 12.0) * 1.05 < gemm_h16_time(ctx, p) && gemm_tc_eligible(ctx, p);
 }
 
 std::string gemm_inline_tile(const b200_ctx* ctx, const GemmProblem& p) {
