@@ -1,4 +1,4 @@
-"""index_select where its kernels change over: the width of a row, index lists with a stride, an index out of range."""
+"""index_select and scatter_add where their kernels change over: the width of a row, index lists with a stride, indices out of range, an axis in front."""
 import numpy as np
 import pytest
 
@@ -78,3 +78,28 @@ def test_an_empty_axis_has_no_rows_to_select(backend, width):
     none = DeviceTensor.empty(backend, (0,), DType.I64)
     backend.compute([NodeDesc(int(Op.INDEX_SELECT), empty.desc, [a.desc, none.desc], graph.axis_params(0))])  # (none is asked for)
     backend.synchronize()
+
+
+# lines of sources and chains, an axis in front of the destinations, every second word of the index list, indices out of range
+@pytest.mark.parametrize("outer,extent,count,width", [(1, 500, 900, 33), (3, 500, 700, 33), (2, 40, 3000, 130), (2, (1 << 18) + 3, 900, 16)])
+@pytest.mark.parametrize("beyond", [False, True])
+def test_rows_are_added(backend, outer, extent, count, width, beyond):
+    rng = np.random.default_rng(extent + beyond)
+    src, index = rng.standard_normal((outer, count, width), dtype=np.float32), rng.integers(0, extent, count)
+    index[:40] = extent - 1
+    if beyond:
+        index[50], index[60] = extent, -1
+    spread = np.full(2 * count, -7, np.int64)
+    spread[::2] = index
+    s, i = DeviceTensor.from_host(backend, src), DeviceTensor.from_host(backend, spread)
+    i = DeviceTensor(backend, i.storage, (count,), (16,), i.dtype)
+    out = DeviceTensor.empty(backend, (outer, extent, width))
+    backend.compute([NodeDesc(int(Op.SCATTER_ADD), out.desc, [s.desc, i.desc], graph.axis_params(1))])
+    if beyond:
+        with pytest.raises(IndexError):
+            backend.synchronize()
+    want = np.zeros((outer, extent, width), np.float32)
+    for at, j in enumerate(index):
+        if 0 <= j < extent:
+            want[:, j] += src[:, at]
+    assert np.array_equal(out.numpy(), want)
