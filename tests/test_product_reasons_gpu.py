@@ -39,3 +39,15 @@ def test_reasons(backend, m, k, n, name, words):
         return
     inside = "no planes" in why or "split inside the kernel" in why or "fp32 tiles" in why
     assert any("split" in l for l in labels) != inside, (labels, why)
+
+
+# rows along K that are read a float at a time, by both operands, one and neither: the planes' passes cost less than the first, not than the others
+@pytest.mark.parametrize("m,k,n,layout,inside", [(2348, 421, 123, "nt", False), (200, 462, 2480, "nt", False), (86, 425, 2790, "nt", False),
+                                                 (2348, 421, 123, "tn", True), (681, 1026, 1021, "nn", True), (637, 947, 201, "nt", True)])
+def test_how_a_ragged_product_is_split(backend, m, k, n, layout, inside):
+    def put(r, c, turned):
+        t = DeviceTensor.from_host(backend, np.ones((1, 1) + ((c, r) if turned else (r, c)), np.float32))
+        return t.transpose(2, 3) if turned else t
+    a, b, out = put(m, k, layout[0] == "t"), put(k, n, layout[1] == "t"), DeviceTensor.empty(backend, (1, 1, m, n))
+    why = backend.matmul_kernel(NodeDesc(int(Op.MATMUL), out.desc, [a.desc, b.desc]))[1]
+    assert ("inside the kernel" in why) == inside, why

@@ -130,6 +130,7 @@ void gemm_h16_fold(b200_ctx* ctx, const GemmProblem& p, const float* partial, in
 // The same terms, split inside the product's kernel. gemm_inline.cu
 bool gemm_inline_serves(const b200_ctx* ctx, const GemmProblem& p);
 void gemm_inline_tf32(b200_ctx* ctx, const GemmProblem& p, float* partial, int64_t splits, int64_t kb_per_split, const char* label);
+double gemm_inline_tf32_block(const GemmProblem& p);
 bool gemm_inline_fits(const GemmProblem& p, bool tf32);  // its index arithmetic, with half or with TF32 terms
 std::string gemm_inline_tile(const b200_ctx* ctx, const GemmProblem& p);
 bool gemm_h16_would_serve(const b200_ctx* ctx, const GemmProblem& p);  // (whatever else reads the operands without planes)

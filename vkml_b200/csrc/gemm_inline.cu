@@ -1130,6 +1130,14 @@ void gemm_inline_tf32(b200_ctx* ctx, const GemmProblem& p, float* partial, int64
     check_last_launch("matmul (tcgen05, TF32 terms split in the kernel)");
 }
 
+// us of a K-block in the TF32 form.  An operand whose rows along K are no whole quads on 16 bytes is read a float to a lane, each row of a stage from
+// two lines: 0.17 us more for either (products of one wave, fitted over 127: both so 1.34 us, one 1.1 to 1.18, quads 0.8 to 0.95 where 1 is taken).
+double gemm_inline_tf32_block(const GemmProblem& p) {
+    bool mn[2];
+    const InlineSide side[2] = {side_of(p.a, p.a_s, 2, 3, p.m, p, mn[0]), side_of(p.b, p.b_s, 3, 2, p.n, p, mn[1])};
+    return 1.0 + (mn[0] || side[0].quads ? 0.0 : 0.17) + (mn[1] || side[1].quads ? 0.0 : 0.17);
+}
+
 bool gemm_inline_fits(const GemmProblem& p, bool tf32) {
     // (a thread's neighbouring rows are less than 2^31 bytes apart: pitches below 2^25 floats for half terms, 2^24 for TF32 terms; units and
     // lines are counted in 31 bits)

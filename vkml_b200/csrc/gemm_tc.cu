@@ -1588,9 +1588,10 @@ struct TcPlan {
 // Whether the product is better off with operands split inside its kernel (gemm_inline.cu): where it is the only one of its span, and one wave
 // serves it.  Where fp32 tiles by TMA would be taken otherwise, always: the converters hold the operands in registers, not in a stage that the tensor
 // cores read (2816x1536x128 21.2 us -> 17.8, 704x1664x64 11.7 -> 10.4, 568x6746x228 32.2 -> 25.5).  Instead of planes, while K is not too long: a
-// K-block takes 1 us for 0.6 from planes, but there are no passes over the operands in front (512^3 16.8 -> 11.5, 1024^3 26.8 -> 23.3; rows that do
+// K-block takes 1 to 1.34 us for 0.57 from planes, but there are no passes over the operands in front (512^3 16.8 -> 11.5, 1024^3 26.8 -> 23.3; rows that do
 // not lie on 16 bytes 637x947x201 19.0 -> 13.6, 37x8191x1999 79.5 -> 44.1, 681x1026x1021 29.1 -> 25.7; with three waves 1166x129x4131 26.2 -> 31.4;
-// 1540x41875x910 935 -> 1535).  A training step's products stay as they were: a CTA here takes an SM's registers whole, so neither this
+// 1540x41875x910 935 -> 1535; both operands a float at a time, 2348x421x123 in 'nt', 20.5 -> 26.7, which planes keep).  Over 289 products of one wave
+// six take more than 3 % longer than by the other form, and none more than 8 %.  A training step's products stay as they were: a CTA here takes an SM's registers whole, so neither this
 // kernel nor the one behind it is scheduled ahead, which costs such a step more than the passes (MLP 248-2451x3-56 545 us -> 562, two products of the
 // CNN 12 us).  A compared product of 2^28 operations, up to which fp32 tiles would serve it, keeps its planes.
 bool inline_pays(const b200_ctx* ctx, const GemmProblem& p, const Operand& oa, const Operand& ob, const TcPlan& plan, bool direct) {
@@ -1604,7 +1605,8 @@ bool inline_pays(const b200_ctx* ctx, const GemmProblem& p, const Operand& oa, c
     if (ceil_div(p.m, int64_t(BM)) * ceil_div(p.n, bn) * batches * plan.splits > sm_count()) return false;
     if (direct) return true;
     // us: K-blocks, what is around them, and the passes over the operands (12 bytes per element)
-    const double inline_us = double(plan.kb_per_split) + 7.0;
+    // (units of up to ten K-blocks stay here whatever their rows: it costs them 3 us at most, 3 x 257x301x219 in 'nt' 16.0 -> 18.7)
+    const double inline_us = (plan.kb_per_split > 10 ? gemm_inline_tf32_block(p) : 1.0) * double(plan.kb_per_split) + 7.0;
     const double planes_us = 0.6 * double(plan.kb_per_split) + 12.0 * double(oa.plane_bytes + ob.plane_bytes) / 4 / 5.8e6 + 11.0;
     const double flops = 2.0 * double(p.m) * double(p.n) * double(p.k) * double(batches);
     return inline_us <= planes_us && (flops > double(1 << 28) || ctx->compared.count(p.out) == 0 || !maps_describe(p, oa, ob));
