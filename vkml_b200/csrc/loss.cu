@@ -180,8 +180,9 @@ __device__ __forceinline__ float head_total(const LossArgs& a, float scale, floa
 }
 
 // A group of threads per row -- a warp up to 1024 classes, a block up to 4096 -- with the row's logits in registers.  Up to 128 classes, where the
-// machine's warps would take more than one row each, eight threads: a warp to a row of 47 leaves most of its lanes idle ([17795, 47] 24.7 us with the
-// loss's value, 17.1 with eight; [60000, 33] 59.5 and 32.9; but 278 rows of 107 9.8 and 14.4).
+// machine's warps would take more than one row each, eight threads: a warp to a row of 47 leaves most of its lanes idle (forward and backward
+// with the loss's value, [17795, 47] 25.0 us with a warp, 18.7 with eight threads; [60000, 33] 55.7 and 29.0; [9473, 107] 20.8 and 18.8, where the line
+// lies; but 278 rows of 107 9.8 and 14.4).
 constexpr int64_t kManyRows = 64;  // per SM: eight blocks of eight warps
 template <bool HEAD, bool BACK, int GROUP, int ITEMS>
 __global__ void __launch_bounds__(256) loss_rows_kernel(LossArgs a) {
@@ -258,7 +259,8 @@ __global__ void __launch_bounds__(256) loss_rows_kernel(LossArgs a) {
 // logits never stops the writing.  (Rows re-read from L2 by three smaller blocks per SM took 245 us at [1024, 32000]
 // -- 1024 rows make 2.3 waves of those -- against 218 here.)
 // Rows of up to 16384 and 8192 classes leave room for more and smaller blocks, so that one block's rows are written while another reduces
-// its own ([689, 6337]: 53 us with one block of 1024 threads, 32 with six of 256; [4000, 4500] 222 and 119).  A row's head planes do not depend on
+// its own (this launch by itself, [689, 6337]: 51 us with one block of 1024 threads, 32 with six of 256, of 64 and 45 for the whole loss; [4000, 4500]
+// 222 and 119).  A row's head planes do not depend on
 // its logits and are written first: they drain while the row is reduced.
 constexpr int kLongThreads = 1024;
 constexpr int kLongChunks = 8;
@@ -564,7 +566,8 @@ __global__ void __launch_bounds__(256) loss_value_kernel(ValueArgs v) {
     constexpr int kInWarp = GROUP < 32 ? 32 / GROUP : 1;  // (as in loss_rows_kernel)
     const uint32_t in_warp = GROUP < 32 ? (threadIdx.x & 31) / GROUP : 0;
     for (int64_t first = int64_t(blockIdx.x) * kRows + threadIdx.x / (GROUP * kInWarp) * kInWarp; first < v.rows; first += int64_t(gridDim.x) * kRows) {
-        const int64_t r = min(first + in_warp, v.rows - 1);
+        // (a bound that a group of a warp or more does not need cost its kernel eight registers: [17388, 205] 41.3 us forward and backward, 39.5 without)
+        const int64_t r = GROUP >= 32 ? first : min(first + in_warp, v.rows - 1);
         const bool live = GROUP >= 32 || first + in_warp < v.rows;
         const int64_t base = r * v.cols;
         float s = 0.0F;
