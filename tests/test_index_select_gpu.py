@@ -103,3 +103,18 @@ def test_rows_are_added(backend, outer, extent, count, width, beyond):
         if 0 <= j < extent:
             want[:, j] += src[:, at]
     assert np.array_equal(out.numpy(), want)
+
+
+# every width of a task and one column more, by quads and by words, lists of all lengths
+@pytest.mark.parametrize("width", [1, 32, 33, 64, 65, 127, 128, 129, 132, 257])
+@pytest.mark.parametrize("extent,count", [(70, 4000), (3000, 5000)])
+def test_widths_of_tasks(backend, width, extent, count):
+    rng = np.random.default_rng(width)
+    src = rng.standard_normal((count, width), dtype=np.float32)
+    index = np.minimum(extent - 1, np.exp(rng.random(count) * np.log(extent)) - 1).astype(np.int64)  # as words of a text
+    s, i, out = DeviceTensor.from_host(backend, src), DeviceTensor.from_host(backend, index), DeviceTensor.empty(backend, (extent, width))
+    backend.compute([NodeDesc(int(Op.SCATTER_ADD), out.desc, [s.desc, i.desc], graph.axis_params(0))])
+    want = np.zeros((extent, width), np.float32)
+    for at, j in enumerate(index):
+        want[j] += src[at]
+    assert np.array_equal(out.numpy(), want)

@@ -1125,9 +1125,10 @@ scatter_chain_gather_kernel(float* __restrict__ out, const float* __restrict__ s
             }
         };
         auto add_few = [&](int held, int m) { add(held, m, Int<4>{}, Int<Q>{}, Int<0>{}); };
-        auto add_32 = [&](int held, int m) {  // a full set of lanes: eight in flight, half of the columns at a time
-            add(held, m, Int<8>{}, Int<Q / 2>{}, Int<0>{});
-            add(held, m, Int<8>{}, Int<Q / 2>{}, Int<Q / 2>{});
+        auto add_32 = [&](int held, int m) {  // a full set of lanes: eight in flight, half of the columns at a time where there are many
+            constexpr int C = Q * W <= 2 ? Q : (Q + 1) / 2;
+            add(held, m, Int<8>{}, Int<C>{}, Int<0>{});
+            if constexpr (C < Q) add(held, m, Int<8>{}, Int<Q - C>{}, Int<C>{});
         };
         const int c = count[j];
         if (c == 1) {  // (most lists, where destinations are many)
@@ -1645,24 +1646,27 @@ void launch_movement(b200_ctx* ctx, const b200_node& node) {
                 ctx->count_launch(2);
                 const bool quads = inner % 4 == 0 && reinterpret_cast<uintptr_t>(sp) % 16 == 0 && reinterpret_cast<uintptr_t>(o) % 16 == 0;
                 const bool long_lists = n_idx >= 8 * extent;  // (eight sources to a destination on average)
-                // (rows that are no quads: as many single elements to a lane as are in flight with quads, half of it for short rows and for long lists,
-                // where more tasks are worth more: 16384 indices into 100 rows of 1023, distributed as 1/rank, 663 us, 1133 with 256 to a task)
-                const bool wide = quads || (inner > 128 && !long_lists);
-                const int64_t pieces = ceil_div(inner, wide ? 256 : 128), tasks = total / inner * pieces;
+                // Columns of a task: no more than the row has, as a load past it costs as much as one in it (18411 indices into 1537 rows of 53,
+                // distributed as 1/rank, 208 us with 128, 140 with 64), and 128 at most where rows are no quads: longer tasks leave fewer warps to the
+                // longest lists (8462 into 165745 of 362 likewise 271 and 171 us; 735 into 35526 of 278, uniform, 26 and 18 forward and backward).
+                const int64_t columns = !quads ? (inner <= 32 ? 32 : inner <= 64 ? 64 : 128) : (inner <= 128 ? 128 : 256);  // of a task
+                const int64_t pieces = ceil_div(inner, columns), tasks = total / inner * pieces;
                 const unsigned grid = grid_for(tasks * 32, kThreads);
                 auto gather = [&](auto kernel) {
                     launch_kernel(ctx, kernel, grid, kThreads, 0, o, sp, static_cast<const int*>(count), static_cast<const int*>(head),
                                   static_cast<const int*>(next), ip, istride, n, FastDiv(static_cast<uint32_t>(pieces)),
                                   FastDiv(static_cast<uint32_t>(extent)), static_cast<uint32_t>(inner), static_cast<uint32_t>(tasks));
                 };
-                if (long_lists) {
-                    if (quads) gather(scatter_chain_gather_kernel<4, 2, 4>);
-                    else gather(scatter_chain_gather_kernel<1, 4, 4>);
-                } else {
-                    if (quads) gather(scatter_chain_gather_kernel<4, 2, 1>);
-                    else if (wide) gather(scatter_chain_gather_kernel<1, 8, 1>);
-                    else gather(scatter_chain_gather_kernel<1, 4, 1>);
-                }
+                auto widths = [&](auto look) {
+                    constexpr int L = decltype(look)::value;
+                    if (columns == 256) gather(scatter_chain_gather_kernel<4, 2, L>);
+                    else if (quads) gather(scatter_chain_gather_kernel<4, 1, L>);
+                    else if (columns == 128) gather(scatter_chain_gather_kernel<1, 4, L>);
+                    else if (columns == 64) gather(scatter_chain_gather_kernel<1, 2, L>);
+                    else gather(scatter_chain_gather_kernel<1, 1, L>);
+                };
+                if (long_lists) widths(Int<4>{});
+                else widths(Int<1>{});
                 break;
             }
             if (n_idx > 0) {
