@@ -1073,9 +1073,11 @@ scatter_chain_kernel(int* __restrict__ count, int* __restrict__ head, int* __res
 }
 
 // One warp per piece of 32*Q*W elements of a destination row, with at most 32 registers of sources in flight: 64 left two
-// blocks on an SM, which took 71 us where this takes 45.  LOOK pieces of 32 indices are in flight where a destination's list is long; four
+// blocks on an SM, which took 71 us where this takes 45.  A row's last piece begins early enough to be whole -- what two pieces have in common both
+// write alike -- so that no load stands under a condition, where each waits for the one before it, nor needs an address of its own; only
+// rows of less than a piece (SHORT) read their last columns again instead.  LOOK pieces of 32 indices are in flight where a destination's list is long; four
 // of them spill a few registers, which costs 3 % where no list is.
-template <int W, int Q, int LOOK>
+template <int W, int Q, int LOOK, bool SHORT>
 __global__ void __launch_bounds__(kThreads, 4)
 scatter_chain_gather_kernel(float* __restrict__ out, const float* __restrict__ src, const int* __restrict__ count,
                             const int* __restrict__ head, const int* __restrict__ next, const int64_t* __restrict__ idx,
@@ -1088,8 +1090,8 @@ scatter_chain_gather_kernel(float* __restrict__ out, const float* __restrict__ s
         uint32_t piece, row, outer, j;
         by_pieces.divmod(task, row, piece);
         by_extent.divmod(row, outer, j);
-        const uint32_t c0 = piece * (32 * Q * W) + lane * W;
-        const float* from = src + int64_t(outer) * n * inner;
+        const uint32_t c0 = (SHORT ? 0 : min(piece * (32 * Q * W), inner - 32 * Q * W)) + lane * W;
+        const float* from = src + int64_t(outer) * n * inner + (SHORT ? 0 : c0);
         float acc[Q][W] = {};
         // Adds the sources held by the lanes, `m` of them, in lane order, F at a time for C column groups from q0 on.
         auto add = [&](int held, int m, auto f, auto cols, auto first) {
@@ -1098,12 +1100,12 @@ scatter_chain_gather_kernel(float* __restrict__ out, const float* __restrict__ s
                 float v[F][C][W];
 #pragma unroll
                 for (int i = 0; i < F; ++i) {
-                    // (past the list the last source is read again, past the row its last columns: a load under a condition waits for the one before it)
+                    // (past the list the last source is read again)
                     const int k = __shfl_sync(0xffffffffu, held, min(i0 + i, m - 1));
                     const float* p = from + int64_t(k) * inner;
 #pragma unroll
                     for (int q = 0; q < C; ++q) {
-                        const uint32_t c = min(c0 + (q0 + q) * 32 * W, inner - W);
+                        const uint32_t c = SHORT ? min(c0 + (q0 + q) * 32 * W, inner - W) : (q0 + q) * 32 * W;
                         if constexpr (W == 4) {
                             const float4 t = __ldg(reinterpret_cast<const float4*>(p + c));
                             v[i][q][0] = t.x; v[i][q][1] = t.y; v[i][q][2] = t.z; v[i][q][3] = t.w;
@@ -1184,7 +1186,7 @@ scatter_chain_gather_kernel(float* __restrict__ out, const float* __restrict__ s
         float* to = out + int64_t(row) * inner + c0;
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
-            if (c0 + q * 32 * W < inner) {
+            if (!SHORT || c0 + q * 32 * W < inner) {
                 if constexpr (W == 4) *reinterpret_cast<float4*>(to + q * 128) = make_float4(acc[q][0], acc[q][1], acc[q][2], acc[q][3]);
                 else to[q * 32] = acc[q][0];
             }
@@ -1646,10 +1648,12 @@ void launch_movement(b200_ctx* ctx, const b200_node& node) {
                 ctx->count_launch(2);
                 const bool quads = inner % 4 == 0 && reinterpret_cast<uintptr_t>(sp) % 16 == 0 && reinterpret_cast<uintptr_t>(o) % 16 == 0;
                 const bool long_lists = n_idx >= 8 * extent;  // (eight sources to a destination on average)
-                // Columns of a task: no more than the row has, as a load past it costs as much as one in it (18411 indices into 1537 rows of 53,
-                // distributed as 1/rank, 208 us with 128, 140 with 64), and 128 at most where rows are no quads: longer tasks leave fewer warps to the
-                // longest lists (8462 into 165745 of 362 likewise 271 and 171 us; 735 into 35526 of 278, uniform, 26 and 18 forward and backward).
-                const int64_t columns = !quads ? (inner <= 32 ? 32 : inner <= 64 ? 64 : 128) : (inner <= 128 ? 128 : 256);  // of a task
+                // Columns of a task.  No more than the row has, as a load past it costs as much as one in it (18411 indices into 1537 rows of 53,
+                // distributed as 1/rank, 208 us with 128, 139 with 64).  Where lists are long few, as the longest ones decide and each is one warp's
+                // for its columns (16384 into 100 rows of 1024 likewise, 345 us with 256 and 205 with 128; of 1023, 335 with 128 and 192 with
+                // 64); otherwise most destinations have no source and every task costs its look at the count (110 into 319148 rows of 188
+                // 66 us with 256, 87 with 128), but no more than 128 by words (735 into 35526 of 278 and their selection 26 us with 256, 18 with 128).
+                const int64_t columns = quads ? (inner <= 128 || long_lists ? 128 : 256) : (inner <= 32 ? 32 : inner <= 64 || long_lists ? 64 : 128);
                 const int64_t pieces = ceil_div(inner, columns), tasks = total / inner * pieces;
                 const unsigned grid = grid_for(tasks * 32, kThreads);
                 auto gather = [&](auto kernel) {
@@ -1659,11 +1663,16 @@ void launch_movement(b200_ctx* ctx, const b200_node& node) {
                 };
                 auto widths = [&](auto look) {
                     constexpr int L = decltype(look)::value;
-                    if (columns == 256) gather(scatter_chain_gather_kernel<4, 2, L>);
-                    else if (quads) gather(scatter_chain_gather_kernel<4, 1, L>);
-                    else if (columns == 128) gather(scatter_chain_gather_kernel<1, 4, L>);
-                    else if (columns == 64) gather(scatter_chain_gather_kernel<1, 2, L>);
-                    else gather(scatter_chain_gather_kernel<1, 1, L>);
+                    const bool whole = inner >= columns;
+                    if (columns == 256 && whole) gather(scatter_chain_gather_kernel<4, 2, L, false>);
+                    else if (columns == 256) gather(scatter_chain_gather_kernel<4, 2, L, true>);
+                    else if (quads && whole) gather(scatter_chain_gather_kernel<4, 1, L, false>);
+                    else if (quads) gather(scatter_chain_gather_kernel<4, 1, L, true>);
+                    else if (columns == 128 && whole) gather(scatter_chain_gather_kernel<1, 4, L, false>);
+                    else if (columns == 128) gather(scatter_chain_gather_kernel<1, 4, L, true>);
+                    else if (columns == 64 && whole) gather(scatter_chain_gather_kernel<1, 2, L, false>);
+                    else if (columns == 64) gather(scatter_chain_gather_kernel<1, 2, L, true>);
+                    else gather(scatter_chain_gather_kernel<1, 1, L, true>);
                 };
                 if (long_lists) widths(Int<4>{});
                 else widths(Int<1>{});
