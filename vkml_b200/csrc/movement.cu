@@ -1027,10 +1027,10 @@ scatter_gather4_kernel(float4* __restrict__ out, const float4* __restrict__ src,
 // ascending order by itself -- up to 32 of them lie one per lane and are ranked by comparing -- or, for a destination
 // with more, finds them in order by reading the index list (at most n / 33 destinations have more, so that all of them
 // together read it a bounded number of times).  The sums and their order are those of the pull form, bit for bit.
-// [8192, 1024] into [50000, 1024]: 152 -> 50 us; 239 MB, nearly all of it the result.  Rows that are no quads, 7548 of 898 into 4760: 40 -> 17 us since
-// no load stands under a condition (each then waited for the one before it).  Long lists, buckets against chains: 16384 indices
-// into 100 rows of 1024, uniform 130 and 92 us, as words of a text are distributed (1/rank) 573 and 445; into 256 of 512 90 and 72, 504 and 381;
-// all into one 3633 and 2594.  (One piece of 32 indices at a time instead of four in flight: 156, 461, 146, 390 and 2797.)
+// [8192, 1024] into [50000, 1024]: 152 -> 49.5 us; 239 MB, nearly all of it the result.  Rows that are no quads, 7548 of 898 into 4760: 26 -> 16 us since
+// no load stands under a condition (each then waited for the one before it).  Long lists, buckets against this: 16384 indices
+// into 100 rows of 1024, uniform 130 and 70 us, as words of a text are distributed (1/rank) 573 and 205; into 256 of 512 90 and 57, 504 and 153;
+// all into one 3633 and 900.  (One piece of 32 indices at a time instead of four in flight, and 256 columns to a task: 156, 461, 146, 390 and 2797.)
 constexpr int kChainMax = 65536;
 // While the destinations are not too many for it, the sources lie side by side in a line of 32 per destination instead of a chain: a warp has them with one load
 // where it followed one after the other.
@@ -1074,8 +1074,8 @@ scatter_chain_kernel(int* __restrict__ count, int* __restrict__ head, int* __res
 
 // One warp per piece of 32*Q*W elements of a destination row, with at most 32 registers of sources in flight: 64 left two
 // blocks on an SM, which took 71 us where this takes 45.  A row's last piece begins early enough to be whole -- what two pieces have in common both
-// write alike -- so that no load stands under a condition, where each waits for the one before it, nor needs an address of its own; only
-// rows of less than a piece (SHORT) read their last columns again instead.  LOOK pieces of 32 indices are in flight where a destination's list is long; four
+// write alike -- so that no load stands under a condition, where each waits for the one before it, nor needs an address of its own; in rows of
+// less than a piece (SHORT) the last group of 32*W columns does, and a row of less than a group reads its last columns again.  LOOK pieces of 32 indices are in flight where a destination's list is long; four
 // of them spill a few registers, which costs 3 % where no list is.
 template <int W, int Q, int LOOK, bool SHORT>
 __global__ void __launch_bounds__(kThreads, 4)
@@ -1086,12 +1086,24 @@ scatter_chain_gather_kernel(float* __restrict__ out, const float* __restrict__ s
     __shared__ int found[kThreads / 32][64];
     const uint32_t lane = threadIdx.x & 31;
     int* mine = found[threadIdx.x >> 5];
-    for (uint32_t task = (blockIdx.x * kThreads + threadIdx.x) >> 5; task < tasks; task += (gridDim.x * kThreads) >> 5) {
+    const uint32_t step = (gridDim.x * kThreads) >> 5;
+    // A task without sources costs little more than its look at the count.  Short rows have it on its way while the task before is written (110
+    // indices into 319148 rows of 188 65 us without, 56 with); in the other forms the registers would be missed more (8192 into 50000 of 1024 49.5 and 57).
+    auto sources = [&](uint32_t t) {
+        const uint32_t r = by_pieces.div(min(t, tasks - 1));
+        return count[r - by_extent.div(r) * by_extent.d];
+    };
+    uint32_t task = (blockIdx.x * kThreads + threadIdx.x) >> 5;
+    int ahead = SHORT ? sources(task) : 0;
+    for (; task < tasks; task += step) {
         uint32_t piece, row, outer, j;
         by_pieces.divmod(task, row, piece);
         by_extent.divmod(row, outer, j);
+        const int c = SHORT ? ahead : count[j];
+        if constexpr (SHORT) ahead = sources(task + step);
         const uint32_t c0 = (SHORT ? 0 : min(piece * (32 * Q * W), inner - 32 * Q * W)) + lane * W;
-        const float* from = src + int64_t(outer) * n * inner + (SHORT ? 0 : c0);
+        const float* from = src + int64_t(outer) * n * inner + (SHORT && Q == 1 ? min(c0, inner - W) : c0);
+        auto group = [&](int q) { return SHORT && Q > 1 ? min(static_cast<uint32_t>(q * 32 * W), inner - 32 * W) : static_cast<uint32_t>(q * 32 * W); };
         float acc[Q][W] = {};
         // Adds the sources held by the lanes, `m` of them, in lane order, F at a time for C column groups from q0 on.
         auto add = [&](int held, int m, auto f, auto cols, auto first) {
@@ -1105,7 +1117,7 @@ scatter_chain_gather_kernel(float* __restrict__ out, const float* __restrict__ s
                     const float* p = from + int64_t(k) * inner;
 #pragma unroll
                     for (int q = 0; q < C; ++q) {
-                        const uint32_t c = SHORT ? min(c0 + (q0 + q) * 32 * W, inner - W) : (q0 + q) * 32 * W;
+                        const uint32_t c = group(q0 + q);
                         if constexpr (W == 4) {
                             const float4 t = __ldg(reinterpret_cast<const float4*>(p + c));
                             v[i][q][0] = t.x; v[i][q][1] = t.y; v[i][q][2] = t.z; v[i][q][3] = t.w;
@@ -1132,7 +1144,6 @@ scatter_chain_gather_kernel(float* __restrict__ out, const float* __restrict__ s
             add(held, m, Int<8>{}, Int<C>{}, Int<0>{});
             if constexpr (C < Q) add(held, m, Int<8>{}, Int<Q - C>{}, Int<C>{});
         };
-        const int c = count[j];
         if (c == 1) {  // (most lists, where destinations are many)
             add(head[next == nullptr ? int64_t(j) * 32 : int64_t(j)], 1, Int<1>{}, Int<Q>{}, Int<0>{});
         } else if (c > 1 && c <= 32) {
@@ -1186,9 +1197,9 @@ scatter_chain_gather_kernel(float* __restrict__ out, const float* __restrict__ s
         float* to = out + int64_t(row) * inner + c0;
 #pragma unroll
         for (int q = 0; q < Q; ++q) {
-            if (!SHORT || c0 + q * 32 * W < inner) {
-                if constexpr (W == 4) *reinterpret_cast<float4*>(to + q * 128) = make_float4(acc[q][0], acc[q][1], acc[q][2], acc[q][3]);
-                else to[q * 32] = acc[q][0];
+            if (!SHORT || Q > 1 || c0 < inner) {
+                if constexpr (W == 4) *reinterpret_cast<float4*>(to + group(q)) = make_float4(acc[q][0], acc[q][1], acc[q][2], acc[q][3]);
+                else to[group(q)] = acc[q][0];
             }
         }
     }
