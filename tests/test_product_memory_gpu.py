@@ -25,7 +25,7 @@ def test_planes_that_stand_by_are_bounded(backend, m, k, n, kernel):
 
 
 def test_a_product_runs_without_room_for_planes(backend):
-    import torch
+    from vkml_b200.backend import OutOfMemoryError
     m, k, n = 64, 524288, 64
     rng = np.random.default_rng(1)
     x, w = rng.standard_normal((m, k), dtype=np.float32), rng.standard_normal((k, n), dtype=np.float32)
@@ -34,9 +34,15 @@ def test_a_product_runs_without_room_for_planes(backend):
     node = NodeDesc(int(Op.MATMUL), out.desc, [dx.desc, dw.desc])
     assert backend.matmul_kernel(node)[0] == "tcgen05_3xf16"
     backend.synchronize()
-    torch.cuda.empty_cache()
-    room = 384 << 20  # (the planes that stand by are 512 MB)
-    taken = backend.allocate(torch.cuda.mem_get_info()[0] - room)
+    backend.trim()
+    room, taken, size = backend.allocate(384 << 20), [], 64 << 30  # (the planes that stand by are 512 MB)
+    while size >= 32 << 20:
+        try:
+            taken.append(backend.allocate(size))
+        except OutOfMemoryError:
+            size //= 2
+    del room
+    backend.trim()
     try:
         backend.compute([node])
         got = out.numpy().reshape(m, n)
