@@ -254,10 +254,12 @@ Route route_of(const b200_ctx* ctx, const GemmProblem& p) {
 }
 
 // Whether the kernel that writes the product's last sum can write an epilogue as well.
-// A launch inside a step costs 6 to 8 us whatever it does, and these nodes are such launches: an MLP's training step has 13 in place of 15
-// (784-128-10, batch 64: 51.0 us, 50.4 now; 315 rows through 160-83-32 63.9 and 61.5) or 35 in place of 41 (93 rows through 284-1130x3-201
-// 222.6 and 214.7).  A small product writes it word by word, which over many elements takes longer than the launch: 361 rows through 307-2484x3-14,
-// whose where follows a result of 361x2484, 323.7 us a step with it and 316.3 without; 560x455 gains.  Behind a small product the group with ReLU's mask stays the launch of its own that a step's profile shows.
+// A launch inside a step costs 6 to 8 us whatever it does by itself, and these nodes are such launches: an MLP's training step has 13 in place of 15
+// (784-128-10, batch 64: 51.4 us, 48.9 now; 315 rows through 160-83-32 63.9 and 61.5) or 35 in place of 44 (93 rows through 284-1130x3-201
+// 233.5 and 214.4).  A small product writes it word by word, which over many elements takes longer than the launch: a step of 361 rows through
+// 200-h-14, whose where follows a result of 361 x h, with and without: h = 300 74.2 and 75.2 us, 850 87.9 and 89.5, 1000 81.6 and 81.4, 1250 102.3 and 100.6,
+// 2000 101.6 and 100.6; the line lies where it still gains or costs nothing.  Behind a small product the group with ReLU's mask stays the
+// launch of its own that a step's profile shows.
 bool takes_epilogue(b200_ctx* ctx, const GemmProblem& p, const ProductEpilogue& e, Route& route) {
     if (p.b0 * p.b1 != 1 || p.m * p.n * p.k == 0 || result_over_operand(p, sizeof(float))) return false;
     route = route_of(ctx, p);

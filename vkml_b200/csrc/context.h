@@ -140,7 +140,8 @@ struct b200_ctx {
     // it (gemm_h16.cu); 0: TF32 terms everywhere (A/B runs).
     bool gemm_half_terms = true;
     // VKML_B200_GEMM_INLINE: products that are split inside their kernel (gemm_inline.cu).  auto (-1): where that is quicker; 0: never;
-    // 1: every product it can serve, whatever its size (A/B runs).
+    // 1: half terms for every product that they can serve there, whatever its size; 2 to 5: the same with one tile by force (256x256, 128x64, and the
+    // two with the operands' roles exchanged); 8: TF32 terms for every product that no other kernel streams (A/B runs and tests).
     int gemm_inline = -1;
     void* d_ranges = nullptr;  // RangeSlot[kRangeSlots], cleared at a span's first use
     bool lone_matmul = true;   // the current span has one product at most: no planes to share

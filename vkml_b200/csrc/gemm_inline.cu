@@ -1,7 +1,7 @@
 // F32 products from two half terms per operand, split on the way into shared memory.
 //
 // gemm_h16.cu writes the half planes of both operands to memory before its kernel runs.  For a product that is no
-// large square those passes cost as much as the product: 512 x 65536 x 512 spent 95 of 206 us on them, and a
+// large square those passes cost as much as the product: 512 x 65536 x 512 spent 95 of 207 us on them as a pass of a program, and a
 // product of a few 2^30 operations is a chain of seven launches.  Here warps of the product's own kernel read the
 // caller's floats, whatever their strides, split them in registers and store the halves where the MMA reads them.
 // The terms, the two accumulators, the range rules and what stands by for a wide operand are gemm_h16.cu's.
@@ -23,7 +23,8 @@
 // an infinity or a NaN, which leave a result that is not finite, make the operand wide.
 //
 // What bounds it: a ring of three stages of 64 K.  With the MMAs, the loads or both left out a K-block of the pair's tile takes 2375, 2560 and 1900
-// cycles for 3250: converting, handing over and multiplying add up around the ring.  512x65536x512: 182 us with planes, 119 here.
+// cycles for 3250: converting, handing over and multiplying add up around the ring.  512x65536x512, events around the whole node: 180 us with
+// planes, 120 here; as one pass of a program that has other operands each time 207 and 140.
 #include "gemm.h"
 
 #include <algorithm>
@@ -1000,8 +1001,9 @@ void launch_inline(b200_ctx* ctx, const InlineArgs& g, bool p_mn, bool q_mn, int
 // Where the planes would take longer to write and read than this kernel loses in its main loop: a long K beside a small result, a batch of
 // thin matrices.  Both times are estimated; this path is taken where its own is 5 % less.  (A K-block of the pair's tile takes 1.75 us here -- converting,
 // handing over and multiplying follow one another around a ring of three stages -- and 0.9 us from planes; the passes over the planes take 8 bytes per
-// element at 5.8 TB/s.  Measured, planes / here: 512x65536x512 182 / 119 us, 255x29905x606 105 / 84, 5 x 3335x2687x174 156 / 121,
-// 24 x 366x913x232 59 / 50; but 2048^3 65 / 69, 4096^3 349 / 441, 751x2638x911 45 / 55.)  Planes that another product of the span reads too are kept.
+// element at 5.8 TB/s.  The whole node, planes / here: 512x65536x512 180 / 120 us, 5 x 3335x2687x174 156 / 129,
+// which it takes; 255x29905x606 101 / 90, which its margin leaves to planes; 2048^3 65 / 70, 4096^3 346 / 439, 751x2638x911 55 / 58.  Of 220 products with a long K or many
+// thin matrices the rule takes 40, none of them more than 2 % slower than from planes and 1.33 times quicker in the mean.)  Planes that another product of the span reads too are kept.
 bool gemm_inline_serves(const b200_ctx* ctx, const GemmProblem& p) {
     if (ctx->gemm_inline == 0 || ctx->gemm_inline >= 8 || ctx->gemm_precision != B200_GEMM_3XTF32 || !ctx->gemm_half_terms || ctx->compared.count(p.out) != 0) {
         return false;
