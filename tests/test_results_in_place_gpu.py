@@ -81,3 +81,16 @@ def test_a_filled_choice(backend, m, k, n):
         results.append(z.numpy())
         assert np.array_equal(results[-1], np.where(c, np.float32(-0.5), y.numpy().reshape(m, n)))
     assert np.array_equal(*results)
+
+
+# a product of the wrong rank is refused, with something behind it as without
+@pytest.mark.parametrize("dims", [(), (8,), (2, 4), (1, 2, 4)])
+@pytest.mark.parametrize("behind", [False, True])
+def test_a_product_of_another_rank_is_refused(backend, dims, behind):
+    from vkml_b200.backend import ShapeError
+    a, b, y = (DeviceTensor.empty(backend, dims) for _ in range(3))
+    nodes = [NodeDesc(int(Op.MATMUL), y.desc, [a.desc, b.desc])]
+    if behind:
+        nodes.append(NodeDesc(int(Op.ADD), DeviceTensor.empty(backend, dims).desc, [y.desc, a.desc]))
+    with pytest.raises(ShapeError):
+        backend.compute(nodes)

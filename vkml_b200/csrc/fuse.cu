@@ -604,8 +604,9 @@ static bool apart(const b200_node& product, const b200_node& x) {
 size_t match_product_epilogue(const b200_node& product, const b200_node* const* seq, size_t avail, size_t later, size_t* early, ProductEpilogue& e) {
     *early = 0;
     e = ProductEpilogue{};
+    if (avail == 0 || product.out.ndim != 4 || product.n_src != 2) return 0;  // (what is no product is refused where products are dispatched)
     const int64_t n = numel_of(product.out), cols = product.out.dims[product.out.ndim - 1];
-    if (avail == 0 || n == 0 || n >= (int64_t(1) << 31) || n != product.out.dims[product.out.ndim - 2] * cols || !dense_tensor(product.out)) return 0;
+    if (n == 0 || n >= (int64_t(1) << 31) || n != product.out.dims[product.out.ndim - 2] * cols || !dense_tensor(product.out)) return 0;
     auto whole = [&](const b200_tensor& t, int dtype) { return t.dtype == dtype && t.data != nullptr && numel_of(t) == n && dense_tensor(t); };
     const b200_node& first = *seq[0];
     if (first.op == B200_OP_WHERE) {
